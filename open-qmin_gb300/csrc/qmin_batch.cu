@@ -35,18 +35,6 @@ struct __align__(16) SolveDesc {
     int pad2[2];
 };
 
-// multiplier m = ceil(2^32 / d) for udiv (d >= 2; 0 marks d = 1)
-inline unsigned div_magic(unsigned d) { return d < 2 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d); }
-
-// n / d for n < 2^31: the multiply-high estimate is floor(n / d) or one more
-// (m d - 2^32 < d, so the excess n (m d - 2^32) / (d 2^32) stays below 1)
-__device__ __forceinline__ unsigned udiv(unsigned n, unsigned d, unsigned m)
-{
-    if (m == 0) return n;
-    const unsigned q = __umulhi(n, m);
-    return q * d > n ? q - 1 : q;
-}
-
 struct ChunkDesc {
     int solve;
     int start;  // solve-local index of the chunk's first site (a tile's lowest corner)

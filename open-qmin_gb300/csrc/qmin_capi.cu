@@ -17,6 +17,7 @@
 
 #include "../../include/qmin_gb300.h"
 #include "qmin_bulk_forms.h"
+#include "qmin_fixed.cuh"
 #include "qmin_internal.h"
 
 using namespace qmin;
@@ -82,6 +83,10 @@ struct qmin_ctx {
     int32_t *stage_t = nullptr;
     FireDev *fire = nullptr;
     FireDev *fire_h = nullptr;  // pinned mirror
+    // fixed-point force (FP64): Q 2^56, range flags, coefficients of the current parameters
+    long long *X = nullptr;
+    FixedDev *fx = nullptr;
+    FixedCoef kc{};
     IterDev *iter = nullptr;
     IterDev *iter_h = nullptr;  // pinned mirror
     double *out5 = nullptr;
@@ -245,6 +250,29 @@ static bool ensure_tmap(qmin_ctx *h)
     return h->tmap_ok;
 }
 
+// The fixed-point force of the current parameters (FP64 with a form that has
+// one, no spatially varying field) and its buffers; false where there is none
+// or the buffers do not fit, and the FP64 kernels do the work.
+static bool ensure_fixed(qmin_ctx *h, const Lat<double> &L)
+{
+    h->kc.ok = 0;
+    if (L.Hv || !h->split_cls || 5 * h->P >= (1LL << 31)) return false;
+    double field[5];
+    for (int c = 0; c < 5; ++c) field[c] = (L.efield ? L.fE[c] : 0.0) + (L.hfield ? L.fH[c] : 0.0);
+    h->kc = fixed_coeffs(h->params, h->metric_mode, L.efield || L.hfield ? field : nullptr);
+    if (!h->kc.ok) return false;
+    if (!h->X) {
+        if (cudaMalloc(&h->X, 5 * (size_t)h->P * sizeof(long long)) != cudaSuccess ||
+            (!h->fx && cudaMalloc(&h->fx, sizeof(FixedDev)) != cudaSuccess)) {
+            cudaGetLastError();
+            if (h->X) cudaFree(h->X);
+            h->X = nullptr;
+            return false;
+        }
+    }
+    return true;
+}
+
 template <class T> static Lat<T> make_lat(qmin_ctx *h)
 {
     Lat<T> L;
@@ -267,6 +295,12 @@ template <class T> static Lat<T> make_lat(qmin_ctx *h)
     if (h->prec == QMIN_FP32) ensure_tmap(h);
     L.split = SplitLists{h->split_cls, h->split_sites, h->n_split_sites, h->split_derivs, h->n_split_derivs,
                          h->tmap_ok ? &h->tmap_q : nullptr, h->dev_err};
+    if constexpr (sizeof(T) == 8)
+        if (ensure_fixed(h, L)) {
+            L.X = h->X;
+            L.fx = h->fx;
+            L.fixed = &h->kc;
+        }
     return L;
 }
 
@@ -277,7 +311,7 @@ static void free_ctx(qmin_ctx *h)
     void *bufs[] = {h->Q, h->V, h->F, h->D, h->types, h->objs, h->partials, h->stage, h->stage_t, h->fire, h->iter,
                     h->out5, h->M, h->S, h->alt, h->lbp, h->lbs, h->lby, h->Q2, h->V2, h->F2, h->hvar,
                     h->split_cls, h->split_sites, h->split_derivs, h->cbd, h->dev_err, h->geo_scratch,
-                    h->scan_part, h->scan_out};
+                    h->scan_part, h->scan_out, h->X, h->fx};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (h->fire_h) cudaFreeHost(h->fire_h);
@@ -879,7 +913,7 @@ static int settle_pingpong(qmin_ctx *h, int executed)
 // metric, force form, strategy request and site-class counts) takes the
 // stored choice instead of timing every candidate again.
 struct TuneKey {
-    int Lx, Ly, Lz, prec, metric, multi, l6, l4, fields, mode, variant, tmap;
+    int Lx, Ly, Lz, prec, metric, multi, l6, l4, fields, mode, variant, tmap, fixed;
     long long nTotal, n_sites, n_derivs;
     bool operator==(const TuneKey &o) const { return memcmp(this, &o, sizeof(TuneKey)) == 0; }
 };
@@ -906,6 +940,7 @@ static TuneKey tune_key(const qmin_ctx *h)
     k.mode = h->fire_mode;
     k.variant = h->fire_variant;
     k.tmap = h->tmap_ok;
+    k.fixed = h->prec == QMIN_FP64 && h->kc.ok;
     k.nTotal = h->nTotal;
     k.n_sites = h->n_split_sites;
     k.n_derivs = h->n_split_derivs;
@@ -991,7 +1026,9 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
     // the L6 forms are compiled into the uncapped separate kernels only
     const bool l6 = L.multi && L.L6 != T(0);
     const bool auto_mode = h->fire_mode == QMIN_FIRE_AUTO;
-    const bool split_ok = L.multi && !l6 && h->split_cls;
+    // the one-constant form has the FP64 fixed-point variants and the fused FP32 ones, when none is pinned
+    const bool one_ok = h->fire_variant < 0 && (sizeof(T) == 8 ? L.fixed != nullptr : 5 * h->P < (1LL << 31));
+    const bool split_ok = !l6 && h->split_cls && (L.multi || one_ok);
     // automatic choice: the split path and the separate kernels where the split
     // path exists (the fused and staged paths are measured slower there on
     // GB300 and stay available when pinned), every strategy elsewhere
@@ -1001,16 +1038,28 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
     const bool try_tiled = !l6 && sizeof(T) == 4 && ((auto_mode && !split_ok) || h->fire_mode == QMIN_FIRE_TILED);
     const bool try_fused = !l6 && ((auto_mode && !split_ok) || h->fire_mode == QMIN_FIRE_FUSED);
     if (try_sep || try_tiled || try_split) {
-        const float t_pred = timed([&]() { return launch_fire_pred<T>(LB, h->fire, h->stream); }, kNoBudget);
+        const float t_plain = timed([&]() { return launch_fire_pred<T>(LB, h->fire, h->stream); }, kNoBudget);
         const size_t bytes = 5 * (size_t)h->P * h->esz;
         // the force + kick candidates kick V; it is restored afterwards (their forces equal the resident ones)
         CK(cudaMemcpyAsync(h->V2, h->V, bytes, cudaMemcpyDeviceToDevice, h->stream));
-        if (try_split) {
+        if (try_split && (L.multi || L.fixed)) {
             const SplitLists sl = split_lists(h);
+            float t_fixed = 0.f;  // the fixed-point predictor pass
+            if constexpr (sizeof(T) == 8)
+                if (L.fixed) {
+                    CK(cudaMemsetAsync(h->fx, 0, sizeof(FixedDev), h->stream));
+                    t_fixed = timed([&]() { return launch_fixed_pred(LB, h->fire, h->stream); }, kNoBudget);
+                    CK(cudaMemcpyAsync(h->V2, h->V, bytes, cudaMemcpyDeviceToDevice, h->stream));
+                    // the force candidates read the resident Q and its range
+                    CK(cudaMemsetAsync(h->fx, 0, sizeof(FixedDev), h->stream));
+                    h->launches += launch_fixed_pred(L, nullptr, h->stream);
+                }
             const float t_dl = timed([&]() { return launch_split_derivs<T>(L, sl, h->fire, h->stream); }, kNoBudget);
             for (int cap = 0; cap < kSplitFusedFirst; ++cap) {
                 if (pinned_out(cap) || (sizeof(T) == 8 && cap >= kSplitFp32First)) continue;
                 if (cap == kSplitTma && !h->tmap_ok) continue;
+                if (!L.multi && cap >= 1) continue;
+                const float t_pred = L.fixed && cap == 0 ? t_fixed : t_plain;
                 int np = 0;
                 const float t_fk = timed(
                     [&]() {
@@ -1033,8 +1082,8 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
             if (pinned_out(cap)) continue;
             const float t_fk = timed(
                 [&]() { return launch_force_kick_only<T>(L, h->fire, h->partials, h->grid, h->stream, cap); },
-                budget_for(t_pred + t_der));
-            const float ms = t_pred + t_der + t_fk;
+                budget_for(t_plain + t_der));
+            const float ms = t_plain + t_der + t_fk;
             h->tune_ms[cap] = ms;
             if (ms < best) {
                 best = ms;
@@ -1059,9 +1108,9 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
                         if (n < 0) ok = 0;
                         return n < 0 ? 0 : n;
                     },
-                    budget_for(t_pred + t_der));
+                    budget_for(t_plain + t_der));
                 if (!ok || cudaGetLastError() != cudaSuccess) break;
-                const float ms = t_pred + t_der + t_fk;
+                const float ms = t_plain + t_der + t_fk;
                 h->tune_ms[kSepVariants + 2 * kFusedConfigs + 2 * cfg + v] = ms;
                 if (ms < best) {
                     best = ms;
@@ -1080,6 +1129,7 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
     // the velocities above are restored from the second set)
     for (int cap = kSplitFusedFirst; try_split && cap < kSplitVariants; ++cap) {
         if (pinned_out(cap) || !split_variant_ok(h, cap)) continue;
+        if (!L.multi && (sizeof(T) == 8 || cap >= kSplitFusedFirst + 3)) continue;
         const SplitLists sl = split_lists(h);
         const float ms = timed(
             [&]() {
@@ -1157,6 +1207,8 @@ template <class T> static int fire_impl(qmin_ctx *h, int max_iterations)
     int r = tune_fire<T>(h, L);
     if (r) return r;
     if (h->path == 3 && (r = ensure_aux(h))) return r;
+    const bool fixed = h->path == 3 && h->split_cap == 0 && L.fixed;
+    if (fixed) CK(cudaMemsetAsync(h->fx, 0, sizeof(FixedDev), h->stream));
     Lat<T> LB = L;  // the second buffer set as input
     LB.Q = (T *)h->Q2;
     LB.V = (T *)h->V2;
@@ -1172,7 +1224,7 @@ template <class T> static int fire_impl(qmin_ctx *h, int max_iterations)
         if (h->path == 0) {
             n = launch_fire_pred<T>(L, h->fire, h->stream);
             n += launch_force_kick<T>(L, h->fire, h->partials, h->grid, h->stream, h->sep_cap);
-            n += launch_fire_control(h->fire, h->partials, h->grid, h->stream);
+            n += launch_fire_control(h->fire, h->partials, h->grid, nullptr, h->stream);
         } else if (h->path == 3 && split_fused(h->split_cap)) {
             // predictor fused into the deep-site kernel: one buffer set in, the
             // other out; the listed sites on the side stream form their predicted
@@ -1182,37 +1234,51 @@ template <class T> static int fire_impl(qmin_ctx *h, int max_iterations)
             T *Qo = (T *)(parity == 0 ? h->Q2 : h->Q), *Vo = (T *)(parity == 0 ? h->V2 : h->V),
               *Fo = (T *)(parity == 0 ? h->F2 : h->F);
             parity ^= 1;
-            cudaEventRecord(h->ev_fork, h->stream);
-            cudaStreamWaitEvent(h->aux, h->ev_fork, 0);
+            const bool listed = sl.n_sites > 0;
+            if (listed) {
+                cudaEventRecord(h->ev_fork, h->stream);
+                cudaStreamWaitEvent(h->aux, h->ev_fork, 0);
+            }
             const int nd = launch_split_fused_deep<T>(Lin, Qo, Vo, Fo, sl, h->fire, h->partials,
                                                       h->split_cap - kSplitFusedFirst, h->stream);
             n = 1;
             int nl = 0;
-            n += launch_split_fused_list<T>(Lin, Vo, Fo, sl, h->fire, h->partials + 3 * nd, h->aux, &nl);
-            cudaEventRecord(h->ev_join, h->aux);
-            cudaStreamWaitEvent(h->stream, h->ev_join, 0);
-            n += launch_fire_control(h->fire, h->partials, nd + nl, h->stream);
+            if (listed) {
+                n += launch_split_fused_list<T>(Lin, Vo, Fo, sl, h->fire, h->partials + 3 * nd, h->aux, &nl);
+                cudaEventRecord(h->ev_join, h->aux);
+                cudaStreamWaitEvent(h->stream, h->ev_join, 0);
+            }
+            n += launch_fire_control(h->fire, h->partials, nd + nl, nullptr, h->stream);
         } else if (h->path == 3) {
             // the listed sites (derivative planes, then force + kick) on the
             // high-priority side stream, beside the deep-site kernel
             const SplitLists sl = split_lists(h);
-            n = launch_fire_pred<T>(L, h->fire, h->stream);
-            cudaEventRecord(h->ev_fork, h->stream);
-            cudaStreamWaitEvent(h->aux, h->ev_fork, 0);
+            if constexpr (sizeof(T) == 8)
+                n = fixed ? launch_fixed_pred(L, h->fire, h->stream) : launch_fire_pred<T>(L, h->fire, h->stream);
+            else
+                n = launch_fire_pred<T>(L, h->fire, h->stream);
+            const bool listed = sl.n_sites > 0;
+            if (listed) {
+                cudaEventRecord(h->ev_fork, h->stream);
+                cudaStreamWaitEvent(h->aux, h->ev_fork, 0);
+            }
             const int nd = launch_split_deep<T>(L, sl, h->fire, h->partials, h->grid, h->split_cap, h->stream);
-            n += 1;
-            n += launch_split_derivs<T>(L, sl, h->fire, h->aux);
-            const int nl = launch_split_list<T>(L, sl, h->fire, h->partials + 3 * nd, h->aux);
-            n += nl > 0 ? 1 : 0;
-            cudaEventRecord(h->ev_join, h->aux);
-            cudaStreamWaitEvent(h->stream, h->ev_join, 0);
-            n += launch_fire_control(h->fire, h->partials, nd + nl, h->stream);
+            n += 1 + fixed;
+            int nl = 0;
+            if (listed) {
+                n += launch_split_derivs<T>(L, sl, h->fire, h->aux);
+                nl = launch_split_list<T>(L, sl, h->fire, h->partials + 3 * nd, h->aux);
+                n += 1;
+                cudaEventRecord(h->ev_join, h->aux);
+                cudaStreamWaitEvent(h->stream, h->ev_join, 0);
+            }
+            n += launch_fire_control(h->fire, h->partials, nd + nl, fixed ? h->fx : nullptr, h->stream);
         } else if (h->path == 2) {
             int nb = 0;
             n = launch_fire_pred<T>(L, h->fire, h->stream);
             if (L.multi) n += launch_derivs<T>(L, h->stream);
             n += launch_force_kick_tiled<T>(h->tiled_cfg, L, h->fire, h->partials, h->tiled_zc, h->stream, &nb);
-            n += launch_fire_control(h->fire, h->partials, nb, h->stream);
+            n += launch_fire_control(h->fire, h->partials, nb, nullptr, h->stream);
         } else {
             int nb = 0;
             if (parity == 0)
@@ -1222,7 +1288,7 @@ template <class T> static int fire_impl(qmin_ctx *h, int max_iterations)
                 n = launch_fire_fused<T>(h->fused_cfg, LB, (T *)h->Q, (T *)h->V, (T *)h->F, h->fire, h->partials,
                                          h->fused_zc, h->stream, &nb);
             parity ^= 1;
-            n += launch_fire_control(h->fire, h->partials, nb, h->stream);
+            n += launch_fire_control(h->fire, h->partials, nb, nullptr, h->stream);
         }
         return n;
     });
@@ -1497,13 +1563,17 @@ template <class T> static int fire_profile_impl(qmin_ctx *h, int iterations, dou
     const bool sfused = h->path == 3 && split_fused(h->split_cap);
     const bool fused = h->path == 1, tiled = h->path == 2, split = h->path == 3 && !sfused;
     const SplitLists sl = split_lists(h);
+    const bool fixed = split && h->split_cap == 0 && L.fixed;
+    if (fixed) CK(cudaMemsetAsync(h->fx, 0, sizeof(FixedDev), h->stream));
     Lat<T> LB = L;
     LB.Q = (T *)h->Q2;
     LB.V = (T *)h->V2;
     LB.F = (T *)h->F2;
     for (int it = 0; it < iterations; ++it) {
         CK(cudaEventRecord(ev[0], h->stream));
-        if (!fused && !sfused) h->launches += launch_fire_pred<T>(L, h->fire, h->stream);
+        if (fixed) {
+            if constexpr (sizeof(T) == 8) h->launches += launch_fixed_pred(L, h->fire, h->stream);
+        } else if (!fused && !sfused) h->launches += launch_fire_pred<T>(L, h->fire, h->stream);
         CK(cudaEventRecord(ev[1], h->stream));
         if (split) h->launches += launch_split_derivs<T>(L, sl, h->fire, h->stream);
         else if (!fused && !sfused && L.multi) h->launches += launch_derivs<T>(L, h->stream);
@@ -1536,7 +1606,7 @@ template <class T> static int fire_profile_impl(qmin_ctx *h, int iterations, dou
                                                 h->partials, h->fused_zc, h->stream, &nparts);
         }
         CK(cudaEventRecord(ev[3], h->stream));
-        h->launches += launch_fire_control(h->fire, h->partials, nparts, h->stream);
+        h->launches += launch_fire_control(h->fire, h->partials, nparts, fixed ? h->fx : nullptr, h->stream);
         CK(cudaEventRecord(ev[4], h->stream));
         CK(cudaEventSynchronize(ev[4]));
         for (int k = 0; k < 4; ++k) {

@@ -47,6 +47,18 @@ struct Nb {
     int n[6];  // x-, x+, y-, y+, z-, z+ (cubicLattice::getNeighbors, cubicLattice.cpp:179-244)
 };
 
+// multiplier m = ceil(2^32 / d) for udiv (d >= 2; 0 marks d = 1)
+inline unsigned div_magic(unsigned d) { return d < 2 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d); }
+
+// n / d for n < 2^31: the multiply-high estimate is floor(n / d) or one more
+// (m d - 2^32 < d, so the excess n (m d - 2^32) / (d 2^32) stays below 1)
+__device__ __forceinline__ unsigned udiv(unsigned n, unsigned d, unsigned m)
+{
+    if (m == 0) return n;
+    const unsigned q = __umulhi(n, m);
+    return q * d > n ? q - 1 : q;
+}
+
 template <class T>
 __device__ __forceinline__ Nb neighbours(const Lat<T> &L, int i)
 {

@@ -32,6 +32,16 @@ struct SplitLists {
     int *err;                   // device word set when a TMA wait gives up
 };
 
+struct FixedCoef;  // qmin_fixed.cuh
+
+// Range of Q over the LC sites, for the fixed-point force: wide, a component
+// at or above 3/4; lively, a component at or above 1/8.  The pass that writes
+// Q 2^56 raises them; the force passes after it run in fixed point when
+// lively and not wide, else in FP64.
+struct FixedDev {
+    int wide, lively;
+};
+
 // Everything a lattice kernel needs, passed by value.  Planes are SoA:
 // component k of site i lives at X[k * P + i]; P = N rounded up to 32.
 template <class T> struct Lat {
@@ -53,6 +63,11 @@ template <class T> struct Lat {
     T cqp[sizeof(T) == 4 ? 5 * QMIN_Q25_W : 1];  // FP32: the 25-point form term by term
     const T *cbd;           // merged boundary L2-L4 coefficients [27][5][QMIN_BND_W] in device memory, or null
     SplitLists split;       // deep / listed site classes and lists (all null when not built)
+    // FP64 with a fixed-point force: Q 2^56 (5 planes), the range flags and the
+    // coefficients (host pointer); fixed is null where the form has none
+    long long *X;
+    FixedDev *fx;
+    const FixedCoef *fixed;
 };
 
 // force parameters shared by every kernel (qmin_capi.cu)
@@ -94,7 +109,8 @@ template <class T>
 int launch_force_kick(const Lat<T> &L, FireDev *fd, double *partials, int grid, cudaStream_t s, int cap);
 template <class T>
 int launch_force_kick_only(const Lat<T> &L, FireDev *fd, double *partials, int grid, cudaStream_t s, int cap);
-int launch_fire_control(FireDev *fd, const double *partials, int nparts, cudaStream_t s);
+// fx (may be null): range flags to clear for the next iteration
+int launch_fire_control(FireDev *fd, const double *partials, int nparts, FixedDev *fx, cudaStream_t s);
 template <class T> int launch_fire_finish(const Lat<T> &L, FireDev *fd, cudaStream_t s);
 template <class T>
 int launch_energy_full(const Lat<T> &L, double *partials, int grid, double *out5, const double *E, double eps,
@@ -180,6 +196,10 @@ int launch_split_fused_list(const Lat<T> &Lin, T *Vo, T *Fo, const SplitLists &s
                             cudaStream_t s, int *nblocks);
 template <class T>
 int launch_split_list(const Lat<T> &L, const SplitLists &sl, FireDev *fd, double *partials, cudaStream_t s);
+// FP64 fixed-point passes (qmin_fixed.cu): Q 2^56 and its range (fd: with the FIRE predictor; L.fx cleared before),
+// then the force at deep sites (fd: with kick and sums), a no-op out of range; returns its block count (the partials)
+int launch_fixed_pred(const Lat<double> &L, const FireDev *fd, cudaStream_t s);
+int launch_fixed_force(const Lat<double> &L, const uint8_t *cls, const FireDev *fd, double *partials, cudaStream_t s);
 // polls of the TMA deep-site kernel's waits for its next planes before a block
 // gives up (the waits that let boxes in flight land always use the default)
 constexpr int kSplitWaitPolls = 1 << 22;

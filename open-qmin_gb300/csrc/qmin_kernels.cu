@@ -154,12 +154,13 @@ __global__ void __launch_bounds__(kBlock, CAP + 1)
 
 // fireStepCPU scalar logic (energyMinimizerFIRE.cpp:104-144) and the
 // minimize() loop condition (:160)
-__global__ void __launch_bounds__(kBlock) k_fire_control(FireDev *fd, const double *partials, int nparts)
+__global__ void __launch_bounds__(kBlock) k_fire_control(FireDev *fd, const double *partials, int nparts, FixedDev *fx)
 {
     if (!fd->active) return;
     double v[3];
     sum_partials<3>(partials, nparts, v);
     if (threadIdx.x != 0) return;
+    if (fx) fx->wide = fx->lively = 0;
     const double fn = v[0], vn = v[1], pw = v[2];
     const int it = fd->iterations + 1;
     fd->power = pw;
@@ -867,7 +868,7 @@ template <class T> int launch_derivs(const Lat<T> &L, cudaStream_t s)
 }
 template <class T> int launch_force(const Lat<T> &L, int grid, cudaStream_t s)
 {
-    if (L.multi && L.L6 == T(0) && L.split.cls) return launch_split_force(L, grid, s);
+    if (L.L6 == T(0) && L.split.cls && (L.multi || L.fixed)) return launch_split_force(L, grid, s);
     int n = 0;
     if (L.multi) n += launch_derivs(L, s);
     if (L.L6 != T(0)) k_force<T, true><<<grid, kBlock, 0, s>>>(L);
@@ -896,9 +897,9 @@ int launch_force_kick_only(const Lat<T> &L, FireDev *fd, double *partials, int g
     else k_force_kick<T, 0><<<grid, kBlock, 0, s>>>(L, fd, partials);
     return 1;
 }
-int launch_fire_control(FireDev *fd, const double *partials, int nparts, cudaStream_t s)
+int launch_fire_control(FireDev *fd, const double *partials, int nparts, FixedDev *fx, cudaStream_t s)
 {
-    k_fire_control<<<1, kBlock, 0, s>>>(fd, partials, nparts);
+    k_fire_control<<<1, kBlock, 0, s>>>(fd, partials, nparts, fx);
     return 1;
 }
 template <class T> int launch_fire_finish(const Lat<T> &L, FireDev *fd, cudaStream_t s)

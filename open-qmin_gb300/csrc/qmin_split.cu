@@ -79,12 +79,16 @@ void launch_high(void (*kern)(P...), int grid, cudaStream_t s, A &&...args)
 }  // namespace
 
 // every deep bulk site (cls == 0); partials[0 .. gridDim.x).  KICK = false:
-// forces only (no FIRE state), object sites' forces set to zero
-template <class T, int CAP, bool KICK = true>
+// forces only (no FIRE state), object sites' forces set to zero.  ONE: the
+// one-constant form.  fx (may be null): the fixed-point force ran where the
+// lattice is inside its range.
+template <class T, int CAP, bool KICK = true, bool ONE = false>
 __global__ void __launch_bounds__(kBlock, CAP + 1)
-    k_force_kick_deep(Lat<T> L, const uint8_t *__restrict__ cls, const FireDev *__restrict__ fd, double *partials)
+    k_force_kick_deep(Lat<T> L, const uint8_t *__restrict__ cls, const FireDev *__restrict__ fd, const FixedDev *fx,
+                      double *partials)
 {
     if (KICK && !fd->active) return;
+    if (fx && fx->lively && !fx->wide) return;
     const T hdt = KICK ? T(0.5) * T(fd->dt) : T(0);
     double acc[3] = {0.0, 0.0, 0.0};
     for (int i = blockIdx.x * kBlock + threadIdx.x; i < L.N; i += gridDim.x * kBlock) {
@@ -94,7 +98,13 @@ __global__ void __launch_bounds__(kBlock, CAP + 1)
             for (int k = 0; k < 5; ++k) L.F[k * L.P + i] = T(0);
         if (c != 0) continue;
         T f[5];
-        deep_force(L, i, f);
+        if constexpr (ONE) {
+            GlobalAcc<T> a(L, i);
+            T h[3];
+            site_force_core<T, GlobalAcc<T>, false, false, true>(L, a, 0, f, site_field(L, i, h));
+        } else {
+            deep_force(L, i, f);
+        }
         if constexpr (KICK) {
             kick_and_sum(L, i, hdt, f, acc);
         } else {
@@ -839,8 +849,8 @@ template <int TX, int TY> struct FusedPos {
 };
 
 // force of a deep bulk site from the predicted-Q ring, its own column (planes
-// z-1, z, z+1) from registers
-template <class T, int TS, int SX>
+// z-1, z, z+1) from registers; MULTI = false: the one-constant form
+template <class T, int TS, int SX, bool MULTI>
 __device__ __forceinline__ void deep_force_ring(const Lat<T> &L, const T *sQ, const int (&sb)[3],
                                                 const T (&qc)[3][5], long long i, T *f)
 {
@@ -850,7 +860,14 @@ __device__ __forceinline__ void deep_force_ring(const Lat<T> &L, const T *sQ, co
     (((dx) == 0 && (dy) == 0) ? qc[(dz) + 1][c]                                               \
                               : ((dz) < 0 ? r0 : (dz) == 0 ? r1 : r2)[(c) * TS + (dy) * SX + (dx)])
     T s2[5];
-    if (L.L4 == T(0)) {
+    if constexpr (!MULTI) {
+        // lcForce::bulkL1Force (lcForces.h:26-37)
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+            s2[k] = L.L1 * (T(6) * QQ(0, 0, 0, k) - QQ(-1, 0, 0, k) - QQ(1, 0, 0, k) - QQ(0, -1, 0, k) -
+                            QQ(0, 1, 0, k) - QQ(0, 0, -1, k) - QQ(0, 0, 1, k));
+        l1_cross(s2);
+    } else if (L.L4 == T(0)) {
         QMIN_BULK_Q25_NO_L4(L.cq, s2);
     } else {
         QMIN_BULK_Q25(L.cq, s2);
@@ -861,7 +878,7 @@ __device__ __forceinline__ void deep_force_ring(const Lat<T> &L, const T *sQ, co
 
 // the owned site of plane z: force from the ring, kick, writes to the output
 // set (32-bit component offsets from the site's address), FIRE sums
-template <class T, int TS, int SX, class Acc>
+template <class T, int TS, int SX, bool MULTI, class Acc>
 __device__ __forceinline__ void fused_site_out(const Lat<T> &L, const T *sQ, const int (&sb)[3],
                                                const T (&qc)[3][5], unsigned Pu, unsigned i, uint8_t c,
                                                const T (&vn)[5], T hdt, T *Qo, T *Vo, T *Fo, Acc *sacc)
@@ -873,7 +890,7 @@ __device__ __forceinline__ void fused_site_out(const Lat<T> &L, const T *sQ, con
     auto fo = [&](int k) -> T & { return (Fo + (size_t)k * Pu)[i]; };
     if (c == 0) {
         T f[5], v[5];
-        deep_force_ring<T, TS, SX>(L, sQ, sb, qc, i, f);
+        deep_force_ring<T, TS, SX, MULTI>(L, sQ, sb, qc, i, f);
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
             v[k] = vn[k] + hdt * f[k];
@@ -903,7 +920,7 @@ template <class T, int TX, int TY> constexpr size_t fused_deep_smem()
 
 // raw planes prefetched into registers one plane ahead.  Component offsets are
 // 32-bit (the launcher requires 5 P < 2^31).
-template <class T, int TX, int TY, int MINB>
+template <class T, int TX, int TY, int MINB, bool MULTI>
 __global__ void __launch_bounds__(TX *TY, MINB)
     k_fire_deep_fused(Lat<T> L, T *__restrict__ Qo, T *__restrict__ Vo, T *__restrict__ Fo,
                       const uint8_t *__restrict__ cls, const FireDev *__restrict__ fd, double *partials, int zc)
@@ -981,7 +998,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
             __syncthreads();
             if (fp.own_in) {
                 const int sb[3] = {slot(z - 1) + fp.po, slot(z) + fp.po, slot(z + 1) + fp.po};
-                fused_site_out<T, TS, SX, Acc>(L, sQ, sb, qc, Pu, (unsigned)(sxy * z + fp.colo), c_here, vn_cur,
+                fused_site_out<T, TS, SX, MULTI, Acc>(L, sQ, sb, qc, Pu, (unsigned)(sxy * z + fp.colo), c_here, vn_cur,
                                                hdt, Qo, Vo, Fo, sacc);
             }
 #pragma unroll
@@ -1116,7 +1133,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
             if (z + 2 <= ze) predict(z + 2, vn2, qn);
             if (fp.own_in) {
                 const int sb[3] = {slot(z - 1) + fp.po, slot(z) + fp.po, slot(z + 1) + fp.po};
-                fused_site_out<T, TS, SX, Acc>(L, sQ, sb, qc, Pu, (unsigned)(sxy * z + fp.colo), c_here, vn0,
+                fused_site_out<T, TS, SX, true, Acc>(L, sQ, sb, qc, Pu, (unsigned)(sxy * z + fp.colo), c_here, vn0,
                                                hdt, Qo, Vo, Fo, sacc);
             }
 #pragma unroll
@@ -1328,7 +1345,7 @@ static inline void fused_grid(int Lx, int Ly, int Lz, int TX, int TY, int MINB, 
     nz = (Lz + zc - 1) / zc;
 }
 
-template <class T, int TX, int TY, int MINB>
+template <class T, int TX, int TY, int MINB, bool MULTI>
 static int launch_fused_deep(const Lat<T> &L, T *Qo, T *Vo, T *Fo, const SplitLists &sl, FireDev *fd,
                              double *partials, int zc, cudaStream_t s)
 {
@@ -1336,12 +1353,12 @@ static int launch_fused_deep(const Lat<T> &L, T *Qo, T *Vo, T *Fo, const SplitLi
     static bool attr_set = false;
     if (!attr_set) {
         // a failure here surfaces as the launch's error
-        attr_set = cudaFuncSetAttribute(k_fire_deep_fused<T, TX, TY, MINB>,
+        attr_set = cudaFuncSetAttribute(k_fire_deep_fused<T, TX, TY, MINB, MULTI>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess;
     }
     int ntiles, nz;
     fused_grid(L.Lx, L.Ly, L.Lz, TX, TY, MINB, zc, ntiles, zc, nz);
-    k_fire_deep_fused<T, TX, TY, MINB><<<dim3(ntiles, nz), TX * TY, sm, s>>>(L, Qo, Vo, Fo, sl.cls, fd, partials, zc);
+    k_fire_deep_fused<T, TX, TY, MINB, MULTI><<<dim3(ntiles, nz), TX * TY, sm, s>>>(L, Qo, Vo, Fo, sl.cls, fd, partials, zc);
     return ntiles * nz;
 }
 
@@ -1370,20 +1387,19 @@ static int launch_fused_deep_cp(const Lat<T> &L, T *Qo, T *Vo, T *Fo, const Spli
 // copied into shared memory by 16-byte row chunks two planes ahead; FP32 with
 // Lx % 4 == 0 only, at 2 and 4 blocks per SM).  Returns the block count
 // (partials used), -1 for a variant this lattice or precision does not have.
-template <class T>
-int launch_split_fused_deep(const Lat<T> &Lin, T *Qo, T *Vo, T *Fo, const SplitLists &sl, FireDev *fd,
+template <class T, bool MULTI>
+static int launch_fused_variant(const Lat<T> &Lin, T *Qo, T *Vo, T *Fo, const SplitLists &sl, FireDev *fd,
                             double *partials, int variant, cudaStream_t s)
 {
     constexpr bool f32 = sizeof(T) == 4;
-    if (5 * Lin.P >= (1LL << 31)) return -1;  // the kernels' component offsets are 32-bit
     switch (variant) {
-    case 0: return launch_fused_deep<T, 32, 8, f32 ? 2 : 1>(Lin, Qo, Vo, Fo, sl, fd, partials, 16, s);
-    case 1: return launch_fused_deep<T, 32, 8, f32 ? 2 : 1>(Lin, Qo, Vo, Fo, sl, fd, partials, 0, s);
-    case 2: return launch_fused_deep<T, 32, 4, f32 ? 4 : 2>(Lin, Qo, Vo, Fo, sl, fd, partials, 16, s);
+    case 0: return launch_fused_deep<T, 32, 8, f32 ? 2 : 1, MULTI>(Lin, Qo, Vo, Fo, sl, fd, partials, 16, s);
+    case 1: return launch_fused_deep<T, 32, 8, f32 ? 2 : 1, MULTI>(Lin, Qo, Vo, Fo, sl, fd, partials, 0, s);
+    case 2: return launch_fused_deep<T, 32, 4, f32 ? 4 : 2, MULTI>(Lin, Qo, Vo, Fo, sl, fd, partials, 16, s);
     case 3:
     case 4:
-        // 16-byte row chunks: FP32 with Lx a multiple of 4 only
-        if constexpr (f32) {
+        // 16-byte row chunks: FP32 multi-constant with Lx a multiple of 4 only
+        if constexpr (f32 && MULTI) {
             if (Lin.Lx % 4 != 0) return -1;
             if (variant == 3) return launch_fused_deep_cp<T, 32, 8, 2>(Lin, Qo, Vo, Fo, sl, fd, partials, 0, s);
             return launch_fused_deep_cp<T, 32, 4, 4>(Lin, Qo, Vo, Fo, sl, fd, partials, 0, s);
@@ -1392,6 +1408,15 @@ int launch_split_fused_deep(const Lat<T> &Lin, T *Qo, T *Vo, T *Fo, const SplitL
         }
     default: return -1;
     }
+}
+
+template <class T>
+int launch_split_fused_deep(const Lat<T> &Lin, T *Qo, T *Vo, T *Fo, const SplitLists &sl, FireDev *fd,
+                            double *partials, int variant, cudaStream_t s)
+{
+    if (5 * Lin.P >= (1LL << 31)) return -1;  // the kernels' component offsets are 32-bit
+    return Lin.multi ? launch_fused_variant<T, true>(Lin, Qo, Vo, Fo, sl, fd, partials, variant, s)
+                     : launch_fused_variant<T, false>(Lin, Qo, Vo, Fo, sl, fd, partials, variant, s);
 }
 
 // Fused split iteration, listed part: derivative planes of the predicted Q at
@@ -1403,7 +1428,7 @@ int launch_split_fused_list(const Lat<T> &Lin, T *Vo, T *Fo, const SplitLists &s
 {
     int n = 0;
     *nblocks = 0;
-    if (sl.n_derivs > 0) {
+    if (Lin.multi && sl.n_derivs > 0) {
         launch_high(k_derivs_list_pred<T>, list_grid(sl.n_derivs), s, Lin, (const int *)sl.derivs, sl.n_derivs,
                     (const FireDev *)fd);
         ++n;
@@ -1420,7 +1445,7 @@ int launch_split_fused_list(const Lat<T> &Lin, T *Vo, T *Fo, const SplitLists &s
 
 template <class T> int launch_split_derivs(const Lat<T> &L, const SplitLists &sl, FireDev *fd, cudaStream_t s)
 {
-    if (sl.n_derivs == 0) return 0;
+    if (!L.multi || sl.n_derivs == 0) return 0;
     launch_high(k_derivs_list<T>, list_grid(sl.n_derivs), s, L, (const int *)sl.derivs, sl.n_derivs, (const FireDev *)fd);
     return 1;
 }
@@ -1439,8 +1464,16 @@ int launch_split_deep(const Lat<T> &L, const SplitLists &sl, FireDev *fd, double
             return -1;  // FP32 only (the autotuner does not offer it for FP64)
         }
     }
-    if (cap == 1) k_force_kick_deep<T, 1><<<grid, kBlock, 0, s>>>(L, sl.cls, fd, partials);
-    else k_force_kick_deep<T, 0><<<grid, kBlock, 0, s>>>(L, sl.cls, fd, partials);
+    if constexpr (sizeof(T) == 8)
+        if (L.fixed && cap == 0) {
+            const int g = launch_fixed_force(L, sl.cls, fd, partials, s);
+            if (L.multi) k_force_kick_deep<T, 1><<<g, kBlock, 0, s>>>(L, sl.cls, fd, L.fx, partials);
+            else k_force_kick_deep<T, 1, true, true><<<g, kBlock, 0, s>>>(L, sl.cls, fd, L.fx, partials);
+            return g;
+        }
+    if (!L.multi) return -1;
+    if (cap == 1) k_force_kick_deep<T, 1><<<grid, kBlock, 0, s>>>(L, sl.cls, fd, nullptr, partials);
+    else k_force_kick_deep<T, 0><<<grid, kBlock, 0, s>>>(L, sl.cls, fd, nullptr, partials);
     return grid;
 }
 
@@ -1471,8 +1504,19 @@ template <class T> int launch_split_force(const Lat<T> &L, int grid, cudaStream_
 {
     const SplitLists &sl = L.split;
     int n = launch_split_derivs<T>(L, sl, nullptr, s);
-    if constexpr (sizeof(T) == 4) launch_deep_pair<32, 8, 3, false>(L, sl, nullptr, nullptr, true, s);
-    else k_force_kick_deep<T, 1, false><<<grid, kBlock, 0, s>>>(L, sl.cls, nullptr, nullptr);
+    if constexpr (sizeof(T) == 4) {
+        launch_deep_pair<32, 8, 3, false>(L, sl, nullptr, nullptr, true, s);
+    } else {
+        FixedDev *fx = L.fixed ? L.fx : nullptr;
+        if (fx) {
+            cudaMemsetAsync(fx, 0, sizeof(FixedDev), s);
+            n += launch_fixed_pred(L, nullptr, s);
+            grid = launch_fixed_force(L, sl.cls, nullptr, nullptr, s);
+            ++n;
+        }
+        if (L.multi) k_force_kick_deep<T, 1, false><<<grid, kBlock, 0, s>>>(L, sl.cls, nullptr, fx, nullptr);
+        else k_force_kick_deep<T, 1, false, true><<<grid, kBlock, 0, s>>>(L, sl.cls, nullptr, fx, nullptr);
+    }
     ++n;
     if (sl.n_sites > 0) {
         k_force_kick_list<T, false><<<list_grid(sl.n_sites), kBlock, 0, s>>>(L, sl.sites, sl.n_sites, nullptr, nullptr);
