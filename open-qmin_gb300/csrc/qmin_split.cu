@@ -44,7 +44,13 @@ __device__ __forceinline__ void kick_and_sum(const Lat<T> &L, long long i, T hdt
     }
 }
 
-int list_grid(int n) { return std::max(1, std::min((n + kBlock - 1) / kBlock, 152 * 4)); }
+// Blocks of the list kernels.  A list is short (2 to 10 % of the sites) and a
+// listed site is long (an FP64 one 514 FP64 operations per warp), so the blocks
+// are small enough to reach every SM: at 83 x 61 x 97 with two walls an FP64
+// iteration takes 113 us with 128 threads, 114 with 64 or 32, 120 with 256
+// (87 blocks for 152 SMs); at 200^3 0.959, 0.963, 0.975 and 0.978 ms.
+constexpr int kListBlock = 128, kListPerSm = 8;
+int list_grid(int n) { return std::max(1, std::min((n + kListBlock - 1) / kListBlock, 152 * kListPerSm)); }
 
 // the device's greatest stream priority (the lowest number)
 int high_priority()
@@ -66,7 +72,7 @@ void launch_high(void (*kern)(P...), int grid, cudaStream_t s, A &&...args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kBlock);
+    cfg.blockDim = dim3(kListBlock);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributePriority;
@@ -81,14 +87,17 @@ void launch_high(void (*kern)(P...), int grid, cudaStream_t s, A &&...args)
 // every deep bulk site (cls == 0); partials[0 .. gridDim.x).  KICK = false:
 // forces only (no FIRE state), object sites' forces set to zero.  ONE: the
 // one-constant form.  fx (may be null): the fixed-point force ran where the
-// lattice is inside its range.
+// lattice is inside its range; nparts (with fx): its partials, the entries past
+// this grid set to zero.
 template <class T, int CAP, bool KICK = true, bool ONE = false>
 __global__ void __launch_bounds__(kBlock, CAP + 1)
     k_force_kick_deep(Lat<T> L, const uint8_t *__restrict__ cls, const FireDev *__restrict__ fd, const FixedDev *fx,
-                      double *partials)
+                      double *partials, int nparts = 0)
 {
     if (KICK && !fd->active) return;
     if (fx && fx->lively && !fx->wide) return;
+    if (KICK && fx && blockIdx.x == 0)
+        for (int b = 3 * gridDim.x + threadIdx.x; b < 3 * nparts; b += kBlock) partials[b] = 0.0;
     const T hdt = KICK ? T(0.5) * T(fd->dt) : T(0);
     double acc[3] = {0.0, 0.0, 0.0};
     for (int i = blockIdx.x * kBlock + threadIdx.x; i < L.N; i += gridDim.x * kBlock) {
@@ -122,13 +131,13 @@ __global__ void __launch_bounds__(kBlock, CAP + 1)
 
 // the listed LC sites through the derivative-plane forms (KICK = false: forces only)
 template <class T, bool KICK = true>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kListBlock)
     k_force_kick_list(Lat<T> L, const int *__restrict__ list, int n, const FireDev *__restrict__ fd, double *partials)
 {
     if (KICK && !fd->active) return;
     const T hdt = KICK ? T(0.5) * T(fd->dt) : T(0);
     double acc[3] = {0.0, 0.0, 0.0};
-    for (int e = blockIdx.x * kBlock + threadIdx.x; e < n; e += gridDim.x * kBlock) {
+    for (int e = blockIdx.x * kListBlock + threadIdx.x; e < n; e += gridDim.x * kListBlock) {
         const int i = list[e];
         T f[5];
         site_force<T, false, true>(L, i, f);
@@ -140,7 +149,7 @@ __global__ void __launch_bounds__(kBlock)
         }
     }
     if constexpr (KICK) {
-        block_sum<3>(acc);
+        block_sum<3, kListBlock>(acc);
         if (threadIdx.x == 0)
 #pragma unroll
             for (int k = 0; k < 3; ++k) partials[3 * blockIdx.x + k] = acc[k];
@@ -149,12 +158,12 @@ __global__ void __launch_bounds__(kBlock)
 
 // twice the first derivatives (k_derivs' rules) at the listed sites only
 template <class T>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kListBlock)
     k_derivs_list(Lat<T> L, const int *__restrict__ list, int n, const FireDev *__restrict__ fd)
 {
     if (fd && !fd->active) return;  // fd null: a force-only evaluation
     const long long P = L.P;
-    for (int e = blockIdx.x * kBlock + threadIdx.x; e < n; e += gridDim.x * kBlock) {
+    for (int e = blockIdx.x * kListBlock + threadIdx.x; e < n; e += gridDim.x * kListBlock) {
         const int i = list[e];
         const int t = L.types[i];
         const Nb b = neighbours(L, i);
@@ -1167,13 +1176,13 @@ __device__ __forceinline__ T pred_q_at(const Lat<T> &L, const PredCoef<T> &c, lo
 // twice the first derivatives (k_derivs' rules) of the predicted Q at the listed
 // sites' neighbours, formed from the input buffer set
 template <class T>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kListBlock)
     k_derivs_list_pred(Lat<T> L, const int *__restrict__ list, int n, const FireDev *__restrict__ fd)
 {
     if (!fd->active) return;
     const PredCoef<T> pc = pred_coef<T>(fd);
     const long long P = L.P;
-    for (int e = blockIdx.x * kBlock + threadIdx.x; e < n; e += gridDim.x * kBlock) {
+    for (int e = blockIdx.x * kListBlock + threadIdx.x; e < n; e += gridDim.x * kListBlock) {
         const int i = list[e];
         const int t = L.types[i];
         const Nb b = neighbours(L, i);
@@ -1221,7 +1230,7 @@ template <class T> struct PredAcc {
 // the listed LC sites' force at the predicted Q and kick, from the input buffer
 // set into the output set's V and F (their predicted Q: the fused deep kernel)
 template <class T>
-__global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(kListBlock, sizeof(T) == 4 ? 512 / kListBlock : 1)
     k_force_kick_list_pred(Lat<T> L, T *__restrict__ Vo, T *__restrict__ Fo, const int *__restrict__ list, int n,
                            const FireDev *__restrict__ fd, double *partials)
 {
@@ -1230,7 +1239,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 2 : 1)
     const T hdt = T(0.5) * T(fd->dt);
     const long long P = L.P;
     double acc[3] = {0.0, 0.0, 0.0};
-    for (int e = blockIdx.x * kBlock + threadIdx.x; e < n; e += gridDim.x * kBlock) {
+    for (int e = blockIdx.x * kListBlock + threadIdx.x; e < n; e += gridDim.x * kListBlock) {
         const int i = list[e];
         const int t = L.types[i];
         PredAcc<T> a(L, i, pc);
@@ -1251,11 +1260,15 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 2 : 1)
             acc[2] += (double)dot_qt(f, v);
         }
     }
-    block_sum<3>(acc);
+    block_sum<3, kListBlock>(acc);
     if (threadIdx.x == 0)
 #pragma unroll
         for (int k = 0; k < 3; ++k) partials[3 * blockIdx.x + k] = acc[k];
 }
+
+// grid of the FP64 deep kernel that stands by for the fixed-point one (two
+// blocks per SM): idle it costs the iteration about 3 us, 608 blocks 4.7
+constexpr int kDeepWideGrid = 152 * 2;
 
 // shared-memory deep kernel over TX x TY columns of kDeepZc planes (more when
 // the grid would not fit the partials buffer); returns its block count
@@ -1466,9 +1479,10 @@ int launch_split_deep(const Lat<T> &L, const SplitLists &sl, FireDev *fd, double
     }
     if constexpr (sizeof(T) == 8)
         if (L.fixed && cap == 0) {
-            const int g = launch_fixed_force(L, sl.cls, fd, partials, s);
-            if (L.multi) k_force_kick_deep<T, 1><<<g, kBlock, 0, s>>>(L, sl.cls, fd, L.fx, partials);
-            else k_force_kick_deep<T, 1, true, true><<<g, kBlock, 0, s>>>(L, sl.cls, fd, L.fx, partials);
+            // one of the two does the step, the other returns at once
+            const int g = launch_fixed_force(L, sl.cls, fd, partials, s), gw = std::min(g, kDeepWideGrid);
+            if (L.multi) k_force_kick_deep<T, 1><<<gw, kBlock, 0, s>>>(L, sl.cls, fd, L.fx, partials, g);
+            else k_force_kick_deep<T, 1, true, true><<<gw, kBlock, 0, s>>>(L, sl.cls, fd, L.fx, partials, g);
             return g;
         }
     if (!L.multi) return -1;
@@ -1511,7 +1525,7 @@ template <class T> int launch_split_force(const Lat<T> &L, int grid, cudaStream_
         if (fx) {
             cudaMemsetAsync(fx, 0, sizeof(FixedDev), s);
             n += launch_fixed_pred(L, nullptr, s);
-            grid = launch_fixed_force(L, sl.cls, nullptr, nullptr, s);
+            grid = std::min(launch_fixed_force(L, sl.cls, nullptr, nullptr, s), kDeepWideGrid);
             ++n;
         }
         if (L.multi) k_force_kick_deep<T, 1, false><<<grid, kBlock, 0, s>>>(L, sl.cls, nullptr, fx, nullptr);
@@ -1519,7 +1533,7 @@ template <class T> int launch_split_force(const Lat<T> &L, int grid, cudaStream_
     }
     ++n;
     if (sl.n_sites > 0) {
-        k_force_kick_list<T, false><<<list_grid(sl.n_sites), kBlock, 0, s>>>(L, sl.sites, sl.n_sites, nullptr, nullptr);
+        k_force_kick_list<T, false><<<list_grid(sl.n_sites), kListBlock, 0, s>>>(L, sl.sites, sl.n_sites, nullptr, nullptr);
         ++n;
     }
     return n;
