@@ -333,9 +333,10 @@ int qmin_energy_noalloc(const qmin_lattice_desc *desc, const qmin_ldg_params *p,
  * FIRE scalars, stopping rule and iteration count), converged solves retire.
  * qmin_batch_fire_run runs all iterations of all solves in one persistent
  * cooperative launch (grid barriers between the phases of an iteration; FP32
- * one-constant batches run the predictor, force and kick as one phase over two
- * state sets, and the device memory for the second set is allocated on their
- * first run).  All
+ * batches run the predictor, force and kick as one phase over two state sets,
+ * and the device memory for the second set is allocated on their first run).
+ * Site classes and lists are taken from the types at the first run after a
+ * solve's types changed.  All
  * solves share the force parameters; each has up to 16 objects.  No reference
  * counterpart for the batching itself (the reference minimises one lattice per
  * process). */
@@ -363,6 +364,8 @@ int qmin_batch_set_barrier_limit(qmin_batch b, long long spins);
 /* the chunk shape the tuner chose (-1 before the first run; 0: 256
  * consecutive sites, 1-4: tiles of 32x8x1, 16x16x1, 16x4x4, 8x8x4 sites, as
  * tile[3]) and the force + kick time of each shape in ms (-1: not timed).
+ * FP32 batches take it for the entry forces only: their iterations run on
+ * tiles and z chunks cut from each solve's box.
  * No reference counterpart (execution strategy). */
 int qmin_batch_tuning(qmin_batch b, int *shape, int tile[3], double ms[5]);
 /* pin the chunk shape (0-4 as in qmin_batch_tuning) or hand it back to the

@@ -126,39 +126,9 @@ template <class T> struct BatchSet {
     T *Q, *V, *F;
 };
 
-// accessor over the predicted Q of a packed solve, formed on the fly from an
-// input state set (one-constant forms: no derivative planes)
-template <class T> struct BatchPredAcc {
-    const T *Q, *V, *F;
-    const int8_t *types;
-    const ObjDev<T> *objs;
-    long long P;
-    int i;
-    int nb[6];
-    PredCoef<T> c;
-    __device__ __forceinline__ BatchPredAcc(const Lat<T> &L, const BatchSet<T> &in, const PredCoef<T> &c_,
-                                            const SolveDesc &sd, int li, int x, int y, int z)
-        : Q(in.Q), V(in.V), F(in.F), types(L.types), objs(L.objs + sd.obj_base), P(L.P), i(sd.off + li), c(c_)
-    {
-        const int sx = sd.Lx, sy = sd.Lx * sd.Ly;
-        nb[0] = i + (x == 0 ? sd.Lx - 1 : -1);
-        nb[1] = i + (x == sd.Lx - 1 ? -(sd.Lx - 1) : 1);
-        nb[2] = i + (y == 0 ? (sd.Ly - 1) * sx : -sx);
-        nb[3] = i + (y == sd.Ly - 1 ? -(sd.Ly - 1) * sx : sx);
-        nb[4] = i + (z == 0 ? (sd.Lz - 1) * sy : -sy);
-        nb[5] = i + (z == sd.Lz - 1 ? -(sd.Lz - 1) * sy : sy);
-    }
-    __device__ __forceinline__ T at(int j, int k) const
-    {
-        const long long o = (long long)k * P + j;
-        return pred_q(c, ld(Q + o), pred_v(c, ld(V + o), ld(F + o)));
-    }
-    __device__ __forceinline__ int tn(int s) const { return types[nb[s]]; }
-    __device__ __forceinline__ T q(int k) const { return at(i, k); }
-    __device__ __forceinline__ T nq(int s, int k) const { return at(nb[s], k); }
-    __device__ __forceinline__ T dn(int, int) const { return T(0); }  // multi-constant forms only
-    __device__ __forceinline__ ObjDev<T> obj(int t) const { return objs[t - 1]; }
-};
+}  // namespace qmin
+#include "qmin_batch_tile.cuh"
+namespace qmin {
 
 // ----------------------------------------------------- per-chunk phases
 // The deferred mix folded into the Verlet coefficients, as k_fire_pred does:
@@ -276,82 +246,16 @@ __device__ __forceinline__ void b_force_chunk(const BatchArgs<T> &B, const FireD
     }
 }
 
-// One fused FIRE iteration of chunk c (one-constant forms): the predicted Q of
-// the site and of its six neighbours formed on the fly from the input set, the
-// force there, the half kick, the output set written (Q', V', F) and each
-// warp's FIRE sums, as b_force_chunk lays them out
-template <class T>
-__device__ __forceinline__ void b_fused_chunk(const BatchArgs<T> &B, const BatchSet<T> &in, const BatchSet<T> &out,
-                                              const FireDev *fds, double *partials, int c)
-{
-    const ChunkDesc ch = B.chunks[c];
-    // coefficients formed in FP64 by one lane per warp
-    double cf[3] = {0.0, 0.0, 0.0};
-    if ((threadIdx.x & 31) == 0) {
-        const FireDev &fd = fds[ch.solve];
-        const double dt = fd.dt, hdt = 0.5 * dt;
-        double mv = 1.0, mf = 0.0;
-        if (fd.pending) {
-            mv = fd.reset ? 0.0 : 1.0 - fd.mixA;
-            mf = fd.reset ? 0.0 : fd.mixA * fd.mixS;
-        }
-        cf[0] = mv;
-        cf[1] = mf + hdt;
-        cf[2] = dt;
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) cf[k] = __shfl_sync(0xffffffffu, cf[k], 0);
-    const PredCoef<T> pc{T(cf[0]), T(cf[1]), T(cf[2])};
-    const T hdt = T(0.5) * T(cf[2]);  // the kick's half step, as b_force_chunk forms it
-    const SolveDesc sd = B.solves[ch.solve];
-    int li, x, y, z;
-    const bool inb = chunk_site(B, sd, ch, threadIdx.x, li, x, y, z);
-    T acc[3] = {T(0), T(0), T(0)};
-    if (inb) {
-        const int gi = sd.off + li;
-        const BatchPredAcc<T> a(B.L, in, pc, sd, li, x, y, z);
-        T f[5], v[5];
-        site_force_core<T, BatchPredAcc<T>, false, false, true>(B.L, a, B.L.types[gi], f);
-        const long long P = B.L.P;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            const long long o = k * P + gi;
-            const T vp = pred_v(pc, ld(in.V + o), ld(in.F + o));
-            out.Q[o] = pred_q(pc, ld(in.Q + o), vp);
-            v[k] = vp + hdt * f[k];
-            out.V[o] = v[k];
-            out.F[o] = f[k];
-        }
-        acc[0] = dot_qt(f, f);
-        acc[1] = dot_qt(v, v);
-        acc[2] = dot_qt(f, v);
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-    if ((threadIdx.x & 31) == 0) {
-        double *p = partials + 3 * ((long long)kBatchWarps * c + threadIdx.x / 32);
-        p[0] = (double)acc[0];
-        p[1] = (double)acc[1];
-        p[2] = (double)acc[2];
-    }
-}
-
-// one warp, solve w: deterministic sum of its chunks' partials, then the
-// fireStepCPU scalar logic (energyMinimizerFIRE.cpp:104-144) and the loop
-// condition of minimize(); returns (in lane 0) whether the solve retired now
-__device__ __forceinline__ bool b_control_solve(FireDev *fds, const SolveDesc *solves, int w, const double *partials)
+// one warp: deterministic sum of a solve's n partials p, then the fireStepCPU
+// scalar logic (energyMinimizerFIRE.cpp:104-144) and the loop condition of
+// minimize(); returns (in lane 0) whether the solve retired now
+__device__ __forceinline__ bool b_control_solve(FireDev *fd, const double *p, int n)
 {
     const int lane = threadIdx.x & 31;
-    FireDev *fd = fds + w;
     if (!fd->active) return false;  // uniform per warp
-    const SolveDesc sd = solves[w];
     double v[3] = {0.0, 0.0, 0.0};
     // eight strides' loads in flight; each lane adds its entries in index order
     constexpr int U = 8;
-    const int n = kBatchWarps * sd.nchunks;
-    const double *p = partials + 3LL * kBatchWarps * sd.chunk0;
     for (int c0 = lane; c0 < n; c0 += 32 * U) {
         double x[U][3];
 #pragma unroll
@@ -440,7 +344,19 @@ __global__ void k_b_clear_pending(FireDev *fds, int n)
     if (s < n) fds[s].pending = 0;
 }
 
-// after a fused run: the solves whose last iteration wrote the second state
+// a solve's Q from AoS, V = F = 0
+template <class T>
+__global__ void __launch_bounds__(kBlock) k_b_set(const double *__restrict__ aos, T *Q, T *V, T *F, int n, long long P)
+{
+    for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock)
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            Q[k * P + i] = T(aos[5 * (size_t)i + k]);
+            V[k * P + i] = F[k * P + i] = T(0);
+        }
+}
+
+// after an FP32 run: the solves whose last iteration wrote the second state
 // set get their Q, V, F copied back into the first
 template <class T>
 __global__ void __launch_bounds__(kBlock) k_b_settle(BatchArgs<T> B, BatchSet<T> s1, const int *in_second)
@@ -470,9 +386,9 @@ struct BatchRun {
     int pad;
     long long spin_limit;
     int retired[3];
+    int next[6];  // tile loop: items taken, per iteration modulo 3 and phase
     int pad2;
 };
-
 
 // grid-wide barrier between two phases; bounded: a block that has waited
 // spin_limit polls raises the abort flag, and every block leaves at its next
@@ -508,106 +424,237 @@ __device__ __forceinline__ bool b_grid_sync(BatchRun *run)
     return ok != 0;
 }
 
-// Every FIRE iteration of every solve in one cooperative launch: predictor,
-// (derivative planes,) force + half kick + per-chunk sums, per-solve control,
-// a grid barrier after each phase.  The work of a phase is the chunks of the
-// active solves: each block holds the same list of active solves and the
-// prefix sums of their chunk counts in shared memory, rebuilt (in solve order)
-// when a solve retires, so retired solves cost nothing.
+// Every FIRE iteration of every solve in one cooperative launch, a grid barrier
+// after each phase.  The work of a phase is that of the active solves: each
+// block holds the same list of them and the prefix sums of their work counts
+// in shared memory, rebuilt (in solve order) when a solve retires, so retired
+// solves cost nothing.
 constexpr int kMaxBatchSolves = 16384;  // the lists take 8 (nsolves + 1) bytes of shared memory
 
-// (the one-constant forms ask for three blocks per SM, the FP32 multi-constant
-// form for two: the force phase would otherwise hold the registers of fewer)
-//
-// FUSED (FP32 one-constant forms; in FP64 the neighbours' predictions formed
-// again at every site cost more FP64 FMAs than the separate predictor phase
-// saves): one phase per iteration instead of predictor and force: iteration it reads state set it & 1 (0: B.L's planes, 1: s1) and
-// writes the other, forming the predicted Q of every neighbour on the fly
-// (b_fused_chunk); a solve that retires leaves in_second[solve] = 1 when its
-// final state is in s1 (k_b_settle copies it back)
-template <class T, bool ONE_CONST, bool FUSED = false>
-__global__ void __launch_bounds__(kBlock, ONE_CONST ? 3 : (sizeof(T) == 4 ? 2 : 1))
-    k_b_fire_persistent(BatchArgs<T> B, BatchSet<T> s1, FireDev *fds, double *partials, int *in_second,
-                        int nsolves, BatchRun *run)
+// the active solves in solve order and the prefix sums of their work counts,
+// kept by every block in shared memory
+struct ActiveList {
+    int *act, *pre;
+    int n, all;  // active solves; whether that is every solve
+};
+
+// one warp's ballot over the solves in order; count(s): the work of solve s
+template <class COUNT> __device__ __forceinline__ void b_rebuild(ActiveList *al, const FireDev *fds, int nsolves, COUNT count)
 {
-    static_assert(!FUSED || (ONE_CONST && sizeof(T) == 4), "the fused iteration covers the FP32 one-constant forms");
-    extern __shared__ int b_lists[];
-    int *act = b_lists;                // active solve ids, in solve order
-    int *pre = b_lists + nsolves + 1;  // prefix sums of their chunk counts
-    __shared__ int n_act;
-    __shared__ int all_act;  // every solve active: work item w is chunk w
-    auto rebuild = [&]() {
-        // one warp: ballot over the solves in order
-        if (threadIdx.x < 32) {
-            int n = 0, tot = 0;
-            for (int s0 = 0; s0 < nsolves; s0 += 32) {
-                const int s = s0 + threadIdx.x;
-                const bool a = s < nsolves && fds[s].active;
-                const int nc = a ? B.solves[s].nchunks : 0;
-                const unsigned m = __ballot_sync(0xffffffffu, a);
-                int inc = nc;
+    if (threadIdx.x < 32) {
+        int n = 0, tot = 0;
+        for (int s0 = 0; s0 < nsolves; s0 += 32) {
+            const int s = s0 + threadIdx.x;
+            const bool a = s < nsolves && fds[s].active;
+            const int nc = a ? count(s) : 0;
+            const unsigned m = __ballot_sync(0xffffffffu, a);
+            int inc = nc;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (threadIdx.x >= o) inc += v;
-                }
-                if (a) {
-                    const int k = n + __popc(m & ((1u << threadIdx.x) - 1u));
-                    act[k] = s;
-                    pre[k] = tot + inc - nc;
-                }
-                n += __popc(m);
-                tot += __shfl_sync(0xffffffffu, inc, 31);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (threadIdx.x >= o) inc += v;
             }
-            if (threadIdx.x == 0) {
-                n_act = n;
-                all_act = n == nsolves;
-                pre[n] = tot;
+            if (a) {
+                const int k = n + __popc(m & ((1u << threadIdx.x) - 1u));
+                al->act[k] = s;
+                al->pre[k] = tot + inc - nc;
             }
+            n += __popc(m);
+            tot += __shfl_sync(0xffffffffu, inc, 31);
         }
-        __syncthreads();
-    };
-    // chunk of work item w: binary search in the prefix sums
+        if (threadIdx.x == 0) {
+            al->n = n;
+            al->all = n == nsolves;
+            al->pre[n] = tot;
+        }
+    }
+    __syncthreads();
+}
+
+// entry of the active list that work item w belongs to
+__device__ __forceinline__ int b_find(const ActiveList &al, int w)
+{
+    int lo = 0, hi = al.n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (al.pre[mid] <= w) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// FP64: predictor, (derivative planes,) force + kick and control, a grid
+// barrier after each (the one-constant form asks for three blocks per SM: the
+// force phase would otherwise hold the registers of fewer)
+template <class T, bool ONE_CONST>
+__global__ void __launch_bounds__(kBlock, ONE_CONST ? 3 : 1)
+    k_b_fire_persistent(const __grid_constant__ BatchArgs<T> B, FireDev *fds, double *partials, int nsolves, BatchRun *run)
+{
+    extern __shared__ int b_lists[];
+    __shared__ ActiveList al;
+    if (threadIdx.x == 0) {
+        al.act = b_lists;
+        al.pre = b_lists + nsolves + 1;
+    }
+    __syncthreads();
+    auto count = [&](int s) { return B.solves[s].nchunks; };
+    // chunk of work item w (every solve active: the item itself)
     auto chunk_of = [&](int w) {
-        if (all_act) return w;
-        int lo = 0, hi = n_act - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (pre[mid] <= w) lo = mid;
-            else hi = mid - 1;
-        }
-        return B.solves[act[lo]].chunk0 + (w - pre[lo]);
+        if (al.all) return w;
+        const int k = b_find(al, w);
+        return B.solves[al.act[k]].chunk0 + (w - al.pre[k]);
     };
-    rebuild();
+    b_rebuild(&al, fds, nsolves, count);
     const int nwarps = gridDim.x * (kBlock / 32);
     const int gwarp = blockIdx.x * (kBlock / 32) + threadIdx.x / 32;
-    const BatchSet<T> s0{B.L.Q, B.L.V, B.L.F};
-    for (int it = 0; n_act > 0; ++it) {
+    for (int it = 0; al.n > 0; ++it) {
         if (blockIdx.x == 0 && threadIdx.x == 0) run->retired[it % 3] = 0;
-        const int nw = pre[n_act];
-        if constexpr (FUSED) {
-            const BatchSet<T> in = (it & 1) ? s1 : s0, out = (it & 1) ? s0 : s1;
-            for (int w = blockIdx.x; w < nw; w += gridDim.x) b_fused_chunk<T>(B, in, out, fds, partials, chunk_of(w));
-            if (!b_grid_sync(run)) return;
-        } else {
-            for (int w = blockIdx.x; w < nw; w += gridDim.x) b_pred_chunk<T>(B, fds, chunk_of(w));
-            if (!b_grid_sync(run)) return;
-            if (!ONE_CONST && B.L.multi) {
-                for (int w = blockIdx.x; w < nw; w += gridDim.x) b_derivs_chunk<T>(B, fds, chunk_of(w));
-                if (!b_grid_sync(run)) return;
-            }
-            for (int w = blockIdx.x; w < nw; w += gridDim.x)
-                b_force_chunk<T, 1, ONE_CONST>(B, fds, partials, chunk_of(w));
+        const int nw = al.pre[al.n];
+        for (int w = blockIdx.x; w < nw; w += gridDim.x) b_pred_chunk<T>(B, fds, chunk_of(w));
+        if (!b_grid_sync(run)) return;
+        if (!ONE_CONST && B.L.multi) {
+            for (int w = blockIdx.x; w < nw; w += gridDim.x) b_derivs_chunk<T>(B, fds, chunk_of(w));
             if (!b_grid_sync(run)) return;
         }
-        // per-solve control, one warp per active solve (its warps' sums added in order)
-        for (int k = gwarp; k < n_act; k += nwarps)
-            if (b_control_solve(fds, B.solves, act[k], partials) && (threadIdx.x & 31) == 0) {
-                atomicAdd(&run->retired[it % 3], 1);
-                if (FUSED) in_second[act[k]] = (it & 1) == 0;
-            }
+        for (int w = blockIdx.x; w < nw; w += gridDim.x) b_force_chunk<T, 1, ONE_CONST>(B, fds, partials, chunk_of(w));
         if (!b_grid_sync(run)) return;
-        if (*(volatile int *)&run->retired[it % 3] > 0) rebuild();
+        // per-solve control, one warp per active solve (its warps' sums added in order)
+        for (int k = gwarp; k < al.n; k += nwarps) {
+            const SolveDesc sd = B.solves[al.act[k]];
+            if (b_control_solve(fds + al.act[k], partials + 3LL * kBatchWarps * sd.chunk0, kBatchWarps * sd.nchunks) &&
+                (threadIdx.x & 31) == 0)
+                atomicAdd(&run->retired[it % 3], 1);
+        }
+        if (!b_grid_sync(run)) return;
+        if (*(volatile int *)&run->retired[it % 3] > 0) b_rebuild(&al, fds, nsolves, count);
+    }
+}
+
+// the predictor's coefficients and the kick's half step of one solve
+__device__ __forceinline__ void b_set_coef(float4 *coefs, const FireDev *fds, int s)
+{
+    const PredCoef<float> pc = pred_coef<float>(fds + s);
+    coefs[s] = make_float4(pc.cvv, pc.cvf, pc.tdt, 0.5f * pc.tdt);
+}
+
+// the items of one phase that this block does: the first by its index, the
+// others from a counter (the next one is asked for before an item is done)
+struct TileItems {
+    int w, nxt, *counter;
+    __device__ __forceinline__ TileItems(const ActiveList &al, int *counter_) : w(blockIdx.x), nxt(0), counter(counter_)
+    {
+        ask(al);
+    }
+    __device__ __forceinline__ void ask(const ActiveList &al)
+    {
+        if (threadIdx.x == 0 && w < al.pre[al.n]) nxt = gridDim.x + atomicAdd(counter, 1);
+    }
+    __device__ __forceinline__ bool more(const ActiveList &al) const { return w < al.pre[al.n]; }
+    __device__ __forceinline__ void item(const ActiveList &al, int &s, int &k) const
+    {
+        const int e = b_find(al, w);
+        s = al.act[e];
+        k = w - al.pre[e];
+    }
+    __device__ __forceinline__ void take(int *sh)
+    {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            *sh = nxt;
+            nxt = gridDim.x + atomicAdd(counter, 1);
+        }
+        __syncthreads();
+        w = *sh;
+    }
+};
+
+// FP32: one phase per iteration for predictor, force and kick (b_tile_item),
+// before it for multi-constant solves the derivative planes the listed sites
+// read, after it the control.  Iteration it reads state set it & 1 (0: B.L's
+// planes, 1: s1) and writes the other; a solve that retires leaves
+// in_second[solve] = 1 when its final state is in s1 (k_b_settle copies it
+// back).  Blocks take the items in turn from a counter, listed sites first in
+// each solve; every item's sums have their own place, so the totals do not
+// depend on who did it.
+template <bool MULTI>
+__global__ void __launch_bounds__(kTileThreads, kTilePerSm)
+    k_b_fire_tiled(const __grid_constant__ BatchArgs<float> B, const SolveTile *tiles,
+                   const __grid_constant__ BatchSet<float> s1, FireDev *fds, float4 *coefs,
+                   double *partials, int *in_second, int nsolves, BatchRun *run)
+{
+    extern __shared__ __align__(16) float b_ring[];  // the plane ring, then the lists
+    __shared__ ActiveList al;
+    __shared__ int sh_w;
+    if (threadIdx.x == 0) {
+        al.act = reinterpret_cast<int *>(b_ring + kTileRing);
+        al.pre = al.act + nsolves + 1;
+    }
+    __syncthreads();
+    auto count = [&](int s) { return tiles[s].items; };
+    for (int s = blockIdx.x * kTileThreads + threadIdx.x; s < nsolves; s += gridDim.x * kTileThreads)
+        b_set_coef(coefs, fds, s);
+    b_rebuild(&al, fds, nsolves, count);
+    if (!b_grid_sync(run)) return;
+    const int nwarps = gridDim.x * (kTileThreads / 32);
+    const int gwarp = blockIdx.x * (kTileThreads / 32) + threadIdx.x / 32;
+    const BatchSet<float> s0{B.L.Q, B.L.V, B.L.F};
+    for (int it = 0; al.n > 0; ++it) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            run->retired[it % 3] = 0;
+            run->next[2 * ((it + 1) % 3)] = run->next[2 * ((it + 1) % 3) + 1] = 0;
+        }
+        const BatchSet<float> in = (it & 1) ? s1 : s0, out = (it & 1) ? s0 : s1;
+        if (MULTI) {
+            for (TileItems q(al, &run->next[2 * (it % 3)]); q.more(al); q.take(&sh_w)) {
+                int s, k;
+                q.item(al, s, k);
+                const SolveTile st = tiles[s];
+                if (k * kTileThreads >= st.nderiv) continue;
+                const float4 c = __ldcg(coefs + s);
+                b_deriv_item(B.L, in, PredCoef<float>{c.x, c.y, c.z}, B.solves[s], st, k);
+            }
+            if (!b_grid_sync(run)) return;
+        }
+        for (TileItems q(al, &run->next[2 * (it % 3) + 1]); q.more(al); q.take(&sh_w)) {
+            int s, k;
+            q.item(al, s, k);
+            const SolveTile st = tiles[s];
+            const int nli = (st.nlist + kTileThreads - 1) / kTileThreads;
+            if (k >= nli + st.ntile) continue;
+            const float4 c = __ldcg(coefs + s);
+            const PredCoef<float> pc{c.x, c.y, c.z};
+            const SolveDesc sd = B.solves[s];
+            float a[3] = {0.f, 0.f, 0.f};
+            // the two orders of the sets as they stand in the parameters: plane bases in uniform registers
+            if (k < nli) b_list_item<MULTI>(B.L, in, out, pc, c.w, sd, st, k, a);
+            else if (it & 1) b_tile_item<MULTI>(B.L, B.cls, s1, s0, pc, c.w, sd, st, k - nli, b_ring, a);
+            else b_tile_item<MULTI>(B.L, B.cls, s0, s1, pc, c.w, sd, st, k - nli, b_ring, a);
+            // FP32 over a thread's column, FP64 from there on
+            double acc[3] = {(double)a[0], (double)a[1], (double)a[2]};
+            block_sum<3, kTileThreads>(acc);
+            if (threadIdx.x == 0) {
+                double *p = partials + 3LL * (st.item0 + k);
+                p[0] = acc[0];
+                p[1] = acc[1];
+                p[2] = acc[2];
+            }
+        }
+        if (!b_grid_sync(run)) return;
+        for (int k = gwarp; k < al.n; k += nwarps) {
+            const int s = al.act[k];
+            const SolveTile st = tiles[s];
+            const int n = st.ntile + (st.nlist + kTileThreads - 1) / kTileThreads;
+            const bool retired = b_control_solve(fds + s, partials + 3LL * st.item0, n);
+            if ((threadIdx.x & 31) == 0) {
+                b_set_coef(coefs, fds, s);
+                if (retired) {
+                    atomicAdd(&run->retired[it % 3], 1);
+                    in_second[s] = (it & 1) == 0;
+                }
+            }
+        }
+        if (!b_grid_sync(run)) return;
+        if (*(volatile int *)&run->retired[it % 3] > 0) b_rebuild(&al, fds, nsolves, count);
     }
 }
 
@@ -650,13 +697,29 @@ struct qmin_batch_ctx {
     SolveDesc *solves = nullptr;
     ChunkDesc *chunks = nullptr;
     void *Q = nullptr, *V = nullptr, *F = nullptr, *D = nullptr, *objs = nullptr;
-    void *Q2 = nullptr, *V2 = nullptr, *F2 = nullptr;  // second state set of the fused iteration
+    void *Q2 = nullptr, *V2 = nullptr, *F2 = nullptr;  // second state set of the FP32 iteration
+    // FP32: the items of each solve, its predictor coefficients, their sums
+    SolveTile *tiles = nullptr;
+    float4 *coefs = nullptr;
+    double *tile_partials = nullptr;
+    size_t tile_partials_cap = 0;
+    std::vector<SolveTile> tiles_h;
+    // per solve: its site types (host), its listed sites and derivative sites
+    // (device, multi-constant FP32) and whether classes and lists are those of its types
+    struct SolveLists {
+        std::vector<int8_t> types;
+        int *sites = nullptr, *derivs = nullptr;
+        int sites_cap = 0, derivs_cap = 0, n_sites = 0, n_derivs = 0;
+        bool classified = false;
+    };
+    std::vector<SolveLists> lists;
+    bool tiles_multi = false, classified_multi = false;
+    void *geo_scratch = nullptr;
     int *in_second = nullptr;                          // per solve: final state in the second set
     int8_t *types = nullptr;
     uint8_t *cls = nullptr, *needd = nullptr;  // per packed site (multi-constant split of the force)
     void *cbd = nullptr;                       // merged boundary coefficients (multi-constant)
     double *partials = nullptr, *stage = nullptr;
-    int32_t *stage_t = nullptr;
     FireDev *fds = nullptr;
     std::vector<FireDev> fds_h;
     cudaStream_t stream = nullptr;
@@ -714,7 +777,7 @@ template <class T> static BatchArgs<T> batch_args(qmin_batch_ctx *b)
     B.L.objs = (const ObjDev<T> *)b->objs;
     fill_lat_params(B.L, b->params, b->metric_mode);
     B.L.cbd = (const T *)b->cbd;
-    B.cls = b->params.multi_constant ? b->cls : nullptr;
+    B.cls = b->cls;
     B.needd = b->params.multi_constant ? b->needd : nullptr;
     B.solves = b->solves;
     B.chunks = b->chunks;
@@ -809,32 +872,139 @@ template <class T> static int tune_shape(qmin_batch_ctx *b)
     return set_layout(b, best_k);
 }
 
-// the persistent FIRE loop as one cooperative launch of as many blocks as can
-// be resident together
-template <class T, bool ONE_CONST, bool FUSED>
-static int launch_persistent(qmin_batch_ctx *b, const BatchArgs<T> &B)
+// Site classes of every solve whose types changed since they were last taken,
+// on the device: classes, the derivative-plane marks and the two lists
+// (multi-constant), or the boundary sites (one-constant FP32).
+static int classify_solves(qmin_batch_ctx *b)
 {
-    const size_t smem = sizeof(int) * 2 * ((size_t)b->nsolves + 1);
-    auto kern = k_b_fire_persistent<T, ONE_CONST, FUSED>;
+    const bool multi = b->params.multi_constant != 0;
+    if (b->classified_multi != multi)
+        for (auto &l : b->lists) l.classified = false;
+    b->classified_multi = multi;
+
+    for (int s = 0; s < b->nsolves; ++s) {
+        auto &l = b->lists[s];
+        if (l.classified || l.types.empty()) continue;
+        const SolveDesc &sd = b->solves_h[s];
+        if (!b->geo_scratch && cudaMalloc(&b->geo_scratch, split_scratch_bytes(b->maxN)) != cudaSuccess) {
+            cudaGetLastError();
+            return bfail(QMIN_ENOMEM, "batch site lists: scratch allocation failed");
+        }
+        int totals[32];
+        int n = multi ? build_split_lists_dev(b->types + sd.off, sd.Lx, sd.Ly, sd.Lz, b->cls + sd.off, b->geo_scratch,
+                                            totals, &l.sites, &l.sites_cap, &l.n_sites, &l.derivs, &l.derivs_cap,
+                                            &l.n_derivs, b->stream)
+                          : build_boundary_list_dev(b->types + sd.off, sd.Lx * sd.Ly * sd.Lz, b->cls + sd.off,
+                                                    b->geo_scratch, &l.sites, &l.sites_cap, &l.n_sites, b->stream);
+        if (n == -2) {
+            cudaGetLastError();
+            return bfail(QMIN_ENOMEM, "batch site lists: allocation failed");
+        }
+        if (n < 0) return bfail(QMIN_ECUDA, std::string("batch site lists: ") + cudaGetErrorString(cudaGetLastError()));
+        b->launches += n;
+        if (multi) {
+            b->launches += launch_need_marks(b->geo_scratch, sd.Lx * sd.Ly * sd.Lz, b->needd + sd.off, b->stream);
+            // derivative planes of a previous geometry: object sites' are read as zero and never written
+            for (int k = 0; k < 15; ++k)
+                BCK(cudaMemsetAsync((char *)b->D + ((size_t)k * b->P + sd.off) * b->esz, 0,
+                                    (size_t)sd.Lx * sd.Ly * sd.Lz * b->esz, b->stream));
+        }
+        l.classified = true;
+        b->tiles_h.clear();
+    }
+    return QMIN_OK;
+}
+
+// the items of every solve: tiles of about 128 sites cut evenly (at most 32
+// wide and 32 high), z chunks of 4 to 16 planes so that there are about four
+// items per resident block (two, three and six measured within 5 %)
+static int lay_out_tiles(qmin_batch_ctx *b, bool multi)
+{
+    if (!b->tiles_h.empty() && b->tiles_multi == multi) return QMIN_OK;
+    auto cut = [](int n, int most) { return (n + most - 1) / most; };
+    std::vector<SolveTile> t((size_t)b->nsolves);
+    long long planes = 0;
+    for (int s = 0; s < b->nsolves; ++s) {
+        const SolveDesc &sd = b->solves_h[s];
+        SolveTile &st = t[s];
+        memset(&st, 0, sizeof st);
+        st.ntx = cut(sd.Lx, kTileWide);
+        st.tx = cut(sd.Lx, st.ntx);
+        st.nty = cut(sd.Ly, std::min(32, kTileThreads / st.tx));
+        st.ty = cut(sd.Ly, st.nty);
+        planes += (long long)st.ntx * st.nty * sd.Lz;
+    }
+    const int zmax = (int)std::min(16LL, std::max(4LL, planes / (152 * kTilePerSm * 4)));
+    long long items = 0;
+    for (int s = 0; s < b->nsolves; ++s) {
+        const SolveDesc &sd = b->solves_h[s];
+        SolveTile &st = t[s];
+        const int nz = cut(sd.Lz, zmax);
+        st.zc = cut(sd.Lz, nz);
+        st.ntile = st.ntx * st.nty * cut(sd.Lz, st.zc);
+        st.nlist = b->lists[s].n_sites;
+        st.sites = b->lists[s].sites;
+        if (multi) {
+            st.nderiv = b->lists[s].n_derivs;
+            st.derivs = b->lists[s].derivs;
+        }
+        st.items = std::max(st.ntile + cut(st.nlist, kTileThreads), cut(st.nderiv, kTileThreads));
+        st.item0 = (int)items;
+        items += st.items;
+    }
+    if (items > b->tile_partials_cap) {
+        if (b->tile_partials) cudaFree(b->tile_partials);
+        b->tile_partials = nullptr;
+        b->tile_partials_cap = 0;
+        if (cudaMalloc(&b->tile_partials, sizeof(double) * 3 * (size_t)items) != cudaSuccess) {
+            cudaGetLastError();
+            return bfail(QMIN_ENOMEM, "batch: partial sums allocation failed");
+        }
+        b->tile_partials_cap = (size_t)items;
+    }
+    if ((!b->tiles && cudaMalloc(&b->tiles, sizeof(SolveTile) * (size_t)b->nsolves) != cudaSuccess) ||
+        (!b->coefs && cudaMalloc(&b->coefs, sizeof(float4) * (size_t)b->nsolves) != cudaSuccess)) {
+        cudaGetLastError();
+        return bfail(QMIN_ENOMEM, "batch: tile table allocation failed");
+    }
+    b->tiles_h = t;
+    b->tiles_multi = multi;
+    BCK(cudaMemcpyAsync(b->tiles, b->tiles_h.data(), sizeof(SolveTile) * t.size(), cudaMemcpyHostToDevice, b->stream));
+    return QMIN_OK;
+}
+
+// a persistent FIRE loop as one cooperative launch of as many blocks as can be
+// resident together
+static int launch_cooperative(qmin_batch_ctx *b, const void *kern, int block, size_t smem, void **args)
+{
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return bfail(QMIN_ECUDA, "batch: shared memory for the active-solve lists");
     int per_sm = 0, nsm = 0, dev = 0;
     BCK(cudaGetDevice(&dev));
     BCK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, smem));
+    BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem));
     if (per_sm < 1) return bfail(QMIN_ECUDA, "batch: the persistent kernel does not fit on an SM");
-    const int grid = per_sm * nsm;
-    BatchArgs<T> a = B;
-    BatchSet<T> s1{(T *)b->Q2, (T *)b->V2, (T *)b->F2};
-    FireDev *fds = b->fds;
-    double *partials = b->partials;
-    int *in_second = b->in_second;
-    int ns = b->nsolves;
-    BatchRun *run = b->run;
-    void *args[] = {&a, &s1, &fds, &partials, &in_second, &ns, &run};
-    BCK(cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(kBlock), args, smem, b->stream));
+    BCK(cudaLaunchCooperativeKernel(kern, dim3(per_sm * nsm), dim3(block), args, smem, b->stream));
     return QMIN_OK;
+}
+
+template <bool MULTI> static int launch_tiled(qmin_batch_ctx *b, const BatchArgs<float> &B)
+{
+    BatchArgs<float> a = B;
+    const SolveTile *tiles = b->tiles;
+    BatchSet<float> s1{(float *)b->Q2, (float *)b->V2, (float *)b->F2};
+    void *args[] = {&a, &tiles, &s1, &b->fds, &b->coefs, &b->tile_partials, &b->in_second, &b->nsolves, &b->run};
+    return launch_cooperative(b, (const void *)k_b_fire_tiled<MULTI>, kTileThreads,
+                              sizeof(float) * kTileRing + sizeof(int) * 2 * ((size_t)b->nsolves + 1), args);
+}
+
+template <bool ONE_CONST> static int launch_persistent(qmin_batch_ctx *b, const BatchArgs<double> &B)
+{
+    BatchArgs<double> a = B;
+    void *args[] = {&a, &b->fds, &b->partials, &b->nsolves, &b->run};
+    return launch_cooperative(b, (const void *)k_b_fire_persistent<double, ONE_CONST>, kBlock,
+                              sizeof(int) * 2 * ((size_t)b->nsolves + 1), args);
 }
 
 // The API functions below take C linkage from their declarations in qmin_gb300.h.
@@ -883,6 +1053,7 @@ int qmin_batch_create(int nsolves, const int32_t *dims, int precision, int metri
     chunk_layout(0, b->solves_h, &b->chunks_h);
     b->nchunks = (int)b->chunks_h.size();
     b->ntotal_h.assign(nsolves, 0);
+    b->lists.resize(nsolves);
     const size_t plane = (size_t)b->P * b->esz;
     bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMalloc(&b->Q, 5 * plane) == cudaSuccess && cudaMalloc(&b->V, 5 * plane) == cudaSuccess &&
@@ -893,8 +1064,7 @@ int qmin_batch_create(int nsolves, const int32_t *dims, int precision, int metri
               cudaMalloc(&b->partials, sizeof(double) * 3 * kBatchWarps * (size_t)b->max_chunks) == cudaSuccess &&
               cudaMalloc(&b->run, sizeof(BatchRun)) == cudaSuccess &&
               cudaMalloc(&b->stage, sizeof(double) * 5 * (size_t)b->maxN) == cudaSuccess &&
-              cudaMalloc(&b->stage_t, sizeof(int32_t) * (size_t)b->maxN) == cudaSuccess &&
-              cudaMalloc(&b->fds, sizeof(FireDev) * nsolves) == cudaSuccess &&
+                            cudaMalloc(&b->fds, sizeof(FireDev) * nsolves) == cudaSuccess &&
               cudaMalloc(&b->cls, (size_t)b->P) == cudaSuccess && cudaMalloc(&b->needd, (size_t)b->P) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
@@ -922,10 +1092,15 @@ int qmin_batch_destroy(qmin_batch b)
 {
     if (!b) return bfail(QMIN_EINVAL, "qmin_batch_destroy: null handle");
     if (b->stream) cudaStreamSynchronize(b->stream);
-    void *bufs[] = {b->Q, b->V, b->F, b->D, b->objs, b->types, b->partials, b->stage, b->stage_t, b->fds,
-                    b->solves, b->chunks, b->cls, b->needd, b->cbd, b->run, b->Q2, b->V2, b->F2, b->in_second};
+    void *bufs[] = {b->Q, b->V, b->F, b->D, b->objs, b->types, b->partials, b->stage, b->fds,
+                    b->solves, b->chunks, b->cls, b->needd, b->cbd, b->run, b->Q2, b->V2, b->F2, b->in_second,
+                    b->tiles, b->coefs, b->tile_partials, b->geo_scratch};
     for (void *p : bufs)
         if (p) cudaFree(p);
+    for (auto &l : b->lists) {
+        if (l.sites) cudaFree(l.sites);
+        if (l.derivs) cudaFree(l.derivs);
+    }
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return QMIN_OK;
@@ -977,55 +1152,36 @@ int qmin_batch_set_solve(qmin_batch b, int s, const double *Q, const int32_t *ty
     if (nobj > kObjPerSolve) return bfail(QMIN_EINVAL, "qmin_batch_set_solve: at most 16 objects per solve");
     const SolveDesc &sd = b->solves_h[s];
     const int n = sd.Lx * sd.Ly * sd.Lz;
-    long long nT = 0;
+    // one pass over the types: range, LC sites, the device's int8 form, whether
+    // they are the ones this solve has
+    std::vector<int8_t> t8((size_t)n);
+    int mn = 0, mx = 0, nT = 0;
     for (int i = 0; i < n; ++i) {
-        if (types[i] < -2 || types[i] > nobj)
-            return bfail(QMIN_EINVAL, "qmin_batch_set_solve: site type out of range for this solve's objects");
-        if (types[i] <= 0) ++nT;
+        const int t = types[i];
+        mn = std::min(mn, t);
+        mx = std::max(mx, t);
+        nT += t <= 0;
+        t8[i] = (int8_t)t;
     }
+    if (mn < -2 || mx > nobj)
+        return bfail(QMIN_EINVAL, "qmin_batch_set_solve: site type out of range for this solve's objects");
     b->ntotal_h[s] = nT;
-    {
-        // site classes of the split force (deep bulk: type 0 with six type-0
-        // neighbours; 1: other LC sites; 2: objects) and the sites whose
-        // derivative planes the class-1 forms read, with this solve's periodic wrap
-        std::vector<uint8_t> cls((size_t)n), need((size_t)n, 0);
-        auto nb = [&](int i, int k) {
-            const int x = i % sd.Lx, r = i / sd.Lx, y = r % sd.Ly, z = r / sd.Ly;
-            switch (k) {
-            case 0: return (x == 0 ? sd.Lx - 1 : x - 1) + sd.Lx * (y + sd.Ly * z);
-            case 1: return (x == sd.Lx - 1 ? 0 : x + 1) + sd.Lx * (y + sd.Ly * z);
-            case 2: return x + sd.Lx * ((y == 0 ? sd.Ly - 1 : y - 1) + sd.Ly * z);
-            case 3: return x + sd.Lx * ((y == sd.Ly - 1 ? 0 : y + 1) + sd.Ly * z);
-            case 4: return x + sd.Lx * (y + sd.Ly * (z == 0 ? sd.Lz - 1 : z - 1));
-            default: return x + sd.Lx * (y + sd.Ly * (z == sd.Lz - 1 ? 0 : z + 1));
-            }
-        };
-        for (int i = 0; i < n; ++i) {
-            if (types[i] > 0) {
-                cls[i] = 2;
-                continue;
-            }
-            bool deep = types[i] == 0;
-            for (int k = 0; k < 6 && deep; ++k) deep = types[nb(i, k)] == 0;
-            cls[i] = deep ? 0 : 1;
-            if (!deep)
-                for (int k = 0; k < 6; ++k) need[nb(i, k)] = 1;
-        }
-        BCK(cudaMemcpyAsync(b->cls + sd.off, cls.data(), (size_t)n, cudaMemcpyHostToDevice, b->stream));
-        BCK(cudaMemcpyAsync(b->needd + sd.off, need.data(), (size_t)n, cudaMemcpyHostToDevice, b->stream));
-        BCK(cudaStreamSynchronize(b->stream));
+    auto &l = b->lists[s];
+    if (l.types != t8) {
+        l.types.swap(t8);
+        l.classified = false;
+        BCK(cudaMemcpyAsync(b->types + sd.off, l.types.data(), (size_t)n, cudaMemcpyHostToDevice, b->stream));
     }
     BCK(cudaMemcpyAsync(b->stage, Q, sizeof(double) * 5 * (size_t)n, cudaMemcpyHostToDevice, b->stream));
-    BCK(cudaMemcpyAsync(b->stage_t, types, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, b->stream));
+    const int grid = std::min((n + kBlock - 1) / kBlock, 152 * 8);
     if (b->prec == QMIN_FP64)
-        b->launches += launch_aos_to_soa<double>(b->stage, (double *)b->Q + sd.off, n, b->P, QMIN_LAYOUT_AOS, b->stream);
+        k_b_set<double><<<grid, kBlock, 0, b->stream>>>(b->stage, (double *)b->Q + sd.off, (double *)b->V + sd.off,
+                                                        (double *)b->F + sd.off, n, b->P);
     else
-        b->launches += launch_aos_to_soa<float>(b->stage, (float *)b->Q + sd.off, n, b->P, QMIN_LAYOUT_AOS, b->stream);
-    b->launches += launch_types_to_i8(b->stage_t, b->types + sd.off, n, b->stream);
-    for (int k = 0; k < 5; ++k) {
-        BCK(cudaMemsetAsync((char *)b->V + ((size_t)k * b->P + sd.off) * b->esz, 0, (size_t)n * b->esz, b->stream));
-        BCK(cudaMemsetAsync((char *)b->F + ((size_t)k * b->P + sd.off) * b->esz, 0, (size_t)n * b->esz, b->stream));
-    }
+        k_b_set<float><<<grid, kBlock, 0, b->stream>>>(b->stage, (float *)b->Q + sd.off, (float *)b->V + sd.off,
+                                                       (float *)b->F + sd.off, n, b->P);
+    b->launches += 1;
+    BCK(cudaGetLastError());
     if (nobj > 0) {
         if (b->prec == QMIN_FP64) {
             std::vector<ObjDev<double>> o(nobj);
@@ -1090,6 +1246,8 @@ int qmin_batch_fire_init(qmin_batch b, const qmin_fire_params *p)
 
 template <class T> static int batch_fire_impl(qmin_batch_ctx *b, bool *timed_out)
 {
+    if (b->params.multi_constant || sizeof(T) == 4)
+        if (int r = classify_solves(b)) return r;
     // every solve's minimize() starts with its forces (energyMinimizerFIRE.cpp:157)
     b->launches += launch_b_force<T>(batch_args<T>(b), b->fds, b->partials, 0, b->stream);
     if (b->shape < 0) {
@@ -1101,9 +1259,9 @@ template <class T> static int batch_fire_impl(qmin_batch_ctx *b, bool *timed_out
     run.spin_limit = b->spin_limit;
     BCK(cudaMemcpyAsync(b->run, &run, sizeof run, cudaMemcpyHostToDevice, b->stream));
     const BatchArgs<T> B = batch_args<T>(b);
-    const bool fused = !B.L.multi && sizeof(T) == 4;
+    const bool fused = sizeof(T) == 4;
     if (fused && !b->Q2) {
-        // the second state set, on the first one-constant run
+        // the second state set, on the first FP32 run
         const size_t bytes = 5 * (size_t)b->P * b->esz;
         if (cudaMalloc(&b->Q2, bytes) != cudaSuccess || cudaMalloc(&b->V2, bytes) != cudaSuccess ||
             cudaMalloc(&b->F2, bytes) != cudaSuccess ||
@@ -1114,10 +1272,12 @@ template <class T> static int batch_fire_impl(qmin_batch_ctx *b, bool *timed_out
     }
     if (fused) BCK(cudaMemsetAsync(b->in_second, 0, sizeof(int) * (size_t)b->nsolves, b->stream));
     int r;
-    if constexpr (sizeof(T) == 4)
-        r = B.L.multi ? launch_persistent<T, false, false>(b, B) : launch_persistent<T, true, true>(b, B);
-    else
-        r = B.L.multi ? launch_persistent<T, false, false>(b, B) : launch_persistent<T, true, false>(b, B);
+    if constexpr (sizeof(T) == 4) {
+        if ((r = lay_out_tiles(b, B.L.multi != 0))) return r;
+        r = B.L.multi ? launch_tiled<true>(b, B) : launch_tiled<false>(b, B);
+    } else {
+        r = B.L.multi ? launch_persistent<false>(b, B) : launch_persistent<true>(b, B);
+    }
     if (r) return r;
     b->launches += 1;
     BCK(cudaMemcpyAsync(&run, b->run, sizeof run, cudaMemcpyDeviceToHost, b->stream));

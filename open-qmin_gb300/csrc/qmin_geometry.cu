@@ -263,10 +263,67 @@ int scan_types(const TT *t, const int8_t *old8, int N, int *part, int *out_dev, 
 template int scan_types<int32_t>(const int32_t *, const int8_t *, int, int *, int *, int *, cudaStream_t);
 template int scan_types<int8_t>(const int8_t *, const int8_t *, int, int *, int *, int *, cudaStream_t);
 
+// class (0 type 0, 1 other LC site, 2 object) and key 0 at the class-1 sites
+__global__ void __launch_bounds__(kScanBlock)
+    k_boundary_classify(const int8_t *__restrict__ t8, int N, uint8_t *cls, uint8_t *key)
+{
+    for (int i = blockIdx.x * kScanBlock + threadIdx.x; i < N; i += gridDim.x * kScanBlock) {
+        const int t = t8[i], c = t > 0 ? 2 : (t < 0 ? 1 : 0);
+        cls[i] = (uint8_t)c;
+        key[i] = c == 1 ? 0 : kNoBucket;
+    }
+}
+
+// 1 where the derivative list of the build_split_lists_dev call that filled `scratch` holds the site
+__global__ void __launch_bounds__(kScanBlock) k_need_marks(const uint8_t *__restrict__ key, int N, uint8_t *need)
+{
+    for (int i = blockIdx.x * kScanBlock + threadIdx.x; i < N; i += gridDim.x * kScanBlock) need[i] = key[i] == 0;
+}
+
+int launch_need_marks(const void *scratch, int N, uint8_t *need, cudaStream_t s)
+{
+    const int grid = std::max(1, std::min((N + kScanBlock - 1) / kScanBlock, 152 * 8));
+    k_need_marks<<<grid, kScanBlock, 0, s>>>(reinterpret_cast<const uint8_t *>(scratch) + N, N, need);
+    return 1;
+}
+
 size_t split_scratch_bytes(int N)
 {
     const size_t nch = ((size_t)N + kBucketChunk - 1) / kBucketChunk;
     return 2 * (size_t)N + 4 * nch * kForms * sizeof(int) + 64 * sizeof(int);
+}
+
+// grows a device list to at least `need` entries
+static bool ensure_list(int **p, int *cap, int need)
+{
+    if (need <= *cap && *p) return true;
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+    *cap = 0;
+    if (cudaMalloc(p, sizeof(int) * (size_t)std::max(need, 1)) != cudaSuccess) return false;
+    *cap = std::max(need, 1);
+    return true;
+}
+
+int build_boundary_list_dev(const int8_t *t8, int N, uint8_t *cls, void *scratch, int **sites, int *sites_cap,
+                            int *n_sites, cudaStream_t s)
+{
+    const int nch = (N + kBucketChunk - 1) / kBucketChunk;
+    uint8_t *key = reinterpret_cast<uint8_t *>(scratch);
+    int *counts = reinterpret_cast<int *>(reinterpret_cast<uintptr_t>(key + N + 15) & ~(uintptr_t)15),
+        *offsets = counts + nch, *total = offsets + nch;
+    const int grid = std::max(1, std::min((N + kScanBlock - 1) / kScanBlock, 152 * 8));
+    k_boundary_classify<<<grid, kScanBlock, 0, s>>>(t8, N, cls, key);
+    k_bucket_count<1><<<nch, kScanBlock, 0, s>>>(key, N, counts);
+    k_bucket_offsets<1><<<1, 1024, 0, s>>>(counts, nch, offsets, total);
+    int n = 0;
+    if (cudaMemcpyAsync(&n, total, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+        return -1;
+    if (!ensure_list(sites, sites_cap, n)) return -2;
+    if (n > 0) k_bucket_scatter<1><<<nch, 32, 0, s>>>(key, N, offsets, *sites);
+    *n_sites = n;
+    return cudaGetLastError() == cudaSuccess ? 3 + (n > 0) : -1;
 }
 
 int build_split_lists_dev(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch, int *host_totals,
@@ -295,16 +352,7 @@ int build_split_lists_dev(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls
     int ns = 0;
     for (int b = 0; b < kForms; ++b) ns += host_totals[b];
     const int nd = host_totals[kForms];
-    auto ensure = [&](int **p, int *cap, int need) -> bool {
-        if (need <= *cap && *p) return true;
-        if (*p) cudaFree(*p);
-        *p = nullptr;
-        *cap = 0;
-        if (cudaMalloc(p, sizeof(int) * (size_t)std::max(need, 1)) != cudaSuccess) return false;
-        *cap = std::max(need, 1);
-        return true;
-    };
-    if (!ensure(sites, sites_cap, ns) || !ensure(derivs, derivs_cap, nd)) return -2;
+    if (!ensure_list(sites, sites_cap, ns) || !ensure_list(derivs, derivs_cap, nd)) return -2;
     if (ns > 0) {
         k_bucket_scatter<kForms><<<nch, 32, 0, s>>>(key, N, offsets, *sites);
         ++n;

@@ -217,35 +217,6 @@ template <int TX> __device__ __forceinline__ void tile_site(int t, int &lx, int 
     ly = (w / NWX) * WY + lane / WX;
 }
 
-// force of a deep bulk site from its Q and its combined bulk form s2, M
-// applied as for type-0 sites (twice in CPU mode, the fields between the two)
-template <class T>
-__device__ __forceinline__ void deep_force_finish(const Lat<T> &L, const T *q, const T *s2, long long i, T *f)
-{
-    phase_force_sub(L.a, L.b, L.c, q, s2, f);
-    if (L.metric_mode == 0 && !L.efield && !L.hfield && !L.Hv) {
-        metric2(f);
-        return;
-    }
-    if (L.metric_mode == 0) metric(f);
-    if (L.efield)
-#pragma unroll
-        for (int k = 0; k < 5; ++k) f[k] -= L.fE[k];
-    if (L.hfield)
-#pragma unroll
-        for (int k = 0; k < 5; ++k) f[k] -= L.fH[k];
-    T h[3];
-    if (const T *hs = site_field(L, i, h)) {
-        const T hx = hs[0], hy = hs[1], hz = hs[2], fp = L.hvp;
-        f[0] -= T(-0.5) * fp * (hx * hx - hz * hz);
-        f[1] -= -fp * hx * hy;
-        f[2] -= -fp * hx * hz;
-        f[3] -= T(-0.5) * fp * (hy * hy - hz * hz);
-        f[4] -= -fp * hy * hz;
-    }
-    metric(f);
-}
-
 // force of a deep bulk site from Q staged in shared memory: plane dz of the
 // site's column starts at sb[dz + 2], components TS apart, rows SX apart
 template <class T, int TS, int SX>
