@@ -20,6 +20,7 @@
 #include <string>
 #include <vector>
 
+#include "qmin_fixed.cuh"
 #include "qmin_force_core.cuh"
 
 namespace qmin {
@@ -120,6 +121,12 @@ template <class T> struct BatchAcc {
 };
 
 constexpr int kBatchWarps = kBlock / 32;  // warp partial sums per chunk
+// Blocks per SM of the FP64 iteration: three (80 registers, the listed sites'
+// form spills) take 367 us an iteration for 40 uneven one-constant solves (2.5 M
+// sites) and 442 for eight 64^3 multi-constant ones (2.1 M), two 401 and 475,
+// four 357 and 493: what bounds it is memory latency between its barriers
+// (floor at the measured HBM rate: 132 us and 109).
+constexpr int kFixedPerSm = 3;
 
 // one set of packed state planes (Q, V, F)
 template <class T> struct BatchSet {
@@ -131,43 +138,64 @@ template <class T> struct BatchSet {
 namespace qmin {
 
 // ----------------------------------------------------- per-chunk phases
+// FP64 fixed-point force (qmin_fixed.cuh): Q 2^56 (5 packed planes, null where
+// the form has none), the range of each solve's predicted Q (x wide, y lively,
+// as FixedDev) and the coefficients
+struct BatchFixed {
+    long long *X;
+    int2 *range;
+    FixedCoef kc;
+};
+
 // The deferred mix folded into the Verlet coefficients, as k_fire_pred does:
-// v' = cvv v + cvf f, q' = q + dt v' (chunk c of an active solve)
-template <class T> __device__ __forceinline__ void b_pred_chunk(const BatchArgs<T> &B, const FireDev *fds, int c)
+// v' = cvv v + cvf f, q' = q + dt v' (sites l0 .. l1 of a solve); with fx.X also
+// Q' 2^56 and the range of the LC sites
+__device__ __forceinline__ void b_pred_item(const BatchArgs<double> &B, const BatchFixed &fx, const FireDev *fds, int s,
+                                            int l0, int l1)
 {
-    const ChunkDesc ch = B.chunks[c];
-    const FireDev &fd = fds[ch.solve];
-    if (!fd.active) return;  // uniform per block
-    // formed in FP64 by one lane per warp
-    double cf[3] = {0.0, 0.0, 0.0};
-    if ((threadIdx.x & 31) == 0) {
-        const double dt = fd.dt, hdt = 0.5 * dt;
-        double mv = 1.0, mf = 0.0;
-        if (fd.pending) {
-            mv = fd.reset ? 0.0 : 1.0 - fd.mixA;
-            mf = fd.reset ? 0.0 : fd.mixA * fd.mixS;
+    const int off = B.solves[s].off;
+    const PredCoef<double> pc = pred_coef<double>(fds + s);
+    int m = 0;
+    for (int i = off + l0 + threadIdx.x; i < off + l1; i += kBlock) {
+        const bool lc = fx.X && B.L.types[i] <= 0;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            const size_t j = k * (size_t)B.L.P + (unsigned)i;
+            const double vn = pred_v(pc, B.L.V[j], B.L.F[j]), q = pred_q(pc, B.L.Q[j], vn);
+            B.L.V[j] = vn;
+            B.L.Q[j] = q;
+            if (fx.X) {
+                fx.X[j] = to_fixed(q);
+                if (lc) m = max(m, fix_magnitude(q));
+            }
         }
-        cf[0] = mv;
-        cf[1] = mf + hdt;
-        cf[2] = dt;
     }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) cf[k] = __shfl_sync(0xffffffffu, cf[k], 0);
-    const T cvv = T(cf[0]), cvf = T(cf[1]), tdt = T(cf[2]);
-    const SolveDesc sd = B.solves[ch.solve];
-    int li;
-    if (!chunk_site(B, sd, ch, threadIdx.x, li)) return;
-    const int i = sd.off + li;
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        const long long j = (long long)k * B.L.P + i;
-        const T vn = cvv * B.L.V[j] + cvf * B.L.F[j];
-        B.L.V[j] = vn;
-        B.L.Q[j] += tdt * vn;
+    if (!fx.X) return;
+    const unsigned wide = __ballot_sync(0xffffffffu, m >= kFixWide), lively = __ballot_sync(0xffffffffu, m >= kFixLively);
+    if ((threadIdx.x & 31) == 0) {  // every warp that raises a flag writes the same value
+        volatile int2 *r = fx.range + s;
+        if (wide && !r->x) r->x = 1;
+        if (lively && !r->y) r->y = 1;
     }
 }
 
 // twice the first derivatives of the LC sites the class-1 forms read (see qmin_force_core.cuh)
+template <class T>
+__device__ __forceinline__ void b_derivs_at(const Lat<T> &L, const BatchAcc<T> &a)
+{
+    const int t = L.types[a.i];
+    const long long P = L.P;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        const int dn = a.nb[2 * ax], up = a.nb[2 * ax + 1];
+        const int td = t < 0 ? L.types[dn] : 0, tu = t < 0 ? L.types[up] : 0;
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+            L.D[(5 * ax + k) * P + a.i] =
+                deriv2_rule(t, td, tu, ld(L.Q + k * P + dn), ld(L.Q + k * P + a.i), ld(L.Q + k * P + up));
+    }
+}
+
 template <class T> __device__ __forceinline__ void b_derivs_chunk(const BatchArgs<T> &B, const FireDev *fds, int c)
 {
     const ChunkDesc ch = B.chunks[c];
@@ -176,18 +204,7 @@ template <class T> __device__ __forceinline__ void b_derivs_chunk(const BatchArg
     int li, x, y, z;
     if (!chunk_site(B, sd, ch, threadIdx.x, li, x, y, z)) return;
     if (B.needd && !B.needd[sd.off + li]) return;
-    BatchAcc<T> a(B.L, sd, li, x, y, z);
-    const int t = B.L.types[a.i];
-    const long long P = B.L.P;
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-        const int dn = a.nb[2 * ax], up = a.nb[2 * ax + 1];
-        const int td = t < 0 ? B.L.types[dn] : 0, tu = t < 0 ? B.L.types[up] : 0;
-#pragma unroll
-        for (int k = 0; k < 5; ++k)
-            B.L.D[(5 * ax + k) * P + a.i] =
-                deriv2_rule(t, td, tu, ld(B.L.Q + k * P + dn), ld(B.L.Q + k * P + a.i), ld(B.L.Q + k * P + up));
-    }
+    b_derivs_at(B.L, BatchAcc<T>(B.L, sd, li, x, y, z));
 }
 
 // force (KICK = 0) or force + half kick + the chunk's FIRE reductions (KICK =
@@ -246,34 +263,97 @@ __device__ __forceinline__ void b_force_chunk(const BatchArgs<T> &B, const FireD
     }
 }
 
-// one warp: deterministic sum of a solve's n partials p, then the fireStepCPU
-// scalar logic (energyMinimizerFIRE.cpp:104-144) and the loop condition of
-// minimize(); returns (in lane 0) whether the solve retired now
-__device__ __forceinline__ bool b_control_solve(FireDev *fd, const double *p, int n)
+// sums of three values over a warp in six additions: lane 0 gets v[0]'s, lane 8
+// v[1]'s, lane 16 v[2]'s (halves of the warp keep different values at the first
+// two levels; FP64 additions are the scarce operation here)
+__device__ __forceinline__ double warp_sum3(const double (&v)[3])
 {
     const int lane = threadIdx.x & 31;
-    if (!fd->active) return false;  // uniform per warp
-    double v[3] = {0.0, 0.0, 0.0};
-    // eight strides' loads in flight; each lane adds its entries in index order
-    constexpr int U = 8;
-    for (int c0 = lane; c0 < n; c0 += 32 * U) {
-        double x[U][3];
+    const bool hi = lane & 16, b3 = lane & 8;
+    double a = (hi ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
+    const double t = __shfl_xor_sync(0xffffffffu, v[1], 16);
+    const double b = hi ? 0.0 : v[1] + t;
+    a = (b3 ? b : a) + __shfl_xor_sync(0xffffffffu, b3 ? a : b, 8);
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+    for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+}
+
+// force, half kick and this thread's FIRE sums at packed site gi of an FP64 solve
+__device__ __forceinline__ void b_kick(const Lat<double> &L, int gi, double hdt, const double (&f)[5], double (&v)[5],
+                                       double (&acc)[3])
+{
 #pragma unroll
-            for (int k = 0; k < 3; ++k) x[u][k] = c0 + 32 * u < n ? p[3 * (c0 + 32 * u) + k] : 0.0;
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (c0 + 32 * u < n)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) v[k] += x[u][k];
+    for (int k = 0; k < 5; ++k) {
+        const size_t j = k * (size_t)L.P + (unsigned)gi;
+        v[k] += hdt * f[k];
+        L.V[j] = v[k];
+        L.F[j] = f[k];
     }
+    dot3_acc(f, v, acc);
+}
+
+// FP64, the bulk sites (class 0) of l0 .. l1 of a solve, in fixed point where the
+// solve is inside its range; the listed sites are items of their own, object
+// sites keep V = F = 0
+template <bool MULTI>
+__device__ __forceinline__ void b_bulk_item(const BatchArgs<double> &B, const BatchFixed &fx, const SolveDesc &sd,
+                                            double hdt, bool fixed, int l0, int l1, double (&acc)[3])
+{
+    const size_t P = (size_t)B.L.P;
+    for (int li = l0 + threadIdx.x; li < l1; li += kBlock) {
+        const int gi = sd.off + li;
+        if (B.cls[gi] != 0) continue;
+        const int r = (int)udiv((unsigned)li, (unsigned)sd.Lx, sd.mx);
+        const int x = li - r * sd.Lx, z = (int)udiv((unsigned)r, (unsigned)sd.Ly, sd.my), y = r - z * sd.Ly;
+        double f[5], v[5];
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
+        for (int k = 0; k < 5; ++k) v[k] = (B.L.V + k * P)[(unsigned)gi];  // in flight during the force
+        if (fixed) {
+            const int sy = sd.Lx, sz = sd.Lx * sd.Ly, n = sz * sd.Lz;
+            const int ox[3] = {x == 0 ? sy - 1 : -1, 0, x == sd.Lx - 1 ? 1 - sy : 1};
+            const int oy[3] = {y == 0 ? sz - sy : -sy, 0, y == sd.Ly - 1 ? sy - sz : sy};
+            const int oz[3] = {z == 0 ? n - sz : -sz, 0, z == sd.Lz - 1 ? sz - n : sz};
+            auto at = [&](int dx, int dy, int dz, int k) {
+                return (fx.X + k * P)[(unsigned)(gi + ox[dx + 1] + oy[dy + 1] + oz[dz + 1])];
+            };
+            long long q[5], lam[5], ax[5], m2[5], m3[5], a[5];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-    if (lane != 0) return false;
-    const double fn = v[0], vn = v[1], pw = v[2];
+            for (int k = 0; k < 5; ++k) q[k] = at(0, 0, 0, k);
+            fixed_axis(at, q, lam, ax);
+            if (MULTI) fixed_mixed(at, m2, m3);
+            fixed_force<MULTI>(fx.kc, q, lam, ax, m2, m3, a);
+            fixed_to_force(fx.kc, a, f);
+        } else if (MULTI) {
+            deep_force_box(B.L, sd.off, sd.Lx, sd.Ly, sd.Lz, li, (long long)gi, f);
+        } else {
+            BatchAcc<double> a(B.L, sd, li, x, y, z);
+            site_force_core<double, BatchAcc<double>, false, false, true>(B.L, a, 0, f);
+        }
+        b_kick(B.L, gi, hdt, f, v, acc);
+    }
+}
+
+// FP64, listed sites of a solve
+template <bool MULTI>
+__device__ __forceinline__ void b_listed_item(const BatchArgs<double> &B, const SolveDesc &sd, const SolveTile &st,
+                                              double hdt, int k, double (&acc)[3])
+{
+    const int e = k * st.lc + threadIdx.x;
+    if (threadIdx.x >= st.lc || e >= st.nlist) return;
+    BatchAcc<double> a(B.L, sd, st.sites[e]);
+    double f[5], v[5];
+    site_force_core<double, BatchAcc<double>, false, MULTI, !MULTI>(B.L, a, B.L.types[a.i], f);
+#pragma unroll
+    for (int k = 0; k < 5; ++k) v[k] = (B.L.V + k * (size_t)B.L.P)[(unsigned)a.i];
+    b_kick(B.L, a.i, hdt, f, v, acc);
+}
+
+// the fireStepCPU scalar logic (energyMinimizerFIRE.cpp:104-144) of one solve on
+// the sums of f.f, v.v, f.v, and the loop condition of minimize(): true when
+// the solve retires
+__device__ __forceinline__ bool b_control_step(FireDev *fd, double fn, double vn, double pw)
+{
     const int it = fd->iterations + 1;
     fd->power = pw;
     fd->forceMax = sqrt(fn) / ((double)fd->nTotal);
@@ -304,6 +384,29 @@ __device__ __forceinline__ bool b_control_solve(FireDev *fd, const double *p, in
     }
     fd->active = (it < fd->max_iters && fd->forceMax > fd->fcut) ? 1 : 0;
     return !fd->active;
+}
+
+// the block that finished a solve's last item: deterministic sum of the
+// solve's n partials p, then its control step (result in thread 0)
+template <int NT> __device__ __forceinline__ bool b_control_block(FireDev *fd, const double *p, int n)
+{
+    double v[3] = {0.0, 0.0, 0.0};
+    // four strides' loads in flight; each thread adds its entries in index order
+    constexpr int U = 4;
+    for (int c0 = threadIdx.x; c0 < n; c0 += NT * U) {
+        double x[U][3];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) x[u][k] = c0 + NT * u < n ? __ldcg(p + 3LL * (c0 + NT * u) + k) : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (c0 + NT * u < n)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) v[k] += x[u][k];
+    }
+    block_sum<3, NT>(v);
+    return threadIdx.x == 0 && b_control_step(fd, v[0], v[1], v[2]);
 }
 
 // ----------------------------------------------- launch-per-phase kernels
@@ -483,53 +586,6 @@ __device__ __forceinline__ int b_find(const ActiveList &al, int w)
     return lo;
 }
 
-// FP64: predictor, (derivative planes,) force + kick and control, a grid
-// barrier after each (the one-constant form asks for three blocks per SM: the
-// force phase would otherwise hold the registers of fewer)
-template <class T, bool ONE_CONST>
-__global__ void __launch_bounds__(kBlock, ONE_CONST ? 3 : 1)
-    k_b_fire_persistent(const __grid_constant__ BatchArgs<T> B, FireDev *fds, double *partials, int nsolves, BatchRun *run)
-{
-    extern __shared__ int b_lists[];
-    __shared__ ActiveList al;
-    if (threadIdx.x == 0) {
-        al.act = b_lists;
-        al.pre = b_lists + nsolves + 1;
-    }
-    __syncthreads();
-    auto count = [&](int s) { return B.solves[s].nchunks; };
-    // chunk of work item w (every solve active: the item itself)
-    auto chunk_of = [&](int w) {
-        if (al.all) return w;
-        const int k = b_find(al, w);
-        return B.solves[al.act[k]].chunk0 + (w - al.pre[k]);
-    };
-    b_rebuild(&al, fds, nsolves, count);
-    const int nwarps = gridDim.x * (kBlock / 32);
-    const int gwarp = blockIdx.x * (kBlock / 32) + threadIdx.x / 32;
-    for (int it = 0; al.n > 0; ++it) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) run->retired[it % 3] = 0;
-        const int nw = al.pre[al.n];
-        for (int w = blockIdx.x; w < nw; w += gridDim.x) b_pred_chunk<T>(B, fds, chunk_of(w));
-        if (!b_grid_sync(run)) return;
-        if (!ONE_CONST && B.L.multi) {
-            for (int w = blockIdx.x; w < nw; w += gridDim.x) b_derivs_chunk<T>(B, fds, chunk_of(w));
-            if (!b_grid_sync(run)) return;
-        }
-        for (int w = blockIdx.x; w < nw; w += gridDim.x) b_force_chunk<T, 1, ONE_CONST>(B, fds, partials, chunk_of(w));
-        if (!b_grid_sync(run)) return;
-        // per-solve control, one warp per active solve (its warps' sums added in order)
-        for (int k = gwarp; k < al.n; k += nwarps) {
-            const SolveDesc sd = B.solves[al.act[k]];
-            if (b_control_solve(fds + al.act[k], partials + 3LL * kBatchWarps * sd.chunk0, kBatchWarps * sd.nchunks) &&
-                (threadIdx.x & 31) == 0)
-                atomicAdd(&run->retired[it % 3], 1);
-        }
-        if (!b_grid_sync(run)) return;
-        if (*(volatile int *)&run->retired[it % 3] > 0) b_rebuild(&al, fds, nsolves, count);
-    }
-}
-
 // the predictor's coefficients and the kick's half step of one solve
 __device__ __forceinline__ void b_set_coef(float4 *coefs, const FireDev *fds, int s)
 {
@@ -559,14 +615,117 @@ struct TileItems {
     __device__ __forceinline__ void take(int *sh)
     {
         __syncthreads();
-        if (threadIdx.x == 0) {
-            *sh = nxt;
-            nxt = gridDim.x + atomicAdd(counter, 1);
-        }
+        if (threadIdx.x == 0) next(sh);
         __syncthreads();
         w = *sh;
     }
+    // as take, after an item of a solve that has n of them in this phase; true
+    // in every thread of the block that did the last one (done: a count per
+    // solve), which then sees what all of them wrote
+    __device__ __forceinline__ bool take_last(int *sh, int *done, int n)
+    {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            const int c = atomicAdd(done, 1);
+            next(sh);
+            sh[1] = c == n - 1;
+            if (c == n - 1) {
+                *done = 0;
+                __threadfence();
+            }
+        }
+        __syncthreads();
+        w = sh[0];
+        return sh[1];
+    }
+    __device__ __forceinline__ void next(int *sh)
+    {
+        *sh = nxt;
+        nxt = gridDim.x + atomicAdd(counter, 1);
+    }
 };
+
+// FP64: predictor, (derivative planes,) force + kick, a grid barrier after
+// each; the block that finishes a solve's last item does its control.  The
+// bulk force runs in fixed point (the FP64 pipe took 948 us an iteration for
+// 2.5 M one-constant sites and 1420 for 2.1 M multi-constant ones, 367 and 442
+// now); listed sites are items of their own, taken first, so that no warp waits
+// for one of them (546 with them inside the bulk runs, each chunk of 256 an
+// item; control as a phase with two more barriers 573).
+template <bool MULTI>
+__global__ void __launch_bounds__(kBlock, kFixedPerSm)
+    k_b_fire_fixed(const __grid_constant__ BatchArgs<double> B, const __grid_constant__ BatchFixed fx,
+                   const SolveTile *tiles, FireDev *fds, double *partials, int *done, int nsolves, BatchRun *run)
+{
+    extern __shared__ int b_lists[];
+    __shared__ ActiveList al;
+    __shared__ int sh_w[2];
+    if (threadIdx.x == 0) {
+        al.act = b_lists;
+        al.pre = b_lists + nsolves + 1;
+    }
+    __syncthreads();
+    auto count = [&](int s) { return tiles[s].items; };
+    b_rebuild(&al, fds, nsolves, count);
+    for (int it = 0; al.n > 0; ++it) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            run->retired[it % 3] = 0;
+            run->next[2 * ((it + 1) % 3)] = run->next[2 * ((it + 1) % 3) + 1] = 0;
+        }
+        for (int w = blockIdx.x; w < al.pre[al.n]; w += gridDim.x) {
+            const int e = b_find(al, w), s = al.act[e], k = w - al.pre[e];
+            const SolveTile st = tiles[s];
+            if (k < st.ntile) b_pred_item(B, fx, fds, s, k * st.zc, min((k + 1) * st.zc, st.n));
+        }
+        if (!b_grid_sync(run)) return;
+        if (MULTI) {
+            for (TileItems q(al, &run->next[2 * (it % 3)]); q.more(al); q.take(sh_w)) {
+                int s, k;
+                q.item(al, s, k);
+                const SolveTile st = tiles[s];
+                const int e = k * kBlock + threadIdx.x;
+                if (e < st.nderiv) b_derivs_at(B.L, BatchAcc<double>(B.L, B.solves[s], st.derivs[e]));
+            }
+            if (!b_grid_sync(run)) return;
+        }
+        TileItems q(al, &run->next[2 * (it % 3) + 1]);
+        while (q.more(al)) {
+            int s, k;
+            q.item(al, s, k);
+            const SolveTile st = tiles[s];
+            const int nli = (st.nlist + st.lc - 1) / st.lc, n = nli + st.ntile;
+            if (k >= n) {
+                q.take(sh_w);
+                continue;
+            }
+            const SolveDesc sd = B.solves[s];
+            const double hdt = 0.5 * fds[s].dt;
+            double acc[3] = {0.0, 0.0, 0.0};
+            if (k < nli) {
+                b_listed_item<MULTI>(B, sd, st, hdt, k, acc);
+            } else {
+                const volatile int2 *rg = fx.range + s;
+                const int l0 = (k - nli) * st.zc;
+                b_bulk_item<MULTI>(B, fx, sd, hdt, fx.X && rg->y && !rg->x, l0, min(l0 + st.zc, st.n), acc);
+            }
+            const double sum = warp_sum3(acc);
+            const int lane = threadIdx.x & 31;
+            if ((lane & 7) == 0 && lane <= 16)
+                partials[3 * ((long long)kBatchWarps * (st.item0 + k) + threadIdx.x / 32) + lane / 8] = sum;
+            if (q.take_last(sh_w, done + s, n)) {
+                const bool retired =
+                    b_control_block<kBlock>(fds + s, partials + 3LL * kBatchWarps * st.item0, kBatchWarps * n);
+                if (threadIdx.x == 0) {
+                    if (fx.X) fx.range[s] = make_int2(0, 0);
+                    if (retired) atomicAdd(&run->retired[it % 3], 1);
+                }
+            }
+        }
+        if (!b_grid_sync(run)) return;
+        if (*(volatile int *)&run->retired[it % 3] > 0) b_rebuild(&al, fds, nsolves, count);
+    }
+}
 
 // FP32: one phase per iteration for predictor, force and kick (b_tile_item),
 // before it for multi-constant solves the derivative planes the listed sites
@@ -580,11 +739,11 @@ template <bool MULTI>
 __global__ void __launch_bounds__(kTileThreads, kTilePerSm)
     k_b_fire_tiled(const __grid_constant__ BatchArgs<float> B, const SolveTile *tiles,
                    const __grid_constant__ BatchSet<float> s1, FireDev *fds, float4 *coefs,
-                   double *partials, int *in_second, int nsolves, BatchRun *run)
+                   double *partials, int *in_second, int *done, int nsolves, BatchRun *run)
 {
     extern __shared__ __align__(16) float b_ring[];  // the plane ring, then the lists
     __shared__ ActiveList al;
-    __shared__ int sh_w;
+    __shared__ int sh_w[2];
     if (threadIdx.x == 0) {
         al.act = reinterpret_cast<int *>(b_ring + kTileRing);
         al.pre = al.act + nsolves + 1;
@@ -595,8 +754,6 @@ __global__ void __launch_bounds__(kTileThreads, kTilePerSm)
         b_set_coef(coefs, fds, s);
     b_rebuild(&al, fds, nsolves, count);
     if (!b_grid_sync(run)) return;
-    const int nwarps = gridDim.x * (kTileThreads / 32);
-    const int gwarp = blockIdx.x * (kTileThreads / 32) + threadIdx.x / 32;
     const BatchSet<float> s0{B.L.Q, B.L.V, B.L.F};
     for (int it = 0; al.n > 0; ++it) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -605,7 +762,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilePerSm)
         }
         const BatchSet<float> in = (it & 1) ? s1 : s0, out = (it & 1) ? s0 : s1;
         if (MULTI) {
-            for (TileItems q(al, &run->next[2 * (it % 3)]); q.more(al); q.take(&sh_w)) {
+            for (TileItems q(al, &run->next[2 * (it % 3)]); q.more(al); q.take(sh_w)) {
                 int s, k;
                 q.item(al, s, k);
                 const SolveTile st = tiles[s];
@@ -615,12 +772,16 @@ __global__ void __launch_bounds__(kTileThreads, kTilePerSm)
             }
             if (!b_grid_sync(run)) return;
         }
-        for (TileItems q(al, &run->next[2 * (it % 3) + 1]); q.more(al); q.take(&sh_w)) {
+        TileItems q(al, &run->next[2 * (it % 3) + 1]);
+        while (q.more(al)) {
             int s, k;
             q.item(al, s, k);
             const SolveTile st = tiles[s];
-            const int nli = (st.nlist + kTileThreads - 1) / kTileThreads;
-            if (k >= nli + st.ntile) continue;
+            const int nli = (st.nlist + kTileThreads - 1) / kTileThreads, n = nli + st.ntile;
+            if (k >= n) {
+                q.take(sh_w);
+                continue;
+            }
             const float4 c = __ldcg(coefs + s);
             const PredCoef<float> pc{c.x, c.y, c.z};
             const SolveDesc sd = B.solves[s];
@@ -630,26 +791,19 @@ __global__ void __launch_bounds__(kTileThreads, kTilePerSm)
             else if (it & 1) b_tile_item<MULTI>(B.L, B.cls, s1, s0, pc, c.w, sd, st, k - nli, b_ring, a);
             else b_tile_item<MULTI>(B.L, B.cls, s0, s1, pc, c.w, sd, st, k - nli, b_ring, a);
             // FP32 over a thread's column, FP64 from there on
-            double acc[3] = {(double)a[0], (double)a[1], (double)a[2]};
-            block_sum<3, kTileThreads>(acc);
-            if (threadIdx.x == 0) {
-                double *p = partials + 3LL * (st.item0 + k);
-                p[0] = acc[0];
-                p[1] = acc[1];
-                p[2] = acc[2];
-            }
-        }
-        if (!b_grid_sync(run)) return;
-        for (int k = gwarp; k < al.n; k += nwarps) {
-            const int s = al.act[k];
-            const SolveTile st = tiles[s];
-            const int n = st.ntile + (st.nlist + kTileThreads - 1) / kTileThreads;
-            const bool retired = b_control_solve(fds + s, partials + 3LL * st.item0, n);
-            if ((threadIdx.x & 31) == 0) {
-                b_set_coef(coefs, fds, s);
-                if (retired) {
-                    atomicAdd(&run->retired[it % 3], 1);
-                    in_second[s] = (it & 1) == 0;
+            const double sum = warp_sum3({(double)a[0], (double)a[1], (double)a[2]});
+            const int lane = threadIdx.x & 31;
+            if ((lane & 7) == 0 && lane <= 16)
+                partials[3 * ((long long)kTileWarps * (st.item0 + k) + threadIdx.x / 32) + lane / 8] = sum;
+            if (q.take_last(sh_w, done + s, n)) {
+                const bool retired = b_control_block<kTileThreads>(
+                    fds + s, partials + 3LL * kTileWarps * st.item0, kTileWarps * n);
+                if (threadIdx.x == 0) {
+                    b_set_coef(coefs, fds, s);
+                    if (retired) {
+                        atomicAdd(&run->retired[it % 3], 1);
+                        in_second[s] = (it & 1) == 0;
+                    }
                 }
             }
         }
@@ -698,14 +852,14 @@ struct qmin_batch_ctx {
     ChunkDesc *chunks = nullptr;
     void *Q = nullptr, *V = nullptr, *F = nullptr, *D = nullptr, *objs = nullptr;
     void *Q2 = nullptr, *V2 = nullptr, *F2 = nullptr;  // second state set of the FP32 iteration
-    // FP32: the items of each solve, its predictor coefficients, their sums
+    // the items of each solve, its predictor coefficients (FP32), their sums
     SolveTile *tiles = nullptr;
     float4 *coefs = nullptr;
     double *tile_partials = nullptr;
     size_t tile_partials_cap = 0;
     std::vector<SolveTile> tiles_h;
     // per solve: its site types (host), its listed sites and derivative sites
-    // (device, multi-constant FP32) and whether classes and lists are those of its types
+    // (device; those of multi-constant solves) and whether classes and lists are those of its types
     struct SolveLists {
         std::vector<int8_t> types;
         int *sites = nullptr, *derivs = nullptr;
@@ -715,6 +869,9 @@ struct qmin_batch_ctx {
     std::vector<SolveLists> lists;
     bool tiles_multi = false, classified_multi = false;
     void *geo_scratch = nullptr;
+    long long *X = nullptr;  // FP64: Q 2^56 of the fixed-point force
+    int2 *range = nullptr;
+    int *done = nullptr;  // per solve: items of the phase that are done
     int *in_second = nullptr;                          // per solve: final state in the second set
     int8_t *types = nullptr;
     uint8_t *cls = nullptr, *needd = nullptr;  // per packed site (multi-constant split of the force)
@@ -874,7 +1031,7 @@ template <class T> static int tune_shape(qmin_batch_ctx *b)
 
 // Site classes of every solve whose types changed since they were last taken,
 // on the device: classes, the derivative-plane marks and the two lists
-// (multi-constant), or the boundary sites (one-constant FP32).
+// (multi-constant), or the boundary sites (one-constant).
 static int classify_solves(qmin_batch_ctx *b)
 {
     const bool multi = b->params.multi_constant != 0;
@@ -915,19 +1072,24 @@ static int classify_solves(qmin_batch_ctx *b)
     return QMIN_OK;
 }
 
-// the items of every solve: tiles of about 128 sites cut evenly (at most 32
-// wide and 32 high), z chunks of 4 to 16 planes so that there are about four
-// items per resident block (two, three and six measured within 5 %)
-static int lay_out_tiles(qmin_batch_ctx *b, bool multi)
+// the items of every solve.  FP32: tiles of about 128 sites cut evenly (at most
+// 32 wide and 32 high), z chunks of 4 to 16 planes so that there are about four
+// items per resident block (two, three and six measured within 5 %).  FP64:
+// runs of 1 to 8 blocks' sites, by the same rule (40 uneven solves, 2.5 M sites:
+// 431 us with runs of one block's sites, 389 two, 370 four, 367 eight, 382 ten).
+static int lay_out_items(qmin_batch_ctx *b, bool multi)
 {
     if (!b->tiles_h.empty() && b->tiles_multi == multi) return QMIN_OK;
     auto cut = [](int n, int most) { return (n + most - 1) / most; };
+    const bool fp32 = b->prec == QMIN_FP32;
+    const int block = fp32 ? kTileThreads : kBlock;
     std::vector<SolveTile> t((size_t)b->nsolves);
     long long planes = 0;
     for (int s = 0; s < b->nsolves; ++s) {
         const SolveDesc &sd = b->solves_h[s];
         SolveTile &st = t[s];
         memset(&st, 0, sizeof st);
+        st.n = sd.Lx * sd.Ly * sd.Lz;
         st.ntx = cut(sd.Lx, kTileWide);
         st.tx = cut(sd.Lx, st.ntx);
         st.nty = cut(sd.Ly, std::min(32, kTileThreads / st.tx));
@@ -935,35 +1097,47 @@ static int lay_out_tiles(qmin_batch_ctx *b, bool multi)
         planes += (long long)st.ntx * st.nty * sd.Lz;
     }
     const int zmax = (int)std::min(16LL, std::max(4LL, planes / (152 * kTilePerSm * 4)));
+    // a listed site costs ten bulk ones on the FP64 pipe: few of them are spread over the SMs (eight
+    // solves of 16^3 to 24^3: 56 us an iteration, 77 with 256 to an item)
+    long long nl = 0;
+    for (const auto &l : b->lists) nl += l.n_sites;
+    const int lc = fp32 ? kTileThreads : 32 * (int)std::min(8LL, 1 + nl / (32LL * 152 * kFixedPerSm));
+    const int run = kBlock * (int)std::min(8, std::max(1, b->N / (kBlock * 152 * kFixedPerSm * 4)));
     long long items = 0;
     for (int s = 0; s < b->nsolves; ++s) {
         const SolveDesc &sd = b->solves_h[s];
         SolveTile &st = t[s];
-        const int nz = cut(sd.Lz, zmax);
-        st.zc = cut(sd.Lz, nz);
-        st.ntile = st.ntx * st.nty * cut(sd.Lz, st.zc);
+        if (fp32) {
+            st.zc = cut(sd.Lz, cut(sd.Lz, zmax));
+            st.ntile = st.ntx * st.nty * cut(sd.Lz, st.zc);
+        } else {
+            st.zc = run;
+            st.ntile = cut(st.n, run);
+        }
         st.nlist = b->lists[s].n_sites;
         st.sites = b->lists[s].sites;
         if (multi) {
             st.nderiv = b->lists[s].n_derivs;
             st.derivs = b->lists[s].derivs;
         }
-        st.items = std::max(st.ntile + cut(st.nlist, kTileThreads), cut(st.nderiv, kTileThreads));
+        st.lc = lc;
+        st.items = std::max(st.ntile + cut(st.nlist, lc), cut(st.nderiv, block));
         st.item0 = (int)items;
         items += st.items;
     }
-    if (items > b->tile_partials_cap) {
+    if (items > (long long)b->tile_partials_cap) {
         if (b->tile_partials) cudaFree(b->tile_partials);
         b->tile_partials = nullptr;
         b->tile_partials_cap = 0;
-        if (cudaMalloc(&b->tile_partials, sizeof(double) * 3 * (size_t)items) != cudaSuccess) {
+        if (cudaMalloc(&b->tile_partials, sizeof(double) * 3 * (block / 32) * (size_t)items) != cudaSuccess) {
             cudaGetLastError();
             return bfail(QMIN_ENOMEM, "batch: partial sums allocation failed");
         }
         b->tile_partials_cap = (size_t)items;
     }
     if ((!b->tiles && cudaMalloc(&b->tiles, sizeof(SolveTile) * (size_t)b->nsolves) != cudaSuccess) ||
-        (!b->coefs && cudaMalloc(&b->coefs, sizeof(float4) * (size_t)b->nsolves) != cudaSuccess)) {
+        (!b->coefs && cudaMalloc(&b->coefs, sizeof(float4) * (size_t)b->nsolves) != cudaSuccess) ||
+        (!b->done && cudaMalloc(&b->done, sizeof(int) * (size_t)b->nsolves) != cudaSuccess)) {
         cudaGetLastError();
         return bfail(QMIN_ENOMEM, "batch: tile table allocation failed");
     }
@@ -994,17 +1168,44 @@ template <bool MULTI> static int launch_tiled(qmin_batch_ctx *b, const BatchArgs
     BatchArgs<float> a = B;
     const SolveTile *tiles = b->tiles;
     BatchSet<float> s1{(float *)b->Q2, (float *)b->V2, (float *)b->F2};
-    void *args[] = {&a, &tiles, &s1, &b->fds, &b->coefs, &b->tile_partials, &b->in_second, &b->nsolves, &b->run};
+    void *args[] = {&a, &tiles, &s1, &b->fds, &b->coefs, &b->tile_partials, &b->in_second, &b->done, &b->nsolves, &b->run};
     return launch_cooperative(b, (const void *)k_b_fire_tiled<MULTI>, kTileThreads,
                               sizeof(float) * kTileRing + sizeof(int) * 2 * ((size_t)b->nsolves + 1), args);
 }
 
-template <bool ONE_CONST> static int launch_persistent(qmin_batch_ctx *b, const BatchArgs<double> &B)
+template <bool MULTI> static int launch_fixed(qmin_batch_ctx *b, const BatchArgs<double> &B, const BatchFixed &fx)
 {
     BatchArgs<double> a = B;
-    void *args[] = {&a, &b->fds, &b->partials, &b->nsolves, &b->run};
-    return launch_cooperative(b, (const void *)k_b_fire_persistent<double, ONE_CONST>, kBlock,
+    BatchFixed f = fx;
+    const SolveTile *tiles = b->tiles;
+    void *args[] = {&a, &f, &tiles, &b->fds, &b->tile_partials, &b->done, &b->nsolves, &b->run};
+    return launch_cooperative(b, (const void *)k_b_fire_fixed<MULTI>, kBlock,
                               sizeof(int) * 2 * ((size_t)b->nsolves + 1), args);
+}
+
+// the fixed-point force of the current parameters and its buffers (X null: the
+// form has none, or they do not fit)
+static BatchFixed batch_fixed(qmin_batch_ctx *b, const Lat<double> &L)
+{
+    BatchFixed fx;
+    memset(&fx, 0, sizeof fx);
+    double field[5];
+    for (int c = 0; c < 5; ++c) field[c] = (L.efield ? L.fE[c] : 0.0) + (L.hfield ? L.fH[c] : 0.0);
+    fx.kc = fixed_coeffs(b->params, b->metric_mode, L.efield || L.hfield ? field : nullptr);
+    if (!fx.kc.ok) return fx;
+    if (!b->X && cudaMalloc(&b->X, 5 * (size_t)b->P * sizeof(long long)) != cudaSuccess) {
+        cudaGetLastError();
+        b->X = nullptr;
+        return fx;
+    }
+    if (!b->range && cudaMalloc(&b->range, sizeof(int2) * (size_t)b->nsolves) != cudaSuccess) {
+        cudaGetLastError();
+        b->range = nullptr;
+        return fx;
+    }
+    fx.X = b->X;
+    fx.range = b->range;
+    return fx;
 }
 
 // The API functions below take C linkage from their declarations in qmin_gb300.h.
@@ -1094,7 +1295,7 @@ int qmin_batch_destroy(qmin_batch b)
     if (b->stream) cudaStreamSynchronize(b->stream);
     void *bufs[] = {b->Q, b->V, b->F, b->D, b->objs, b->types, b->partials, b->stage, b->fds,
                     b->solves, b->chunks, b->cls, b->needd, b->cbd, b->run, b->Q2, b->V2, b->F2, b->in_second,
-                    b->tiles, b->coefs, b->tile_partials, b->geo_scratch};
+                    b->tiles, b->coefs, b->tile_partials, b->geo_scratch, b->X, b->range, b->done};
     for (void *p : bufs)
         if (p) cudaFree(p);
     for (auto &l : b->lists) {
@@ -1246,8 +1447,7 @@ int qmin_batch_fire_init(qmin_batch b, const qmin_fire_params *p)
 
 template <class T> static int batch_fire_impl(qmin_batch_ctx *b, bool *timed_out)
 {
-    if (b->params.multi_constant || sizeof(T) == 4)
-        if (int r = classify_solves(b)) return r;
+    if (int r = classify_solves(b)) return r;
     // every solve's minimize() starts with its forces (energyMinimizerFIRE.cpp:157)
     b->launches += launch_b_force<T>(batch_args<T>(b), b->fds, b->partials, 0, b->stream);
     if (b->shape < 0) {
@@ -1271,12 +1471,15 @@ template <class T> static int batch_fire_impl(qmin_batch_ctx *b, bool *timed_out
         }
     }
     if (fused) BCK(cudaMemsetAsync(b->in_second, 0, sizeof(int) * (size_t)b->nsolves, b->stream));
-    int r;
+    int r = lay_out_items(b, B.L.multi != 0);
+    if (r) return r;
+    BCK(cudaMemsetAsync(b->done, 0, sizeof(int) * (size_t)b->nsolves, b->stream));
     if constexpr (sizeof(T) == 4) {
-        if ((r = lay_out_tiles(b, B.L.multi != 0))) return r;
         r = B.L.multi ? launch_tiled<true>(b, B) : launch_tiled<false>(b, B);
     } else {
-        r = B.L.multi ? launch_persistent<false>(b, B) : launch_persistent<true>(b, B);
+        const BatchFixed fx = batch_fixed(b, B.L);
+        if (fx.X) BCK(cudaMemsetAsync(fx.range, 0, sizeof(int2) * (size_t)b->nsolves, b->stream));
+        r = B.L.multi ? launch_fixed<true>(b, B, fx) : launch_fixed<false>(b, B, fx);
     }
     if (r) return r;
     b->launches += 1;

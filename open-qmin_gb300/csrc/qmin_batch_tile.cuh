@@ -27,15 +27,17 @@ namespace qmin {
 // at every site and 91 stencil reads through L1 (multi-constant).  Now 34 % of
 // the issue slots and 44 % of the measured HBM rate: plane loads one plane
 // ahead at 12 warps per SM.
-constexpr int kTileThreads = 128, kTilePerSm = 3, kTileWide = 32;
+constexpr int kTileThreads = 128, kTileWarps = kTileThreads / 32, kTilePerSm = 3, kTileWide = 32;
 constexpr int kTilePlane = 204;  // sites of a staged plane: at most (32 + 2) x (4 + 2)
 constexpr int kTileHalo = 96;  // halo entries of a plane: at most 2 (32 + 2) + 2 x 8, 2 (4 + 2) + 2 x 32
 constexpr int kTileRing = 4 * 5 * kTilePlane + 15 * kTileHalo;  // floats: the ring, one plane's raw halo
 
 // the items of one solve: list items (kTileThreads listed sites each), then tile items
 struct SolveTile {
-    int tx, ty, ntx, nty, zc;  // sites of a tile, tiles along x and y, planes of an item
+    int n;                     // sites of the solve
+    int tx, ty, ntx, nty, zc;  // sites of a tile, tiles along x and y, planes of an item (FP64: its sites)
     int ntile, nlist, nderiv;  // tile items; listed sites and derivative sites (multi-constant)
+    int lc;                    // listed sites of an item
     int items, item0;          // items of the solve (at least its derivative items), the first one
     const int *sites, *derivs; // solve-local indices
 };
@@ -168,12 +170,12 @@ __device__ __forceinline__ void b_tile_item(const Lat<float> &L, const uint8_t *
                                         QQ(0, 1, 0, c) - QQ(0, 0, -1, c) - QQ(0, 0, 1, c));
                     l1_cross(s2);
                 } else if (L.L4 == 0.f) {
-                    QMIN_BULK_Q25_NO_L4(L.cq, s2);
+                    QMIN_BULK_Q25_NO_L4_PLAIN(L.cqp, s2);  // as deep_force_box
                 } else {
                     QMIN_BULK_Q25(L.cq, s2);
                 }
 #undef QQ
-                deep_force_finish(L, qc[1], s2, (long long)i, f);
+                deep_force_finish<float, MULTI>(L, qc[1], s2, (long long)i, f);  // the bits of the site form
                 float v[5];
 #pragma unroll
                 for (int c = 0; c < 5; ++c) {

@@ -418,12 +418,14 @@ template <class T> __device__ __forceinline__ const T *site_field(const Lat<T> &
 }
 
 // force of a deep bulk site from its Q and its combined bulk form s2, M
-// applied as for type-0 sites (twice in CPU mode, the fields between the two)
-template <class T>
+// applied as for type-0 sites (twice in CPU mode, the fields between the two);
+// SQUARED: M M in one where no field comes between, as the other deep forms
+// (site_force_core's one-constant form has it twice)
+template <class T, bool SQUARED = true>
 __device__ __forceinline__ void deep_force_finish(const Lat<T> &L, const T *q, const T *s2, long long i, T *f)
 {
     phase_force_sub(L.a, L.b, L.c, q, s2, f);
-    if (L.metric_mode == 0 && !L.efield && !L.hfield && !L.Hv) {
+    if (SQUARED && L.metric_mode == 0 && !L.efield && !L.hfield && !L.Hv) {
         metric2(f);
         return;
     }
