@@ -67,6 +67,7 @@ struct qmin_ctx {
     // side stream (highest priority) and fork/join events for the listed sites of the split path
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    ForceFork fork{};
     void *Q = nullptr, *V = nullptr, *F = nullptr, *D = nullptr;
     void *cbd = nullptr;  // merged boundary coefficients (multi-constant)
     int8_t *types = nullptr;
@@ -92,6 +93,7 @@ struct qmin_ctx {
     double *out5 = nullptr;
     double *out5_h = nullptr;
     void *M = nullptr, *S = nullptr, *alt = nullptr, *lbp = nullptr, *lbs = nullptr, *lby = nullptr;
+    LbGram *lbg = nullptr;  // FP32: products of the L-BFGS pairs
     int lb_m = 0;
     qmin_ldg_params params{};
     bool have_params = false, have_state = false, fire_ready = false;
@@ -273,6 +275,18 @@ static bool ensure_fixed(qmin_ctx *h, const Lat<double> &L)
     return true;
 }
 
+static int ensure_aux(qmin_ctx *h)
+{
+    int least = 0, greatest = 0;
+    if (!h->aux) {
+        CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        CK(cudaStreamCreateWithPriority(&h->aux, cudaStreamNonBlocking, greatest));
+    }
+    if (!h->ev_fork) CK(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
+    if (!h->ev_join) CK(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
+    return QMIN_OK;
+}
+
 template <class T> static Lat<T> make_lat(qmin_ctx *h)
 {
     Lat<T> L;
@@ -295,6 +309,10 @@ template <class T> static Lat<T> make_lat(qmin_ctx *h)
     if (h->prec == QMIN_FP32) ensure_tmap(h);
     L.split = SplitLists{h->split_cls, h->split_sites, h->n_split_sites, h->split_derivs, h->n_split_derivs,
                          h->tmap_ok ? &h->tmap_q : nullptr, h->dev_err};
+    if (h->n_split_sites > 0 && ensure_aux(h) == QMIN_OK) {
+        h->fork = ForceFork{h->aux, h->ev_fork, h->ev_join};
+        L.fork = &h->fork;
+    }
     if constexpr (sizeof(T) == 8)
         if (ensure_fixed(h, L)) {
             L.X = h->X;
@@ -309,7 +327,7 @@ static void free_ctx(qmin_ctx *h)
     for (int g = 0; g < 5; ++g)
         if (h->graph[g]) cudaGraphExecDestroy(h->graph[g]);
     void *bufs[] = {h->Q, h->V, h->F, h->D, h->types, h->objs, h->partials, h->stage, h->stage_t, h->fire, h->iter,
-                    h->out5, h->M, h->S, h->alt, h->lbp, h->lbs, h->lby, h->Q2, h->V2, h->F2, h->hvar,
+                    h->out5, h->M, h->S, h->alt, h->lbp, h->lbs, h->lby, h->lbg, h->Q2, h->V2, h->F2, h->hvar,
                     h->split_cls, h->split_sites, h->split_derivs, h->cbd, h->dev_err, h->geo_scratch,
                     h->scan_part, h->scan_out, h->X, h->fx};
     for (void *b : bufs)
@@ -393,6 +411,7 @@ int qmin_create(const qmin_lattice_desc *desc, qmin_handle *out)
     cudaMemsetAsync(h->types, 0, (size_t)h->P, h->stream);
     memset(h->fire_h, 0, sizeof(FireDev));
     memset(h->iter_h, 0, sizeof(IterDev));
+    if (ensure_aux(h) != QMIN_OK) cudaGetLastError();  // here, so that no first call waits for it
     *out = h;
     return QMIN_OK;
 }
@@ -779,8 +798,8 @@ int qmin_energy(qmin_handle h, double *e_per_active, double comps[5])
 }
 
 // ------------------------------------------------------------- graphs
-// Record `per_iter` launches of one iteration kChunk times into a graph.
-template <class F> static int capture_chunk(qmin_ctx *h, int slot, const double (&args)[4], F &&one_iteration)
+// Record the launches of one iteration `chunk` times into a graph.
+template <class F> static int capture_chunk(qmin_ctx *h, int slot, const double (&args)[4], F &&one_iteration, int chunk = kChunk)
 {
     if (h->graph[slot] && h->graph_key[slot] == h->version &&
         memcmp(h->graph_args[slot], args, sizeof(args)) == 0)
@@ -792,14 +811,14 @@ template <class F> static int capture_chunk(qmin_ctx *h, int slot, const double 
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int per = 0;
-    for (int k = 0; k < kChunk; ++k) per = one_iteration();
+    for (int k = 0; k < chunk; ++k) per = one_iteration();
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     if (e != cudaSuccess) return fail(QMIN_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     // per-node priorities: the side stream's list kernels carry the greatest one
     e = cudaGraphInstantiate(&h->graph[slot], g, cudaGraphInstantiateFlagUseNodePriority);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(QMIN_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    h->graph_per_iter[slot] = per;
+    h->graph_per_iter[slot] = per * chunk;
     h->graph_key[slot] = h->version;
     memcpy(h->graph_args[slot], args, sizeof(args));
     return QMIN_OK;
@@ -811,7 +830,7 @@ template <class S> static int run_chunks(qmin_ctx *h, int slot, S *dev, S *host,
 {
     for (int c = 0; c < max_chunks; ++c) {
         CK(cudaGraphLaunch(h->graph[slot], h->stream));
-        h->launches += (long long)kChunk * h->graph_per_iter[slot];
+        h->launches += h->graph_per_iter[slot];
         CK(cudaMemcpyAsync(host, dev, sizeof(S), cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
         if (!host->active) break;
@@ -867,17 +886,6 @@ int qmin_fire_set_state(qmin_handle h, const qmin_fire_state *st)
     f->reset = 0;
     CK(cudaMemcpyAsync(h->fire, f, sizeof(FireDev), cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    return QMIN_OK;
-}
-
-static int ensure_aux(qmin_ctx *h)
-{
-    if (h->aux) return QMIN_OK;
-    int least = 0, greatest = 0;
-    CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    CK(cudaStreamCreateWithPriority(&h->aux, cudaStreamNonBlocking, greatest));
-    CK(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
     return QMIN_OK;
 }
 
@@ -1373,10 +1381,21 @@ static int iter_begin(qmin_ctx *h, int reset, double fm0, double fcut, int max_i
     return QMIN_OK;
 }
 
+// Adam and Nesterov step from the forces at the old Q.  A run that ends inside
+// a chunk leaves F at the new Q.
+template <class T> static int force_at_end(qmin_ctx *h, int first)
+{
+    if ((h->iter_h->iterations - first) % kChunk != 0)
+        h->launches += launch_force<T>(make_lat<T>(h), h->grid, h->stream);
+    return QMIN_OK;
+}
+
 template <class T>
 static int adam_impl(qmin_ctx *h, double b1, double b2, double eps, double dt, int max_iterations)
 {
     Lat<T> L = make_lat<T>(h);
+    const int first = h->iter_h->iterations;
+    L.go = &h->iter->active;
     const double args[4] = {b1, b2, eps, dt};
     int r = capture_chunk(h, 1, args, [&]() {
         int n = launch_force<T>(L, h->grid, h->stream);
@@ -1385,7 +1404,8 @@ static int adam_impl(qmin_ctx *h, double b1, double b2, double eps, double dt, i
         return n;
     });
     if (r) return r;
-    return run_chunks(h, 1, h->iter, h->iter_h, max_iterations / kChunk + 2);
+    if ((r = run_chunks(h, 1, h->iter, h->iter_h, max_iterations / kChunk + 2))) return r;
+    return force_at_end<T>(h, first);
 }
 
 int qmin_adam_run(qmin_handle h, double beta1, double beta2, double eps, double dt, double force_cutoff,
@@ -1423,6 +1443,8 @@ int qmin_adam_run(qmin_handle h, double beta1, double beta2, double eps, double 
 template <class T> static int nesterov_impl(qmin_ctx *h, double dt, double mu, int max_iterations)
 {
     Lat<T> L = make_lat<T>(h);
+    const int first = h->iter_h->iterations;
+    L.go = &h->iter->active;
     const double args[4] = {dt, mu, 0, 0};
     int r = capture_chunk(h, 2, args, [&]() {
         int n = launch_force<T>(L, h->grid, h->stream);
@@ -1431,7 +1453,8 @@ template <class T> static int nesterov_impl(qmin_ctx *h, double dt, double mu, i
         return n;
     });
     if (r) return r;
-    return run_chunks(h, 2, h->iter, h->iter_h, max_iterations / kChunk + 2);
+    if ((r = run_chunks(h, 2, h->iter, h->iter_h, max_iterations / kChunk + 2))) return r;
+    return force_at_end<T>(h, first);
 }
 
 int qmin_nesterov_run(qmin_handle h, double dt, double mu, double force_cutoff, int max_iterations, int reset,
@@ -1463,6 +1486,7 @@ int qmin_nesterov_run(qmin_handle h, double dt, double mu, double force_cutoff, 
 template <class T> static int gd_impl(qmin_ctx *h, double dt, int max_iterations)
 {
     Lat<T> L = make_lat<T>(h);
+    L.go = &h->iter->active;
     const double args[4] = {dt, 0, 0, 0};
     int r = capture_chunk(h, 4, args, [&]() {
         int n = launch_gd_move<T>(L, h->iter, dt, h->stream);
@@ -1501,18 +1525,30 @@ int qmin_gd_run(qmin_handle h, double dt, double force_cutoff, int max_iteration
 template <class T> static int lbfgs_impl(qmin_ctx *h, int m, double eta, int max_iterations)
 {
     Lat<T> L = make_lat<T>(h);
+    // FP32 without room for the products: the passes
+    LbGram *gram = sizeof(T) == 4 && m <= kLbGram ? h->lbg : nullptr;
     if (h->iter_h->iterations == 0) {
         // LoLBFGSStepCPU step 1 (energyMinimizerLoLBFGS.cpp:110-116): p = forces at Q,
         // which the iteration's first pass reads from F
         h->launches += launch_force<T>(L, h->grid, h->stream);
+        if (gram) CK(cudaMemsetAsync(gram, 0, sizeof(LbGram), h->stream));
+    } else if (gram) {
+        // a resumed run (the pairs may come from a file): all products afresh
+        if constexpr (sizeof(T) == 4)
+            h->launches += launch_lbfgs_products(L, (T *)h->lbs, (T *)h->lby, h->iter, gram, m, h->partials, h->stream);
     }
+    // an iteration has up to 27 launches and takes 0.9 ms at 200^3: from 10^6 sites
+    // the wait for the host after a chunk of eight is below 2 %, and the capture
+    // and the empty rest of the last chunk cost a quarter
+    const int chunk = h->N >= 1000000 ? 8 : kChunk;
     const double args[4] = {(double)m, eta, 0, 0};
+    L.go = &h->iter->active;
     int r = capture_chunk(h, 3, args, [&]() {
-        return launch_lbfgs_iteration<T>(L, (T *)h->lbp, (T *)h->lbs, (T *)h->lby, h->iter, m, eta, h->partials,
+        return launch_lbfgs_iteration<T>(L, (T *)h->lbp, (T *)h->lbs, (T *)h->lby, h->iter, gram, m, eta, h->partials,
                                          h->grid, h->stream);
-    });
+    }, chunk);
     if (r) return r;
-    return run_chunks(h, 3, h->iter, h->iter_h, max_iterations / kChunk + 2);
+    return run_chunks(h, 3, h->iter, h->iter_h, max_iterations / chunk + 2);
 }
 
 int qmin_lbfgs_run(qmin_handle h, int m, double eta, double force_cutoff, int max_iterations, int reset,
@@ -1530,6 +1566,10 @@ int qmin_lbfgs_run(qmin_handle h, int m, double eta, double force_cutoff, int ma
     }
     if ((r = alloc_planes(h, &h->lbp, 1)) || (r = alloc_planes(h, &h->lbs, m)) || (r = alloc_planes(h, &h->lby, m)))
         return r;
+    if (h->esz == 4 && !h->lbg && cudaMalloc(&h->lbg, sizeof(LbGram)) != cudaSuccess) {
+        cudaGetLastError();
+        h->lbg = nullptr;
+    }
     if (reset) {
         CK(cudaMemsetAsync(h->lbs, 0, (size_t)m * 5 * (size_t)h->P * h->esz, h->stream));
         CK(cudaMemsetAsync(h->lby, 0, (size_t)m * 5 * (size_t)h->P * h->esz, h->stream));

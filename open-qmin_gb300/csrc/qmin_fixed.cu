@@ -30,9 +30,9 @@ template <bool MOVE>
 __global__ void __launch_bounds__(kBlock)
     k_fixed_pred(double *__restrict__ Q, double *__restrict__ V, const double *__restrict__ F,
                  const int8_t *__restrict__ types, long long *__restrict__ X, long long P,
-                 const FireDev *__restrict__ fd, FixedDev *fx)
+                 const FireDev *__restrict__ fd, const int *go, FixedDev *fx)
 {
-    if (MOVE && !fd->active) return;
+    if (MOVE ? !fd->active : go && !*go) return;
     PredCoef<double> pc{0, 0, 0};
     if (MOVE) pc = pred_coef<double>(fd);
     int m = 0;  // largest |Q| as its upper word
@@ -140,8 +140,8 @@ __global__ void __launch_bounds__(kFixBlock, kFixPerSm)
 int launch_fixed_pred(const Lat<double> &L, const FireDev *fd, cudaStream_t s)
 {
     const int g = (int)((L.P / 2 + kBlock - 1) / kBlock);
-    if (fd) k_fixed_pred<true><<<g, kBlock, 0, s>>>(L.Q, L.V, L.F, L.types, L.X, L.P, fd, L.fx);
-    else k_fixed_pred<false><<<g, kBlock, 0, s>>>(L.Q, L.V, L.F, L.types, L.X, L.P, nullptr, L.fx);
+    if (fd) k_fixed_pred<true><<<g, kBlock, 0, s>>>(L.Q, L.V, L.F, L.types, L.X, L.P, fd, nullptr, L.fx);
+    else k_fixed_pred<false><<<g, kBlock, 0, s>>>(L.Q, L.V, L.F, L.types, L.X, L.P, nullptr, L.go, L.fx);
     return 1;
 }
 

@@ -68,6 +68,16 @@ template <class T> struct Lat {
     long long *X;
     FixedDev *fx;
     const FixedCoef *fixed;
+    // force-only launches: a device flag that turns them into nothing while it
+    // is 0 (the iterations of a captured chunk past the last one), or null
+    const int *go;
+    // force-only launches: the stream the listed sites' kernels run on beside
+    // the bulk ones, with its two events (host), or null
+    const struct ForceFork *fork;
+};
+struct ForceFork {
+    cudaStream_t aux;
+    cudaEvent_t fork, join;
 };
 
 // force parameters shared by every kernel (qmin_capi.cu)
@@ -90,6 +100,15 @@ struct IterDev {
     int iterations, max_iters, active, status;
     long long ndof;
     double lb[64];  // L-BFGS scalars: sy[0..m), alpha[0..m), scratch
+};
+
+// Products of the stored L-BFGS pairs, by slot (row stride kLbGram), and the
+// coefficients of the next step over the y and the s (F has 1)
+constexpr int kLbGram = 8;
+struct LbGram {
+    double sy[kLbGram * kLbGram], yy[kLbGram * kLbGram];  // s_i . y_j, y_i . y_j
+    double sf[kLbGram], yf[kLbGram];                      // s_i . F, y_i . F
+    float cs[kLbGram], cy[kLbGram];
 };
 
 constexpr int kBlock = 256;
@@ -138,9 +157,13 @@ int launch_norm_control(IterDev *it, const double *partials, int nparts, int ada
                         cudaStream_t s);
 // one L-BFGS iteration; p enters as L.F (the forces at Q), so the forces
 // must be current when the first iteration starts
+// gram: the pair products (FP32, m <= kLbGram), or null
 template <class T>
-int launch_lbfgs_iteration(const Lat<T> &L, T *p, T *sbase, T *ybase, IterDev *it, int m, double eta,
+int launch_lbfgs_iteration(const Lat<T> &L, T *p, T *sbase, T *ybase, IterDev *it, LbGram *gram, int m, double eta,
                            double *partials, int grid, cudaStream_t s);
+// all of gram from the stored pairs and F
+int launch_lbfgs_products(const Lat<float> &L, float *sbase, float *ybase, IterDev *it, LbGram *gram, int m,
+                          double *partials, cudaStream_t s);
 
 int reduction_grid(int N);
 

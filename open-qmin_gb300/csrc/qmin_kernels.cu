@@ -42,6 +42,7 @@ __device__ __forceinline__ void site_derivs(const Lat<T> &L, int i, int t, const
 template <class T>
 __global__ void __launch_bounds__(kBlock) k_derivs(Lat<T> L)
 {
+    if (L.go && !*L.go) return;
     const long long P = L.P;
     for (int i = blockIdx.x * kBlock + threadIdx.x; i < L.N; i += gridDim.x * kBlock) {
         const int t = L.types[i];
@@ -70,6 +71,7 @@ __global__ void __launch_bounds__(kBlock) k_derivs(Lat<T> L)
 template <class T, bool WITH_L6 = false>
 __global__ void __launch_bounds__(kBlock) k_force(Lat<T> L)
 {
+    if (L.go && !*L.go) return;
     for (int i = blockIdx.x * kBlock + threadIdx.x; i < L.N; i += gridDim.x * kBlock) {
         T f[5];
         site_force<T, WITH_L6>(L, i, f);
@@ -470,33 +472,95 @@ __global__ void k_fill(T *x, T v, long long n)
         x[j] = v;
 }
 
-// ------------------------------------------------------------------- Adam
-// energyMinimizerAdam::adamStepCPU (energyMinimizerAdam.cpp:25-54), the force
-// already computed at the current Q
+// ---------------------------------------------- Adam, Nesterov, descent
+// The 5 P values of Q, F and the minimiser's planes as 16-byte vectors (the
+// planes' padding is zero and stays so).
+template <class T> struct Vec16;
+template <> struct Vec16<float> {
+    using V = float4;
+};
+template <> struct Vec16<double> {
+    using V = double2;
+};
+
+// a . b over one 16-byte vector, summed in the element type (FP32: four
+// products, one FP64 addition per two vectors in the caller)
+__device__ __forceinline__ float vdot(const float4 &a, const float4 &b)
+{
+    return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
+}
+__device__ __forceinline__ double vdot(const double2 &a, const double2 &b) { return a.x * b.x + a.y * b.y; }
+// x + c y value by value (host_dVec_plusEqual_dVec), c x, x + y
+__device__ __forceinline__ float4 vaxpy(const float4 &x, float c, const float4 &y)
+{
+    return make_float4(x.x + c * y.x, x.y + c * y.y, x.z + c * y.z, x.w + c * y.w);
+}
+__device__ __forceinline__ double2 vaxpy(const double2 &x, double c, const double2 &y)
+{
+    return make_double2(x.x + c * y.x, x.y + c * y.y);
+}
+__device__ __forceinline__ float4 vscale(float c, const float4 &x)
+{
+    return make_float4(c * x.x, c * x.y, c * x.z, c * x.w);
+}
+__device__ __forceinline__ double2 vscale(double c, const double2 &x) { return make_double2(c * x.x, c * x.y); }
+__device__ __forceinline__ float4 vadd(const float4 &x, const float4 &y)
+{
+    return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+}
+__device__ __forceinline__ double2 vadd(const double2 &x, const double2 &y) { return make_double2(x.x + y.x, x.y + y.y); }
+
+// one value of energyMinimizerAdam::adamStepCPU (energyMinimizerAdam.cpp:25-54)
+template <class T> struct AdamCoef {
+    T beta1, beta2, eps, dt, c1, c2;
+};
+template <class T> __device__ __forceinline__ T adam_value(const AdamCoef<T> &a, T f, T &m, T &s)
+{
+    m = a.beta1 * m + (a.beta1 - T(1)) * f;
+    s = a.beta2 * s + (T(1) - a.beta2) * (f * f);
+    const T mc = m * a.c1, vc = s * a.c2;
+    T root = sqrt(vc);
+    if (root == T(0)) root = a.eps;
+    return -a.dt * mc / root;
+}
+__device__ __forceinline__ float4 adam_vec(const AdamCoef<float> &a, const float4 &f, float4 &m, float4 &s)
+{
+    return make_float4(adam_value(a, f.x, m.x, s.x), adam_value(a, f.y, m.y, s.y), adam_value(a, f.z, m.z, s.z),
+                       adam_value(a, f.w, m.w, s.w));
+}
+__device__ __forceinline__ double2 adam_vec(const AdamCoef<double> &a, const double2 &f, double2 &m, double2 &s)
+{
+    return make_double2(adam_value(a, f.x, m.x, s.x), adam_value(a, f.y, m.y, s.y));
+}
+
+// the step, the force already computed at the current Q.  Bound by memory: 140
+// bytes a site in FP32; 34 us at 120 x 136 x 104 (50 with single values and the
+// two FP64 divisions of the bias corrections in every thread).
 template <class T>
 __global__ void __launch_bounds__(kBlock) k_adam(Lat<T> L, T *M, T *S, const IterDev *__restrict__ it, T beta1,
                                                  T beta2, T eps, T dt, double *partials)
 {
     if (!it->active) return;
-    const T c1 = T(1.0 / (1.0 - it->b1t)), c2 = T(1.0 / (1.0 - it->b2t));
+    using V = typename Vec16<T>::V;
+    __shared__ T corr[2];
+    if (threadIdx.x == 0) {
+        corr[0] = T(1.0 / (1.0 - it->b1t));
+        corr[1] = T(1.0 / (1.0 - it->b2t));
+    }
+    __syncthreads();
+    const AdamCoef<T> a{beta1, beta2, eps, dt, corr[0], corr[1]};
+    const long long n = 5 * L.P / (16 / sizeof(T));
+    const V *F = reinterpret_cast<const V *>(L.F);
+    V *Q = reinterpret_cast<V *>(L.Q), *M4 = reinterpret_cast<V *>(M), *S4 = reinterpret_cast<V *>(S);
     double acc[1] = {0.0};
-    for (int i = blockIdx.x * kBlock + threadIdx.x; i < L.N; i += gridDim.x * kBlock) {
-        T ff = T(0);
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            const long long j = k * L.P + i;
-            const T f = L.F[j];
-            ff += f * f;
-            const T m = beta1 * M[j] + (beta1 - T(1)) * f;
-            const T s = beta2 * S[j] + (T(1) - beta2) * (f * f);
-            M[j] = m;
-            S[j] = s;
-            const T mc = m * c1, vc = s * c2;
-            T root = sqrt(vc);
-            if (root == T(0)) root = eps;
-            L.Q[j] += -dt * mc / root;
-        }
-        acc[0] += (double)ff;
+    for (long long j = blockIdx.x * (long long)kBlock + threadIdx.x; j < n; j += (long long)gridDim.x * kBlock) {
+        const V f = F[j], q = Q[j];
+        V m = M4[j], s = S4[j];
+        const V d = adam_vec(a, f, m, s);
+        M4[j] = m;
+        S4[j] = s;
+        Q[j] = vadd(q, d);
+        acc[0] += (double)vdot(f, f);
     }
     block_sum<1>(acc);
     if (threadIdx.x == 0) partials[blockIdx.x] = acc[0];
@@ -508,20 +572,16 @@ __global__ void __launch_bounds__(kBlock) k_nesterov(Lat<T> L, T *alt, const Ite
                                                      double *partials)
 {
     if (!it->active) return;
+    using V = typename Vec16<T>::V;
+    const long long n = 5 * L.P / (16 / sizeof(T));
+    const V *F = reinterpret_cast<const V *>(L.F);
+    V *Q = reinterpret_cast<V *>(L.Q), *A = reinterpret_cast<V *>(alt);
     double acc[1] = {0.0};
-    for (int i = blockIdx.x * kBlock + threadIdx.x; i < L.N; i += gridDim.x * kBlock) {
-        T ff = T(0);
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            const long long j = k * L.P + i;
-            const T f = L.F[j];
-            ff += f * f;
-            const T old = alt[j];
-            const T a = L.Q[j] + dt * f;
-            alt[j] = a;
-            L.Q[j] = a + mu * (a - old);
-        }
-        acc[0] += (double)ff;
+    for (long long j = blockIdx.x * (long long)kBlock + threadIdx.x; j < n; j += (long long)gridDim.x * kBlock) {
+        const V f = F[j], old = A[j], a = vaxpy(Q[j], dt, f);
+        A[j] = a;
+        Q[j] = vaxpy(a, mu, vaxpy(a, T(-1), old));
+        acc[0] += (double)vdot(f, f);
     }
     block_sum<1>(acc);
     if (threadIdx.x == 0) partials[blockIdx.x] = acc[0];
@@ -533,9 +593,12 @@ template <class T>
 __global__ void __launch_bounds__(kBlock) k_gd_move(Lat<T> L, const IterDev *__restrict__ it, T dt)
 {
     if (!it->active) return;
-    for (int i = blockIdx.x * kBlock + threadIdx.x; i < L.N; i += gridDim.x * kBlock)
-#pragma unroll
-        for (int k = 0; k < 5; ++k) L.Q[k * L.P + i] += dt * L.F[k * L.P + i];
+    using V = typename Vec16<T>::V;
+    const long long n = 5 * L.P / (16 / sizeof(T));
+    const V *F = reinterpret_cast<const V *>(L.F);
+    V *Q = reinterpret_cast<V *>(L.Q);
+    for (long long j = blockIdx.x * (long long)kBlock + threadIdx.x; j < n; j += (long long)gridDim.x * kBlock)
+        Q[j] = vaxpy(Q[j], dt, F[j]);
 }
 
 // sum_i F_i . F_i (plain dot, energyMinimizerGradientDescent.cpp:75-79)
@@ -543,15 +606,13 @@ template <class T>
 __global__ void __launch_bounds__(kBlock) k_ff_dot(Lat<T> L, const IterDev *__restrict__ it, double *partials)
 {
     if (!it->active) return;
+    using V = typename Vec16<T>::V;
+    const long long n = 5 * L.P / (16 / sizeof(T));
+    const V *F = reinterpret_cast<const V *>(L.F);
     double acc[1] = {0.0};
-    for (int i = blockIdx.x * kBlock + threadIdx.x; i < L.N; i += gridDim.x * kBlock) {
-        T ff = T(0);
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            const T f = L.F[k * L.P + i];
-            ff += f * f;
-        }
-        acc[0] += (double)ff;
+    for (long long j = blockIdx.x * (long long)kBlock + threadIdx.x; j < n; j += (long long)gridDim.x * kBlock) {
+        const V f = F[j];
+        acc[0] += (double)vdot(f, f);
     }
     block_sum<1>(acc);
     if (threadIdx.x == 0) partials[blockIdx.x] = acc[0];
@@ -655,41 +716,6 @@ __device__ __forceinline__ int lb_slot(const IterDev *it, int m, int ii)
     return (cur - ii - 1 + m) % m;
 }
 
-template <class T> struct LbVec;
-template <> struct LbVec<float> {
-    using V = float4;
-};
-template <> struct LbVec<double> {
-    using V = double2;
-};
-
-// a . b over one 16-byte vector, summed in the element type (FP32: four
-// products, one FP64 addition per two vectors in the caller)
-__device__ __forceinline__ float vdot(const float4 &a, const float4 &b)
-{
-    return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
-}
-__device__ __forceinline__ double vdot(const double2 &a, const double2 &b) { return a.x * b.x + a.y * b.y; }
-// x + c y lane by lane (host_dVec_plusEqual_dVec), c x, x + y
-__device__ __forceinline__ float4 vaxpy(const float4 &x, float c, const float4 &y)
-{
-    return make_float4(x.x + c * y.x, x.y + c * y.y, x.z + c * y.z, x.w + c * y.w);
-}
-__device__ __forceinline__ double2 vaxpy(const double2 &x, double c, const double2 &y)
-{
-    return make_double2(x.x + c * y.x, x.y + c * y.y);
-}
-__device__ __forceinline__ float4 vscale(float c, const float4 &x)
-{
-    return make_float4(c * x.x, c * x.y, c * x.z, c * x.w);
-}
-__device__ __forceinline__ double2 vscale(double c, const double2 &x) { return make_double2(c * x.x, c * x.y); }
-__device__ __forceinline__ float4 vadd(const float4 &x, const float4 &y)
-{
-    return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
-}
-__device__ __forceinline__ double2 vadd(const double2 &x, const double2 &y) { return make_double2(x.x + y.x, x.y + y.y); }
-
 // KIND 0: step 2 at ii < m - 1;  KIND 1: step 2 at ii = m - 1 with step 3;
 // KIND 2: step 4 at ii >= 1.  p_in is F in an iteration's first pass.  Two
 // 16-byte vectors per thread per trip; the dot's block partial in partials[b].
@@ -699,7 +725,7 @@ __global__ void __launch_bounds__(kBlock) k_lb_pass(const IterDev *__restrict__ 
                                                     long long n5, double *partials)
 {
     if (!it->active) return;
-    using V = typename LbVec<T>::V;
+    using V = typename Vec16<T>::V;
     const double *lb = it->lb;
     const long long n = n5 / (16 / sizeof(T));
     const V *x, *z = nullptr, *w = nullptr;
@@ -759,7 +785,7 @@ __global__ void __launch_bounds__(kBlock) k_lb_step(const IterDev *__restrict__ 
                                                     T *sb, T *yb, const T *F, T *Q, long long n5)
 {
     if (!it->active) return;
-    using V = typename LbVec<T>::V;
+    using V = typename Vec16<T>::V;
     const double *lb = it->lb;
     const long long n = n5 / (16 / sizeof(T));
     const int t0 = lb_slot(it, m, 0), cur = it->iterations % m;
@@ -785,7 +811,7 @@ __global__ void __launch_bounds__(kBlock) k_lb_post(const IterDev *__restrict__ 
                                                     T *yb, const T *__restrict__ F, long long n5, double *partials)
 {
     if (!it->active) return;
-    using V = typename LbVec<T>::V;
+    using V = typename Vec16<T>::V;
     const long long n = n5 / (16 / sizeof(T));
     const int cur = it->iterations % m;
     const V *s = reinterpret_cast<const V *>(sb + cur * n5), *F4 = reinterpret_cast<const V *>(F);
@@ -852,6 +878,226 @@ __global__ void __launch_bounds__(kBlock) k_lb_close(IterDev *it, int m, const d
         return;
     }
     it->active = (it->iterations < it->max_iters && it->forceMax > it->fcut) ? 1 : 0;
+}
+
+// FP32 and up to kLbGram pairs: the two-loop recursion on coefficients.  The
+// step is p = F + sum cy_j y_j + sum cs_j s_j, and every dot product the
+// recursion takes is a sum over s_i . y_j, y_i . y_j, s_i . F and y_i . F.  Of
+// these an iteration changes those of the new pair and of F: one pass over the
+// pairs after the force forms them (k_lbg_post), one block runs the recursion in
+// FP64 (k_lbg_solve), one pass applies it with the step (k_lbg_step): 6 m - 1
+// vectors of 5 N values move, force aside, instead of the 8 m + 7 of the passes above.
+// Bound by HBM: at 200^3 and m = 5 0.67 ms (6.9 and 6.3 TB/s) instead of 1.24.
+// FP64 keeps the passes: 5 m + 1 products a value would bound it on the FP64 pipe.
+template <int M>
+__global__ void __launch_bounds__(kBlock)
+    k_lbg_step(const IterDev *__restrict__ it, const LbGram *__restrict__ g, float eta, float *sb, float *yb,
+               const float *F, float *Q, long long n5)
+{
+    if (!it->active) return;
+    const long long n = n5 / 4;
+    const int cur = it->iterations % M;
+    float cs[M], cy[M];
+#pragma unroll
+    for (int t = 0; t < M; ++t) {
+        cs[t] = g->cs[t];
+        cy[t] = g->cy[t];
+    }
+    const float4 *F4 = reinterpret_cast<const float4 *>(F);
+    float4 *S4 = reinterpret_cast<float4 *>(sb), *Y4 = reinterpret_cast<float4 *>(yb), *Q4 = reinterpret_cast<float4 *>(Q);
+    for (long long j = blockIdx.x * (long long)kBlock + threadIdx.x; j < n; j += (long long)gridDim.x * kBlock) {
+        float4 s[M], y[M];
+#pragma unroll
+        for (int t = 0; t < M; ++t) {
+            y[t] = Y4[t * n + j];
+            s[t] = S4[t * n + j];
+        }
+        const float4 f = F4[j], q = Q4[j];
+        float4 v = f;
+#pragma unroll
+        for (int t = 0; t < M; ++t) v = vaxpy(v, cy[t], y[t]);
+#pragma unroll
+        for (int t = 0; t < M; ++t) v = vaxpy(v, cs[t], s[t]);
+        const float4 sv = vscale(eta, v);
+        S4[cur * n + j] = sv;
+        Y4[cur * n + j] = f;  // the old forces
+        Q4[j] = vadd(q, sv);
+    }
+}
+
+// hi + lo += x, exact up to the rounding of lo
+__device__ __forceinline__ void add_twice(float &hi, float &lo, float x)
+{
+    const float s = __fadd_rn(hi, x), b = __fsub_rn(s, hi);
+    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
+    hi = s;
+}
+
+// Pair `cur` against all: per slot t, s_cur . y_t, s_t . y_cur, y_t . y_cur,
+// s_t . F, y_t . F, then F . F; dot d of block b in partials[d gridDim.x + b].
+// slot < 0: the iteration's pair, y_cur += -F first; else the products of a
+// stored pair.  Four products in FP32, their sums in pairs of FP32 numbers (a
+// conversion to FP64 costs as much as an FP64 addition here, and there are 26
+// sums at m = 5).
+constexpr int kLbPostBlock = 128;
+template <int M> constexpr int lb_post_per_sm() { return M <= 5 ? 4 : 3; }
+template <int M>
+__global__ void __launch_bounds__(kLbPostBlock, lb_post_per_sm<M>())
+    k_lbg_post(const IterDev *__restrict__ it, int slot, const float *sb, float *yb, const float *F, long long n5,
+               double *partials)
+{
+    if (!it->active) return;
+    constexpr int ND = 5 * M + 1;
+    const long long n = n5 / 4;
+    const int cur = slot < 0 ? it->iterations % M : slot;
+    const float4 *F4 = reinterpret_cast<const float4 *>(F), *S4 = reinterpret_cast<const float4 *>(sb);
+    float4 *Y4 = reinterpret_cast<float4 *>(yb);
+    float hi[ND], lo[ND];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) hi[d] = lo[d] = 0.f;
+    for (long long j = blockIdx.x * (long long)kLbPostBlock + threadIdx.x; j < n;
+         j += (long long)gridDim.x * kLbPostBlock) {
+        float4 s[M], y[M], sc, yc;
+        const float4 f = F4[j];
+#pragma unroll
+        for (int t = 0; t < M; ++t) {
+            s[t] = S4[t * n + j];
+            y[t] = Y4[t * n + j];
+        }
+#pragma unroll
+        for (int t = 0; t < M; ++t)
+            if (t == cur) {
+                if (slot < 0) {
+                    y[t] = vaxpy(y[t], -1.f, f);
+                    Y4[t * n + j] = y[t];
+                }
+                sc = s[t];
+                yc = y[t];
+            }
+#pragma unroll
+        for (int t = 0; t < M; ++t) {
+            add_twice(hi[5 * t], lo[5 * t], vdot(sc, y[t]));
+            add_twice(hi[5 * t + 1], lo[5 * t + 1], vdot(s[t], yc));
+            add_twice(hi[5 * t + 2], lo[5 * t + 2], vdot(y[t], yc));
+            add_twice(hi[5 * t + 3], lo[5 * t + 3], vdot(s[t], f));
+            add_twice(hi[5 * t + 4], lo[5 * t + 4], vdot(y[t], f));
+        }
+        add_twice(hi[5 * M], lo[5 * M], vdot(f, f));
+    }
+    // one warp's sums over its lanes, then the block's warps in order
+    __shared__ double sh[ND][kLbPostBlock / 32];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float h = __shfl_down_sync(0xffffffffu, hi[d], o), l = __shfl_down_sync(0xffffffffu, lo[d], o);
+            lo[d] = __fadd_rn(lo[d], l);
+            add_twice(hi[d], lo[d], h);
+        }
+        if ((threadIdx.x & 31) == 0) sh[d][threadIdx.x / 32] = (double)hi[d] + (double)lo[d];
+    }
+    __syncthreads();
+    if (threadIdx.x < ND) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < kLbPostBlock / 32; ++w) v += sh[threadIdx.x][w];
+        partials[(long long)threadIdx.x * gridDim.x + blockIdx.x] = v;
+    }
+}
+
+// One block, a warp per dot product: the products of k_lbg_post into gram;
+// slot < 0: the iteration's close as k_lb_close, and the next step's
+// coefficients; else the coefficients with the last slot.
+__global__ void __launch_bounds__(1024)
+    k_lbg_solve(IterDev *it, LbGram *g, int slot, int m, const double *__restrict__ partials, int nparts)
+{
+    if (!it->active) return;
+    __shared__ double v[5 * kLbGram + 1], sy[kLbGram * kLbGram], yy[kLbGram * kLbGram];
+    const int lane = threadIdx.x & 31, nd = 5 * m + 1;
+    for (int k = threadIdx.x; k < kLbGram * kLbGram; k += blockDim.x) {
+        sy[k] = g->sy[k];
+        yy[k] = g->yy[k];
+    }
+    for (int d = threadIdx.x / 32; d < nd; d += blockDim.x / 32) {
+        const double *p = partials + (long long)d * nparts;
+        double a = 0.0;
+        constexpr int U = 8;
+        for (int b0 = lane; b0 < nparts; b0 += 32 * U) {
+            double x[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) x[u] = b0 + 32 * u < nparts ? p[b0 + 32 * u] : 0.0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) a += x[u];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0) v[d] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    int cur = slot < 0 ? it->iterations % m : slot;
+    if (lane < m) {
+        const int r = cur * kLbGram + lane, c = lane * kLbGram + cur;
+        g->sy[r] = sy[r] = v[5 * lane];
+        g->sy[c] = sy[c] = v[5 * lane + 1];
+        g->yy[r] = g->yy[c] = yy[r] = yy[c] = v[5 * lane + 2];
+        g->sf[lane] = v[5 * lane + 3];
+        g->yf[lane] = v[5 * lane + 4];
+    }
+    if (slot < 0) {
+        int n = it->iterations + 1;
+        __syncwarp();
+        if (lane == 0) {
+            double *lb = it->lb;
+            const double sy = v[5 * cur];
+            lb[cur] = sy;
+            lb[16 + cur] = v[5 * cur + 2];
+            lb[32] = sy != 0 ? v[5 * cur + 3] / sy : 0.0;
+            it->forceMax = sqrt(v[5 * m]) / (double)it->ndof;
+            it->iterations = n;
+            if (!isfinite(v[5 * m])) {
+                it->status = 1;
+                it->active = 0;
+            } else {
+                it->active = (n < it->max_iters && it->forceMax > it->fcut) ? 1 : 0;
+            }
+        }
+        cur = n % m;  // the next iteration's slot
+    } else {
+        if (slot < m - 1) return;
+        cur = it->iterations % m;
+    }
+    __syncwarp();
+    // lane j < m: slot j's coefficients; sums over groups of eight lanes
+    double cs = 0.0, cy = 0.0, al = 0.0;
+    auto sum8 = [](double a) {
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        return a;
+    };
+    const bool mine = lane < m;
+    for (int ii = 0; ii < m; ++ii) {
+        const int t = (cur - ii - 1 + m) % m;
+        const double d = sy[t * kLbGram + t];
+        const double sp = sum8(mine ? cy * sy[t * kLbGram + lane] : 0.0) + v[5 * t + 3];
+        if (lane == t) {
+            al = d != 0 ? sp / d : 0.0;
+            cy -= al;
+        }
+    }
+    const int t0 = (cur - 1 + m) % m;
+    if (lane == t0 && yy[t0 * kLbGram + t0] != 0) cy += sy[t0 * kLbGram + t0] / yy[t0 * kLbGram + t0];
+    for (int ii = m - 1; ii >= 0; --ii) {
+        const int t = (cur - ii - 1 + m) % m;
+        const double d = sy[t * kLbGram + t];
+        const double yp =
+            sum8(mine ? cy * yy[t * kLbGram + lane] + cs * sy[lane * kLbGram + t] : 0.0) + v[5 * t + 4];
+        if (lane == t && d != 0) cs += al - yp / d;
+    }
+    if (mine) {
+        g->cs[lane] = (float)cs;
+        g->cy[lane] = (float)cy;
+    }
 }
 
 // ---------------------------------------------------------------- launchers
@@ -977,10 +1223,50 @@ int launch_norm_control(IterDev *it, const double *partials, int nparts, int ada
     k_norm_control<<<1, kBlock, 0, s>>>(it, partials, nparts, adam, beta1, beta2);
     return 1;
 }
-template <class T>
-int launch_lbfgs_iteration(const Lat<T> &L, T *p, T *sb, T *yb, IterDev *it, int m, double eta, double *partials,
-                           int grid, cudaStream_t s)
+template <int M>
+static void launch_lbg_post(const Lat<float> &L, int slot, float *sb, float *yb, IterDev *it, LbGram *gram,
+                            double *partials, cudaStream_t s)
 {
+    const int grid = 152 * lb_post_per_sm<M>();
+    k_lbg_post<M><<<grid, kLbPostBlock, 0, s>>>(it, slot, sb, yb, L.F, 5 * L.P, partials);
+    k_lbg_solve<<<1, 32 * std::min(32, 5 * M + 1), 0, s>>>(it, gram, slot, M, partials, grid);
+}
+template <int M>
+static int launch_lbg(const Lat<float> &L, float *sb, float *yb, IterDev *it, LbGram *gram, double eta, bool products,
+                      double *partials, cudaStream_t s)
+{
+    if (products) {
+        for (int c = 0; c < M; ++c) launch_lbg_post<M>(L, c, sb, yb, it, gram, partials, s);
+        return 2 * M;
+    }
+    k_lbg_step<M><<<elem_grid(5 * L.P / 4), kBlock, 0, s>>>(it, gram, (float)eta, sb, yb, L.F, L.Q, 5 * L.P);
+    const int n = launch_force(L, reduction_grid(L.N), s);
+    launch_lbg_post<M>(L, -1, sb, yb, it, gram, partials, s);
+    return n + 3;
+}
+static int launch_lbg_iteration(const Lat<float> &L, float *sb, float *yb, IterDev *it, LbGram *gram, int m, double eta,
+                                double *partials, cudaStream_t s, bool products = false)
+{
+    switch (m) {
+#define QMIN_LBG(M) \
+    case M: return launch_lbg<M>(L, sb, yb, it, gram, eta, products, partials, s);
+        QMIN_LBG(1) QMIN_LBG(2) QMIN_LBG(3) QMIN_LBG(4) QMIN_LBG(5) QMIN_LBG(6) QMIN_LBG(7) QMIN_LBG(8)
+#undef QMIN_LBG
+    }
+    return 0;
+}
+int launch_lbfgs_products(const Lat<float> &L, float *sb, float *yb, IterDev *it, LbGram *gram, int m,
+                          double *partials, cudaStream_t s)
+{
+    return launch_lbg_iteration(L, sb, yb, it, gram, m, 0.0, partials, s, true);
+}
+
+template <class T>
+int launch_lbfgs_iteration(const Lat<T> &L, T *p, T *sb, T *yb, IterDev *it, LbGram *gram, int m, double eta,
+                           double *partials, int grid, cudaStream_t s)
+{
+    if constexpr (sizeof(T) == 4)
+        if (gram) return launch_lbg_iteration(L, sb, yb, it, gram, m, eta, partials, s);
     const long long n5 = 5 * L.P;
     int n = 0;
     for (int ii = 0; ii < m - 1; ++ii) {
@@ -1035,8 +1321,8 @@ int launch_energy_full(const Lat<T> &L, double *partials, int grid, double *out5
                                          cudaStream_t);                                   \
     template int launch_gd_move<T>(const Lat<T> &, IterDev *, double, cudaStream_t);                                 \
     template int launch_ff_dot<T>(const Lat<T> &, IterDev *, double *, int, cudaStream_t);                          \
-    template int launch_lbfgs_iteration<T>(const Lat<T> &, T *, T *, T *, IterDev *, int, double, double *, int,   \
-                                           cudaStream_t);                                                          \
+    template int launch_lbfgs_iteration<T>(const Lat<T> &, T *, T *, T *, IterDev *, LbGram *, int, double, double *, \
+                                           int, cudaStream_t);                                                          \
     template int launch_energy_full<T>(const Lat<T> &, double *, int, double *, const double *, double, double,    \
                                        double, const double *, double, double, double, cudaStream_t);
 
