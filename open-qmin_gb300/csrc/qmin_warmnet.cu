@@ -9,7 +9,8 @@
 // GEMM on the BF16 tensor cores: by default tcgen05.mma with tensor-memory
 // accumulators (a direct kernel with TMA-staged halo planes for the 3^3
 // stride-1 layers of 32 and 48 output channels, a gathering kernel
-// otherwise), or mma.sync m16n8k16 (tensor path 0; the weight gradient
+// otherwise; the weight gradient of the 3^3 layers in qmin_wgrad.cuh), or
+// mma.sync m16n8k16 (tensor path 0; the weight gradient of the 1^3 layers
 // always), FP32 accumulate:
 //   forward:      out[v][co]      = sum_{tap,ci} in[src(v,tap)][ci] * W[co][tap][ci]
 //   data grad:    din[u][ci]      = sum_{tap,co} dout[src'(u,tap)][co] * W'[ci][tap][co]
@@ -1195,6 +1196,12 @@ static void conv_gemm(const Geo &g, const bf16 *in, const bf16 *w, const float *
     }
 }
 
+}  // namespace nn
+}  // namespace qmin
+#include "qmin_wgrad.cuh"
+namespace qmin {
+namespace nn {
+
 struct Layer {
     int cin, cout, taps, stride, level;  // level of the input grid
     bool relu;
@@ -1330,7 +1337,7 @@ void layer_backward(qmin_warmnet_ctx *n, int i, const float *gout, const bf16 *a
     k_bias_grad<<<dim3((unsigned)std::min<long long>((rows_out + 7) / 8, 1024), (unsigned)((L.cout + 31) / 32)), 256, 0,
                   s>>>(gout, act_out, n->g + L.boff, rows_out, L.cout);
     const Geo g = fwd_geo(n, L);
-    {
+    if (n->path == 0 || !wgrad_umma(g, n->gbf, act_in, n->g + L.woff, s)) {
         const int tiles = ((L.cout + 63) / 64) * ((L.cin + 63) / 64);
         const long long want = std::max<long long>(1, 152 * 8 / (L.taps * tiles));
         long long chunk = (rows_out + want - 1) / want;
