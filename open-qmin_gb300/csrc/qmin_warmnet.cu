@@ -184,8 +184,20 @@ __global__ void __launch_bounds__(128) k_conv_gemm(Geo g, const bf16 *__restrict
 // 128 and their stride (M/N) byte offset cin/8 * 128.  One thread issues
 // cin/16 tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, M = 128, N = cout,
 // K = 16) into an accumulator in tensor memory and commits them to the
-// stage's mbarrier; two stage buffers let the next tap's gather overlap the
-// MMAs.  The epilogue reads each warp's 32 accumulator rows with tcgen05.ld.
+// stage's mbarrier.  The epilogue reads each warp's 32 accumulator rows with
+// tcgen05.ld.
+//
+// The stages (four, or three where they are large) are filled by cp.async one
+// or two taps ahead, consecutive threads on consecutive 16-byte pieces of a
+// row; the rows' source coordinates are worked out once per CTA.  The
+// transposed gather of a stride-2 convolution (mode 1) takes the fine voxels by
+// parity: the rows of a CTA share theirs, and only the 1, 2, 4 or 8 taps that
+// reach a coarse voxel from it run, 27 of 216.  With one tap a CTA walks
+// several row tiles, its weights staged once.  Bound by the latency of its
+// gathers.  The first convolution of stride 2 at 200^3 takes 606 us (834 with
+// a thread per row, two stages and the loads waited for), the data gradient of
+// eight 64^3 samples' 535 (990 with all 27 taps of every voxel), the head at
+// 200^3 312 (330).
 // Every wait is bounded; a wait that gives up sets g_conv_err, and the CTA
 // still frees its tensor memory.
 __device__ int g_conv_err;
@@ -231,16 +243,29 @@ static int umma_cols(int n)
     while (c < n) c <<= 1;
     return c;
 }
-// dynamic shared memory of k_conv_umma: two stages of A and B, two mbarriers,
-// the tensor-memory address; padded so that at most 512 / cols CTAs share an SM
-// and a tcgen05.alloc never waits
+constexpr int kUmmaStages = 4;
+// stages of A and B: four where one has at most 16 KB, else three
+__host__ __device__ constexpr int umma_stages(int cin, int n) { return (128 + n) * cin * 2 <= 16384 ? kUmmaStages : 3; }
+// dynamic shared memory of k_conv_umma: the stages, the rows' sources, the
+// mbarriers, the tensor-memory address; padded so that at most 512 / cols CTAs
+// share an SM and a tcgen05.alloc never waits
 static size_t umma_smem(int cin, int n)
 {
-    const size_t need = 2 * (size_t)(128 + n) * cin * 2 + 64;
+    const size_t need = umma_stages(cin, n) * (size_t)(128 + n) * cin * 2 + 128 * 16 + 8 * kUmmaStages + 16;
     const int per_sm = 512 / umma_cols(n);
     const size_t floor_bytes = (size_t)(232448 / per_sm) - 1024 + 1;  // more than 1/(per_sm+1) of the SM's 227 KB
     return std::max(need, std::min<size_t>(floor_bytes, 232448 - 1024));
 }
+
+__device__ __forceinline__ void cp_async16(unsigned saddr, const void *g, bool in)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(g), "r"(in ? 16 : 0) : "memory");
+}
+
+// one axis of the transposed gather: taps of a fine voxel of parity p, the
+// k of the i-th and its coarse voxel's distance from the fine voxel's half
+__device__ __forceinline__ int up_tap(int p, int i) { return p ? 2 * i : 1; }
+__device__ __forceinline__ int up_shift(int p, int i) { return p && i == 0; }
 
 template <int N, bool OUT_BF16>
 __global__ void __launch_bounds__(128) k_conv_umma(Geo g, const bf16 *__restrict__ in, const bf16 *__restrict__ w,
@@ -250,14 +275,13 @@ __global__ void __launch_bounds__(128) k_conv_umma(Geo g, const bf16 *__restrict
     static_assert(N % 16 == 0 && N >= 16 && N <= 256, "tcgen05 M=128 needs N a multiple of 16 in [16, 256]");
     constexpr int COLS = N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256));
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int cin = g.cin, kc8 = cin >> 3, K = g.taps * cin;
-    const size_t a_bytes = (size_t)128 * cin * 2, b_bytes = (size_t)N * cin * 2;
-    unsigned char *bufA[2] = {smem_raw, smem_raw + a_bytes + b_bytes};
-    unsigned char *bufB[2] = {smem_raw + a_bytes, smem_raw + 2 * a_bytes + b_bytes};
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw + 2 * (a_bytes + b_bytes));
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar + 2);
+    const int cin = g.cin, kc8 = cin >> 3, K = g.taps * cin, st = umma_stages(cin, N), pf = st - 2;
+    const unsigned a_bytes = 128u * cin * 2, stage = a_bytes + (unsigned)N * cin * 2;
+    const unsigned mul = 65536u / kc8 + 1;  // e / kc8 = e mul >> 16 for e < 2048
+    int4 *src = reinterpret_cast<int4 *>(smem_raw + (size_t)st * stage);  // per row: flat voxel of tap 0, x, y, z
+    uint64_t *bar = reinterpret_cast<uint64_t *>(src + 128);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar + kUmmaStages);
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int row = blockIdx.x * 128 + tid;
     // an earlier CTA's wait gave up: the launch's results are void, do no more work
     if (*(volatile int *)&g_conv_err) return;
 
@@ -268,48 +292,116 @@ __global__ void __launch_bounds__(128) k_conv_umma(Geo g, const bf16 *__restrict
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(s_addr(&bar[0])) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(s_addr(&bar[1])) : "memory");
+        for (int k = 0; k < kUmmaStages; ++k)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(s_addr(&bar[k])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    // this thread's row: its sources and its place in the output
+    const bool flat = g.taps == 1;
+    int par = 0, orow = -1, nt = g.taps;
+    if (!flat) {
+        const bool up = g.mode == 1;
+        const int Dr = up ? g.Di : g.Do, Hr = up ? g.Hi : g.Ho, Wr = up ? g.Wi : g.Wo;
+        const int nrows = g.nb * Dr * Hr * Wr;  // mode 1: the rows of one parity
+        int r = blockIdx.x;
+        if (up) {
+            const int nblk = (nrows + 127) / 128, q = blockIdx.x / nblk;
+            par = 0x01243567 >> (4 * q) & 7;  // parities (z y x) in the order of falling tap counts
+            r -= q * nblk;
+            nt = 1 << __popc(par);
+        }
+        r = r * 128 + tid;
+        int4 c = make_int4(0, -0x40000000, 0, 0);
+        if (r < nrows) {
+            const int x = r % Wr, y = r / Wr % Hr, z = r / (Wr * Hr) % Dr, b = r / (Wr * Hr * Dr);
+            if (up) {
+                c = make_int4(r, x, y, z);
+                orow = ((b * g.Do + 2 * z + (par >> 2)) * g.Ho + 2 * y + (par >> 1 & 1)) * g.Wo + 2 * x + (par & 1);
+            } else {
+                c.y = x * g.stride - 1;
+                c.z = y * g.stride - 1;
+                c.w = z * g.stride - 1;
+                c.x = ((b * g.Di + c.w) * g.Hi + c.z) * g.Wi + c.y;
+                orow = r;
+            }
+        }
+        src[tid] = c;
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tmem_slot;
 
-    bool ok = true;
-    for (int tap = 0; tap < g.taps; ++tap) {
-        const int b = tap & 1;
-        if (tap >= 2) {
-            // the MMAs of tap - 2 have read this buffer
-            const bool w_ok = mbar_wait_bounded(s_addr(&bar[b]), (unsigned)((tap - 2) >> 1) & 1u);
-            if (__syncthreads_or(!w_ok)) {
-                ok = false;
-                break;
-            }
+    // one tap of one tile a step; tiles of 128 rows, several to a CTA with one tap
+    const int tiles = flat ? ((rows + 127) / 128 - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 1;
+    const int steps = tiles * nt;
+    const unsigned base = s_addr(smem_raw);
+    auto load = [&](int t) {
+        const unsigned sa = base + (unsigned)(t % st) * stage, sb = sa + a_bytes;
+        int tap = t, dx = 0, dy = 0, dz = 0;
+        if (flat) {
+            tap = 0;
+        } else if (g.mode == 1) {
+            const int px = par & 1, py = par >> 1 & 1, pz = par >> 2;
+            const int ix = t & px, iy = t >> px & py, iz = t >> (px + py);
+            tap = (up_tap(pz, iz) * 3 + up_tap(py, iy)) * 3 + up_tap(px, ix);
+            dx = up_shift(px, ix);
+            dy = up_shift(py, iy);
+            dz = up_shift(pz, iz);
+        } else {
+            dx = t % 3;
+            dy = t / 3 % 3;
+            dz = t / 9;
         }
-        // A: this thread's row, cin channels of the tap's source voxel (zeros outside)
-        {
-            const int src = row < rows ? gather_src(g, row, tap) : -1;
-            const uint4 *sp = reinterpret_cast<const uint4 *>(in + (size_t)(src < 0 ? 0 : src) * cin);
-            unsigned char *dst = bufA[b] + (size_t)(tid >> 3) * kc8 * 128 + (tid & 7) * 16;
-            for (int k8 = 0; k8 < kc8; ++k8) {
-                const uint4 v = src >= 0 ? sp[k8] : make_uint4(0, 0, 0, 0);
-                *reinterpret_cast<uint4 *>(dst + k8 * 128) = v;
+        const int off = (dz * g.Hi + dy) * g.Wi + dx, row0 = ((int)blockIdx.x + t * (int)gridDim.x) * 128;
+        for (int e = tid; e < 128 * kc8; e += 128) {
+            const int r = (int)((unsigned)e * mul >> 16), k8 = e - r * kc8;
+            int v;
+            bool ok;
+            if (flat) {
+                v = row0 + r;
+                ok = v < rows;
+            } else {
+                const int4 c = src[r];
+                v = c.x + off;
+                ok = (unsigned)(c.y + dx) < (unsigned)g.Wi && (unsigned)(c.z + dy) < (unsigned)g.Hi &&
+                     (unsigned)(c.w + dz) < (unsigned)g.Di;
             }
+            cp_async16(sa + (unsigned)((r >> 3) * kc8 + k8) * 128 + (r & 7) * 16, in + (size_t)(ok ? v : 0) * cin + k8 * 8,
+                       ok);
         }
-        // B: the tap's weights, N x cin
+        if (flat && t >= st) return;  // the stage has the weights
         for (int e = tid; e < N * kc8; e += 128) {
-            const int co = e / kc8, k8 = e - co * kc8;
-            const uint4 v = *reinterpret_cast<const uint4 *>(w + (size_t)co * K + (size_t)tap * cin + k8 * 8);
-            *reinterpret_cast<uint4 *>(bufB[b] + ((size_t)(co >> 3) * kc8 + k8) * 128 + (co & 7) * 16) = v;
+            const int co = (int)((unsigned)e * mul >> 16), k8 = e - co * kc8;
+            cp_async16(sb + (unsigned)((co >> 3) * kc8 + k8) * 128 + (co & 7) * 16,
+                       w + (size_t)co * K + (size_t)tap * cin + k8 * 8, true);
         }
-        // generic-proxy stores -> visible to the tensor cores' async proxy
+    };
+    for (int t = 0; t < pf; ++t) {
+        if (t < steps) load(t);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    bool ok = true;
+    int t = 0;
+    for (int tile = 0, tap = 0; t < steps; ++t) {
+        bool w_ok = true;
+        if (t + pf < steps) {
+            // its stage was last read by the MMAs of step t - 2
+            if (t >= 2) w_ok = mbar_wait_bounded(s_addr(&bar[(t - 2) % st]), (unsigned)((t - 2) / st) & 1u);
+            if (w_ok) load(t + pf);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        if (st == 4) asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+        else asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        // the copies -> visible to the tensor cores' async proxy
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        __syncthreads();
+        if (__syncthreads_or(!w_ok)) {
+            ok = false;
+            break;
+        }
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const unsigned sa = s_addr(bufA[b]), sb = s_addr(bufB[b]);
+            const unsigned sa = base + (unsigned)(t % st) * stage, sb = sa + a_bytes;
             const unsigned sbo = (unsigned)kc8 * 128u;
             for (int kk = 0; kk < (cin >> 4); ++kk) {
                 const uint64_t da = umma_desc(sa + kk * 256, 128, sbo);
@@ -322,17 +414,23 @@ __global__ void __launch_bounds__(128) k_conv_umma(Geo g, const bf16 *__restrict
                     : "memory");
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                             s_addr(&bar[b]))
+                             s_addr(&bar[t % st]))
                          : "memory");
         }
-    }
-    if (ok) {
-        // the last commit covers every MMA this CTA issued
-        const int last = g.taps - 1;
-        const bool w_ok = mbar_wait_bounded(s_addr(&bar[last & 1]), (unsigned)(last >> 1) & 1u);
-        ok = !__syncthreads_or(!w_ok);
-    }
-    if (ok) {
+        if (++tap < nt) continue;
+        // the tile is complete with this commit
+        tap = 0;
+        w_ok = mbar_wait_bounded(s_addr(&bar[t % st]), (unsigned)(t / st) & 1u);
+        if (__syncthreads_or(!w_ok)) {
+            ok = false;
+            ++t;
+            break;
+        }
+        if (flat) {
+            orow = ((int)blockIdx.x + tile * (int)gridDim.x) * 128 + tid;
+            if (orow >= rows) orow = -1;
+        }
+        ++tile;
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
 #pragma unroll
@@ -349,17 +447,17 @@ __global__ void __launch_bounds__(128) k_conv_umma(Geo g, const bf16 *__restrict
                 v[e] = __uint_as_float(r[e]) + (bias ? bias[c0 + e] : 0.f);
                 if (relu) v[e] = fmaxf(v[e], 0.f);
             }
-            if (row < rows) {
+            if (orow >= 0) {
                 if (OUT_BF16) {
-                    bf16 *o = reinterpret_cast<bf16 *>(out) + (size_t)row * N + c0;
+                    bf16 *o = reinterpret_cast<bf16 *>(out) + (size_t)orow * N + c0;
                     __nv_bfloat162 h[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
                     *reinterpret_cast<uint4 *>(o) = *reinterpret_cast<const uint4 *>(h);
                 } else {
-                    float *o = reinterpret_cast<float *>(out) + (size_t)row * N + c0;
+                    float *o = reinterpret_cast<float *>(out) + (size_t)orow * N + c0;
                     if (addend) {
-                        const float *a = addend + (size_t)row * N + c0;
+                        const float *a = addend + (size_t)orow * N + c0;
 #pragma unroll
                         for (int e = 0; e < 8; ++e) v[e] += a[e];
                     }
@@ -368,9 +466,13 @@ __global__ void __launch_bounds__(128) k_conv_umma(Geo g, const bf16 *__restrict
                 }
             }
         }
-    } else if (tid == 0) {
+        // the accumulator is read before the next tile's MMAs, which follow a barrier
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    if (!ok && tid == 0) {
         // a wait gave up: let the MMAs in flight finish (bounded) before the buffers go away
-        for (int b = 0; b < 2; ++b) mbar_wait_bounded(s_addr(&bar[b]), 0u), mbar_wait_bounded(s_addr(&bar[b]), 1u);
+        for (int q = max(0, t - st); q < t; ++q) mbar_wait_bounded(s_addr(&bar[q % st]), (unsigned)(q / st) & 1u);
         atomicExch(&g_conv_err, 1);
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -1069,7 +1171,11 @@ static void conv_umma(const Geo &g, const bf16 *in, const bf16 *w, const float *
             cudaSuccess)
             attr_bytes = (int)sm;
     }
-    k_conv_umma<N, OB><<<(rows + 127) / 128, 128, sm, s>>>(g, in, w, bias, addend, out, relu, rows);
+    // one tap: eight CTAs an SM walk the tiles; mode 1: the coarse voxels once per parity
+    const int tiles = (rows + 127) / 128;
+    const int grid = g.taps == 1 ? std::min(tiles, 152 * 8)
+                                 : (g.mode == 1 ? 8 * ((g.nb * g.Di * g.Hi * g.Wi + 127) / 128) : tiles);
+    k_conv_umma<N, OB><<<grid, 128, sm, s>>>(g, in, w, bias, addend, out, relu, rows);
 }
 
 template <int N>

@@ -32,11 +32,6 @@
 namespace qmin {
 namespace nn {
 
-__device__ __forceinline__ void cp_async16(unsigned saddr, const void *g, bool in)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(g), "r"(in ? 16 : 0) : "memory");
-}
-
 template <int CI, int CO, int S> struct Wgrad {
     static constexpr int NDY = CI <= 48 ? 3 : 1;      // dy taps of a CTA
     static constexpr int NG = 9 / NDY;                // groups: dz, and dy where NDY = 1
