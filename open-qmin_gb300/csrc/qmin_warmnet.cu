@@ -670,17 +670,23 @@ __global__ void __launch_bounds__(128) k_conv3_direct_z(Geo g, const bf16 *__res
 // as [18][10][8 channels], the canonical K-major core-matrix layout the
 // descriptors read, in a slab padded to 2944 bytes so that every box starts on
 // a 128-byte boundary; the leading byte offset of the A descriptor is that
-// slab pitch.  One thread issues the boxes against one mbarrier per ring slot
-// (the expected bytes count the whole box, zero fill included), waits for
-// plane z + 1 before it issues the MMAs of plane z, and reloads a slot only
-// after the MMAs that read it have committed.  All waits are bounded; a wait
+// slab pitch.  The MMAs go by input plane: for one (dx, dy) its rows meet the
+// weights of dz = 2, 1, 0 side by side (N = 3 cout), which adds to the output
+// planes before it, at it and after it, whose accumulators are neighbours in a
+// ring of four (split where the ring wraps and where a plane begins).  A small
+// MMA costs about as much as one of three times its N: with one per tap, 32 ->
+// 32 at 200^3 took 930 us, 16 -> 32 422 and 48 -> 48 at 100^3 352; 720, 392 and
+// 290 now.  The sums keep their order.  One thread issues the boxes against one
+// mbarrier per ring slot (the expected bytes count the whole box, zero fill
+// included) and reloads a slot only after the MMAs that read it have
+// committed.  All waits are bounded; a wait
 // that gives up leaves the copies and MMAs in flight to land (bounded again)
 // before the CTA frees its tensor memory and reports through g_conv_err.
 constexpr int kTmaSlab = 2944;  // 2880 bytes of box, padded to a multiple of 128
 static size_t direct_z_tma_smem(int cin, int n)
 {
     const size_t need = (size_t)27 * n * cin * 2 + (size_t)4 * (cin / 8) * kTmaSlab + 128 + 128;
-    const int per_sm = 512 / umma_cols(2 * n);
+    const int per_sm = 512 / umma_cols(4 * n);
     const size_t floor_bytes = (size_t)(232448 / per_sm) - 1024 + 1;
     return std::max(need, std::min<size_t>(floor_bytes, 232448 - 1024));
 }
@@ -697,15 +703,16 @@ __device__ __forceinline__ void tma_box_5d(unsigned dst, const CUtensorMap *map,
 }
 }  // namespace
 
-template <int N, int CIN>
+template <int N, int CIN, bool OUT_BF16>
 __global__ void __launch_bounds__(128) k_conv3_direct_z_tma(Geo g, const __grid_constant__ CUtensorMap tmap,
                                                             const bf16 *__restrict__ w,
-                                                            const float *__restrict__ bias, bf16 *__restrict__ out,
+                                                            const float *__restrict__ bias,
+                                                            const float *__restrict__ addend, void *out,
                                                             int relu, int zt)
 {
-    static_assert(N % 16 == 0 && N >= 16 && 2 * N <= 256, "two M=128 accumulators of N columns");
+    static_assert(N % 16 == 0 && N >= 16 && 4 * N <= 256, "four M=128 accumulators of N columns");
     static_assert(CIN % 16 == 0 && CIN >= 16, "input channels a multiple of 16");
-    constexpr int COLS = 2 * N <= 32 ? 32 : (2 * N <= 64 ? 64 : (2 * N <= 128 ? 128 : 256));
+    constexpr int COLS = 4 * N <= 64 ? 64 : (4 * N <= 128 ? 128 : 256);
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int cin = CIN, kc8 = CIN / 8, K = 27 * CIN;
     const int W = g.Wo, H = g.Ho, D = g.Do;
@@ -725,7 +732,7 @@ __global__ void __launch_bounds__(128) k_conv3_direct_z_tma(Geo g, const __grid_
     const int y0 = (bidx % ty) * 16;
     bidx /= ty;
     const int z0 = (bidx % tz) * zt, b = bidx / tz;
-    const int nz = min(zt, D - z0);
+    const int nz = min(zt, D - z0), ni = nz + 2;  // output planes; input planes z0 - 1 + i, i < ni
     if (*(volatile int *)&g_conv_err) return;
 
     if (warp == 0) {
@@ -739,32 +746,29 @@ __global__ void __launch_bounds__(128) k_conv3_direct_z_tma(Geo g, const __grid_
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(s_addr(&bar[k])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    auto slot_of = [&](int iz) { return (iz - z0 + 1) & 3; };            // iz >= z0 - 1
-    auto use_of = [&](int iz) { return (unsigned)((iz - z0 + 1) >> 2); };  // how many loads the slot had before
-    // plane iz's boxes into its ring slot (one thread)
-    auto load_plane = [&](int iz) {
-        const int sl = slot_of(iz);
-        const unsigned bs = s_addr(&bar[2 + sl]);
+    // input plane i's boxes into its ring slot (one thread)
+    auto load_plane = [&](int i) {
+        const unsigned bs = s_addr(&bar[2 + (i & 3)]);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bs), "r"(kc8 * 2880u)
                      : "memory");
-        const unsigned dst = s_addr(ring) + (unsigned)sl * slot_bytes;
-        for (int k8 = 0; k8 < kc8; ++k8) tma_box_5d(dst + (unsigned)k8 * kTmaSlab, &tmap, k8 * 8, x0 - 1, y0 - 1, iz, b, bs);
+        const unsigned dst = s_addr(ring) + (unsigned)(i & 3) * slot_bytes;
+        for (int k8 = 0; k8 < kc8; ++k8)
+            tma_box_5d(dst + (unsigned)k8 * kTmaSlab, &tmap, k8 * 8, x0 - 1, y0 - 1, z0 - 1 + i, b, bs);
     };
     const int polls = *(volatile int *)&g_conv_wait_limit;
-    auto wait_plane = [&](int iz, int lim) {
-        return mbar_wait_bounded(s_addr(&bar[2 + slot_of(iz)]), use_of(iz) & 1u, lim);
+    auto wait_plane = [&](int i, int lim) {
+        return mbar_wait_bounded(s_addr(&bar[2 + (i & 3)]), (unsigned)(i >> 2) & 1u, lim);
     };
-    int issued_hi = z0 - 2;  // the last plane whose boxes were issued
-    __syncthreads();         // the barriers are initialised
-    if (tid == 0) {
-        for (int iz = z0 - 1; iz <= z0 + 1; ++iz) load_plane(iz);
-        issued_hi = z0 + 1;
-    }
-    // all 27 taps' weights, [tap][co][cin] with each tap's [co][cin] in the canonical layout
+    int issued = 0;   // planes whose boxes were issued
+    __syncthreads();  // the barriers are initialised
+    if (tid == 0)
+        for (; issued < 3; ++issued) load_plane(issued);  // ni >= 3
+    // all 27 taps' weights: for each (dy, dx) the [co][cin] of dz = 2, 1, 0, in the canonical layout
     for (int e = tid; e < 27 * N * kc8; e += 128) {
-        const int tap = e / (N * kc8), rem = e - tap * N * kc8, co = rem / kc8, k8 = rem - co * kc8;
+        const int blk = e / (N * kc8), rem = e - blk * N * kc8, co = rem / kc8, k8 = rem - co * kc8;
+        const int tap = (2 - blk % 3) * 9 + blk / 3;
         const uint4 v = *reinterpret_cast<const uint4 *>(w + (size_t)co * K + (size_t)tap * cin + k8 * 8);
-        *reinterpret_cast<uint4 *>(wts + (size_t)tap * N * cin * 2 + ((size_t)(co >> 3) * kc8 + k8) * 128 +
+        *reinterpret_cast<uint4 *>(wts + (size_t)blk * N * cin * 2 + ((size_t)(co >> 3) * kc8 + k8) * 128 +
                                    (co & 7) * 16) = v;
     }
     // descriptors of the ring's and the weights' first core matrices; a
@@ -773,58 +777,90 @@ __global__ void __launch_bounds__(128) k_conv3_direct_z_tma(Geo g, const __grid_
     // the descriptor itself: the issuing thread does one add per operand per MMA
     const uint64_t da0 = umma_desc(s_addr(ring), kTmaSlab, 160);
     const uint64_t db0 = umma_desc(s_addr(wts), 128, (unsigned)kc8 * 128u);
-    auto issue = [&](int z, int acc_idx) {
+    auto mma = [&](uint32_t dst, uint64_t da, uint64_t db, uint32_t idesc, unsigned acc) {
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dst),
+            "l"(da), "l"(db), "r"(idesc), "r"(acc)
+            : "memory");
+    };
+    // input plane i: block j of the weights (dz = 2 - j) adds to output plane
+    // i - 2 + j, whose accumulator is at (i - 2 + j) % 4
+    auto issue = [&](int i) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const uint32_t dst = *tmem_slot + (uint32_t)(acc_idx * N);
-        const uint64_t das[3] = {da0 + ((uint64_t)slot_of(z - 1) * slot_bytes >> 4),
-                                 da0 + ((uint64_t)slot_of(z) * slot_bytes >> 4),
-                                 da0 + ((uint64_t)slot_of(z + 1) * slot_bytes >> 4)};
+        const uint32_t tm = *tmem_slot;
+        const uint64_t da_i = da0 + ((uint64_t)(i & 3) * slot_bytes >> 4);
+        const int j0 = max(0, 2 - i), j1 = min(2, nz + 1 - i);  // the planes this CTA owns
+        // blocks whose accumulators lie side by side go in one MMA: [j0, js) and [js, j1]
+        int js = j1 + 1;
+        for (int j = j0 + 1; j <= j1; ++j)
+            if (((i - 2 + j) & 3) == 0) js = j;
+        const uint32_t c0 = tm + (uint32_t)(((i - 2 + j0) & 3) * N), c1 = tm;
+        const uint32_t id0 = umma_idesc((js - j0) * N), id1 = umma_idesc((j1 - js + 1) * N);
+        constexpr uint64_t blk = (uint64_t)(N * CIN * 2 >> 4);
 #pragma unroll
-        for (int tap = 0; tap < 27; ++tap) {
-            const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
+        for (int t9 = 0; t9 < 9; ++t9) {
+            const int dy = t9 / 3, dx = t9 % 3;
 #pragma unroll
             for (int kk = 0; kk < CIN / 16; ++kk) {
-                const uint64_t da = das[dz] + (uint64_t)((2 * kk * kTmaSlab + (dy * 10 + dx) * 16) >> 4);
-                const uint64_t db = db0 + (uint64_t)((tap * N * CIN * 2 + kk * 256) >> 4);
-                const unsigned acc = (tap > 0 || kk > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dst),
-                    "l"(da), "l"(db), "r"(umma_idesc(N)), "r"(acc)
-                    : "memory");
+                const uint64_t da = da_i + (uint64_t)((2 * kk * kTmaSlab + (dy * 10 + dx) * 16) >> 4);
+                const uint64_t db = db0 + (uint64_t)((t9 * 3 * N * CIN * 2 + kk * 256) >> 4);
+                if (t9 == 0 && kk == 0) {
+                    // plane i (block 2) starts here, the others go on
+                    for (int j = j0; j <= j1; ++j)
+                        mma(tm + (uint32_t)(((i - 2 + j) & 3) * N), da, db + j * blk, umma_idesc(N), j < 2 ? 1u : 0u);
+                } else {
+                    mma(c0, da, db + j0 * blk, id0, 1u);
+                    if (js <= j1) mma(c1, da, db + js * blk, id1, 1u);
+                }
             }
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                         s_addr(&bar[acc_idx]))
+                         s_addr(&bar[i & 1]))
                      : "memory");
     };
-    auto epilogue = [&](int z, int acc_idx, uint32_t tmem) {
+    auto epilogue = [&](int o, uint32_t tmem) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(acc_idx * N);
+        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((o & 3) * N);
         const int ox = x0 + (tid & 7), oy = y0 + (tid >> 3);
         const bool inside = ox < W && oy < H;
-        bf16 *o = out + ((((size_t)b * D + z) * H + oy) * W + ox) * N;
+        const size_t at = ((((size_t)b * D + z0 + o) * H + oy) * W + ox) * N;
 #pragma unroll
-        for (int c0 = 0; c0 < N; c0 += 8) {
-            uint32_t r[8];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                           "=r"(r[7])
-                         : "r"(taddr + c0));
+        for (int c0 = 0; c0 < N; c0 += 16) {
+            uint32_t r[16];
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
+                "[%16];\n"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                : "r"(taddr + c0));
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            if (inside) {
-                __nv_bfloat162 hh[4];
+            if (!inside) continue;
+            float v[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                v[e] = __uint_as_float(r[e]) + (bias ? bias[c0 + e] : 0.f);
+                if (relu) v[e] = fmaxf(v[e], 0.f);
+            }
+            if constexpr (OUT_BF16) {
+                __nv_bfloat162 hh[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) hh[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+                uint4 *o4 = reinterpret_cast<uint4 *>(reinterpret_cast<bf16 *>(out) + at + c0);
+                o4[0] = reinterpret_cast<const uint4 *>(hh)[0];
+                o4[1] = reinterpret_cast<const uint4 *>(hh)[1];
+            } else {
+                float4 *o4 = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + at + c0);
+                const float4 *a4 = reinterpret_cast<const float4 *>(addend + (addend ? at + c0 : 0));
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    float v0 = __uint_as_float(r[2 * e]) + bias[c0 + 2 * e];
-                    float v1 = __uint_as_float(r[2 * e + 1]) + bias[c0 + 2 * e + 1];
-                    if (relu) {
-                        v0 = fmaxf(v0, 0.f);
-                        v1 = fmaxf(v1, 0.f);
+                    float4 q = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+                    if (addend) {
+                        const float4 p = a4[e];
+                        q = make_float4(q.x + p.x, q.y + p.y, q.z + p.z, q.w + p.w);
                     }
-                    hh[e] = __floats2bfloat162_rn(v0, v1);
+                    o4[e] = q;
                 }
-                *reinterpret_cast<uint4 *>(o + c0) = *reinterpret_cast<const uint4 *>(hh);
             }
         }
     };
@@ -835,47 +871,43 @@ __global__ void __launch_bounds__(128) k_conv3_direct_z_tma(Geo g, const __grid_
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tmem_slot;
     bool ok = true;
-    int committed = 0;  // planes whose MMAs were committed
-    for (int p = 0; p < nz; ++p) {
-        const int z = z0 + p;
+    int committed = 0;  // input planes whose MMAs were committed
+    for (int i = 0; i < ni; ++i) {
         bool good = true;
         if (tid == 0) {
-            // planes z - 1 and z were waited for by earlier steps (all three at the first)
-            if (p == 0) good = wait_plane(z - 1, polls) && wait_plane(z, polls);
-            good = good && wait_plane(z + 1, polls);
-            if (good) issue(z, p & 1);
+            good = wait_plane(i, polls);
+            if (good) issue(i);
         }
         if (__syncthreads_or(!good)) {
             ok = false;
             break;
         }
-        committed = p + 1;
-        if (p >= 1) {
-            // the MMAs of plane p - 1: done with their accumulator and with slot z - 2
-            const bool w_ok = mbar_wait_bounded(s_addr(&bar[(p - 1) & 1]), (unsigned)((p - 1) >> 1) & 1u, polls);
+        committed = i + 1;
+        if (i >= 1) {
+            // the MMAs of plane i - 1: done with its slot and with output plane i - 3
+            const bool w_ok = mbar_wait_bounded(s_addr(&bar[(i - 1) & 1]), (unsigned)((i - 1) >> 1) & 1u, polls);
             if (__syncthreads_or(!w_ok)) {
                 ok = false;
                 break;
             }
-            epilogue(z - 1, (p - 1) & 1, tmem);
-        }
-        if (tid == 0 && p + 1 < nz) {
-            load_plane(z + 2);
-            issued_hi = z + 2;
+            if (tid == 0 && issued < ni) load_plane(issued++);
+            if (i >= 3) epilogue(i - 3, tmem);
+        } else if (tid == 0 && issued < ni) {
+            load_plane(issued++);  // the fourth slot
         }
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         __syncthreads();
     }
     if (ok) {
-        const int last = nz - 1;
+        const int last = ni - 1;
         const bool w_ok = mbar_wait_bounded(s_addr(&bar[last & 1]), (unsigned)(last >> 1) & 1u, polls);
         ok = !__syncthreads_or(!w_ok);
-        if (ok) epilogue(z0 + last, last & 1, tmem);
+        if (ok) epilogue(nz - 1, tmem);
     }
     if (!ok && tid == 0) {
         // a wait gave up: let the boxes and the MMAs in flight land (bounded,
         // at the full poll count) before the buffers go away
-        for (int iz = max(z0 - 1, issued_hi - 3); iz <= issued_hi; ++iz) wait_plane(iz, kWaitPolls);
+        for (int i = max(0, issued - 4); i < issued; ++i) wait_plane(i, kWaitPolls);
         for (int q = max(0, committed - 2); q < committed; ++q)
             mbar_wait_bounded(s_addr(&bar[q & 1]), (unsigned)(q >> 1) & 1u);
         atomicExch(&g_conv_err, 1);
@@ -1215,9 +1247,9 @@ static PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder()
 // the TMA-staged direct kernel; false (nothing launched) where its tensor map
 // cannot describe the input: no encoder, an input not 16-byte aligned, or a
 // grid smaller than one halo box (10 x 18)
-template <int N, int CIN>
-static bool conv3_direct_z_tma(const Geo &g, const bf16 *in, const bf16 *w, const float *bias, bf16 *out, int relu,
-                               cudaStream_t s)
+template <int N, int CIN, bool OB>
+static bool conv3_direct_z_tma(const Geo &g, const bf16 *in, const bf16 *w, const float *bias,
+                               const float *addend, void *out, int relu, cudaStream_t s)
 {
     auto enc = tmap_encoder();
     if (!enc || (reinterpret_cast<uintptr_t>(in) & 15) || g.Wi < 10 || g.Hi < 18 || g.cin != CIN) return false;
@@ -1238,47 +1270,45 @@ static bool conv3_direct_z_tma(const Geo &g, const bf16 *in, const bf16 *w, cons
     if (sm > 232448 - 1024) return false;
     if ((int)sm > attr_bytes) {
         // a failure here surfaces as the launch's error
-        if (cudaFuncSetAttribute(k_conv3_direct_z_tma<N, CIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(k_conv3_direct_z_tma<N, CIN, OB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sm) == cudaSuccess)
             attr_bytes = (int)sm;
     }
     const int zt = std::min(g.Do, 16);
     const long long tiles = (long long)((g.Wo + 7) / 8) * ((g.Ho + 15) / 16) * ((g.Do + zt - 1) / zt) * g.nb;
-    k_conv3_direct_z_tma<N, CIN><<<(unsigned)tiles, 128, sm, s>>>(g, map, w, bias, out, relu, zt);
+    k_conv3_direct_z_tma<N, CIN, OB><<<(unsigned)tiles, 128, sm, s>>>(g, map, w, bias, addend, out, relu, zt);
     return true;
 }
 
-// path 1 or 2: the 5th-generation tensor-core kernels above (the direct kernel
-// for 3x3x3 stride-1 forward convolutions with BF16 output, its halo planes
-// staged by TMA on path 1 where the tensor map applies, by the threads on path
-// 2; the gathering kernel otherwise); path 0: mma.sync
+// path 1 or 2: the 5th-generation tensor-core kernels above (for 3x3x3 stride-1
+// convolutions the direct kernel: on path 1 its halo planes staged by TMA where
+// the tensor map applies, on path 2, forward only, by the threads; the
+// gathering kernel otherwise); path 0: mma.sync
 template <bool OB>
 static void conv_gemm(const Geo &g, const bf16 *in, const bf16 *w, const float *bias, const float *addend, void *out,
                       int relu, int rows, cudaStream_t s, int path)
 {
     const bool tcgen05 = path != 0;
-    // the direct kernel wins where a dz plane's weights are small (measured at
-    // 128^3: 16->32 0.29 ms vs 0.49 gathering, 32->32 0.77 vs 0.95; at 48->48
-    // and 64->64 the 135-216 KB of staging leave one CTA per SM and it loses)
-    if (tcgen05 && OB && g.mode == 0 && g.taps == 27 && g.stride == 1 && !addend && bias &&
-        direct_z_smem(g.cin, g.cout) <= 232448 - 1024) {
-        if (g.cout == 32) {
-            // the network's direct layers: 16 -> 32 and 32 -> 32 (TMA kernel per input width)
-            if (path == 1 && g.cin == 16 &&
-                conv3_direct_z_tma<32, 16>(g, in, w, bias, reinterpret_cast<bf16 *>(out), relu, s))
-                return;
-            if (path == 1 && g.cin == 32 &&
-                conv3_direct_z_tma<32, 32>(g, in, w, bias, reinterpret_cast<bf16 *>(out), relu, s))
-                return;
-            conv3_direct_z<32>(g, in, w, bias, reinterpret_cast<bf16 *>(out), relu, s);
-            return;
+    // the direct kernel wins where the weights of all taps stay in shared memory
+    // (data gradients of eight 64^3 samples, direct against gathering: 32 -> 32
+    // 265 us against 1130, 48 -> 48 86 against 255); at 64 -> 64 they take 216 KB
+    if (tcgen05 && g.mode == 0 && g.taps == 27 && g.stride == 1) {
+        if (path == 1) {
+            if constexpr (OB)
+                if (g.cout == 32 && g.cin == 16 && conv3_direct_z_tma<32, 16, OB>(g, in, w, bias, addend, out, relu, s))
+                    return;
+            if (g.cout == 32 && g.cin == 32 && conv3_direct_z_tma<32, 32, OB>(g, in, w, bias, addend, out, relu, s)) return;
+            if (g.cout == 48 && g.cin == 48 && conv3_direct_z_tma<48, 48, OB>(g, in, w, bias, addend, out, relu, s)) return;
         }
-        if (g.cout == 48) {
-            if (path == 1 && g.cin == 48 &&
-                conv3_direct_z_tma<48, 48>(g, in, w, bias, reinterpret_cast<bf16 *>(out), relu, s))
+        if (OB && !addend && bias && direct_z_smem(g.cin, g.cout) <= 232448 - 1024) {
+            if (g.cout == 32) {
+                conv3_direct_z<32>(g, in, w, bias, reinterpret_cast<bf16 *>(out), relu, s);
                 return;
-            conv3_direct_z<48>(g, in, w, bias, reinterpret_cast<bf16 *>(out), relu, s);
-            return;
+            }
+            if (g.cout == 48) {
+                conv3_direct_z<48>(g, in, w, bias, reinterpret_cast<bf16 *>(out), relu, s);
+                return;
+            }
         }
     }
     if (tcgen05) {
