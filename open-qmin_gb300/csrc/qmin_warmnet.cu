@@ -675,8 +675,9 @@ __global__ void __launch_bounds__(128) k_conv3_direct_z(Geo g, const bf16 *__res
 // planes before it, at it and after it, whose accumulators are neighbours in a
 // ring of four (split where the ring wraps and where a plane begins).  A small
 // MMA costs about as much as one of three times its N: with one per tap, 32 ->
-// 32 at 200^3 took 930 us, 16 -> 32 422 and 48 -> 48 at 100^3 352; 720, 392 and
-// 290 now.  The sums keep their order.  One thread issues the boxes against one
+// 32 at 200^3 took 930 us, 16 -> 32 422 and 48 -> 48 at 100^3 352; 661, 298 and
+// 256 now, the accumulators read by four warps while a thread of a fifth issues
+// (720, 392 and 290 where one of the four issues).  The sums keep their order.  One thread issues the boxes against one
 // mbarrier per ring slot (the expected bytes count the whole box, zero fill
 // included) and reloads a slot only after the MMAs that read it have
 // committed.  All waits are bounded; a wait
@@ -703,8 +704,11 @@ __device__ __forceinline__ void tma_box_5d(unsigned dst, const CUtensorMap *map,
 }
 }  // namespace
 
+// four warps read the accumulators out, one thread of a fifth issues copies and MMAs
+constexpr int kDirectThreads = 160;
+
 template <int N, int CIN, bool OUT_BF16>
-__global__ void __launch_bounds__(128) k_conv3_direct_z_tma(Geo g, const __grid_constant__ CUtensorMap tmap,
+__global__ void __launch_bounds__(kDirectThreads) k_conv3_direct_z_tma(Geo g, const __grid_constant__ CUtensorMap tmap,
                                                             const bf16 *__restrict__ w,
                                                             const float *__restrict__ bias,
                                                             const float *__restrict__ addend, void *out,
@@ -722,8 +726,9 @@ __global__ void __launch_bounds__(128) k_conv3_direct_z_tma(Geo g, const __grid_
     unsigned char *base = smem_raw + ((128u - (s_addr(smem_raw) & 127u)) & 127u);
     unsigned char *wts = base;
     unsigned char *ring = base + w_bytes;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(ring + 4 * (size_t)slot_bytes);  // [0..1] MMAs, [2..5] ring slots
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar + 6);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(ring + 4 * (size_t)slot_bytes);  // [0..3] MMAs, [4..7] ring slots, [8..11] epilogues
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar + 12);
+    volatile int *bad = reinterpret_cast<volatile int *>(tmem_slot + 1);  // a wait gave up
     const int tid = threadIdx.x, warp = tid >> 5;
     const int tx = (W + 7) >> 3, ty = (H + 15) >> 4, tz = (D + zt - 1) / zt;
     int bidx = blockIdx.x;
@@ -741,14 +746,16 @@ __global__ void __launch_bounds__(128) k_conv3_direct_z_tma(Geo g, const __grid_
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    if (tid == 0) {
-        for (int k = 0; k < 6; ++k)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(s_addr(&bar[k])) : "memory");
+    if (tid == 128) {
+        *bad = 0;
+        for (int k = 0; k < 12; ++k)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(s_addr(&bar[k])), "r"(k < 8 ? 1 : 128)
+                         : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     // input plane i's boxes into its ring slot (one thread)
     auto load_plane = [&](int i) {
-        const unsigned bs = s_addr(&bar[2 + (i & 3)]);
+        const unsigned bs = s_addr(&bar[4 + (i & 3)]);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bs), "r"(kc8 * 2880u)
                      : "memory");
         const unsigned dst = s_addr(ring) + (unsigned)(i & 3) * slot_bytes;
@@ -756,15 +763,21 @@ __global__ void __launch_bounds__(128) k_conv3_direct_z_tma(Geo g, const __grid_
             tma_box_5d(dst + (unsigned)k8 * kTmaSlab, &tmap, k8 * 8, x0 - 1, y0 - 1, z0 - 1 + i, b, bs);
     };
     const int polls = *(volatile int *)&g_conv_wait_limit;
-    auto wait_plane = [&](int i, int lim) {
-        return mbar_wait_bounded(s_addr(&bar[2 + (i & 3)]), (unsigned)(i >> 2) & 1u, lim);
+    // bounded; also gives up when another thread of the CTA has
+    auto wait = [&](int at, int n, int lim) {
+        const unsigned bs = s_addr(&bar[at + (n & 3)]), parity = (unsigned)(n >> 2) & 1u;
+        for (int it = 0; it < lim; it += 64) {
+            if (mbar_wait_bounded(bs, parity, min(64, lim - it))) return true;
+            if (*bad) return false;
+        }
+        return false;
     };
     int issued = 0;   // planes whose boxes were issued
     __syncthreads();  // the barriers are initialised
-    if (tid == 0)
+    if (tid == 128)
         for (; issued < 3; ++issued) load_plane(issued);  // ni >= 3
     // all 27 taps' weights: for each (dy, dx) the [co][cin] of dz = 2, 1, 0, in the canonical layout
-    for (int e = tid; e < 27 * N * kc8; e += 128) {
+    for (int e = tid; e < 27 * N * kc8; e += kDirectThreads) {
         const int blk = e / (N * kc8), rem = e - blk * N * kc8, co = rem / kc8, k8 = rem - co * kc8;
         const int tap = (2 - blk % 3) * 9 + blk / 3;
         const uint4 v = *reinterpret_cast<const uint4 *>(w + (size_t)co * K + (size_t)tap * cin + k8 * 8);
@@ -816,7 +829,7 @@ __global__ void __launch_bounds__(128) k_conv3_direct_z_tma(Geo g, const __grid_
             }
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                         s_addr(&bar[i & 1]))
+                         s_addr(&bar[i & 3]))
                      : "memory");
     };
     auto epilogue = [&](int o, uint32_t tmem) {
@@ -870,46 +883,41 @@ __global__ void __launch_bounds__(128) k_conv3_direct_z_tma(Geo g, const __grid_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tmem_slot;
-    bool ok = true;
     int committed = 0;  // input planes whose MMAs were committed
-    for (int i = 0; i < ni; ++i) {
-        bool good = true;
-        if (tid == 0) {
-            good = wait_plane(i, polls);
-            if (good) issue(i);
+    if (tid == 128) {
+        // the issuing thread: at most four output planes ahead of the epilogues
+        bool ok = true;
+        for (int i = 0; i < ni && ok; ++i) {
+            ok = wait(4, i, polls) && (i < 4 || wait(8, i - 4, polls));
+            if (!ok) break;
+            issue(i);
+            committed = i + 1;
+            if (issued < ni) {
+                // the slot of plane i + 3: its MMAs are those of plane i - 1
+                ok = i == 0 || wait(0, i - 1, polls);
+                if (ok) load_plane(issued++);
+            }
         }
-        if (__syncthreads_or(!good)) {
-            ok = false;
-            break;
-        }
-        committed = i + 1;
-        if (i >= 1) {
-            // the MMAs of plane i - 1: done with its slot and with output plane i - 3
-            const bool w_ok = mbar_wait_bounded(s_addr(&bar[(i - 1) & 1]), (unsigned)((i - 1) >> 1) & 1u, polls);
-            if (__syncthreads_or(!w_ok)) {
-                ok = false;
+        if (!ok) *bad = 1;
+    } else if (tid < 128) {
+        for (int o = 0; o < nz; ++o) {
+            if (!__all_sync(0xffffffffu, wait(0, o + 2, polls))) {  // the warp leaves together
+                *bad = 1;
                 break;
             }
-            if (tid == 0 && issued < ni) load_plane(issued++);
-            if (i >= 3) epilogue(i - 3, tmem);
-        } else if (tid == 0 && issued < ni) {
-            load_plane(issued++);  // the fourth slot
+            epilogue(o, tmem);
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(s_addr(&bar[8 + (o & 3)])) : "memory");
         }
-        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-        __syncthreads();
     }
-    if (ok) {
-        const int last = ni - 1;
-        const bool w_ok = mbar_wait_bounded(s_addr(&bar[last & 1]), (unsigned)(last >> 1) & 1u, polls);
-        ok = !__syncthreads_or(!w_ok);
-        if (ok) epilogue(nz - 1, tmem);
-    }
-    if (!ok && tid == 0) {
+    __syncthreads();
+    if (*bad && tid == 128) {
         // a wait gave up: let the boxes and the MMAs in flight land (bounded,
         // at the full poll count) before the buffers go away
-        for (int i = max(0, issued - 4); i < issued; ++i) wait_plane(i, kWaitPolls);
-        for (int q = max(0, committed - 2); q < committed; ++q)
-            mbar_wait_bounded(s_addr(&bar[q & 1]), (unsigned)(q >> 1) & 1u);
+        for (int i = max(0, issued - 4); i < issued; ++i)
+            mbar_wait_bounded(s_addr(&bar[4 + (i & 3)]), (unsigned)(i >> 2) & 1u);
+        for (int q = max(0, committed - 4); q < committed; ++q)
+            mbar_wait_bounded(s_addr(&bar[q & 3]), (unsigned)(q >> 2) & 1u);
         atomicExch(&g_conv_err, 1);
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -990,10 +998,46 @@ __global__ void k_f32_to_bf16(const float *x, bf16 *y, long long n)
     GRID_STRIDE(i, n) y[i] = __float2bfloat16(x[i]);
 }
 
-// gradient through the ReLU (mask from the stored BF16 activation), as BF16
-__global__ void k_relu_grad_bf16(const float *g, const bf16 *act, bf16 *y, long long n)
+// the gradient at a layer's output, through its ReLU (mask from the stored BF16
+// activation) where act is given: as BF16, and its sum over the rows added to
+// the bias gradient.  One pass over g: 12 launches of it and of a separate sum
+// took 0.95 ms of a training pass of eight 64^3 samples, 0.32 now.  A thread
+// keeps its four channels (the block size is a multiple of c / 4).
+constexpr int kGradBlock = 192;
+__global__ void __launch_bounds__(kGradBlock)
+    k_grad_in(const float *__restrict__ g, const bf16 *__restrict__ act, bf16 *__restrict__ y, float *__restrict__ db,
+              long long n4, int c)
 {
-    GRID_STRIDE(i, n) y[i] = __float2bfloat16(__bfloat162float(act[i]) > 0.f ? g[i] : 0.f);
+    extern __shared__ float sum[];
+    for (int k = threadIdx.x; k < c; k += kGradBlock) sum[k] = 0.f;
+    __syncthreads();
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    const long long i0 = blockIdx.x * (long long)kGradBlock + threadIdx.x;
+    for (long long i = i0; i < n4; i += (long long)gridDim.x * kGradBlock) {
+        float4 v = reinterpret_cast<const float4 *>(g)[i];
+        if (act) {
+            const uint2 a = reinterpret_cast<const uint2 *>(act)[i];
+            const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&a.x));
+            const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&a.y));
+            v.x = lo.x > 0.f ? v.x : 0.f;
+            v.y = lo.y > 0.f ? v.y : 0.f;
+            v.z = hi.x > 0.f ? v.z : 0.f;
+            v.w = hi.y > 0.f ? v.w : 0.f;
+        }
+        s.x += v.x;
+        s.y += v.y;
+        s.z += v.z;
+        s.w += v.w;
+        const __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+        reinterpret_cast<uint2 *>(y)[i] = *reinterpret_cast<const uint2 *>(h);
+    }
+    const int k0 = 4 * (int)(i0 % (c / 4));
+    atomicAdd(sum + k0, s.x);
+    atomicAdd(sum + k0 + 1, s.y);
+    atomicAdd(sum + k0 + 2, s.z);
+    atomicAdd(sum + k0 + 3, s.w);
+    __syncthreads();
+    for (int k = threadIdx.x; k < c; k += kGradBlock) atomicAdd(db + k, sum[k]);
 }
 
 // data-gradient weights: Wd[ci][tap'][co] = W[co][tap][ci], tap' = 26 - tap
@@ -1068,22 +1112,6 @@ __global__ void k_up2_grad(const float *g2, float *g, Dims d, int c)
                 for (int dx = 0; dx < 2; ++dx)
                     s += g2[((((long long)b * Z + 2 * z + dz) * Y + 2 * y + dy) * X + 2 * x + dx) * c + ch];
         g[i] = s;
-    }
-}
-
-// bias gradient db[c] += sum_v g[v][c] (masked by the ReLU when act != NULL);
-// one block per (row chunk, 32-channel group), a thread per channel and row lane
-__global__ void k_bias_grad(const float *g, const bf16 *act, float *db, long long rows, int c)
-{
-    const int ch = blockIdx.y * 32 + (threadIdx.x & 31);
-    const int lanes = blockDim.x >> 5;
-    float s = 0.f;
-    if (ch < c) {
-        for (long long v = blockIdx.x * (long long)lanes + (threadIdx.x >> 5); v < rows; v += (long long)gridDim.x * lanes) {
-            const float x = g[v * c + ch];
-            s += (act == nullptr || __bfloat162float(act[v * c + ch]) > 0.f) ? x : 0.f;
-        }
-        atomicAdd(db + ch, s);
     }
 }
 
@@ -1276,7 +1304,7 @@ static bool conv3_direct_z_tma(const Geo &g, const bf16 *in, const bf16 *w, cons
     }
     const int zt = std::min(g.Do, 16);
     const long long tiles = (long long)((g.Wo + 7) / 8) * ((g.Ho + 15) / 16) * ((g.Do + zt - 1) / zt) * g.nb;
-    k_conv3_direct_z_tma<N, CIN, OB><<<(unsigned)tiles, 128, sm, s>>>(g, map, w, bias, addend, out, relu, zt);
+    k_conv3_direct_z_tma<N, CIN, OB><<<(unsigned)tiles, kDirectThreads, sm, s>>>(g, map, w, bias, addend, out, relu, zt);
     return true;
 }
 
@@ -1291,7 +1319,7 @@ static void conv_gemm(const Geo &g, const bf16 *in, const bf16 *w, const float *
     const bool tcgen05 = path != 0;
     // the direct kernel wins where the weights of all taps stay in shared memory
     // (data gradients of eight 64^3 samples, direct against gathering: 32 -> 32
-    // 265 us against 1130, 48 -> 48 86 against 255); at 64 -> 64 they take 216 KB
+    // 237 us against 1130, 48 -> 48 76 against 255); at 64 -> 64 they take 216 KB
     if (tcgen05 && g.mode == 0 && g.taps == 27 && g.stride == 1) {
         if (path == 1) {
             if constexpr (OB)
@@ -1468,10 +1496,8 @@ void layer_backward(qmin_warmnet_ctx *n, int i, const float *gout, const bf16 *a
     const long long rows_out = rows_at(n, out_level(L)), rows_in = rows_at(n, L.level);
     const bf16 *act_out = L.relu ? n->act[i] : nullptr;
     const long long ne = rows_out * L.cout;
-    if (act_out) k_relu_grad_bf16<<<grid1(ne), 256, 0, s>>>(gout, act_out, n->gbf, ne);
-    else k_f32_to_bf16<<<grid1(ne), 256, 0, s>>>(gout, n->gbf, ne);
-    k_bias_grad<<<dim3((unsigned)std::min<long long>((rows_out + 7) / 8, 1024), (unsigned)((L.cout + 31) / 32)), 256, 0,
-                  s>>>(gout, act_out, n->g + L.boff, rows_out, L.cout);
+    k_grad_in<<<(unsigned)std::min<long long>((ne / 4 + kGradBlock - 1) / kGradBlock, 152 * 10), kGradBlock,
+                L.cout * sizeof(float), s>>>(gout, act_out, n->gbf, n->g + L.boff, ne / 4, L.cout);
     const Geo g = fwd_geo(n, L);
     if (n->path == 0 || !wgrad_umma(g, n->gbf, act_in, n->g + L.woff, s)) {
         const int tiles = ((L.cout + 63) / 64) * ((L.cin + 63) / 64);
@@ -1481,7 +1507,7 @@ void layer_backward(qmin_warmnet_ctx *n, int i, const float *gout, const bf16 *a
         const dim3 grid((unsigned)((rows_out + chunk - 1) / chunk), (unsigned)L.taps, (unsigned)tiles);
         k_conv_wgrad<<<grid, 128, 0, s>>>(g, n->gbf, act_in, n->g + L.woff, (int)rows_out, (int)chunk);
     }
-    n->launches += 3;
+    n->launches += 2;
     if (!gin) return;
     Geo d;
     d.Di = g.Do;
