@@ -48,6 +48,9 @@ SPLIT_FUSED_FIRST = 7
 # FP64 instructions per deep bulk site of the split force + kick (135 DFMA, 15.2 DMUL,
 # 22.7 DADD counted by ncu; 106 of them the 25-point form over shared sums)
 FP64_OPS_PER_DEEP_SITE = 173
+# the fixed-point force (split variant 0, fields within its range) leaves the metric (4), the
+# kick (5) and the FIRE sums (17); everything else runs on the integer pipes
+FP64_OPS_PER_FIXED_SITE = 26
 
 
 def kernel_roofline(lat, esz, N, peak, peak_kind, tag):
@@ -185,7 +188,7 @@ def make_lattice(q, consts, g, precision):
 # the older strategies on a 128^3 case, scaled by the number of sites (their
 # traffic grows in proportion to the sites they process).
 DRAM_BYTES_PER_LAUNCH = {
-    ("force_kick_split", "f64"): 1715513856.0,   # 214.4 B/site (161 algorithmic)
+    ("force_kick_split", "f64"): 1031700000.0,   # 129.0 B/site (fixed-point force, 128^3 capture; 161 algorithmic)
     ("force_kick_split", "f32"): 648814080.0,    # 81.1 B/site (81 algorithmic)
     ("fire_fused_split", "f32"): 939452544.0,    # 117.4 B/site (121 algorithmic)
     ("force_kick_reduce", "f64"): 2872800000.0,  # 359.1 B/site
@@ -282,16 +285,18 @@ def run_ours(args, rank, world):
     it_ms = ms / (K)
     roofline["iteration_achieved_gbs_at_241B"] = 241 * N / (it_ms / 1e3) / 1e9
     if roofline["kernel"] == "force_kick_split":
-        # the FP64 force + kick is bound by the FP64 pipe, not by HBM: the same launch
-        # against GB300's FP64 instruction rate (2 per SM per cycle, 304 per cycle over
-        # the 152 SMs) at the SM clock sampled during the timed region
+        # the same launch against GB300's FP64 instruction rate (2 per SM per cycle, 304 per
+        # cycle over the 152 SMs) at the SM clock sampled during the timed region
         mhz = (clocks or {}).get("sm_mhz") or 2070.0
         t = roofline["kernel_ms"]["force_kick_split"] / 1e3
-        achieved = FP64_OPS_PER_DEEP_SITE * N / t / 1e9
+        fixed = roofline["autotuned"]["variant"] == 0
+        ops = FP64_OPS_PER_FIXED_SITE if fixed else FP64_OPS_PER_DEEP_SITE
+        achieved = ops * N / t / 1e9
         peak_ops = 304 * mhz * 1e6 / 1e9
-        roofline["fp64_pipe"] = {"ops_per_site": FP64_OPS_PER_DEEP_SITE, "achieved": achieved, "peak": peak_ops,
+        roofline["fp64_pipe"] = {"ops_per_site": ops, "achieved": achieved, "peak": peak_ops,
                                  "unit": "G FP64 instructions/s", "frac": achieved / peak_ops,
-                                 "source": "ncu dfma + dmul + dadd per deep site of the FP64 deep-site kernel "
+                                 "source": "FP64 instructions left per deep site of the fixed-point force" if fixed else
+                                           "ncu dfma + dmul + dadd per deep site of the FP64 deep-site kernel "
                                            "(128^3 capture); every site counted at the deep-site figure"}
     fire_state = {"forceMax": r["forceMax"], "iterations": r["iterations"]}
     lat.close()

@@ -241,7 +241,8 @@ int qmin_gd_run(qmin_handle h, double dt, double force_cutoff, int max_iteration
                                 tiles (FP32 form only) */
 #define QMIN_FIRE_SPLIT 4    /* deep bulk sites' force + kick over Q on the 25-point stencil (no derivative
                                 planes), the sites near objects through the plane forms (multi-constant
-                                form without L6; otherwise the separate kernels run) */
+                                form without L6, and one-constant lattices: FP64 variant 0, FP32 variants
+                                7 to 9 when no variant is pinned; otherwise the separate kernels run) */
 /* Choose how qmin_fire_run executes an iteration; all strategies give the
  * same results to rounding.  No reference counterpart (execution strategy). */
 int qmin_set_fire_kernel(qmin_handle h, int mode);
@@ -268,7 +269,9 @@ int qmin_set_fire_variant(qmin_handle h, int variant);
  * iteration of every candidate: ms[0..2] separate (1, 2, 3 blocks per SM),
  * ms[3 + 2*cfg + v] fused (4 shapes, v = 0/1 for the two z extents tried),
  * ms[11 + 2*cfg + v] staged (3 shapes), ms[17 + v] split (v = 0, 1: deep
- * sites from global memory at 1 or 2 blocks per SM; v = 2, 3: deep sites
+ * sites from global memory at 1 or 2 blocks per SM; v = 0 in FP64: in 64-bit
+ * fixed point where |Q| < 3/4 at every site the minimiser moves, with the
+ * former kernel standing by for fields outside; v = 2, 3: deep sites
  * from shared-memory tiles of 32 x 8 or 16 x 16 sites; v = 4, 5, FP32
  * only: two x-adjacent sites per thread on 32 x 8 tiles, z chunks of 8
  * planes or long enough that the grid is about two waves; v = 6, FP32 only:

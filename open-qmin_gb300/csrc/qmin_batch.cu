@@ -1,17 +1,19 @@
 // Batched minimisation: many independent lattices of uneven sizes minimised
 // together.  Every solve is an independent energyMinimizerFIRE::minimize
 // (energyMinimizerFIRE.cpp:151-170) on its own lattice; the batch packs all of
-// them into one set of SoA planes, cut into chunks of 256 sites that never
-// straddle two solves (256 consecutive sites, or tiles of the solve's box; the
-// tuner picks the shape by timing the force + kick).  qmin_batch_fire_run runs
-// every iteration of every solve in one persistent cooperative launch: per
-// iteration the predictor, the force + half kick + per-chunk FIRE sums and the
-// per-solve FIRE control, separated by bounded grid barriers (FP32
-// one-constant batches: predictor, force and kick as one phase from one state
-// set into the other, then the control).  Per-solve FIRE
-// scalars live on the device; a solve that converged or ran out of iterations
-// retires, and the phases then cover only the chunks of the solves still
-// active.
+// them into one set of SoA planes.  qmin_batch_fire_run runs every iteration of
+// every solve in one persistent cooperative launch: work items (tiles or runs
+// of a solve's bulk sites; its listed sites, near objects) taken from a
+// counter, the phases of an iteration separated by bounded grid barriers; the
+// block that finishes a solve's last item takes its FIRE control step.  FP32:
+// predictor, force and kick as one phase from one state set into the other;
+// FP64: the predictor, then the force and kick in fixed point; multi-constant
+// solves have a phase for the derivative planes of the listed sites.  Per-solve
+// FIRE scalars live on the device; a solve that converged or ran out of
+// iterations retires, and the phases then cover only the solves still active.
+// The entry force evaluation goes by chunks of 256 sites that never straddle
+// two solves (256 consecutive sites, or tiles of the solve's box; the tuner
+// picks the shape).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -729,7 +731,8 @@ __global__ void __launch_bounds__(kBlock, kFixedPerSm)
 
 // FP32: one phase per iteration for predictor, force and kick (b_tile_item),
 // before it for multi-constant solves the derivative planes the listed sites
-// read, after it the control.  Iteration it reads state set it & 1 (0: B.L's
+// read; the block that finishes a solve's last item does its control.
+// Iteration it reads state set it & 1 (0: B.L's
 // planes, 1: s1) and writes the other; a solve that retires leaves
 // in_second[solve] = 1 when its final state is in s1 (k_b_settle copies it
 // back).  Blocks take the items in turn from a counter, listed sites first in

@@ -18,9 +18,9 @@
 
 namespace qmin {
 
-// 128 threads, three blocks per SM (168 registers, nothing spilled): 64 uneven
-// one-constant solves (4.4 M sites) take 180 us an iteration and eight 64^3
-// multi-constant ones (2.1 M sites) 180; four blocks per SM 183 and 199 (864
+// 128 threads, three blocks per SM (168 registers; the multi-constant form
+// spills 270 bytes): 64 uneven one-constant solves (4.4 M sites) take 180 us an
+// iteration and eight 64^3 multi-constant ones (2.1 M sites) 183; four blocks per SM 183 and 199 (864
 // bytes spilled), five 235 and 202, 256 threads 182 and 210, tiles at most 16
 // wide 202 and 221.  The site-by-site form this replaced took 290 and 465:
 // every neighbour's prediction formed again (one-constant), derivative planes

@@ -287,7 +287,8 @@ static int ensure_aux(qmin_ctx *h)
     return QMIN_OK;
 }
 
-template <class T> static Lat<T> make_lat(qmin_ctx *h)
+// fire: for FIRE iterations, whose FP64 force runs in fixed point at every size
+template <class T> static Lat<T> make_lat(qmin_ctx *h, bool fire = false)
 {
     Lat<T> L;
     memset(&L, 0, sizeof L);
@@ -314,7 +315,7 @@ template <class T> static Lat<T> make_lat(qmin_ctx *h)
         L.fork = &h->fork;
     }
     if constexpr (sizeof(T) == 8)
-        if (ensure_fixed(h, L)) {
+        if ((fire || h->N >= kFixedForceSites) && ensure_fixed(h, L)) {
             L.X = h->X;
             L.fx = h->fx;
             L.fixed = &h->kc;
@@ -1208,7 +1209,7 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
 
 template <class T> static int fire_impl(qmin_ctx *h, int max_iterations)
 {
-    Lat<T> L = make_lat<T>(h);
+    Lat<T> L = make_lat<T>(h, true);
     const int it0 = h->fire_h->iterations;
     // minimize(): forces at the current Q first (energyMinimizerFIRE.cpp:157)
     h->launches += launch_force<T>(L, h->grid, h->stream);
@@ -1594,7 +1595,7 @@ int qmin_lbfgs_run(qmin_handle h, int m, double eta, double force_cutoff, int ma
 // ------------------------------------------------------------ diagnostics
 template <class T> static int fire_profile_impl(qmin_ctx *h, int iterations, double *ms)
 {
-    Lat<T> L = make_lat<T>(h);
+    Lat<T> L = make_lat<T>(h, true);
     int r = tune_fire<T>(h, L);
     if (r) return r;
     cudaEvent_t ev[5];

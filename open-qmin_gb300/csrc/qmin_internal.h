@@ -34,6 +34,11 @@ struct SplitLists {
 
 struct FixedCoef;  // qmin_fixed.cuh
 
+// sites from which a force-only FP64 evaluation runs in fixed point: its passes
+// beside the listed sites take 62 against 65 us at 40^3, 58 against 80 at 50^3
+// (multi-constant; one-constant from 10^5, launch_force)
+constexpr int kFixedForceSites = 50000;
+
 // Range of Q over the LC sites, for the fixed-point force: wide, a component
 // at or above 3/4; lively, a component at or above 1/8.  The pass that writes
 // Q 2^56 raises them; the force passes after it run in fixed point when

@@ -1507,7 +1507,7 @@ template <class T> int launch_split_force(const Lat<T> &L, int grid, cudaStream_
     if constexpr (sizeof(T) == 4) {
         launch_deep_pair<32, 8, 3, false>(L, sl, nullptr, nullptr, true, s);
     } else {
-        FixedDev *fx = L.fixed ? L.fx : nullptr;
+        FixedDev *fx = L.fixed && L.N >= kFixedForceSites ? L.fx : nullptr;
         if (fx) {
             cudaMemsetAsync(fx, 0, sizeof(FixedDev), s);
             n += launch_fixed_pred(L, nullptr, s);
