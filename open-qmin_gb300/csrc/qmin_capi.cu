@@ -1272,7 +1272,7 @@ template <class T> static int fire_impl(qmin_ctx *h, int max_iterations)
                 cudaStreamWaitEvent(h->aux, h->ev_fork, 0);
             }
             const int nd = launch_split_deep<T>(L, sl, h->fire, h->partials, h->grid, h->split_cap, h->stream);
-            n += 1 + fixed;
+            n += 1 + (fixed && L.multi);
             int nl = 0;
             if (listed) {
                 n += launch_split_derivs<T>(L, sl, h->fire, h->aux);

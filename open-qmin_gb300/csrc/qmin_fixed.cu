@@ -9,15 +9,6 @@ namespace qmin {
 
 namespace {
 
-// what the force kernel needs of a lattice
-struct FixedLat {
-    int Lx, Ly, Lz, N;
-    unsigned P, mx, my;  // multipliers of udiv for Lx and Ly
-    const long long *X;
-    double *V, *F;
-    const uint8_t *cls;
-};
-
 constexpr int kFixBlock = 128, kFixPerSm = 4;
 
 }  // namespace
@@ -66,7 +57,11 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 // Force at deep bulk sites from X; KICK: half kick and the FIRE sums,
-// partials[0 .. 3 gridDim.x), otherwise forces only, zero at object sites.
+// partials[0 .. 3 gridDim.x), otherwise forces only, zero at object sites.  A
+// one-constant lattice outside the fixed-point range takes the FP64 form here
+// (50^3: 3.09 ms per 100 iterations, 3.25 with a kernel of its own standing by).
+// Multi-constant lattices leave it to k_force_kick_deep: with both forms in one
+// kernel the fixed-point one spills (83 x 61 x 97: 8.3 ms instead of 7.3).
 //
 // 1,080 instructions per warp and site group against 173 FP64 operations (2,770
 // cycles of the FP64 pipe) of k_force_kick_deep; 26 FP64 operations are left
@@ -78,29 +73,56 @@ __global__ void __launch_bounds__(kBlock)
 // is left partly empty on a small or odd lattice.
 template <bool MULTI, bool KICK>
 __global__ void __launch_bounds__(kFixBlock, kFixPerSm)
-    k_fixed_force(FixedLat L, const __grid_constant__ FixedCoef kc, const FireDev *__restrict__ fd, const FixedDev *fx,
-                  double *partials)
+    k_fixed_force(const __grid_constant__ Lat<double> L, const uint8_t *__restrict__ cls,
+                  const __grid_constant__ FixedCoef kc, unsigned mx, unsigned my, const FireDev *__restrict__ fd, double *partials)
 {
-    if (KICK && !fd->active) return;
-    if (fx->wide || !fx->lively) return;  // k_force_kick_deep does the step
+    if (KICK ? !fd->active : L.go && !*L.go) return;
+    const bool fixed = L.fx->lively && !L.fx->wide;
+    if (MULTI && !fixed) return;  // k_force_kick_deep does the step
     const double hdt = KICK ? 0.5 * fd->dt : 0.0;
-    const int sy = L.Lx, sz = L.Lx * L.Ly;
-    const unsigned P = L.P;
+    const int Lx = L.Lx, Ly = L.Ly, Lz = L.Lz, N = L.N, sy = Lx, sz = Lx * Ly;
+    const unsigned P = (unsigned)L.P;
     double acc[3] = {0.0, 0.0, 0.0};
-    for (int i = blockIdx.x * kFixBlock + threadIdx.x; i < L.N; i += gridDim.x * kFixBlock) {
-        const int c = L.cls[i];
+    auto finish = [&](int i, double(&v)[5], const double(&f)[5]) {
+        if (KICK) {
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                v[k] += hdt * f[k];
+                (L.V + (size_t)k * P)[(unsigned)i] = v[k];
+                (L.F + (size_t)k * P)[(unsigned)i] = f[k];
+            }
+            dot3_acc(f, v, acc);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 5; ++k) (L.F + (size_t)k * P)[(unsigned)i] = f[k];
+        }
+    };
+    for (int i = blockIdx.x * kFixBlock + threadIdx.x; i < N; i += gridDim.x * kFixBlock) {
+        const int c = cls[i];
         if (c != 0) {
             if (!KICK && c == 2)
 #pragma unroll
                 for (int k = 0; k < 5; ++k) (L.F + (size_t)k * P)[(unsigned)i] = 0.0;
             continue;
         }
-        const int r = (int)udiv((unsigned)i, (unsigned)L.Lx, L.mx);
-        const int x = i - r * L.Lx, z = (int)udiv((unsigned)r, (unsigned)L.Ly, L.my), y = r - z * L.Ly;
+        if constexpr (!MULTI) {
+            if (!fixed) {
+                GlobalAcc<double> a(L, i);
+                double f[5], v[5], h[3];
+                site_force_core<double, GlobalAcc<double>, false, false, true>(L, a, 0, f, site_field(L, i, h));
+                if (KICK)
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) v[k] = (L.V + (size_t)k * P)[(unsigned)i];
+                finish(i, v, f);
+                continue;
+            }
+        }
+        const int r = (int)udiv((unsigned)i, (unsigned)Lx, mx);
+        const int x = i - r * Lx, z = (int)udiv((unsigned)r, (unsigned)Ly, my), y = r - z * Ly;
         // neighbour offsets by direction, -1 and +1
-        const int ox[3] = {x == 0 ? L.Lx - 1 : -1, 0, x == L.Lx - 1 ? 1 - L.Lx : 1};
-        const int oy[3] = {y == 0 ? sz - sy : -sy, 0, y == L.Ly - 1 ? sy - sz : sy};
-        const int oz[3] = {z == 0 ? L.N - sz : -sz, 0, z == L.Lz - 1 ? sz - L.N : sz};
+        const int ox[3] = {x == 0 ? Lx - 1 : -1, 0, x == Lx - 1 ? 1 - Lx : 1};
+        const int oy[3] = {y == 0 ? sz - sy : -sy, 0, y == Ly - 1 ? sy - sz : sy};
+        const int oz[3] = {z == 0 ? N - sz : -sz, 0, z == Lz - 1 ? sz - N : sz};
         auto at = [&](int dx, int dy, int dz, int k) {
             return __ldg(L.X + (size_t)k * P + (unsigned)(i + ox[dx + 1] + oy[dy + 1] + oz[dz + 1]));
         };
@@ -116,18 +138,7 @@ __global__ void __launch_bounds__(kFixBlock, kFixPerSm)
         fixed_force<MULTI>(kc, q, lam, ax, m2, m3, a);
         double f[5];
         fixed_to_force(kc, a, f);
-        if (KICK) {
-#pragma unroll
-            for (int k = 0; k < 5; ++k) {
-                v[k] += hdt * f[k];
-                (L.V + (size_t)k * P)[(unsigned)i] = v[k];
-                (L.F + (size_t)k * P)[(unsigned)i] = f[k];
-            }
-            dot3_acc(f, v, acc);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 5; ++k) (L.F + (size_t)k * P)[(unsigned)i] = f[k];
-        }
+        finish(i, v, f);
     }
     if (KICK) {
         block_sum<3, kFixBlock>(acc);
@@ -149,9 +160,9 @@ template <bool MULTI>
 static void launch_fixed(const Lat<double> &L, const uint8_t *cls, const FireDev *fd, double *partials, int grid,
                          cudaStream_t s)
 {
-    const FixedLat fl{L.Lx, L.Ly, L.Lz, L.N, (unsigned)L.P, div_magic(L.Lx), div_magic(L.Ly), L.X, L.V, L.F, cls};
-    if (fd) k_fixed_force<MULTI, true><<<grid, kFixBlock, 0, s>>>(fl, *L.fixed, fd, L.fx, partials);
-    else k_fixed_force<MULTI, false><<<grid, kFixBlock, 0, s>>>(fl, *L.fixed, nullptr, L.fx, nullptr);
+    const unsigned mx = div_magic(L.Lx), my = div_magic(L.Ly);  // multipliers of udiv
+    if (fd) k_fixed_force<MULTI, true><<<grid, kFixBlock, 0, s>>>(L, cls, *L.fixed, mx, my, fd, partials);
+    else k_fixed_force<MULTI, false><<<grid, kFixBlock, 0, s>>>(L, cls, *L.fixed, mx, my, nullptr, nullptr);
 }
 
 int launch_fixed_force(const Lat<double> &L, const uint8_t *cls, const FireDev *fd, double *partials, cudaStream_t s)

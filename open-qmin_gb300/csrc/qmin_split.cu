@@ -85,11 +85,11 @@ void launch_high(void (*kern)(P...), int grid, cudaStream_t s, A &&...args)
 }  // namespace
 
 // every deep bulk site (cls == 0); partials[0 .. gridDim.x).  KICK = false:
-// forces only (no FIRE state), object sites' forces set to zero.  ONE: the
-// one-constant form.  fx (may be null): the fixed-point force ran where the
+// forces only (no FIRE state), object sites' forces set to zero.  fx (may be
+// null): the fixed-point force ran where the
 // lattice is inside its range; nparts (with fx): its partials, the entries past
 // this grid set to zero.
-template <class T, int CAP, bool KICK = true, bool ONE = false>
+template <class T, int CAP, bool KICK = true>
 __global__ void __launch_bounds__(kBlock, CAP + 1)
     k_force_kick_deep(Lat<T> L, const uint8_t *__restrict__ cls, const FireDev *__restrict__ fd, const FixedDev *fx,
                       double *partials, int nparts = 0)
@@ -107,13 +107,7 @@ __global__ void __launch_bounds__(kBlock, CAP + 1)
             for (int k = 0; k < 5; ++k) L.F[k * L.P + i] = T(0);
         if (c != 0) continue;
         T f[5];
-        if constexpr (ONE) {
-            GlobalAcc<T> a(L, i);
-            T h[3];
-            site_force_core<T, GlobalAcc<T>, false, false, true>(L, a, 0, f, site_field(L, i, h));
-        } else {
-            deep_force(L, i, f);
-        }
+        deep_force(L, i, f);
         if constexpr (KICK) {
             kick_and_sum(L, i, hdt, f, acc);
         } else {
@@ -1450,10 +1444,9 @@ int launch_split_deep(const Lat<T> &L, const SplitLists &sl, FireDev *fd, double
     }
     if constexpr (sizeof(T) == 8)
         if (L.fixed && cap == 0) {
-            // one of the two does the step, the other returns at once
+            // multi-constant: one of the two does the step, the other returns at once
             const int g = launch_fixed_force(L, sl.cls, fd, partials, s), gw = std::min(g, kDeepWideGrid);
             if (L.multi) k_force_kick_deep<T, 1><<<gw, kBlock, 0, s>>>(L, sl.cls, fd, L.fx, partials, g);
-            else k_force_kick_deep<T, 1, true, true><<<gw, kBlock, 0, s>>>(L, sl.cls, fd, L.fx, partials, g);
             return g;
         }
     if (!L.multi) return -1;
@@ -1512,10 +1505,10 @@ template <class T> int launch_split_force(const Lat<T> &L, int grid, cudaStream_
             cudaMemsetAsync(fx, 0, sizeof(FixedDev), s);
             n += launch_fixed_pred(L, nullptr, s);
             grid = std::min(launch_fixed_force(L, sl.cls, nullptr, nullptr, s), kDeepWideGrid);
-            ++n;
+            n += L.multi;
         }
+        // one-constant lattices come here with a fixed-point form only (launch_force)
         if (L.multi) k_force_kick_deep<T, 1, false><<<grid, kBlock, 0, s>>>(L, sl.cls, nullptr, fx, nullptr);
-        else k_force_kick_deep<T, 1, false, true><<<grid, kBlock, 0, s>>>(L, sl.cls, nullptr, fx, nullptr);
     }
     ++n;
     if (sl.n_sites > 0 && L.fork) cudaStreamWaitEvent(s, L.fork->join, 0);
