@@ -88,9 +88,9 @@ struct FixAcc {
     // hi 2^up + mid 2^(up - 32), 0 < up < 32
     QMIN_DEV long long get(int up) const
     {
-        return (long long)((unsigned long long)hi << up) + (mid >> (32 - up));
+        return (long long)((unsigned long long)hi << up) + (mid >> (32 - up));  // the caller's mid has half a unit
     }
-    QMIN_DEV long long get32() const { return hi + (mid >> 32); }
+    QMIN_DEV long long get32() const { return hi + ((mid + (1LL << 31)) >> 32); }
 };
 
 #ifdef __CUDACC__
@@ -293,15 +293,19 @@ QMIN_DEV void fixed_force(const FixedCoef &k, const long long (&q)[5], const lon
     p03.add(y[0], y[3]);
     const long long h24 = sq[2].hi + sq[4].hi, n24 = sq[2].mid + sq[4].mid;
     const long long h03 = sq[0].hi + sq[3].hi, n03 = sq[0].mid + sq[3].mid;
-    const long long s = (h03 + h24 + sq[1].hi + p03.hi) + ((n03 + n24 + sq[1].mid) >> 31) + (p03.mid >> 32);
+    // every shift rounds to nearest: a floor's half unit would add up over the iterations of a run
+    constexpr long long half = 1LL << 30;
+    const long long s =
+        (h03 + h24 + sq[1].hi + p03.hi) + ((n03 + n24 + sq[1].mid + half) >> 31) + ((p03.mid + 2 * half) >> 32);
     FixAcc g;
-    g.zero();
+    g.hi = 0;
+    g.mid = 1LL << (31 - k.c8up);
     g.add(fix_split(s), k.c8);
     const long long mg = g.get(k.c8up) + k.a2;  // -g2 at 2^(R + 3)
     const Fix2 g2 = fix_split(mg), g4 = fix_split(2 * mg);
     // at 2^58: X0 = q3^2 + q4^2 + w, X3 = q0^2 + q2^2 + w with w = 2 q0 q3 - q1^2; X1 = q1 (q0 + q3) + q2 q4,
     // X2 = q1 q4 - q2 q3, X4 = q1 q2 - q0 q4
-    const long long wh = 2 * p03.hi - sq[1].hi, wm = p03.mid - sq[1].mid;
+    const long long wh = 2 * p03.hi - sq[1].hi, wm = p03.mid - sq[1].mid + half;
     const Fix2 X0 = fix_split(sq[3].hi + sq[4].hi + wh + ((sq[3].mid + sq[4].mid + wm) >> 31));
     const Fix2 X3 = fix_split(sq[0].hi + sq[2].hi + wh + ((sq[0].mid + sq[2].mid + wm) >> 31));
     FixAcc x1, x2, x4, xn;
