@@ -252,6 +252,20 @@ static bool ensure_tmap(qmin_ctx *h)
     return h->tmap_ok;
 }
 
+// the buffers of the fixed-point force; false (nothing allocated) without room
+static bool alloc_fixed(qmin_ctx *h)
+{
+    if (h->X) return true;
+    if (cudaMalloc(&h->X, 5 * (size_t)h->P * sizeof(long long)) != cudaSuccess ||
+        (!h->fx && cudaMalloc(&h->fx, sizeof(FixedDev)) != cudaSuccess)) {
+        cudaGetLastError();
+        if (h->X) cudaFree(h->X);
+        h->X = nullptr;
+        return false;
+    }
+    return true;
+}
+
 // The fixed-point force of the current parameters (FP64 with a form that has
 // one, no spatially varying field) and its buffers; false where there is none
 // or the buffers do not fit, and the FP64 kernels do the work.
@@ -263,16 +277,7 @@ static bool ensure_fixed(qmin_ctx *h, const Lat<double> &L)
     for (int c = 0; c < 5; ++c) field[c] = (L.efield ? L.fE[c] : 0.0) + (L.hfield ? L.fH[c] : 0.0);
     h->kc = fixed_coeffs(h->params, h->metric_mode, L.efield || L.hfield ? field : nullptr);
     if (!h->kc.ok) return false;
-    if (!h->X) {
-        if (cudaMalloc(&h->X, 5 * (size_t)h->P * sizeof(long long)) != cudaSuccess ||
-            (!h->fx && cudaMalloc(&h->fx, sizeof(FixedDev)) != cudaSuccess)) {
-            cudaGetLastError();
-            if (h->X) cudaFree(h->X);
-            h->X = nullptr;
-            return false;
-        }
-    }
-    return true;
+    return alloc_fixed(h);
 }
 
 static int ensure_aux(qmin_ctx *h)
@@ -412,7 +417,10 @@ int qmin_create(const qmin_lattice_desc *desc, qmin_handle *out)
     cudaMemsetAsync(h->types, 0, (size_t)h->P, h->stream);
     memset(h->fire_h, 0, sizeof(FireDev));
     memset(h->iter_h, 0, sizeof(IterDev));
-    if (ensure_aux(h) != QMIN_OK) cudaGetLastError();  // here, so that no first call waits for it
+    // here, so that no first call waits for them: the side stream, and for small FP64 lattices (at most 16 MB),
+    // whose first run is short, the fixed-point force's buffers
+    if (ensure_aux(h) != QMIN_OK) cudaGetLastError();
+    if (h->prec == QMIN_FP64 && 40 * (size_t)h->P <= (16u << 20)) alloc_fixed(h);
     *out = h;
     return QMIN_OK;
 }
