@@ -270,7 +270,7 @@ int qmin_set_fire_variant(qmin_handle h, int variant);
  * ms[3 + 2*cfg + v] fused (4 shapes, v = 0/1 for the two z extents tried),
  * ms[11 + 2*cfg + v] staged (3 shapes), ms[17 + v] split (v = 0, 1: deep
  * sites from global memory at 1 or 2 blocks per SM; v = 0 in FP64: in 64-bit
- * fixed point where |Q| < 3/4 at every site the minimiser moves, with the
+ * fixed point where |Q| < 1 at every site the minimiser moves, with the
  * FP64 form taken for fields outside; v = 2, 3: deep sites
  * from shared-memory tiles of 32 x 8 or 16 x 16 sites; v = 4, 5, FP32
  * only: two x-adjacent sites per thread on 32 x 8 tiles, z chunks of 8

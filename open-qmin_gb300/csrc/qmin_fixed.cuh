@@ -19,7 +19,8 @@
 // of the FP64 evaluation, whose partial sums reach 10 to 30: against 80-bit
 // arithmetic the error of the force is 0.2 to 0.6 of the FP64 form's over
 // random and smooth nematic fields, 0.6 to 0.75 at 0.4 of the nematic order.
-// The sums need every component's |Q| < 3/4 at LC sites, the relative
+// The sums need every component's |Q| < 1 at LC sites (with 3/4, 350 of the
+// first 520 iterations at 200^3 left the range: FIRE overshoots to 0.85), the relative
 // accuracy some |Q| >= 1/8: a lattice outside that takes the FP64 kernel
 // (FixedDev).  QMIN_DEV functions also compile for the host.
 #pragma once
@@ -112,8 +113,8 @@ inline unsigned fix_lo_word(double d)
 #endif
 
 // |d| as the upper word of its bits, ordered like |d|: >= kFixWide for |d| >=
-// 3/4 (Inf and NaN too), >= kFixLively for |d| >= 1/8
-constexpr int kFixWide = 0x3fe80000, kFixLively = 0x3fc00000;
+// 1 (Inf and NaN too), >= kFixLively for |d| >= 1/8
+constexpr int kFixWide = 0x3ff00000, kFixLively = 0x3fc00000;
 QMIN_DEV int fix_magnitude(double d) { return fix_hi_word(d) & 0x7fffffff; }
 
 // d 2^56 towards zero, |d| < 1 (some number for the rest)
@@ -158,7 +159,7 @@ inline FixedCoef fixed_coeffs(const qmin_ldg_params &p, int metric_mode, const d
     const double L2 = p.multi_constant ? p.L2 : 0.0, L3 = p.multi_constant ? p.L3 : 0.0;
     const double a2 = p.A, b3 = p.B, c8 = 2.0 * p.C;  // 2 (A / 2), 3 (B / 3), 8 (C / 4)
     const double lmax = fmax(fabs(p.L1), fmax(fabs(L2 + L3), fmax(fabs(L2), fabs(L3)) / 8));
-    const double gmax = 3.375 * fabs(c8) + fabs(a2);  // |8 c s + 2 a|, s <= 6 (3/4)^2
+    const double gmax = 6 * fabs(c8) + fabs(a2);  // |8 c s + 2 a|, s <= 6
     if (!isfinite(lmax) || !isfinite(gmax) || !isfinite(b3)) return c;
     if (p.multi_constant && (p.L4 != 0.0 || p.L6 != 0.0)) return c;
     auto bits = [](double v) {  // v < 2^bits
@@ -171,13 +172,13 @@ inline FixedCoef fixed_coeffs(const qmin_ldg_params &p, int metric_mode, const d
     int R = 60 - 8 - bits(lmax);
     R = R < 60 - 6 - bits(fabs(b3)) ? R : 60 - 6 - bits(fabs(b3));
     R = R < 60 - 3 - bits(gmax) ? R : 60 - 3 - bits(gmax);
-    // |result| for |Q| < 3/4: 36 L1 and 12 (L2 + L3) from the axis terms, 16 / 8 (|L2| + |L3|) from the face
-    // diagonals, g2 u with |u| <= 9/4, 3 b X with |X| <= 45/16 or 6 b X with |X| <= 27/16, the fields
+    // |result| for |Q| < 1: 36 L1 and 12 (L2 + L3) from the axis terms, 16 / 8 (|L2| + |L3|) from the face
+    // diagonals, g2 u with |u| <= 3, 3 b X with |X| <= 5 or 6 b X with |X| <= 3, the fields
     double fsum = 0.0;
     if (field)
         for (int k = 0; k < 5; ++k) fsum = fmax(fsum, fabs(field[k]));
     const double bound =
-        27 * fabs(p.L1) + 10.5 * (fabs(L2) + fabs(L3)) + 2.25 * gmax + 3.375 * fabs(b3) + 2 * fsum;
+        36 * fabs(p.L1) + 14 * (fabs(L2) + fabs(L3)) + 3 * gmax + 18 * fabs(b3) + 2 * fsum;
     if (!isfinite(bound) || bound == 0.0) return c;
     const int room = 62 - bits(bound);  // R + up
     if (R > room - 1) R = room - 1;

@@ -40,7 +40,7 @@ struct FixedCoef;  // qmin_fixed.cuh
 constexpr int kFixedForceSites = 50000;
 
 // Range of Q over the LC sites, for the fixed-point force: wide, a component
-// at or above 3/4; lively, a component at or above 1/8.  The pass that writes
+// at or above 1; lively, a component at or above 1/8.  The pass that writes
 // Q 2^56 raises them; the force passes after it run in fixed point when
 // lively and not wide, else in FP64.
 struct FixedDev {
