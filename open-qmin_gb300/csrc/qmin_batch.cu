@@ -491,9 +491,20 @@ struct BatchRun {
     int pad;
     long long spin_limit;
     int retired[3];
-    int next[6];  // tile loop: items taken, per iteration modulo 3 and phase
+    int next[6];  // items taken, per iteration modulo 3 and phase
     int pad2;
 };
+
+// The words of the next iteration (slot: its number modulo 3), cleared by one
+// thread of this one.  Their last readers are two iterations back, before a
+// grid barrier every block has passed; their next writers are behind the
+// barrier that ends this iteration.  An iteration's own words are in use from
+// its first statement on: a block that enters it early may retire a solve
+// before the clearing thread has run.
+__device__ __forceinline__ void b_clear_next(BatchRun *run, int slot)
+{
+    run->retired[slot] = run->next[2 * slot] = run->next[2 * slot + 1] = 0;
+}
 
 // grid-wide barrier between two phases; bounded: a block that has waited
 // spin_limit polls raises the abort flag, and every block leaves at its next
@@ -671,10 +682,7 @@ __global__ void __launch_bounds__(kBlock, kFixedPerSm)
     auto count = [&](int s) { return tiles[s].items; };
     b_rebuild(&al, fds, nsolves, count);
     for (int it = 0; al.n > 0; ++it) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            run->retired[it % 3] = 0;
-            run->next[2 * ((it + 1) % 3)] = run->next[2 * ((it + 1) % 3) + 1] = 0;
-        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) b_clear_next(run, (it + 1) % 3);
         for (int w = blockIdx.x; w < al.pre[al.n]; w += gridDim.x) {
             const int e = b_find(al, w), s = al.act[e], k = w - al.pre[e];
             const SolveTile st = tiles[s];
@@ -759,10 +767,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilePerSm)
     if (!b_grid_sync(run)) return;
     const BatchSet<float> s0{B.L.Q, B.L.V, B.L.F};
     for (int it = 0; al.n > 0; ++it) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            run->retired[it % 3] = 0;
-            run->next[2 * ((it + 1) % 3)] = run->next[2 * ((it + 1) % 3) + 1] = 0;
-        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) b_clear_next(run, (it + 1) % 3);
         const BatchSet<float> in = (it & 1) ? s1 : s0, out = (it & 1) ? s0 : s1;
         if (MULTI) {
             for (TileItems q(al, &run->next[2 * (it % 3)]); q.more(al); q.take(sh_w)) {
