@@ -91,7 +91,9 @@ __device__ __forceinline__ bool chunk_site(const BatchArgs<T> &B, const SolveDes
     return chunk_site(B, sd, ch, t, li, x, y, z);
 }
 
-// accessor for a site of a packed solve: neighbours wrap inside that solve's box
+// accessor for a site of a packed solve: neighbours wrap inside that solve's box.
+// Ordinary loads: the persistent loop reads Q and D that it wrote itself an
+// iteration phase before, which the read-only path of ld does not allow.
 template <class T> struct BatchAcc {
     const T *Q;
     const T *D;
@@ -116,9 +118,9 @@ template <class T> struct BatchAcc {
         nb[5] = i + (z == sd.Lz - 1 ? -(sd.Lz - 1) * sy : sy);
     }
     __device__ __forceinline__ int tn(int s) const { return types[nb[s]]; }
-    __device__ __forceinline__ T q(int k) const { return ld(Q + (long long)k * P + i); }
-    __device__ __forceinline__ T nq(int s, int k) const { return ld(Q + (long long)k * P + nb[s]); }
-    __device__ __forceinline__ T dn(int s, int d) const { return ld(D + (long long)d * P + nb[s]); }
+    __device__ __forceinline__ T q(int k) const { return Q[(long long)k * P + i]; }
+    __device__ __forceinline__ T nq(int s, int k) const { return Q[(long long)k * P + nb[s]]; }
+    __device__ __forceinline__ T dn(int s, int d) const { return D[(long long)d * P + nb[s]]; }
     __device__ __forceinline__ ObjDev<T> obj(int t) const { return objs[t - 1]; }
 };
 
@@ -194,7 +196,7 @@ __device__ __forceinline__ void b_derivs_at(const Lat<T> &L, const BatchAcc<T> &
 #pragma unroll
         for (int k = 0; k < 5; ++k)
             L.D[(5 * ax + k) * P + a.i] =
-                deriv2_rule(t, td, tu, ld(L.Q + k * P + dn), ld(L.Q + k * P + a.i), ld(L.Q + k * P + up));
+                deriv2_rule(t, td, tu, L.Q[k * P + dn], L.Q[k * P + a.i], L.Q[k * P + up]);
     }
 }
 
@@ -327,7 +329,7 @@ __device__ __forceinline__ void b_bulk_item(const BatchArgs<double> &B, const Ba
             fixed_force<MULTI>(fx.kc, q, lam, ax, m2, m3, a);
             fixed_to_force(fx.kc, a, f);
         } else if (MULTI) {
-            deep_force_box(B.L, sd.off, sd.Lx, sd.Ly, sd.Lz, li, (long long)gi, f);
+            deep_force_box<double, false>(B.L, sd.off, sd.Lx, sd.Ly, sd.Lz, li, (long long)gi, f);
         } else {
             BatchAcc<double> a(B.L, sd, li, x, y, z);
             site_force_core<double, BatchAcc<double>, false, false, true>(B.L, a, 0, f);

@@ -457,8 +457,9 @@ __device__ __forceinline__ int wrap_near(int v, int m) { return v < 0 ? v + m : 
 // x + Lx (y + Ly z) of a periodic Lx x Ly x Lz box whose planes start at
 // element `base` (0 for a lattice, the solve's offset in a batch); i is its
 // index in the planes.  M is applied as the reference does for type-0 sites
-// (twice in CPU mode, the fields between the two).
-template <class T>
+// (twice in CPU mode, the fields between the two).  READ_ONLY: Q is not written
+// in this launch (ld); otherwise ordinary loads.
+template <class T, bool READ_ONLY = true>
 __device__ __forceinline__ void deep_force_box(const Lat<T> &L, long long base, int Lx, int Ly, int Lz, int li,
                                                long long i, T *f)
 {
@@ -473,7 +474,8 @@ __device__ __forceinline__ void deep_force_box(const Lat<T> &L, long long base, 
     }
     const T *Q = L.Q + base;
     const long long P = L.P;
-#define QQ(dx, dy, dz, c) ld(Q + (long long)(c) * P + (xi[(dx) + 2] + yo[(dy) + 2] + zo[(dz) + 2]))
+    auto get = [](const T *p) { return READ_ONLY ? ld(p) : *p; };
+#define QQ(dx, dy, dz, c) get(Q + (long long)(c) * P + (xi[(dx) + 2] + yo[(dy) + 2] + zo[(dz) + 2]))
     T q[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) q[k] = QQ(0, 0, 0, k);
