@@ -1,0 +1,62 @@
+// Block counts of the tiled bulk kernels and of the list kernels beside them.
+// One iteration's kernels leave one triple of FIRE sums a block in a buffer of
+// kMaxFusedBlocks triples, the bulk kernel's first and the listed sites' behind
+// them, so the two counts have to fit it together.  Host arithmetic only.
+#pragma once
+#include <algorithm>
+
+namespace qmin {
+
+constexpr int kMaxFusedBlocks = 16384;
+
+// Blocks of the list kernels.  A list is short (2 to 10 % of the sites) and a
+// listed site is long (an FP64 one 514 FP64 operations per warp), so the blocks
+// are small enough to reach every SM: at 83 x 61 x 97 with two walls an FP64
+// iteration takes 113 us with 128 threads, 114 with 64 or 32, 120 with 256
+// (87 blocks for 152 SMs); at 200^3 0.959, 0.963, 0.975 and 0.978 ms.
+constexpr int kListBlock = 128, kListPerSm = 8, kMaxListBlocks = 152 * kListPerSm;
+inline int list_grid(int n) { return std::max(1, std::min((n + kListBlock - 1) / kListBlock, kMaxListBlocks)); }
+
+// what a bulk kernel may use of the buffer when listed sites run beside it
+constexpr int kMaxDeepBlocks = kMaxFusedBlocks - kMaxListBlocks;
+
+constexpr int kDeepZc = 8;  // planes of a z chunk of the deep kernels
+
+// tiles of TX x TY columns, cut along z into nz chunks of zc planes
+struct TileGrid {
+    int ntiles, zc, nz;
+    int blocks() const { return ntiles * nz; }
+};
+
+// chunks of zc planes, or more where they would not fit the buffer
+inline TileGrid tile_grid(int ntiles, int Lz, int zc)
+{
+    while ((long long)ntiles * ((Lz + zc - 1) / zc) > kMaxDeepBlocks) ++zc;
+    return TileGrid{ntiles, zc, (Lz + zc - 1) / zc};
+}
+
+inline int tiles_xy(int Lx, int Ly, int TX, int TY) { return ((Lx + TX - 1) / TX) * ((Ly + TY - 1) / TY); }
+
+// planes of a chunk for a grid of about two waves of minb blocks on each of the 152 SMs
+inline int two_waves_zc(int ntiles, int Lz, int minb)
+{
+    const long long nz = std::max(1LL, 2LL * 152 * minb / ntiles);
+    return (int)((Lz + nz - 1) / nz);
+}
+
+// deep kernels: chunks of kDeepZc planes; fitted_minb > 0: about two waves (fewer, longer columns)
+inline TileGrid deep_grid(int Lx, int Ly, int Lz, int TX, int TY, int fitted_minb)
+{
+    const int ntiles = tiles_xy(Lx, Ly, TX, TY);
+    return tile_grid(ntiles, Lz, fitted_minb ? std::max(kDeepZc, two_waves_zc(ntiles, Lz, fitted_minb)) : kDeepZc);
+}
+
+// fused deep kernels: chunks of zc planes; zc = 0: about two waves
+inline TileGrid fused_grid(int Lx, int Ly, int Lz, int TX, int TY, int minb, int zc)
+{
+    const int ntiles = tiles_xy(Lx, Ly, TX, TY);
+    if (zc <= 0) zc = two_waves_zc(ntiles, Lz, minb);
+    return tile_grid(ntiles, Lz, std::max(1, std::min(zc, Lz)));
+}
+
+}  // namespace qmin

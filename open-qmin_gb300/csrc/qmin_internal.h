@@ -10,6 +10,7 @@
 #include "qmin_bulk_forms.h"
 #include "qmin_bulk_q25.h"
 #include "qmin_boundary_forms.h"
+#include "qmin_grids.h"
 
 namespace qmin {
 
@@ -175,7 +176,6 @@ int reduction_grid(int N);
 // fused tiled FIRE iteration (qmin_fused.cu): tile configuration cfg in
 // [0, kFusedConfigs), z planes per block zc; returns launches or -1
 constexpr int kFusedConfigs = 4;
-constexpr int kMaxFusedBlocks = 16384;
 template <class T>
 int launch_fire_fused(int cfg, const Lat<T> &L, T *Qn, T *Vn, T *Fn, FireDev *fd, double *partials, int zc,
                       cudaStream_t s, int *nblocks);

@@ -44,14 +44,6 @@ __device__ __forceinline__ void kick_and_sum(const Lat<T> &L, long long i, T hdt
     }
 }
 
-// Blocks of the list kernels.  A list is short (2 to 10 % of the sites) and a
-// listed site is long (an FP64 one 514 FP64 operations per warp), so the blocks
-// are small enough to reach every SM: at 83 x 61 x 97 with two walls an FP64
-// iteration takes 113 us with 128 threads, 114 with 64 or 32, 120 with 256
-// (87 blocks for 152 SMs); at 200^3 0.959, 0.963, 0.975 and 0.978 ms.
-constexpr int kListBlock = 128, kListPerSm = 8;
-int list_grid(int n) { return std::max(1, std::min((n + kListBlock - 1) / kListBlock, 152 * kListPerSm)); }
-
 // the device's greatest stream priority (the lowest number)
 int high_priority()
 {
@@ -190,7 +182,7 @@ __device__ __forceinline__ int wrap_any(int v, int m)
     int r = v % m;
     return r < 0 ? r + m : r;
 }
-constexpr int kDeepNS = 6, kDeepZc = 8;
+constexpr int kDeepNS = 6;
 template <class T, int TX, int TY> constexpr size_t deep_tiled_smem()
 {
     return (size_t)kDeepNS * 5 * (TX + 4) * (TY + 4) * sizeof(T);
@@ -1247,17 +1239,12 @@ static int launch_deep_tiled(const Lat<T> &L, const SplitLists &sl, FireDev *fd,
         attr_set = cudaFuncSetAttribute(k_force_kick_deep_tiled<T, TX, TY>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess;
     }
-    const int ntiles = ((L.Lx + TX - 1) / TX) * ((L.Ly + TY - 1) / TY);
-    int zc = kDeepZc;
-    while ((long long)ntiles * ((L.Lz + zc - 1) / zc) > kMaxFusedBlocks - 1024) ++zc;
-    const int nz = (L.Lz + zc - 1) / zc;
-    k_force_kick_deep_tiled<T, TX, TY><<<dim3(ntiles, nz), TX * TY, sm, s>>>(L, sl.cls, fd, partials, zc);
-    return ntiles * nz;
+    const TileGrid g = deep_grid(L.Lx, L.Ly, L.Lz, TX, TY, 0);
+    k_force_kick_deep_tiled<T, TX, TY><<<dim3(g.ntiles, g.nz), TX * TY, sm, s>>>(L, sl.cls, fd, partials, g.zc);
+    return g.blocks();
 }
 
 // the FP32 two-sites-per-thread deep kernel over TX x TY columns
-// fitted = true: z chunks sized so that the grid is about two waves of MINB
-// blocks on each of the 152 SMs (fewer, longer columns), else kDeepZc planes
 template <int TX, int TY, int MINB, bool KICK = true>
 static int launch_deep_pair(const Lat<float> &L, const SplitLists &sl, FireDev *fd, double *partials, bool fitted,
                             cudaStream_t s)
@@ -1269,17 +1256,9 @@ static int launch_deep_pair(const Lat<float> &L, const SplitLists &sl, FireDev *
         attr_set = cudaFuncSetAttribute(k_force_kick_deep_pair<TX, TY, MINB, KICK>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess;
     }
-    const int ntiles = ((L.Lx + TX - 1) / TX) * ((L.Ly + TY - 1) / TY);
-    int zc = kDeepZc;
-    if (fitted) {
-        // about two waves: each block walks a long column
-        const long long nz = std::max(1LL, 2LL * 152 * MINB / ntiles);
-        zc = std::max(kDeepZc, (int)((L.Lz + nz - 1) / nz));
-    }
-    while ((long long)ntiles * ((L.Lz + zc - 1) / zc) > kMaxFusedBlocks - 1024) ++zc;
-    const int nz = (L.Lz + zc - 1) / zc;
-    k_force_kick_deep_pair<TX, TY, MINB, KICK><<<dim3(ntiles, nz), TX / 2 * TY, sm, s>>>(L, sl.cls, fd, partials, zc);
-    return ntiles * nz;
+    const TileGrid g = deep_grid(L.Lx, L.Ly, L.Lz, TX, TY, fitted ? MINB : 0);
+    k_force_kick_deep_pair<TX, TY, MINB, KICK><<<dim3(g.ntiles, g.nz), TX / 2 * TY, sm, s>>>(L, sl.cls, fd, partials, g.zc);
+    return g.blocks();
 }
 
 // the TMA-staged two-sites-per-thread kernel (FP32, z chunks of about two
@@ -1296,31 +1275,10 @@ static int launch_deep_pair_tma(const Lat<float> &L, const SplitLists &sl, FireD
         attr_set = cudaFuncSetAttribute(k_force_kick_deep_pair_tma<TX, TY, MINB, KICK>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess;
     }
-    const int ntiles = ((L.Lx + TX - 1) / TX) * ((L.Ly + TY - 1) / TY);
-    const long long nzt = std::max(1LL, 2LL * 152 * MINB / ntiles);
-    int zc = std::max(kDeepZc, (int)((L.Lz + nzt - 1) / nzt));
-    while ((long long)ntiles * ((L.Lz + zc - 1) / zc) > kMaxFusedBlocks - 1024) ++zc;
-    const int nz = (L.Lz + zc - 1) / zc;
+    const TileGrid g = deep_grid(L.Lx, L.Ly, L.Lz, TX, TY, MINB);
     k_force_kick_deep_pair_tma<TX, TY, MINB, KICK>
-        <<<dim3(ntiles, nz), TX / 2 * TY, sm, s>>>(L, *sl.tmap_q, sl.cls, fd, partials, zc, sl.err);
-    return ntiles * nz;
-}
-
-// grid of the fused deep kernels over TX x TY columns; zc > 0: z chunks of zc
-// planes, zc = 0: chunks long enough that the grid is about two waves of
-// MINB blocks on each of the 152 SMs
-static inline void fused_grid(int Lx, int Ly, int Lz, int TX, int TY, int MINB, int zc, int &ntiles, int &zc_out,
-                              int &nz)
-{
-    ntiles = ((Lx + TX - 1) / TX) * ((Ly + TY - 1) / TY);
-    if (zc <= 0) {
-        const long long nzt = std::max(1LL, 2LL * 152 * MINB / ntiles);
-        zc = (int)((Lz + nzt - 1) / nzt);
-    }
-    zc = std::max(1, std::min(zc, Lz));
-    while ((long long)ntiles * ((Lz + zc - 1) / zc) > kMaxFusedBlocks - 1024) ++zc;
-    zc_out = zc;
-    nz = (Lz + zc - 1) / zc;
+        <<<dim3(g.ntiles, g.nz), TX / 2 * TY, sm, s>>>(L, *sl.tmap_q, sl.cls, fd, partials, g.zc, sl.err);
+    return g.blocks();
 }
 
 template <class T, int TX, int TY, int MINB, bool MULTI>
@@ -1334,10 +1292,10 @@ static int launch_fused_deep(const Lat<T> &L, T *Qo, T *Vo, T *Fo, const SplitLi
         attr_set = cudaFuncSetAttribute(k_fire_deep_fused<T, TX, TY, MINB, MULTI>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess;
     }
-    int ntiles, nz;
-    fused_grid(L.Lx, L.Ly, L.Lz, TX, TY, MINB, zc, ntiles, zc, nz);
-    k_fire_deep_fused<T, TX, TY, MINB, MULTI><<<dim3(ntiles, nz), TX * TY, sm, s>>>(L, Qo, Vo, Fo, sl.cls, fd, partials, zc);
-    return ntiles * nz;
+    const TileGrid g = fused_grid(L.Lx, L.Ly, L.Lz, TX, TY, MINB, zc);
+    k_fire_deep_fused<T, TX, TY, MINB, MULTI>
+        <<<dim3(g.ntiles, g.nz), TX * TY, sm, s>>>(L, Qo, Vo, Fo, sl.cls, fd, partials, g.zc);
+    return g.blocks();
 }
 
 template <class T, int TX, int TY, int MINB>
@@ -1351,11 +1309,10 @@ static int launch_fused_deep_cp(const Lat<T> &L, T *Qo, T *Vo, T *Fo, const Spli
         attr_set = cudaFuncSetAttribute(k_fire_deep_fused_cp<T, TX, TY, MINB>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess;
     }
-    int ntiles, nz;
-    fused_grid(L.Lx, L.Ly, L.Lz, TX, TY, MINB, zc, ntiles, zc, nz);
+    const TileGrid g = fused_grid(L.Lx, L.Ly, L.Lz, TX, TY, MINB, zc);
     k_fire_deep_fused_cp<T, TX, TY, MINB>
-        <<<dim3(ntiles, nz), TX * TY, sm, s>>>(L, Qo, Vo, Fo, sl.cls, fd, partials, zc);
-    return ntiles * nz;
+        <<<dim3(g.ntiles, g.nz), TX * TY, sm, s>>>(L, Qo, Vo, Fo, sl.cls, fd, partials, g.zc);
+    return g.blocks();
 }
 
 // Fused split iteration, deep part: variant 0 = 32 x 8 tiles, z chunks of 16;
