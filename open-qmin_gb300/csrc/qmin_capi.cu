@@ -399,7 +399,7 @@ int qmin_create(const qmin_lattice_desc *desc, qmin_handle *out)
     size_t plane = (size_t)h->P * h->esz;
     bool ok = cudaMalloc(&h->Q, 5 * plane) == cudaSuccess && cudaMalloc(&h->V, 5 * plane) == cudaSuccess &&
               cudaMalloc(&h->F, 5 * plane) == cudaSuccess && cudaMalloc(&h->types, (size_t)h->P) == cudaSuccess &&
-              cudaMalloc(&h->partials, sizeof(double) * std::max(8 * (size_t)h->grid, (size_t)3 * kMaxFusedBlocks)) == cudaSuccess &&
+              cudaMalloc(&h->partials, sizeof(double) * std::max(8 * (size_t)h->grid, 3 * (size_t)sum_blocks(h->Lx, h->Ly))) == cudaSuccess &&
               cudaMalloc(&h->fire, sizeof(FireDev)) == cudaSuccess &&
               cudaMalloc(&h->iter, sizeof(IterDev)) == cudaSuccess &&
               cudaMalloc(&h->out5, sizeof(double) * 8) == cudaSuccess &&
@@ -1114,8 +1114,7 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
             tiled_tile_shape(cfg, &tx, &ty);
             const int ntiles = ((h->Lx + tx - 1) / tx) * ((h->Ly + ty - 1) / ty);
             // short z chunks: many blocks per SM over the launch keep the last wave small
-            int zc0 = 4;
-            while ((long long)ntiles * ((h->Lz + zc0 - 1) / zc0) > kMaxFusedBlocks) ++zc0;
+            const int zc0 = tile_grid(ntiles, h->Lz, 4, kMaxFusedBlocks).zc;
             for (int v = 0; v < 2; ++v) {
                 const int zc = std::min(h->Lz, zc0 << v);
                 int nb = 0, ok = 1;

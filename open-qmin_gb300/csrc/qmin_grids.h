@@ -1,6 +1,6 @@
 // Block counts of the tiled bulk kernels and of the list kernels beside them.
 // One iteration's kernels leave one triple of FIRE sums a block in a buffer of
-// kMaxFusedBlocks triples, the bulk kernel's first and the listed sites' behind
+// sum_blocks triples, the bulk kernel's first and the listed sites' behind
 // them, so the two counts have to fit it together.  Host arithmetic only.
 #pragma once
 #include <algorithm>
@@ -28,14 +28,19 @@ struct TileGrid {
     int blocks() const { return ntiles * nz; }
 };
 
-// chunks of zc planes, or more where they would not fit the buffer
-inline TileGrid tile_grid(int ntiles, int Lz, int zc)
+inline int tiles_xy(int Lx, int Ly, int TX, int TY) { return ((Lx + TX - 1) / TX) * ((Ly + TY - 1) / TY); }
+
+// chunks of zc planes, or more where they would come to over `most` blocks (at
+// worst one chunk: a box may have more tiles than that)
+inline TileGrid tile_grid(int ntiles, int Lz, int zc, int most = kMaxDeepBlocks)
 {
-    while ((long long)ntiles * ((Lz + zc - 1) / zc) > kMaxDeepBlocks) ++zc;
+    while (zc < Lz && (long long)ntiles * ((Lz + zc - 1) / zc) > most) ++zc;
     return TileGrid{ntiles, zc, (Lz + zc - 1) / zc};
 }
 
-inline int tiles_xy(int Lx, int Ly, int TX, int TY) { return ((Lx + TX - 1) / TX) * ((Ly + TY - 1) / TY); }
+// triples of the buffer: kMaxFusedBlocks, or what one chunk of the smallest
+// tiles needs (none is smaller than 16 x 4)
+inline int sum_blocks(int Lx, int Ly) { return std::max(kMaxFusedBlocks, tiles_xy(Lx, Ly, 16, 4) + kMaxListBlocks); }
 
 // planes of a chunk for a grid of about two waves of minb blocks on each of the 152 SMs
 inline int two_waves_zc(int ntiles, int Lz, int minb)

@@ -56,3 +56,35 @@ def test_sums_of_bulk_and_listed_blocks_fit(tmp_path):
     assert r.returncode == 0, r.stderr
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout
+
+
+WIDE = r"""
+#include <cstdio>
+#include "qmin_grids.h"
+using namespace qmin;
+int main()
+{
+    const int box[][3] = {{2048, 2048, 3}, {4096, 4096, 3}, {20000, 20000, 3}, {300000, 3, 3}, {3, 150000000, 3}, {7000, 11, 9}};
+    for (const auto &b : box) {
+        const int x = b[0], y = b[1], z = b[2];
+        const TileGrid g[] = {deep_grid(x, y, z, 32, 8, 0),     deep_grid(x, y, z, 16, 16, 0),
+                              deep_grid(x, y, z, 32, 8, 3),     fused_grid(x, y, z, 32, 8, 2, 16),
+                              fused_grid(x, y, z, 32, 4, 4, 0), tile_grid(tiles_xy(x, y, 16, 16), z, 4, kMaxFusedBlocks)};
+        for (const TileGrid &t : g)
+            if (t.blocks() < t.ntiles || t.blocks() + kMaxListBlocks > sum_blocks(x, y) + (&t == g + 5 ? kMaxListBlocks : 0) ||
+                (long long)t.nz * t.zc < z)
+                return printf("%d x %d x %d: %d blocks\n", x, y, z, t.blocks()), 1;
+    }
+    return sum_blocks(512, 512) != kMaxFusedBlocks;
+}
+"""
+
+
+def test_boxes_of_more_tiles_than_the_usual_buffer(tmp_path):
+    src, exe = tmp_path / "wide.cpp", tmp_path / "wide"
+    src.write_text(WIDE)
+    csrc = os.path.join(ROOT, "open-qmin_gb300", "csrc")
+    r = subprocess.run(["g++", "-std=c++17", "-O2", "-I", csrc, str(src), "-o", str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout
