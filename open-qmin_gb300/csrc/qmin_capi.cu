@@ -84,8 +84,7 @@ struct qmin_ctx {
     int32_t *stage_t = nullptr;
     FireDev *fire = nullptr;
     FireDev *fire_h = nullptr;  // pinned mirror
-    // fixed-point force (FP64): Q 2^56, range flags, coefficients of the current parameters
-    long long *X = nullptr;
+    // fixed-point force (FP64): range flags, coefficients of the current parameters (Q 2^56 is in stage)
     FixedDev *fx = nullptr;
     FixedCoef kc{};
     IterDev *iter = nullptr;
@@ -252,18 +251,27 @@ static bool ensure_tmap(qmin_ctx *h)
     return h->tmap_ok;
 }
 
-// the buffers of the fixed-point force; false (nothing allocated) without room
+// the staging buffer of uploads and read-backs: 5 planes of doubles, in use only within such a call
+static bool alloc_stage(qmin_ctx *h)
+{
+    if (h->stage) return true;
+    if (cudaMalloc(&h->stage, sizeof(double) * 5 * (size_t)h->P) == cudaSuccess) return true;
+    cudaGetLastError();
+    h->stage = nullptr;
+    return false;
+}
+
+// The buffers of the fixed-point force; false without room.  Q 2^56 goes into
+// the staging buffer, which an upload has allocated: every force pass writes it
+// afresh, on the stream that the uploads and read-backs are on.
 static bool alloc_fixed(qmin_ctx *h)
 {
-    if (h->X) return true;
-    if (cudaMalloc(&h->X, 5 * (size_t)h->P * sizeof(long long)) != cudaSuccess ||
-        (!h->fx && cudaMalloc(&h->fx, sizeof(FixedDev)) != cudaSuccess)) {
+    if (!h->fx && cudaMalloc(&h->fx, sizeof(FixedDev)) != cudaSuccess) {
         cudaGetLastError();
-        if (h->X) cudaFree(h->X);
-        h->X = nullptr;
+        h->fx = nullptr;
         return false;
     }
-    return true;
+    return alloc_stage(h);
 }
 
 // The fixed-point force of the current parameters (FP64 with a form that has
@@ -321,7 +329,7 @@ template <class T> static Lat<T> make_lat(qmin_ctx *h, bool fire = false)
     }
     if constexpr (sizeof(T) == 8)
         if ((fire || h->N >= kFixedForceSites) && ensure_fixed(h, L)) {
-            L.X = h->X;
+            L.X = (long long *)h->stage;
             L.fx = h->fx;
             L.fixed = &h->kc;
         }
@@ -335,7 +343,7 @@ static void free_ctx(qmin_ctx *h)
     void *bufs[] = {h->Q, h->V, h->F, h->D, h->types, h->objs, h->partials, h->stage, h->stage_t, h->fire, h->iter,
                     h->out5, h->M, h->S, h->alt, h->lbp, h->lbs, h->lby, h->lbg, h->Q2, h->V2, h->F2, h->hvar,
                     h->split_cls, h->split_sites, h->split_derivs, h->cbd, h->dev_err, h->geo_scratch,
-                    h->scan_part, h->scan_out, h->X, h->fx};
+                    h->scan_part, h->scan_out, h->fx};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (h->fire_h) cudaFreeHost(h->fire_h);
@@ -417,10 +425,6 @@ int qmin_create(const qmin_lattice_desc *desc, qmin_handle *out)
     cudaMemsetAsync(h->types, 0, (size_t)h->P, h->stream);
     memset(h->fire_h, 0, sizeof(FireDev));
     memset(h->iter_h, 0, sizeof(IterDev));
-    // here, so that no first call waits for them: the side stream, and for small FP64 lattices (at most 16 MB),
-    // whose first run is short, the fixed-point force's buffers
-    if (ensure_aux(h) != QMIN_OK) cudaGetLastError();
-    if (h->prec == QMIN_FP64 && 40 * (size_t)h->P <= (16u << 20)) alloc_fixed(h);
     *out = h;
     return QMIN_OK;
 }
@@ -513,12 +517,11 @@ int qmin_set_objects(qmin_handle h, const qmin_object *objs, int n)
 
 static int ensure_stage(qmin_ctx *h)
 {
-    if (!h->stage) {
-        if (cudaMalloc(&h->stage, sizeof(double) * 5 * (size_t)h->N) != cudaSuccess ||
-            cudaMalloc(&h->stage_t, sizeof(int32_t) * (size_t)h->N) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(QMIN_ENOMEM, "staging buffer allocation failed");
-        }
+    if (!alloc_stage(h)) return fail(QMIN_ENOMEM, "staging buffer allocation failed");
+    if (!h->stage_t && cudaMalloc(&h->stage_t, sizeof(int32_t) * (size_t)h->N) != cudaSuccess) {
+        cudaGetLastError();
+        h->stage_t = nullptr;
+        return fail(QMIN_ENOMEM, "staging buffer allocation failed");
     }
     return QMIN_OK;
 }
