@@ -138,6 +138,17 @@ static bool split_variant_ok(const qmin_ctx *h, int cap)
     return true;
 }
 
+// whether this handle can launch split variant cap on L: one-constant lattices
+// have the FP64 fixed-point variant, where the form is there (L.fixed), and the
+// first three fused FP32 ones
+template <class T> static bool split_usable(const qmin_ctx *h, const Lat<T> &L, int cap)
+{
+    if (cap < 0 || cap >= kSplitVariants || !h->split_cls || (L.multi && L.L6 != T(0))) return false;
+    if (!split_variant_ok(h, cap) || (cap == kSplitTma && !h->tmap_ok)) return false;
+    if (L.multi) return true;
+    return sizeof(T) == 8 ? cap == 0 && L.fixed : split_fused(cap) && cap < kSplitFusedFirst + 3;
+}
+
 static const int kChunk = 32;  // iterations per captured graph
 
 namespace qmin {
@@ -944,7 +955,7 @@ struct TuneChoice {
 static std::mutex g_tune_mutex;
 static std::vector<std::pair<TuneKey, TuneChoice>> g_tune_cache;
 
-static TuneKey tune_key(const qmin_ctx *h)
+static TuneKey tune_key(const qmin_ctx *h, bool fixed)
 {
     TuneKey k;
     memset(&k, 0, sizeof k);  // padding included: the key is compared bytewise
@@ -960,7 +971,7 @@ static TuneKey tune_key(const qmin_ctx *h)
     k.mode = h->fire_mode;
     k.variant = h->fire_variant;
     k.tmap = h->tmap_ok;
-    k.fixed = h->prec == QMIN_FP64 && h->kc.ok;
+    k.fixed = fixed;
     k.nTotal = h->nTotal;
     k.n_sites = h->n_split_sites;
     k.n_derivs = h->n_split_derivs;
@@ -980,7 +991,7 @@ static TuneKey tune_key(const qmin_ctx *h)
 template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
 {
     // a strategy restored from a checkpoint that this handle cannot launch is tuned afresh
-    if (h->path == 3 && h->split_cap == kSplitTma && !h->tmap_ok) h->path = -1;
+    if (h->path == 3 && !split_usable(h, L, h->split_cap)) h->path = -1;
     if (h->path >= 0 && h->tuned_version == h->version && h->tuned_mode == h->fire_mode &&
         h->tuned_variant == h->fire_variant)
         return QMIN_OK;
@@ -988,7 +999,7 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
     auto pinned_out = [&](int v) { return h->fire_variant >= 0 && v != h->fire_variant; };
     int r = ensure_pingpong(h);
     if (r) return r;
-    const TuneKey key = tune_key(h);
+    const TuneKey key = tune_key(h, L.fixed != nullptr);
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         for (const auto &e : g_tune_cache)
@@ -1076,9 +1087,7 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
                 }
             const float t_dl = timed([&]() { return launch_split_derivs<T>(L, sl, h->fire, h->stream); }, kNoBudget);
             for (int cap = 0; cap < kSplitFusedFirst; ++cap) {
-                if (pinned_out(cap) || (sizeof(T) == 8 && cap >= kSplitFp32First)) continue;
-                if (cap == kSplitTma && !h->tmap_ok) continue;
-                if (!L.multi && cap >= 1) continue;
+                if (pinned_out(cap) || !split_usable(h, L, cap)) continue;
                 const float t_pred = L.fixed && cap == 0 ? t_fixed : t_plain;
                 int np = 0;
                 const float t_fk = timed(
@@ -1147,8 +1156,7 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
     // the second buffer set, the derivative planes and the partials (timed after
     // the velocities above are restored from the second set)
     for (int cap = kSplitFusedFirst; try_split && cap < kSplitVariants; ++cap) {
-        if (pinned_out(cap) || !split_variant_ok(h, cap)) continue;
-        if (!L.multi && (sizeof(T) == 8 || cap >= kSplitFusedFirst + 3)) continue;
+        if (pinned_out(cap) || !split_usable(h, L, cap)) continue;
         const SplitLists sl = split_lists(h);
         const float ms = timed(
             [&]() {
@@ -1233,6 +1241,7 @@ template <class T> static int fire_impl(qmin_ctx *h, int max_iterations)
     LB.V = (T *)h->V2;
     LB.F = (T *)h->F2;
     int parity = 0;
+    bool launched = true;  // every bulk kernel of the split path had a form for this lattice
     const int variant = h->path == 0 ? h->sep_cap
                         : h->path == 1 ? h->fused_cfg
                         : h->path == 2 ? h->tiled_cfg
@@ -1262,7 +1271,8 @@ template <class T> static int fire_impl(qmin_ctx *h, int max_iterations)
                                                       h->split_cap - kSplitFusedFirst, h->stream);
             n = 1;
             int nl = 0;
-            if (listed) {
+            launched = launched && nd >= 0;
+            if (listed && nd >= 0) {
                 n += launch_split_fused_list<T>(Lin, Vo, Fo, sl, h->fire, h->partials + 3 * nd, h->aux, &nl);
                 cudaEventRecord(h->ev_join, h->aux);
                 cudaStreamWaitEvent(h->stream, h->ev_join, 0);
@@ -1284,7 +1294,8 @@ template <class T> static int fire_impl(qmin_ctx *h, int max_iterations)
             const int nd = launch_split_deep<T>(L, sl, h->fire, h->partials, h->grid, h->split_cap, h->stream);
             n += 1 + (fixed && L.multi);
             int nl = 0;
-            if (listed) {
+            launched = launched && nd >= 0;
+            if (listed && nd >= 0) {
                 n += launch_split_derivs<T>(L, sl, h->fire, h->aux);
                 nl = launch_split_list<T>(L, sl, h->fire, h->partials + 3 * nd, h->aux);
                 n += 1;
@@ -1312,6 +1323,10 @@ template <class T> static int fire_impl(qmin_ctx *h, int max_iterations)
         return n;
     });
     if (r) return r;
+    if (!launched) {
+        invalidate_graphs(h);
+        return fail(QMIN_ECUDA, "qmin_fire_run: the chosen strategy has no kernel for this lattice");
+    }
     int remaining = std::max(max_iterations - it0, 1);
     r = run_chunks(h, 0, h->fire, h->fire_h, (remaining + kChunk - 1) / kChunk + 1);
     if (r) return r;

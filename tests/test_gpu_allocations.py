@@ -32,3 +32,56 @@ def test_fixed_point_force_asks_for_no_planes(qmin, oracle, tmp_path):
         Q, V, F = lat.get_state(V=True, F=True)
         assert rel_err(Q, s.Q) <= 1e-9 and rel_err(F, s.force()) <= 1e-9
     """, tmp_path)
+
+
+def test_no_room_for_the_fixed_point_form(qmin, oracle, tmp_path):
+    """A one-constant FP64 handle without the fixed-point form (the allocation of
+    its flags answers out of memory) runs the FP64 kernels, also after a handle of
+    the same shape has left the fixed-point strategy in the process."""
+    malloc_shim.run("""
+        def system():
+            s = oracle.System((33, 17, 21), Ls=(2.32, 0, 0, 0, 0))
+            s.random_nematic(4)
+            s.add_wall(2, 0, 0, 5.3)
+            return s
+        for room in (True, False, True):
+            s = system()
+            lat = gpu_lattice(qmin, s, qmin.FP64)
+            shim.shim_fail(8, 8, 0, 0 if room else 1000)
+            lat.fire_init()
+            r, ro = lat.fire_run(9), s.fire(9)
+            shim.shim_fail(8, 8, 0, 0)
+            assert lat.fire_tuning()["path"] == ("split" if room else "separate"), (room, lat.fire_tuning())
+            assert abs(r["forceMax"] - ro["forceMax"]) <= 1e-9 * ro["forceMax"]
+            assert rel_err(lat.get_state()[0], s.Q) <= 1e-9
+            lat.close()
+    """, tmp_path)
+
+
+def test_checkpoint_into_a_handle_with_a_field_map(qmin, oracle, tmp_path):
+    """The strategy of a checkpoint that a handle cannot launch (fixed point under
+    a spatially varying field) is tuned afresh."""
+    import numpy as np
+
+    from cases import gpu_lattice, rel_err
+    s = oracle.System((33, 17, 21), Ls=(2.32, 0, 0, 0, 0))
+    s.random_nematic(4)
+    s.add_wall(2, 0, 0, 5.3)
+    a, b = gpu_lattice(qmin, s, qmin.FP64), gpu_lattice(qmin, s, qmin.FP64)
+    H = np.random.default_rng(2).standard_normal((s.N, 3))
+    a.set_field_map(H, 1.0, 1.0, 0.5)
+    a.set_field_map(None, 1.0, 1.0, 0.5)  # off; the field constants are part of a checkpoint
+    a.set_fire_kernel(qmin.FIRE_SPLIT)
+    a.fire_init()
+    a.fire_run(5)
+    assert a.fire_tuning()["path"] == "split"
+    a.checkpoint_save(str(tmp_path / "c"))
+    b.set_field_map(H, 1.0, 1.0, 0.5)
+    b.checkpoint_load(str(tmp_path / "c"))
+    s.fire(5)
+    s.set_field_map(H, 1.0, 1.0, 0.5)
+    b.fire_init()
+    r, ro = b.fire_run(9), s.fire(9)
+    assert b.fire_tuning()["path"] == "separate"
+    assert abs(r["forceMax"] - ro["forceMax"]) <= 1e-9 * ro["forceMax"]
+    assert rel_err(b.get_state()[0], s.Q) <= 1e-9
