@@ -1470,12 +1470,14 @@ template <class T> static int batch_fire_impl(qmin_batch_ctx *b, bool *timed_out
     BCK(cudaMemcpyAsync(b->run, &run, sizeof run, cudaMemcpyHostToDevice, b->stream));
     const BatchArgs<T> B = batch_args<T>(b);
     const bool fused = sizeof(T) == 4;
-    if (fused && !b->Q2) {
+    if (fused) {
         // the second state set, on the first FP32 run
         const size_t bytes = 5 * (size_t)b->P * b->esz;
-        if (cudaMalloc(&b->Q2, bytes) != cudaSuccess || cudaMalloc(&b->V2, bytes) != cudaSuccess ||
-            cudaMalloc(&b->F2, bytes) != cudaSuccess ||
-            cudaMalloc(&b->in_second, sizeof(int) * (size_t)b->nsolves) != cudaSuccess) {
+        for (void **p : {&b->Q2, &b->V2, &b->F2})
+            if (!*p && cudaMalloc(p, bytes) != cudaSuccess) *p = nullptr;
+        if (!b->in_second && cudaMalloc(&b->in_second, sizeof(int) * (size_t)b->nsolves) != cudaSuccess)
+            b->in_second = nullptr;
+        if (!b->Q2 || !b->V2 || !b->F2 || !b->in_second) {
             cudaGetLastError();
             return bfail(QMIN_ENOMEM, "qmin_batch_fire_run: second state set allocation failed");
         }

@@ -914,16 +914,16 @@ int qmin_fire_set_state(qmin_handle h, const qmin_fire_state *st)
 
 static int ensure_pingpong(qmin_ctx *h)
 {
-    if (h->Q2) return QMIN_OK;
     const size_t bytes = 5 * (size_t)h->P * h->esz;
-    if (cudaMalloc(&h->Q2, bytes) != cudaSuccess || cudaMalloc(&h->V2, bytes) != cudaSuccess ||
-        cudaMalloc(&h->F2, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(QMIN_ENOMEM, "fused FIRE: second state buffer allocation failed");
+    for (void **p : {&h->Q2, &h->V2, &h->F2}) {
+        if (*p) continue;
+        if (cudaMalloc(p, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            *p = nullptr;
+            return fail(QMIN_ENOMEM, "fused FIRE: second state buffer allocation failed");
+        }
+        CK(cudaMemsetAsync(*p, 0, bytes, h->stream));
     }
-    CK(cudaMemsetAsync(h->Q2, 0, bytes, h->stream));
-    CK(cudaMemsetAsync(h->V2, 0, bytes, h->stream));
-    CK(cudaMemsetAsync(h->F2, 0, bytes, h->stream));
     return QMIN_OK;
 }
 

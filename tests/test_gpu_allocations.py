@@ -85,3 +85,45 @@ def test_checkpoint_into_a_handle_with_a_field_map(qmin, oracle, tmp_path):
     assert b.fire_tuning()["path"] == "separate"
     assert abs(r["forceMax"] - ro["forceMax"]) <= 1e-9 * ro["forceMax"]
     assert rel_err(b.get_state()[0], s.Q) <= 1e-9
+
+
+@pytest.mark.parametrize("precision", ["FP32", "FP64"])
+@pytest.mark.parametrize("passed", [0, 1, 2])
+def test_second_set_that_did_not_fit(qmin, oracle, tmp_path, precision, passed):
+    """A run that found room for only some of the second set's planes answers
+    QMIN_ENOMEM, and so does the next; with room the handle runs as ever."""
+    malloc_shim.run(f"""
+        L, passed, prec = (24, 9, 11), {passed}, qmin.{precision}
+        s = oracle.System(L, Ls=(2.32, 1.0, 0.5, 0, 0))
+        s.random_nematic(4)
+        planes = 5 * (4 if prec == qmin.FP32 else 8) * (s.N + (-s.N) % 32)
+        tol_f, tol_q = (1e-4, 2e-5) if prec == qmin.FP32 else (1e-9, 1e-9)
+        lat = gpu_lattice(qmin, s, prec)
+        for kind in ("lattice", "batch"):
+            if kind == "lattice":
+                run = lambda: (lat.fire_init(), lat.fire_run(7))[1]
+                Q = lambda: lat.get_state()[0]
+            elif prec == qmin.FP32:
+                b = qmin.Batch([L], prec)
+                b.set_params(s.p.A, s.p.B, s.p.C, s.p.L1, s.p.L2, s.p.L3, multi_constant=1)
+                b.set_chunk_shape(0)
+                s.random_nematic(4)
+                b.set_solve(0, s.Q, s.types, [])
+                run = lambda: (b.fire_init(), b.fire_run(7))[1]
+                Q = lambda: b.get_solve(0)
+            else:
+                continue
+            for k in range(2):
+                shim.shim_fail(planes, planes, passed if k == 0 else 0, 100)
+                try:
+                    run()
+                    raise SystemExit("no error")
+                except qmin.QminError as e:
+                    assert e.code == qmin.QMIN_ENOMEM, e
+            shim.shim_fail(planes, planes, 0, 0)
+            r = run()
+            ro = s.fire(7)
+            f = r["forceMax"] if kind == "lattice" else r["forceMax"][0]
+            assert abs(f - ro["forceMax"]) <= tol_f * ro["forceMax"]
+            assert rel_err(Q(), s.Q) <= tol_q
+    """, tmp_path)
