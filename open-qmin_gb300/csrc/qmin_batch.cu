@@ -1061,7 +1061,7 @@ static int classify_solves(qmin_batch_ctx *b)
         int n = multi ? build_split_lists_dev(b->types + sd.off, sd.Lx, sd.Ly, sd.Lz, b->cls + sd.off, b->geo_scratch,
                                             totals, &l.sites, &l.sites_cap, &l.n_sites, &l.derivs, &l.derivs_cap,
                                             &l.n_derivs, b->stream)
-                          : build_boundary_list_dev(b->types + sd.off, sd.Lx * sd.Ly * sd.Lz, b->cls + sd.off,
+                          : build_boundary_list_dev(b->types + sd.off, sd.Lx, sd.Ly, sd.Lz, b->cls + sd.off,
                                                     b->geo_scratch, &l.sites, &l.sites_cap, &l.n_sites, b->stream);
         if (n == -2) {
             cudaGetLastError();

@@ -117,14 +117,18 @@ __global__ void __launch_bounds__(kScanBlock)
         }
         int x, y, z;
         site_xyz(i, Lx, Ly, x, y, z);
-        const int xm = (x == 0 ? Lx - 1 : x - 1) + Lx * (y + Ly * z);
-        const int xp = (x == Lx - 1 ? 0 : x + 1) + Lx * (y + Ly * z);
-        const int ym = x + Lx * ((y == 0 ? Ly - 1 : y - 1) + Ly * z);
-        const int yp = x + Lx * ((y == Ly - 1 ? 0 : y + 1) + Ly * z);
-        const int zm = x + Lx * (y + Ly * (z == 0 ? Lz - 1 : z - 1));
-        const int zp = x + Lx * (y + Ly * (z == Lz - 1 ? 0 : z + 1));
-        const int txm = t8[xm], txp = t8[xp], tym = t8[ym], typ = t8[yp], tzm = t8[zm], tzp = t8[zp];
-        const bool deep = t == 0 && txm == 0 && txp == 0 && tym == 0 && typ == 0 && tzm == 0 && tzp == 0;
+        const int xm = x == 0 ? Lx - 1 : x - 1, xp = x == Lx - 1 ? 0 : x + 1;
+        const int ym = y == 0 ? Ly - 1 : y - 1, yp = y == Ly - 1 ? 0 : y + 1;
+        const int zm = z == 0 ? Lz - 1 : z - 1, zp = z == Lz - 1 ? 0 : z + 1;
+        auto at = [&](int X, int Y, int Z) { return (int)t8[X + Lx * (Y + Ly * Z)]; };
+        const int txm = at(xm, y, z), txp = at(xp, y, z), tym = at(x, ym, z), typ = at(x, yp, z), tzm = at(x, y, zm),
+                  tzp = at(x, y, zp);
+        // deep: no object site in the 19-point stencil (the fixed-point force bounds |Q| at LC sites only).  Beside
+        // six type-0 neighbours a face diagonal is an object's in types that leave its neighbours unmarked.
+        const bool deep = t == 0 && txm == 0 && txp == 0 && tym == 0 && typ == 0 && tzm == 0 && tzp == 0 &&
+                          at(xm, ym, z) <= 0 && at(xm, yp, z) <= 0 && at(xp, ym, z) <= 0 && at(xp, yp, z) <= 0 &&
+                          at(xm, y, zm) <= 0 && at(xm, y, zp) <= 0 && at(xp, y, zm) <= 0 && at(xp, y, zp) <= 0 &&
+                          at(x, ym, zm) <= 0 && at(x, ym, zp) <= 0 && at(x, yp, zm) <= 0 && at(x, yp, zp) <= 0;
         cls[i] = deep ? 0 : 1;
         if (deep) {
             key[i] = kNoBucket;
@@ -273,12 +277,23 @@ int scan_types(const TT *t, const int8_t *old8, int N, int *part, int *out_dev, 
 template int scan_types<int32_t>(const int32_t *, const int8_t *, int, int *, int *, int *, cudaStream_t);
 template int scan_types<int8_t>(const int8_t *, const int8_t *, int, int *, int *, int *, cudaStream_t);
 
-// class (0 type 0, 1 other LC site, 2 object) and key 0 at the class-1 sites
+// class (0 type-0 sites without an object neighbour, 1 other LC sites, 2 objects) and key 0 at the class-1 sites
 __global__ void __launch_bounds__(kScanBlock)
-    k_boundary_classify(const int8_t *__restrict__ t8, int N, uint8_t *cls, uint8_t *key)
+    k_boundary_classify(const int8_t *__restrict__ t8, int Lx, int Ly, int Lz, uint8_t *cls, uint8_t *key)
 {
+    const int N = Lx * Ly * Lz;
     for (int i = blockIdx.x * kScanBlock + threadIdx.x; i < N; i += gridDim.x * kScanBlock) {
-        const int t = t8[i], c = t > 0 ? 2 : (t < 0 ? 1 : 0);
+        const int t = t8[i];
+        int c = t > 0 ? 2 : (t < 0 ? 1 : 0);
+        if (t == 0) {
+            int x, y, z;
+            site_xyz(i, Lx, Ly, x, y, z);
+            auto at = [&](int X, int Y, int Z) { return (int)t8[X + Lx * (Y + Ly * Z)]; };
+            if (at(x == 0 ? Lx - 1 : x - 1, y, z) > 0 || at(x == Lx - 1 ? 0 : x + 1, y, z) > 0 ||
+                at(x, y == 0 ? Ly - 1 : y - 1, z) > 0 || at(x, y == Ly - 1 ? 0 : y + 1, z) > 0 ||
+                at(x, y, z == 0 ? Lz - 1 : z - 1) > 0 || at(x, y, z == Lz - 1 ? 0 : z + 1) > 0)
+                c = 1;
+        }
         cls[i] = (uint8_t)c;
         key[i] = c == 1 ? 0 : kNoBucket;
     }
@@ -315,15 +330,16 @@ static bool ensure_list(int **p, int *cap, int need)
     return true;
 }
 
-int build_boundary_list_dev(const int8_t *t8, int N, uint8_t *cls, void *scratch, int **sites, int *sites_cap,
-                            int *n_sites, cudaStream_t s)
+int build_boundary_list_dev(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch, int **sites,
+                            int *sites_cap, int *n_sites, cudaStream_t s)
 {
+    const int N = Lx * Ly * Lz;
     const int nch = (N + kBucketChunk - 1) / kBucketChunk;
     uint8_t *key = reinterpret_cast<uint8_t *>(scratch);
     int *counts = reinterpret_cast<int *>(reinterpret_cast<uintptr_t>(key + N + 15) & ~(uintptr_t)15),
         *offsets = counts + nch, *total = offsets + nch;
     const int grid = std::max(1, std::min((N + kScanBlock - 1) / kScanBlock, 152 * 8));
-    k_boundary_classify<<<grid, kScanBlock, 0, s>>>(t8, N, cls, key);
+    k_boundary_classify<<<grid, kScanBlock, 0, s>>>(t8, Lx, Ly, Lz, cls, key);
     k_bucket_count<1><<<nch, kScanBlock, 0, s>>>(key, N, counts);
     k_bucket_offsets<1><<<1, 1024, 0, s>>>(counts, nch, offsets, total);
     int n = 0;

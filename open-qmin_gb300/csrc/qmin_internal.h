@@ -213,9 +213,10 @@ int scan_types(const TT *t, const int8_t *old8, int N, int *part, int *out_dev, 
 // cls (N bytes) written, *sites / *derivs grown as needed, host_totals: 29 ints;
 // scratch of split_scratch_bytes(N).  Returns the launch count, < 0 on failure.
 size_t split_scratch_bytes(int N);
-// cls by type (0 type 0, 1 other LC site, 2 object) and the class-1 sites in site order; same scratch and returns
-int build_boundary_list_dev(const int8_t *t8, int N, uint8_t *cls, void *scratch, int **sites, int *sites_cap,
-                            int *n_sites, cudaStream_t s);
+// one-constant classes (0 type 0 without an object neighbour, 1 other LC sites, 2 objects) and the class-1 sites in
+// site order; same scratch and returns
+int build_boundary_list_dev(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch, int **sites,
+                            int *sites_cap, int *n_sites, cudaStream_t s);
 // after build_split_lists_dev, from the same scratch: 1 where a site is in the derivative list
 int launch_need_marks(const void *scratch, int N, uint8_t *need, cudaStream_t s);
 int build_split_lists_dev(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch, int *host_totals,
