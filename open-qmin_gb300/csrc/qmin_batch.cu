@@ -1051,7 +1051,7 @@ static int classify_solves(qmin_batch_ctx *b)
 
     for (int s = 0; s < b->nsolves; ++s) {
         auto &l = b->lists[s];
-        if (l.classified || l.types.empty()) continue;
+        if (l.classified) continue;  // a solve that was never set is all type 0
         const SolveDesc &sd = b->solves_h[s];
         if (!b->geo_scratch && cudaMalloc(&b->geo_scratch, split_scratch_bytes(b->maxN)) != cudaSuccess) {
             cudaGetLastError();
@@ -1286,8 +1286,6 @@ int qmin_batch_create(int nsolves, const int32_t *dims, int precision, int metri
     cudaMemsetAsync(b->V, 0, 5 * plane, b->stream);
     cudaMemsetAsync(b->F, 0, 5 * plane, b->stream);
     cudaMemsetAsync(b->types, 0, (size_t)b->P, b->stream);
-    cudaMemsetAsync(b->cls, 2, (size_t)b->P, b->stream);    // nothing deep until a solve is set
-    cudaMemsetAsync(b->needd, 1, (size_t)b->P, b->stream);  // every derivative until then
     cudaMemsetAsync(b->objs, 0, sizeof(ObjDev<double>) * kObjPerSolve * nsolves, b->stream);
     cudaMemcpyAsync(b->solves, b->solves_h.data(), sizeof(SolveDesc) * nsolves, cudaMemcpyHostToDevice, b->stream);
     cudaMemcpyAsync(b->chunks, b->chunks_h.data(), sizeof(ChunkDesc) * b->nchunks, cudaMemcpyHostToDevice, b->stream);
