@@ -986,8 +986,8 @@ static TuneKey tune_key(const qmin_ctx *h, bool fixed)
 // extents; a candidate whose first launch takes more than twice the best time
 // so far is not timed further.  The timing launches leave the state as it was:
 // the fused kernel writes only the second buffer set and the partials, the
-// predictor is timed on the second buffer set, and the velocities are restored
-// after the force + kick timings (whose forces equal the ones already resident).
+// predictor is timed on the second buffer set, and velocities and forces are
+// restored after the force + kick timings.
 template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
 {
     // a strategy restored from a checkpoint that this handle cannot launch is tuned afresh
@@ -1071,8 +1071,9 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
     if (try_sep || try_tiled || try_split) {
         const float t_plain = timed([&]() { return launch_fire_pred<T>(LB, h->fire, h->stream); }, kNoBudget);
         const size_t bytes = 5 * (size_t)h->P * h->esz;
-        // the force + kick candidates kick V; it is restored afterwards (their forces equal the resident ones)
+        // the force + kick candidates kick V and write F; both are restored afterwards
         CK(cudaMemcpyAsync(h->V2, h->V, bytes, cudaMemcpyDeviceToDevice, h->stream));
+        CK(cudaMemcpyAsync(h->F2, h->F, bytes, cudaMemcpyDeviceToDevice, h->stream));
         if (try_split && (L.multi || L.fixed)) {
             const SplitLists sl = split_lists(h);
             float t_fixed = 0.f;  // the fixed-point predictor pass
@@ -1081,9 +1082,13 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
                     CK(cudaMemsetAsync(h->fx, 0, sizeof(FixedDev), h->stream));
                     t_fixed = timed([&]() { return launch_fixed_pred(LB, h->fire, h->stream); }, kNoBudget);
                     CK(cudaMemcpyAsync(h->V2, h->V, bytes, cudaMemcpyDeviceToDevice, h->stream));
-                    // the force candidates read the resident Q and its range
-                    CK(cudaMemsetAsync(h->fx, 0, sizeof(FixedDev), h->stream));
+                    // the force candidates read the resident Q.  They are timed as inside the range whatever it is
+                    // now: the choice stays for the run and, in the process, for others, and a field that starts
+                    // outside comes in (from noise at 200^3 100 iterations take 92 ms once inside; with the choice made
+                    // outside 286, and 2.90 against 2.87 ms an iteration is what the choice costs outside).
                     h->launches += launch_fixed_pred(L, nullptr, h->stream);
+                    static const FixedDev inside{0, 1};
+                    CK(cudaMemcpyAsync(h->fx, &inside, sizeof inside, cudaMemcpyHostToDevice, h->stream));
                 }
             const float t_dl = timed([&]() { return launch_split_derivs<T>(L, sl, h->fire, h->stream); }, kNoBudget);
             for (int cap = 0; cap < kSplitFusedFirst; ++cap) {
@@ -1151,6 +1156,7 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
             }
         }
         CK(cudaMemcpyAsync(h->V, h->V2, bytes, cudaMemcpyDeviceToDevice, h->stream));
+        CK(cudaMemcpyAsync(h->F, h->F2, bytes, cudaMemcpyDeviceToDevice, h->stream));
     }
     // the fused split variants: the whole iteration but the control, writing only
     // the second buffer set, the derivative planes and the partials (timed after
