@@ -13,7 +13,8 @@
 //     mid += xh yl + xl yh, result hi + mid / 2^32.  The sums of products of
 //     one output share hi and mid, which are put together once;
 //   * every term of an output carries the same scale 2^R, chosen on the host
-//     from the parameters so that no sum can overflow (fixed_coeffs).
+//     from the parameters so that no sum, high or middle, can overflow
+//     (fixed_coeffs).
 //
 // The quantisation of Q (2^-57) and of the products stay below the rounding
 // of the FP64 evaluation, whose partial sums reach 10 to 30: against 80-bit
@@ -183,26 +184,38 @@ inline FixedCoef fixed_coeffs(const qmin_ldg_params &p, int metric_mode, const d
     const int room = 62 - bits(bound);  // R + up
     if (R > room - 1) R = room - 1;
     if (R > 54) R = 54;
-    if (R < 30) return c;
-    int up = room - R;
-    if (up > 8) up = 8;
     auto at = [](double v, int s) { return (long long)llrint(ldexp(v, s)); };
-    c.l1 = fix_split(-at(p.L1, R + 8));
-    c.l1d = fix_split(-at(p.L1, R + 9));
-    c.l23 = fix_split(-at(L2 + L3, R + 8));
-    c.l2 = fix_split(-at(L2, R + 5));
-    c.l3 = fix_split(-at(L3, R + 5));
-    c.b3 = fix_split(at(b3, R + 6));
-    c.b6 = fix_split(-at(b3, R + 7));
-    // 8 c s: s at 2^58 (below 2^60), 8 c at 2^e8 below 2^60, product at 2^(e8 - 6), brought to 2^(R + 3)
-    int e8 = 60 - bits(fabs(c8));
-    if (e8 > R + 8) e8 = R + 8;
-    c.c8up = R + 3 - (e8 - 6);
-    if (c.c8up < 1 || c.c8up > 24) return c;
-    c.c8 = fix_split(-at(c8, e8));
-    c.a2 = -at(a2, R + 3);
-    c.up = up;
-    c.shift = R + up;
+    for (;; --R) {
+        if (R < 30) return c;
+        int up = room - R;
+        if (up > 8) up = 8;
+        c.l1 = fix_split(-at(p.L1, R + 8));
+        c.l1d = fix_split(-at(p.L1, R + 9));
+        c.l23 = fix_split(-at(L2 + L3, R + 8));
+        c.l2 = fix_split(-at(L2, R + 5));
+        c.l3 = fix_split(-at(L3, R + 5));
+        c.b3 = fix_split(at(b3, R + 6));
+        c.b6 = fix_split(-at(b3, R + 7));
+        // 8 c s: s at 2^58 (below 2^60), 8 c at 2^e8 below 2^60, product at 2^(e8 - 6), brought to 2^(R + 3)
+        int e8 = 60 - bits(fabs(c8));
+        if (e8 > R + 8) e8 = R + 8;
+        c.c8up = R + 3 - (e8 - 6);
+        if (c.c8up < 1 || c.c8up > 24) return c;
+        c.c8 = fix_split(-at(c8, e8));
+        c.a2 = -at(a2, R + 3);
+        c.up = up;
+        c.shift = R + up;
+        // The middle sums: a product x y adds at most |xh| |yl| + |xl| |yh|, |yl| <= 2^31.  The largest are those of
+        // components 0 (|2 q0 + q3| <= 3, |X0| <= 4, 36 and 12 from the axis terms, 8 from the face diagonals) and 3
+        // (12 from those); the others stay below 7.5 2^60.  A parameter set whose halves could reach 2^63 takes the
+        // next smaller scale, at which the sum is 7.25 2^60 with every bound at its worst.
+        auto mid = [](double xh, double xl, double y) { return xh * ldexp(1, 31) + xl * (ldexp(y, -32) + 1); };
+        auto term = [&](const Fix2 &x, double y) { return mid(fabs((double)x.h), fabs((double)x.l), y); };
+        const double most = mid(ldexp(gmax, R + 3 - 32) + 1, ldexp(1, 31), 3 * ldexp(1, 61)) + term(c.b3, 4 * ldexp(1, 58)) +
+                            term(c.l1, 36 * ldexp(1, 56)) + term(c.l23, 12 * ldexp(1, 56)) +
+                            term(c.l2, 12 * ldexp(1, 56)) + term(c.l3, 12 * ldexp(1, 56)) + ldexp(1, 33);
+        if (most < 0.999999 * ldexp(1, 63)) break;
+    }
     const bool twice = metric_mode == QMIN_METRIC_CPU;
     c.ma = ldexp(twice ? 20.0 / 9.0 : 4.0 / 3.0, -c.shift);
     c.mb = ldexp(twice ? 16.0 / 9.0 : 2.0 / 3.0, -c.shift);
@@ -212,8 +225,8 @@ inline FixedCoef fixed_coeffs(const qmin_ldg_params &p, int metric_mode, const d
         if (field && twice && k == 0) v += 0.5 * field[3];
         if (field && twice && k == 3) v += 0.5 * field[0];
         const long long b = -at(v, c.shift);  // hi 2^up + mid 2^(up - 32)
-        c.hi0[k] = b >> up;
-        c.mid0[k] = ((b - (long long)((unsigned long long)c.hi0[k] << up)) << (32 - up)) + (1LL << (31 - up));
+        c.hi0[k] = b >> c.up;
+        c.mid0[k] = ((b - (long long)((unsigned long long)c.hi0[k] << c.up)) << (32 - c.up)) + (1LL << (31 - c.up));
     }
     c.ok = 1;
     return c;
