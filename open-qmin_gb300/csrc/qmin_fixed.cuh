@@ -11,15 +11,18 @@
 //   * a product of two 64-bit numbers keeps its upper 64 bits, from the
 //     balanced 32-bit halves x = xh 2^32 + xl (xl signed): hi += xh yh,
 //     mid += xh yl + xl yh, result hi + mid / 2^32.  The sums of products of
-//     one output share hi and mid, which are put together once;
+//     one output share hi and mid, which are put together once; of xl yl the
+//     upper 32 bits go into a sum of their own (FixAcc);
 //   * every term of an output carries the same scale 2^R, chosen on the host
 //     from the parameters so that no sum, high or middle, can overflow
 //     (fixed_coeffs).
 //
-// The quantisation of Q (2^-57) and of the products stay below the rounding
-// of the FP64 evaluation, whose partial sums reach 10 to 30: against 80-bit
-// arithmetic the error of the force is 0.2 to 0.6 of the FP64 form's over
-// random and smooth nematic fields, 0.6 to 0.75 at 0.4 of the nematic order.
+// The quantisation of Q (towards zero at 2^-56, exact from 1/16 on; to the
+// nearest was no better over the 400 runs of FixAcc) and of the products stay
+// below the rounding of the FP64 evaluation, whose partial sums reach 10 to 30:
+// against 80-bit arithmetic the error of the force is 0.06 to 0.52 of the FP64
+// form's over random and smooth nematic fields; where every component is 3/4
+// and the FP64 products are nearly exact, 0.56 to 1.25.
 // The sums need every component's |Q| < 1 at LC sites (with 3/4, 350 of the
 // first 520 iterations at 200^3 left the range: FIRE overshoots to 0.85), the relative
 // accuracy some |Q| >= 1/8: a lattice outside that takes the FP64 kernel
@@ -41,9 +44,9 @@ namespace qmin {
 
 constexpr int kFixQ = 56;  // Q 2^56
 
-// a 64-bit number as balanced halves: v = h 2^32 + l, -2^31 <= l < 2^31
+// a 64-bit number as balanced halves: v = h 2^32 + l, -2^31 <= l < 2^31; q = l / 4
 struct Fix2 {
-    int h, l;
+    int h, l, q;
 };
 
 // what the kernels need of one parameter set
@@ -67,32 +70,53 @@ __host__
 QMIN_DEV Fix2 fix_split(long long v)
 {
     const unsigned l = (unsigned)(unsigned long long)v;
-    return Fix2{(int)(v >> 32) + (int)(l >> 31), (int)l};
+    return Fix2{(int)(v >> 32) + (int)(l >> 31), (int)l, (int)l >> 2};
 }
 
 QMIN_DEV long long fix_mul_wide(int a, int b, long long c) { return (long long)a * (long long)b + c; }
 
-// running sum of products of one output
+// (a b) / 2^32 + c
+QMIN_DEV int fix_mul_high(int a, int b, int c)
+{
+#ifdef __CUDA_ARCH__
+    return __mulhi(a, b) + c;
+#else
+    return (int)((long long)a * b >> 32) + c;
+#endif
+}
+
+// Running sum of products of one output.  The products of the low halves go
+// into lo in units of 4 (the middle sum's unit: 1), six of them below 2^31.
+// Left out, those of the squares are a bias of one sign at every site and
+// iteration: 100 FIRE iterations from random directors at 16^3 then end 10 %
+// farther from quadruple precision than with the FP64 force, with them 1 % +-
+// 2 % (means over 400 starts; from smooth fields 27 and 38 % nearer).  They
+// cost 1.3 to 1.8 % of a run (50^3 one-constant, 100 iterations: 3.10 -> 3.14
+// ms, 83 x 61 x 97, 60: 7.42 -> 7.53, 200^3, 40: 41.9 -> 42.7).
 struct FixAcc {
     long long hi, mid;
-    QMIN_DEV void zero() { hi = mid = 0; }
+    int lo;
+    QMIN_DEV void zero() { hi = mid = lo = 0; }
     QMIN_DEV void add(const Fix2 &x, const Fix2 &y)
     {
         hi = fix_mul_wide(x.h, y.h, hi);
         mid = fix_mul_wide(x.h, y.l, mid);
         mid = fix_mul_wide(x.l, y.h, mid);
+        lo = fix_mul_high(x.q, y.l, lo);
     }
     QMIN_DEV void square(const Fix2 &x)  // x x, its middle products halved: the caller doubles mid
     {
         hi = fix_mul_wide(x.h, x.h, hi);
         mid = fix_mul_wide(x.h, x.l, mid);
+        lo = fix_mul_high(x.q, x.l, lo);
     }
+    QMIN_DEV long long middle() const { return mid + 4LL * lo; }
     // hi 2^up + mid 2^(up - 32), 0 < up < 32
     QMIN_DEV long long get(int up) const
     {
-        return (long long)((unsigned long long)hi << up) + (mid >> (32 - up));  // the caller's mid has half a unit
+        return (long long)((unsigned long long)hi << up) + (middle() >> (32 - up));  // the caller's mid has half a unit
     }
-    QMIN_DEV long long get32() const { return hi + ((mid + (1LL << 31)) >> 32); }
+    QMIN_DEV long long get32() const { return hi + ((middle() + (1LL << 31)) >> 32); }
 };
 
 #ifdef __CUDACC__
@@ -213,7 +237,7 @@ inline FixedCoef fixed_coeffs(const qmin_ldg_params &p, int metric_mode, const d
         auto term = [&](const Fix2 &x, double y) { return mid(fabs((double)x.h), fabs((double)x.l), y); };
         const double most = mid(ldexp(gmax, R + 3 - 32) + 1, ldexp(1, 31), 3 * ldexp(1, 61)) + term(c.b3, 4 * ldexp(1, 58)) +
                             term(c.l1, 36 * ldexp(1, 56)) + term(c.l23, 12 * ldexp(1, 56)) +
-                            term(c.l2, 12 * ldexp(1, 56)) + term(c.l3, 12 * ldexp(1, 56)) + ldexp(1, 33);
+                            term(c.l2, 12 * ldexp(1, 56)) + term(c.l3, 12 * ldexp(1, 56)) + ldexp(1, 34);
         if (most < 0.999999 * ldexp(1, 63)) break;
     }
     const bool twice = metric_mode == QMIN_METRIC_CPU;
@@ -307,21 +331,26 @@ QMIN_DEV void fixed_force(const FixedCoef &k, const long long (&q)[5], const lon
     p03.add(y[0], y[3]);
     const long long h24 = sq[2].hi + sq[4].hi, n24 = sq[2].mid + sq[4].mid;
     const long long h03 = sq[0].hi + sq[3].hi, n03 = sq[0].mid + sq[3].mid;
+    const int o24 = sq[2].lo + sq[4].lo, o03 = sq[0].lo + sq[3].lo;
+    const long long p = p03.middle();
     // every shift rounds to nearest: a floor's half unit would add up over the iterations of a run
     constexpr long long half = 1LL << 30;
     const long long s =
-        (h03 + h24 + sq[1].hi + p03.hi) + ((n03 + n24 + sq[1].mid + half) >> 31) + ((p03.mid + 2 * half) >> 32);
+        (h03 + h24 + sq[1].hi + p03.hi) + ((n03 + n24 + sq[1].mid + 2LL * (o03 + o24 + sq[1].lo) + half) >> 31) +
+        ((p + 2 * half) >> 32);
     FixAcc g;
-    g.hi = 0;
+    g.zero();
     g.mid = 1LL << (31 - k.c8up);
     g.add(fix_split(s), k.c8);
     const long long mg = g.get(k.c8up) + k.a2;  // -g2 at 2^(R + 3)
     const Fix2 g2 = fix_split(mg), g4 = fix_split(2 * mg);
     // at 2^58: X0 = q3^2 + q4^2 + w, X3 = q0^2 + q2^2 + w with w = 2 q0 q3 - q1^2; X1 = q1 (q0 + q3) + q2 q4,
     // X2 = q1 q4 - q2 q3, X4 = q1 q2 - q0 q4
-    const long long wh = 2 * p03.hi - sq[1].hi, wm = p03.mid - sq[1].mid + half;
-    const Fix2 X0 = fix_split(sq[3].hi + sq[4].hi + wh + ((sq[3].mid + sq[4].mid + wm) >> 31));
-    const Fix2 X3 = fix_split(sq[0].hi + sq[2].hi + wh + ((sq[0].mid + sq[2].mid + wm) >> 31));
+    const long long wh = 2 * p03.hi - sq[1].hi, wm = p - sq[1].mid + half;
+    const Fix2 X0 =
+        fix_split(sq[3].hi + sq[4].hi + wh + ((sq[3].mid + sq[4].mid + wm + 2LL * (sq[3].lo + sq[4].lo - sq[1].lo)) >> 31));
+    const Fix2 X3 =
+        fix_split(sq[0].hi + sq[2].hi + wh + ((sq[0].mid + sq[2].mid + wm + 2LL * (sq[0].lo + sq[2].lo - sq[1].lo)) >> 31));
     FixAcc x1, x2, x4, xn;
     x1.zero();
     x1.add(y[1], y03);
@@ -332,17 +361,20 @@ QMIN_DEV void fixed_force(const FixedCoef &k, const long long (&q)[5], const lon
     xn.add(y[2], y[3]);
     x2.hi -= xn.hi;
     x2.mid -= xn.mid;
+    x2.lo -= xn.lo;
     x4.zero();
     x4.add(y[1], y[2]);
     xn.zero();
     xn.add(y[0], y[4]);
     x4.hi -= xn.hi;
     x4.mid -= xn.mid;
+    x4.lo -= xn.lo;
     FixAcc f[5];
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
         f[c].hi = k.hi0[c];
         f[c].mid = k.mid0[c];
+        f[c].lo = 0;
     }
     // -g2 (2 q0 + q3), -2 g2 q1, ..: the q at 2^61
     f[0].add(g2, fix_split((2 * q[0] + q[3]) * 32));
