@@ -13,9 +13,17 @@ constexpr int kMaxFusedBlocks = 16384;
 // listed site is long (an FP64 one 514 FP64 operations per warp), so the blocks
 // are small enough to reach every SM: at 83 x 61 x 97 with two walls an FP64
 // iteration takes 113 us with 128 threads, 114 with 64 or 32, 120 with 256
-// (87 blocks for 152 SMs); at 200^3 0.959, 0.963, 0.975 and 0.978 ms.
-constexpr int kListBlock = 128, kListPerSm = 8, kMaxListBlocks = 152 * kListPerSm;
-inline int list_grid(int n) { return std::max(1, std::min((n + kListBlock - 1) / kListBlock, kMaxListBlocks)); }
+// (87 blocks for 152 SMs); at 200^3 0.959, 0.963, 0.975 and 0.978 ms.  Beside
+// the fused bulk kernels, which fill an SM's registers, it is the other way
+// round: a list block on an SM keeps a bulk block off it, so the list is packed
+// onto fewer SMs (FP32 multi-constant, one wall, the 32 x 4 variant: 56^3 43.7
+// us with 128 threads, 28.8 with 256, 64^3 42.7 and 33.2, 96^3 53.2 and 50.7).
+constexpr int kListBlock = 128, kFusedListBlock = 256;
+constexpr int kMaxListBlocks = 152 * 8;  // of 128 threads; half as many of 256
+inline int list_grid(int n, int block = kListBlock)
+{
+    return std::max(1, std::min((n + block - 1) / block, kMaxListBlocks * kListBlock / block));
+}
 
 // what a bulk kernel may use of the buffer when listed sites run beside it
 constexpr int kMaxDeepBlocks = kMaxFusedBlocks - kMaxListBlocks;

@@ -60,11 +60,11 @@ int high_priority()
 // blocks, so that the two overlap.  Graphs keep the attribute on the kernel
 // node (they are instantiated to honour per-node priorities).
 template <class... P, class... A>
-void launch_high(void (*kern)(P...), int grid, cudaStream_t s, A &&...args)
+void launch_high(void (*kern)(P...), int grid, int block, cudaStream_t s, A &&...args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kListBlock);
+    cfg.blockDim = dim3(block);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributePriority;
@@ -1133,13 +1133,13 @@ __device__ __forceinline__ T pred_q_at(const Lat<T> &L, const PredCoef<T> &c, lo
 // twice the first derivatives (k_derivs' rules) of the predicted Q at the listed
 // sites' neighbours, formed from the input buffer set
 template <class T>
-__global__ void __launch_bounds__(kListBlock)
+__global__ void __launch_bounds__(kFusedListBlock)
     k_derivs_list_pred(Lat<T> L, const int *__restrict__ list, int n, const FireDev *__restrict__ fd)
 {
     if (!fd->active) return;
     const PredCoef<T> pc = pred_coef<T>(fd);
     const long long P = L.P;
-    for (int e = blockIdx.x * kListBlock + threadIdx.x; e < n; e += gridDim.x * kListBlock) {
+    for (int e = blockIdx.x * kFusedListBlock + threadIdx.x; e < n; e += gridDim.x * kFusedListBlock) {
         const int i = list[e];
         const int t = L.types[i];
         const Nb b = neighbours(L, i);
@@ -1187,7 +1187,7 @@ template <class T> struct PredAcc {
 // the listed LC sites' force at the predicted Q and kick, from the input buffer
 // set into the output set's V and F (their predicted Q: the fused deep kernel)
 template <class T>
-__global__ void __launch_bounds__(kListBlock, sizeof(T) == 4 ? 512 / kListBlock : 1)
+__global__ void __launch_bounds__(kFusedListBlock, sizeof(T) == 4 ? 2 : 1)
     k_force_kick_list_pred(Lat<T> L, T *__restrict__ Vo, T *__restrict__ Fo, const int *__restrict__ list, int n,
                            const FireDev *__restrict__ fd, double *partials)
 {
@@ -1196,7 +1196,7 @@ __global__ void __launch_bounds__(kListBlock, sizeof(T) == 4 ? 512 / kListBlock 
     const T hdt = T(0.5) * T(fd->dt);
     const long long P = L.P;
     double acc[3] = {0.0, 0.0, 0.0};
-    for (int e = blockIdx.x * kListBlock + threadIdx.x; e < n; e += gridDim.x * kListBlock) {
+    for (int e = blockIdx.x * kFusedListBlock + threadIdx.x; e < n; e += gridDim.x * kFusedListBlock) {
         const int i = list[e];
         const int t = L.types[i];
         PredAcc<T> a(L, i, pc);
@@ -1217,7 +1217,7 @@ __global__ void __launch_bounds__(kListBlock, sizeof(T) == 4 ? 512 / kListBlock 
             acc[2] += (double)dot_qt(f, v);
         }
     }
-    block_sum<3, kListBlock>(acc);
+    block_sum<3, kFusedListBlock>(acc);
     if (threadIdx.x == 0)
 #pragma unroll
         for (int k = 0; k < 3; ++k) partials[3 * blockIdx.x + k] = acc[k];
@@ -1364,13 +1364,13 @@ int launch_split_fused_list(const Lat<T> &Lin, T *Vo, T *Fo, const SplitLists &s
     int n = 0;
     *nblocks = 0;
     if (Lin.multi && sl.n_derivs > 0) {
-        launch_high(k_derivs_list_pred<T>, list_grid(sl.n_derivs), s, Lin, (const int *)sl.derivs, sl.n_derivs,
-                    (const FireDev *)fd);
+        launch_high(k_derivs_list_pred<T>, list_grid(sl.n_derivs, kFusedListBlock), kFusedListBlock, s, Lin,
+                    (const int *)sl.derivs, sl.n_derivs, (const FireDev *)fd);
         ++n;
     }
     if (sl.n_sites > 0) {
-        const int g = list_grid(sl.n_sites);
-        launch_high(k_force_kick_list_pred<T>, g, s, Lin, Vo, Fo, (const int *)sl.sites, sl.n_sites, (const FireDev *)fd,
+        const int g = list_grid(sl.n_sites, kFusedListBlock);
+        launch_high(k_force_kick_list_pred<T>, g, kFusedListBlock, s, Lin, Vo, Fo, (const int *)sl.sites, sl.n_sites, (const FireDev *)fd,
                     partials);
         *nblocks = g;
         ++n;
@@ -1381,7 +1381,7 @@ int launch_split_fused_list(const Lat<T> &Lin, T *Vo, T *Fo, const SplitLists &s
 template <class T> int launch_split_derivs(const Lat<T> &L, const SplitLists &sl, FireDev *fd, cudaStream_t s)
 {
     if (!L.multi || sl.n_derivs == 0) return 0;
-    launch_high(k_derivs_list<T>, list_grid(sl.n_derivs), s, L, (const int *)sl.derivs, sl.n_derivs, (const FireDev *)fd);
+    launch_high(k_derivs_list<T>, list_grid(sl.n_derivs), kListBlock, s, L, (const int *)sl.derivs, sl.n_derivs, (const FireDev *)fd);
     return 1;
 }
 
@@ -1417,7 +1417,7 @@ int launch_split_list(const Lat<T> &L, const SplitLists &sl, FireDev *fd, double
 {
     if (sl.n_sites <= 0) return 0;
     const int g = list_grid(sl.n_sites);
-    launch_high(k_force_kick_list<T>, g, s, L, (const int *)sl.sites, sl.n_sites, (const FireDev *)fd, partials);
+    launch_high(k_force_kick_list<T>, g, kListBlock, s, L, (const int *)sl.sites, sl.n_sites, (const FireDev *)fd, partials);
     return g;
 }
 
