@@ -196,4 +196,22 @@ __device__ __forceinline__ T anchoring_energy(int kind, T W, T S0, const T *q, c
     return W * e1 + T(0.25) * W * e2 * e2;
 }
 
+// running sum: compensated (Kahan) FP32 for the FP32 form, plain FP64 otherwise
+template <class T> struct RunSum {
+    double s = 0.0;
+    __device__ __forceinline__ void add(T x) { s += (double)x; }
+    __device__ __forceinline__ double value() const { return s; }
+};
+template <> struct RunSum<float> {
+    float s = 0.f, c = 0.f;
+    __device__ __forceinline__ void add(float x)
+    {
+        const float y = x - c;
+        const float t = s + y;
+        c = (t - s) - y;
+        s = t;
+    }
+    __device__ __forceinline__ double value() const { return (double)s - (double)c; }
+};
+
 }  // namespace qmin

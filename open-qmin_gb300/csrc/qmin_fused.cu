@@ -76,24 +76,6 @@ template <class T, int H, int TX, int TY> struct DeepTileAcc : TileAcc<T, H, TX,
     }
 };
 
-// running sum: compensated (Kahan) FP32 for the FP32 form, plain FP64 otherwise
-template <class T> struct RunSum {
-    double s = 0.0;
-    __device__ __forceinline__ void add(T x) { s += (double)x; }
-    __device__ __forceinline__ double value() const { return s; }
-};
-template <> struct RunSum<float> {
-    float s = 0.f, c = 0.f;
-    __device__ __forceinline__ void add(float x)
-    {
-        const float y = x - c;
-        const float t = s + y;
-        c = (t - s) - y;
-        s = t;
-    }
-    __device__ __forceinline__ double value() const { return (double)s - (double)c; }
-};
-
 __device__ __forceinline__ int wrapi(int v, int m)
 {
     int r = v % m;

@@ -842,6 +842,13 @@ __device__ __forceinline__ void deep_force_ring(const Lat<T> &L, const T *sQ, co
     deep_force_finish(L, qc[1], s2, i, f);
 }
 
+// FP32 sum over a thread's column, FP64 from there on
+struct ColumnSum {
+    float s = 0.f;
+    __device__ __forceinline__ void add(float x) { s += x; }
+    __device__ __forceinline__ double value() const { return (double)s; }
+};
+
 // the owned site of plane z: force from the ring, kick, writes to the output
 // set (32-bit component offsets from the site's address), FIRE sums
 template <class T, int TS, int SX, bool MULTI, class Acc>
@@ -864,9 +871,9 @@ __device__ __forceinline__ void fused_site_out(const Lat<T> &L, const T *sQ, con
             vo(k) = v[k];
             fo(k) = f[k];
         }
-        sacc[0] += (Acc)dot_qt(f, f);
-        sacc[1] += (Acc)dot_qt(v, v);
-        sacc[2] += (Acc)dot_qt(f, v);
+        sacc[0].add(dot_qt(f, f));
+        sacc[1].add(dot_qt(v, v));
+        sacc[2].add(dot_qt(f, v));
     } else {
 #pragma unroll
         for (int k = 0; k < 5; ++k) qo(k) = qc[1][k];
@@ -941,8 +948,10 @@ __global__ void __launch_bounds__(TX *TY, MINB)
 #pragma unroll
             for (int k = 0; k < 5; ++k) s[k * TS + fp.ph] = pred_q(pc, rh[k], pred_v(pc, rh[5 + k], rh[10 + k]));
     };
-    using Acc = typename std::conditional<sizeof(T) == 4, float, double>::type;
-    Acc sacc[3] = {Acc(0), Acc(0), Acc(0)};
+    // A thread's column may be hundreds of planes: one-constant FP32 lattices keep compensated sums, as k_fire_fused
+    // (at 200^3 243 us an iteration for 239, forceMax 5e-10 from that of its forces for 4e-9).
+    using Acc = typename std::conditional<sizeof(T) == 4 && MULTI, ColumnSum, RunSum<T>>::type;
+    Acc sacc[3];
     if (zs < L.Lz) {
         T vn_cur[5], vn_nxt[5], qc[3][5];
         load(zs - 1);
@@ -971,7 +980,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
             for (int k = 0; k < 5; ++k) vn_cur[k] = vn_nxt[k];
         }
     }
-    double acc[3] = {(double)sacc[0], (double)sacc[1], (double)sacc[2]};
+    double acc[3] = {sacc[0].value(), sacc[1].value(), sacc[2].value()};
     block_sum<3, NT>(acc);
     if (threadIdx.x == 0) {
         const int b = blockIdx.y * gridDim.x + blockIdx.x;
@@ -1073,8 +1082,8 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     auto cls_at = [&](int z) -> uint8_t {
         return (fp.own_in && z >= zs && z < ze) ? cls[(unsigned)(sxy * z + fp.colo)] : uint8_t(1);
     };
-    using Acc = float;
-    Acc sacc[3] = {0.f, 0.f, 0.f};
+    using Acc = ColumnSum;
+    Acc sacc[3];
     if (zs < L.Lz) {
         // prologue: planes zs-1 .. zs+1 predicted; zs+2 and zs+3 in flight
         T vn0[5], vn1[5], vn2[5], qc[3][5], qn[5];
@@ -1113,7 +1122,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
         }
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
-    double acc[3] = {(double)sacc[0], (double)sacc[1], (double)sacc[2]};
+    double acc[3] = {sacc[0].value(), sacc[1].value(), sacc[2].value()};
     block_sum<3, NT>(acc);
     if (threadIdx.x == 0) {
         const int b = blockIdx.y * gridDim.x + blockIdx.x;
