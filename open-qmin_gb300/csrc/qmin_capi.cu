@@ -1431,8 +1431,8 @@ static int adam_impl(qmin_ctx *h, double b1, double b2, double eps, double dt, i
     const double args[4] = {b1, b2, eps, dt};
     int r = capture_chunk(h, 1, args, [&]() {
         int n = launch_force<T>(L, h->grid, h->stream);
-        n += launch_adam_step<T>(L, (T *)h->M, (T *)h->S, h->iter, b1, b2, eps, dt, h->partials, h->grid, h->stream);
-        n += launch_norm_control(h->iter, h->partials, h->grid, 1, b1, b2, h->stream);
+        n += launch_adam_step<T>(L, (T *)h->M, (T *)h->S, h->iter, b1, b2, eps, dt, h->partials, vector_grid(L), h->stream);
+        n += launch_norm_control(h->iter, h->partials, vector_grid(L), 1, b1, b2, h->stream);
         return n;
     });
     if (r) return r;
@@ -1480,8 +1480,8 @@ template <class T> static int nesterov_impl(qmin_ctx *h, double dt, double mu, i
     const double args[4] = {dt, mu, 0, 0};
     int r = capture_chunk(h, 2, args, [&]() {
         int n = launch_force<T>(L, h->grid, h->stream);
-        n += launch_nesterov_step<T>(L, (T *)h->alt, h->iter, dt, mu, h->partials, h->grid, h->stream);
-        n += launch_norm_control(h->iter, h->partials, h->grid, 0, 0.0, 0.0, h->stream);
+        n += launch_nesterov_step<T>(L, (T *)h->alt, h->iter, dt, mu, h->partials, vector_grid(L), h->stream);
+        n += launch_norm_control(h->iter, h->partials, vector_grid(L), 0, 0.0, 0.0, h->stream);
         return n;
     });
     if (r) return r;
@@ -1523,8 +1523,8 @@ template <class T> static int gd_impl(qmin_ctx *h, double dt, int max_iterations
     int r = capture_chunk(h, 4, args, [&]() {
         int n = launch_gd_move<T>(L, h->iter, dt, h->stream);
         n += launch_force<T>(L, h->grid, h->stream);
-        n += launch_ff_dot<T>(L, h->iter, h->partials, h->grid, h->stream);
-        n += launch_norm_control(h->iter, h->partials, h->grid, 0, 0.0, 0.0, h->stream);
+        n += launch_ff_dot<T>(L, h->iter, h->partials, vector_grid(L), h->stream);
+        n += launch_norm_control(h->iter, h->partials, vector_grid(L), 0, 0.0, 0.0, h->stream);
         return n;
     });
     if (r) return r;

@@ -172,6 +172,15 @@ int launch_lbfgs_products(const Lat<float> &L, float *sbase, float *ybase, IterD
                           double *partials, cudaStream_t s);
 
 int reduction_grid(int N);
+// Grid of the minimisers' passes over the 5 P values in 16-byte vectors, whose blocks leave a sum each: as for the
+// sites, but up to two blocks an SM one vector a thread (by sites an FP64 thread of a small lattice has 2.5 in turn:
+// 64 iterations at 24^3 take 1150 instead of 1244 us in gradient descent, 1620 instead of 2100 in Adam; beyond that the
+// sum of the more blocks costs as much).
+template <class T> int vector_grid(const Lat<T> &L)
+{
+    const long long blocks = (5 * L.P / (long long)(16 / sizeof(T)) + kBlock - 1) / kBlock;
+    return (int)std::max<long long>(reduction_grid(L.N), std::min(blocks, 2LL * 152));
+}
 
 // fused tiled FIRE iteration (qmin_fused.cu): tile configuration cfg in
 // [0, kFusedConfigs), z planes per block zc; returns launches or -1

@@ -1209,7 +1209,7 @@ template <class T> int launch_defects(const Lat<T> &L, int kind, double *out, cu
 }
 template <class T> int launch_gd_move(const Lat<T> &L, IterDev *it, double dt, cudaStream_t s)
 {
-    k_gd_move<T><<<elem_grid(L.N), kBlock, 0, s>>>(L, it, T(dt));
+    k_gd_move<T><<<elem_grid(5 * L.P / (16 / sizeof(T))), kBlock, 0, s>>>(L, it, T(dt));
     return 1;
 }
 template <class T> int launch_ff_dot(const Lat<T> &L, IterDev *it, double *partials, int grid, cudaStream_t s)
