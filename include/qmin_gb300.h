@@ -337,7 +337,9 @@ int qmin_energy_noalloc(const qmin_lattice_desc *desc, const qmin_ldg_params *p,
  * qmin_batch_fire_run runs all iterations of all solves in one persistent
  * cooperative launch (grid barriers between the phases of an iteration; FP32
  * batches run the predictor, force and kick as one phase over two state sets,
- * and the device memory for the second set is allocated on their first run).
+ * and the device memory for the second set is allocated on their first run;
+ * without room for it multi-constant batches run on one, with a phase for the
+ * predictor, and one-constant ones return QMIN_ENOMEM).
  * Site classes and lists are taken from the types at the first run after a
  * solve's types changed.  All
  * solves share the force parameters; each has up to 16 objects.  No reference

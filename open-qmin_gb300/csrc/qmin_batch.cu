@@ -153,28 +153,30 @@ struct BatchFixed {
 
 // The deferred mix folded into the Verlet coefficients, as k_fire_pred does:
 // v' = cvv v + cvf f, q' = q + dt v' (sites l0 .. l1 of a solve); with fx.X also
-// Q' 2^56 and the range of the LC sites
-__device__ __forceinline__ void b_pred_item(const BatchArgs<double> &B, const BatchFixed &fx, const FireDev *fds, int s,
+// Q' 2^56 and the range of the LC sites (FP64)
+template <class T>
+__device__ __forceinline__ void b_pred_item(const BatchArgs<T> &B, const BatchFixed &fx, const FireDev *fds, int s,
                                             int l0, int l1)
 {
     const int off = B.solves[s].off;
-    const PredCoef<double> pc = pred_coef<double>(fds + s);
+    const PredCoef<T> pc = pred_coef<T>(fds + s);
+    constexpr bool f64 = sizeof(T) == 8;
     int m = 0;
     for (int i = off + l0 + threadIdx.x; i < off + l1; i += kBlock) {
-        const bool lc = fx.X && B.L.types[i] <= 0;
+        const bool lc = f64 && fx.X && B.L.types[i] <= 0;
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
             const size_t j = k * (size_t)B.L.P + (unsigned)i;
-            const double vn = pred_v(pc, B.L.V[j], B.L.F[j]), q = pred_q(pc, B.L.Q[j], vn);
+            const T vn = pred_v(pc, B.L.V[j], B.L.F[j]), q = pred_q(pc, B.L.Q[j], vn);
             B.L.V[j] = vn;
             B.L.Q[j] = q;
-            if (fx.X) {
+            if (f64 && fx.X) {
                 fx.X[j] = to_fixed(q);
                 if (lc) m = max(m, fix_magnitude(q));
             }
         }
     }
-    if (!fx.X) return;
+    if (!f64 || !fx.X) return;
     const unsigned wide = __ballot_sync(0xffffffffu, m >= kFixWide), lively = __ballot_sync(0xffffffffu, m >= kFixLively);
     if ((threadIdx.x & 31) == 0) {  // every warp that raises a flag writes the same value
         volatile int2 *r = fx.range + s;
@@ -283,9 +285,9 @@ __device__ __forceinline__ double warp_sum3(const double (&v)[3])
     return a;
 }
 
-// force, half kick and this thread's FIRE sums at packed site gi of an FP64 solve
-__device__ __forceinline__ void b_kick(const Lat<double> &L, int gi, double hdt, const double (&f)[5], double (&v)[5],
-                                       double (&acc)[3])
+// force, half kick and this thread's FIRE sums (FP64) at packed site gi of a solve
+template <class T>
+__device__ __forceinline__ void b_kick(const Lat<T> &L, int gi, T hdt, const T (&f)[5], T (&v)[5], double (&acc)[3])
 {
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
@@ -294,15 +296,21 @@ __device__ __forceinline__ void b_kick(const Lat<double> &L, int gi, double hdt,
         L.V[j] = v[k];
         L.F[j] = f[k];
     }
-    dot3_acc(f, v, acc);
+    if constexpr (sizeof(T) == 8) {
+        dot3_acc(f, v, acc);
+    } else {
+        acc[0] += (double)dot_qt(f, f);
+        acc[1] += (double)dot_qt(v, v);
+        acc[2] += (double)dot_qt(f, v);
+    }
 }
 
-// FP64, the bulk sites (class 0) of l0 .. l1 of a solve, in fixed point where the
+// The bulk sites (class 0) of l0 .. l1 of a solve, FP64 in fixed point where the
 // solve is inside its range; the listed sites are items of their own, object
 // sites keep V = F = 0
-template <bool MULTI>
-__device__ __forceinline__ void b_bulk_item(const BatchArgs<double> &B, const BatchFixed &fx, const SolveDesc &sd,
-                                            double hdt, bool fixed, int l0, int l1, double (&acc)[3])
+template <class T, bool MULTI>
+__device__ __forceinline__ void b_bulk_item(const BatchArgs<T> &B, const BatchFixed &fx, const SolveDesc &sd, T hdt,
+                                            bool fixed, int l0, int l1, double (&acc)[3])
 {
     const size_t P = (size_t)B.L.P;
     for (int li = l0 + threadIdx.x; li < l1; li += kBlock) {
@@ -310,10 +318,10 @@ __device__ __forceinline__ void b_bulk_item(const BatchArgs<double> &B, const Ba
         if (B.cls[gi] != 0) continue;
         const int r = (int)udiv((unsigned)li, (unsigned)sd.Lx, sd.mx);
         const int x = li - r * sd.Lx, z = (int)udiv((unsigned)r, (unsigned)sd.Ly, sd.my), y = r - z * sd.Ly;
-        double f[5], v[5];
+        T f[5], v[5];
 #pragma unroll
         for (int k = 0; k < 5; ++k) v[k] = (B.L.V + k * P)[(unsigned)gi];  // in flight during the force
-        if (fixed) {
+        if (sizeof(T) == 8 && fixed) {
             const int sy = sd.Lx, sz = sd.Lx * sd.Ly, n = sz * sd.Lz;
             const int ox[3] = {x == 0 ? sy - 1 : -1, 0, x == sd.Lx - 1 ? 1 - sy : 1};
             const int oy[3] = {y == 0 ? sz - sy : -sy, 0, y == sd.Ly - 1 ? sy - sz : sy};
@@ -327,27 +335,30 @@ __device__ __forceinline__ void b_bulk_item(const BatchArgs<double> &B, const Ba
             fixed_axis(at, q, lam, ax);
             if (MULTI) fixed_mixed(at, m2, m3);
             fixed_force<MULTI>(fx.kc, q, lam, ax, m2, m3, a);
-            fixed_to_force(fx.kc, a, f);
+            double g[5];
+            fixed_to_force(fx.kc, a, g);
+#pragma unroll
+            for (int k = 0; k < 5; ++k) f[k] = T(g[k]);
         } else if (MULTI) {
-            deep_force_box<double, false>(B.L, sd.off, sd.Lx, sd.Ly, sd.Lz, li, (long long)gi, f);
+            deep_force_box<T, false>(B.L, sd.off, sd.Lx, sd.Ly, sd.Lz, li, (long long)gi, f);
         } else {
-            BatchAcc<double> a(B.L, sd, li, x, y, z);
-            site_force_core<double, BatchAcc<double>, false, false, true>(B.L, a, 0, f);
+            BatchAcc<T> a(B.L, sd, li, x, y, z);
+            site_force_core<T, BatchAcc<T>, false, false, true>(B.L, a, 0, f);
         }
         b_kick(B.L, gi, hdt, f, v, acc);
     }
 }
 
-// FP64, listed sites of a solve
-template <bool MULTI>
-__device__ __forceinline__ void b_listed_item(const BatchArgs<double> &B, const SolveDesc &sd, const SolveTile &st,
-                                              double hdt, int k, double (&acc)[3])
+// listed sites of a solve
+template <class T, bool MULTI>
+__device__ __forceinline__ void b_listed_item(const BatchArgs<T> &B, const SolveDesc &sd, const SolveTile &st, T hdt,
+                                              int k, double (&acc)[3])
 {
     const int e = k * st.lc + threadIdx.x;
     if (threadIdx.x >= st.lc || e >= st.nlist) return;
-    BatchAcc<double> a(B.L, sd, st.sites[e]);
-    double f[5], v[5];
-    site_force_core<double, BatchAcc<double>, false, MULTI, !MULTI>(B.L, a, B.L.types[a.i], f);
+    BatchAcc<T> a(B.L, sd, st.sites[e]);
+    T f[5], v[5];
+    site_force_core<T, BatchAcc<T>, false, MULTI, !MULTI>(B.L, a, B.L.types[a.i], f);
 #pragma unroll
     for (int k = 0; k < 5; ++k) v[k] = (B.L.V + k * (size_t)B.L.P)[(unsigned)a.i];
     b_kick(B.L, a.i, hdt, f, v, acc);
@@ -668,9 +679,11 @@ struct TileItems {
 // now); listed sites are items of their own, taken first, so that no warp waits
 // for one of them (546 with them inside the bulk runs, each chunk of 256 an
 // item; control as a phase with two more barriers 573).
-template <bool MULTI>
-__global__ void __launch_bounds__(kBlock, kFixedPerSm)
-    k_b_fire_fixed(const __grid_constant__ BatchArgs<double> B, const __grid_constant__ BatchFixed fx,
+// FP32 multi-constant solves come here when there is no room for the second
+// state set of k_b_fire_tiled.
+template <class T, bool MULTI>
+__global__ void __launch_bounds__(kBlock, sizeof(T) == 8 ? kFixedPerSm : 2)
+    k_b_fire_fixed(const __grid_constant__ BatchArgs<T> B, const __grid_constant__ BatchFixed fx,
                    const SolveTile *tiles, FireDev *fds, double *partials, int *done, int nsolves, BatchRun *run)
 {
     extern __shared__ int b_lists[];
@@ -697,7 +710,7 @@ __global__ void __launch_bounds__(kBlock, kFixedPerSm)
                 q.item(al, s, k);
                 const SolveTile st = tiles[s];
                 const int e = k * kBlock + threadIdx.x;
-                if (e < st.nderiv) b_derivs_at(B.L, BatchAcc<double>(B.L, B.solves[s], st.derivs[e]));
+                if (e < st.nderiv) b_derivs_at(B.L, BatchAcc<T>(B.L, B.solves[s], st.derivs[e]));
             }
             if (!b_grid_sync(run)) return;
         }
@@ -712,14 +725,14 @@ __global__ void __launch_bounds__(kBlock, kFixedPerSm)
                 continue;
             }
             const SolveDesc sd = B.solves[s];
-            const double hdt = 0.5 * fds[s].dt;
+            const T hdt = T(0.5) * T(fds[s].dt);
             double acc[3] = {0.0, 0.0, 0.0};
             if (k < nli) {
-                b_listed_item<MULTI>(B, sd, st, hdt, k, acc);
+                b_listed_item<T, MULTI>(B, sd, st, hdt, k, acc);
             } else {
                 const volatile int2 *rg = fx.range + s;
                 const int l0 = (k - nli) * st.zc;
-                b_bulk_item<MULTI>(B, fx, sd, hdt, fx.X && rg->y && !rg->x, l0, min(l0 + st.zc, st.n), acc);
+                b_bulk_item<T, MULTI>(B, fx, sd, hdt, fx.X && rg->y && !rg->x, l0, min(l0 + st.zc, st.n), acc);
             }
             const double sum = warp_sum3(acc);
             const int lane = threadIdx.x & 31;
@@ -877,7 +890,7 @@ struct qmin_batch_ctx {
         bool classified = false;
     };
     std::vector<SolveLists> lists;
-    bool tiles_multi = false, classified_multi = false;
+    bool tiles_multi = false, tiles_tiled = false, classified_multi = false;
     void *geo_scratch = nullptr;
     long long *X = nullptr;  // FP64: Q 2^56 of the fixed-point force
     int2 *range = nullptr;
@@ -1082,17 +1095,16 @@ static int classify_solves(qmin_batch_ctx *b)
     return QMIN_OK;
 }
 
-// the items of every solve.  FP32: tiles of about 128 sites cut evenly (at most
+// the items of every solve.  tiled (FP32): tiles of about 128 sites cut evenly (at most
 // 32 wide and 32 high), z chunks of 4 to 16 planes so that there are about four
-// items per resident block (two, three and six measured within 5 %).  FP64:
+// items per resident block (two, three and six measured within 5 %).  Otherwise
 // runs of 1 to 8 blocks' sites, by the same rule (40 uneven solves, 2.5 M sites:
 // 431 us with runs of one block's sites, 389 two, 370 four, 367 eight, 382 ten).
-static int lay_out_items(qmin_batch_ctx *b, bool multi)
+static int lay_out_items(qmin_batch_ctx *b, bool multi, bool tiled)
 {
-    if (!b->tiles_h.empty() && b->tiles_multi == multi) return QMIN_OK;
+    if (!b->tiles_h.empty() && b->tiles_multi == multi && b->tiles_tiled == tiled) return QMIN_OK;
     auto cut = [](int n, int most) { return (n + most - 1) / most; };
-    const bool fp32 = b->prec == QMIN_FP32;
-    const int block = fp32 ? kTileThreads : kBlock;
+    const int block = tiled ? kTileThreads : kBlock;
     std::vector<SolveTile> t((size_t)b->nsolves);
     long long planes = 0;
     for (int s = 0; s < b->nsolves; ++s) {
@@ -1111,13 +1123,13 @@ static int lay_out_items(qmin_batch_ctx *b, bool multi)
     // solves of 16^3 to 24^3: 56 us an iteration, 77 with 256 to an item)
     long long nl = 0;
     for (const auto &l : b->lists) nl += l.n_sites;
-    const int lc = fp32 ? kTileThreads : 32 * (int)std::min(8LL, 1 + nl / (32LL * 152 * kFixedPerSm));
+    const int lc = tiled ? kTileThreads : 32 * (int)std::min(8LL, 1 + nl / (32LL * 152 * kFixedPerSm));
     const int run = kBlock * (int)std::min(8, std::max(1, b->N / (kBlock * 152 * kFixedPerSm * 4)));
     long long items = 0;
     for (int s = 0; s < b->nsolves; ++s) {
         const SolveDesc &sd = b->solves_h[s];
         SolveTile &st = t[s];
-        if (fp32) {
+        if (tiled) {
             st.zc = cut(sd.Lz, cut(sd.Lz, zmax));
             st.ntile = st.ntx * st.nty * cut(sd.Lz, st.zc);
         } else {
@@ -1135,15 +1147,16 @@ static int lay_out_items(qmin_batch_ctx *b, bool multi)
         st.item0 = (int)items;
         items += st.items;
     }
-    if (items > (long long)b->tile_partials_cap) {
+    const size_t warps = (size_t)items * (block / 32);
+    if (warps > b->tile_partials_cap) {
         if (b->tile_partials) cudaFree(b->tile_partials);
         b->tile_partials = nullptr;
         b->tile_partials_cap = 0;
-        if (cudaMalloc(&b->tile_partials, sizeof(double) * 3 * (block / 32) * (size_t)items) != cudaSuccess) {
+        if (cudaMalloc(&b->tile_partials, sizeof(double) * 3 * warps) != cudaSuccess) {
             cudaGetLastError();
             return bfail(QMIN_ENOMEM, "batch: partial sums allocation failed");
         }
-        b->tile_partials_cap = (size_t)items;
+        b->tile_partials_cap = warps;
     }
     if ((!b->tiles && cudaMalloc(&b->tiles, sizeof(SolveTile) * (size_t)b->nsolves) != cudaSuccess) ||
         (!b->coefs && cudaMalloc(&b->coefs, sizeof(float4) * (size_t)b->nsolves) != cudaSuccess) ||
@@ -1153,6 +1166,7 @@ static int lay_out_items(qmin_batch_ctx *b, bool multi)
     }
     b->tiles_h = t;
     b->tiles_multi = multi;
+    b->tiles_tiled = tiled;
     BCK(cudaMemcpyAsync(b->tiles, b->tiles_h.data(), sizeof(SolveTile) * t.size(), cudaMemcpyHostToDevice, b->stream));
     return QMIN_OK;
 }
@@ -1183,13 +1197,13 @@ template <bool MULTI> static int launch_tiled(qmin_batch_ctx *b, const BatchArgs
                               sizeof(float) * kTileRing + sizeof(int) * 2 * ((size_t)b->nsolves + 1), args);
 }
 
-template <bool MULTI> static int launch_fixed(qmin_batch_ctx *b, const BatchArgs<double> &B, const BatchFixed &fx)
+template <class T, bool MULTI> static int launch_fixed(qmin_batch_ctx *b, const BatchArgs<T> &B, const BatchFixed &fx)
 {
-    BatchArgs<double> a = B;
+    BatchArgs<T> a = B;
     BatchFixed f = fx;
     const SolveTile *tiles = b->tiles;
     void *args[] = {&a, &f, &tiles, &b->fds, &b->tile_partials, &b->done, &b->nsolves, &b->run};
-    return launch_cooperative(b, (const void *)k_b_fire_fixed<MULTI>, kBlock,
+    return launch_cooperative(b, (const void *)k_b_fire_fixed<T, MULTI>, kBlock,
                               sizeof(int) * 2 * ((size_t)b->nsolves + 1), args);
 }
 
@@ -1275,7 +1289,7 @@ int qmin_batch_create(int nsolves, const int32_t *dims, int precision, int metri
               cudaMalloc(&b->partials, sizeof(double) * 3 * kBatchWarps * (size_t)b->max_chunks) == cudaSuccess &&
               cudaMalloc(&b->run, sizeof(BatchRun)) == cudaSuccess &&
               cudaMalloc(&b->stage, sizeof(double) * 5 * (size_t)b->maxN) == cudaSuccess &&
-                            cudaMalloc(&b->fds, sizeof(FireDev) * nsolves) == cudaSuccess &&
+              cudaMalloc(&b->fds, sizeof(FireDev) * nsolves) == cudaSuccess &&
               cudaMalloc(&b->cls, (size_t)b->P) == cudaSuccess && cudaMalloc(&b->needd, (size_t)b->P) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
@@ -1467,9 +1481,9 @@ template <class T> static int batch_fire_impl(qmin_batch_ctx *b, bool *timed_out
     run.spin_limit = b->spin_limit;
     BCK(cudaMemcpyAsync(b->run, &run, sizeof run, cudaMemcpyHostToDevice, b->stream));
     const BatchArgs<T> B = batch_args<T>(b);
-    const bool fused = sizeof(T) == 4;
+    bool fused = sizeof(T) == 4;
     if (fused) {
-        // the second state set, on the first FP32 run
+        // the second state set, on the first FP32 run; without room multi-constant solves run in place
         const size_t bytes = 5 * (size_t)b->P * b->esz;
         for (void **p : {&b->Q2, &b->V2, &b->F2})
             if (!*p && cudaMalloc(p, bytes) != cudaSuccess) *p = nullptr;
@@ -1477,19 +1491,26 @@ template <class T> static int batch_fire_impl(qmin_batch_ctx *b, bool *timed_out
             b->in_second = nullptr;
         if (!b->Q2 || !b->V2 || !b->F2 || !b->in_second) {
             cudaGetLastError();
-            return bfail(QMIN_ENOMEM, "qmin_batch_fire_run: second state set allocation failed");
+            if (!B.L.multi) return bfail(QMIN_ENOMEM, "qmin_batch_fire_run: second state set allocation failed");
+            fused = false;
+            for (void **p : {&b->Q2, &b->V2, &b->F2}) {
+                if (*p) cudaFree(*p);
+                *p = nullptr;
+            }
         }
     }
     if (fused) BCK(cudaMemsetAsync(b->in_second, 0, sizeof(int) * (size_t)b->nsolves, b->stream));
-    int r = lay_out_items(b, B.L.multi != 0);
+    int r = lay_out_items(b, B.L.multi != 0, fused);
     if (r) return r;
     BCK(cudaMemsetAsync(b->done, 0, sizeof(int) * (size_t)b->nsolves, b->stream));
     if constexpr (sizeof(T) == 4) {
-        r = B.L.multi ? launch_tiled<true>(b, B) : launch_tiled<false>(b, B);
+        BatchFixed none;
+        memset(&none, 0, sizeof none);
+        r = !fused ? launch_fixed<T, true>(b, B, none) : B.L.multi ? launch_tiled<true>(b, B) : launch_tiled<false>(b, B);
     } else {
         const BatchFixed fx = batch_fixed(b, B.L);
         if (fx.X) BCK(cudaMemsetAsync(fx.range, 0, sizeof(int2) * (size_t)b->nsolves, b->stream));
-        r = B.L.multi ? launch_fixed<true>(b, B, fx) : launch_fixed<false>(b, B, fx);
+        r = B.L.multi ? launch_fixed<T, true>(b, B, fx) : launch_fixed<T, false>(b, B, fx);
     }
     if (r) return r;
     b->launches += 1;

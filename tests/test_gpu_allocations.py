@@ -105,7 +105,8 @@ def test_second_set_that_did_not_fit(qmin, oracle, tmp_path, precision, passed):
                 Q = lambda: lat.get_state()[0]
             elif prec == qmin.FP32:
                 b = qmin.Batch([L], prec)
-                b.set_params(s.p.A, s.p.B, s.p.C, s.p.L1, s.p.L2, s.p.L3, multi_constant=1)
+                s = oracle.System(L, Ls=(2.32, 0, 0, 0, 0))  # multi-constant batches run without it
+                b.set_params(s.p.A, s.p.B, s.p.C, s.p.L1)
                 b.set_chunk_shape(0)
                 s.random_nematic(4)
                 b.set_solve(0, s.Q, s.types, [])
