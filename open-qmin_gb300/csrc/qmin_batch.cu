@@ -808,13 +808,12 @@ __global__ void __launch_bounds__(kTileThreads, kTilePerSm)
             const float4 c = __ldcg(coefs + s);
             const PredCoef<float> pc{c.x, c.y, c.z};
             const SolveDesc sd = B.solves[s];
-            float a[3] = {0.f, 0.f, 0.f};
+            RunSum<float> a[3];
             // the two orders of the sets as they stand in the parameters: plane bases in uniform registers
             if (k < nli) b_list_item<MULTI>(B.L, in, out, pc, c.w, sd, st, k, a);
             else if (it & 1) b_tile_item<MULTI>(B.L, B.cls, s1, s0, pc, c.w, sd, st, k - nli, b_ring, a);
             else b_tile_item<MULTI>(B.L, B.cls, s0, s1, pc, c.w, sd, st, k - nli, b_ring, a);
-            // FP32 over a thread's column, FP64 from there on
-            const double sum = warp_sum3({(double)a[0], (double)a[1], (double)a[2]});
+            const double sum = warp_sum3({a[0].value(), a[1].value(), a[2].value()});
             const int lane = threadIdx.x & 31;
             if ((lane & 7) == 0 && lane <= 16)
                 partials[3 * ((long long)kTileWarps * (st.item0 + k) + threadIdx.x / 32) + lane / 8] = sum;
