@@ -1062,12 +1062,21 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
     const bool split_ok = !l6 && h->split_cls && (L.multi || one_ok);
     // automatic choice: the split path and the separate kernels where the split
     // path exists (the fused and staged paths are measured slower there on
-    // GB300 and stay available when pinned), every strategy elsewhere
+    // GB300 and stay available when pinned), every strategy elsewhere and for
+    // FP32 one-constant lattices with listed sites: with few of them split is
+    // the fastest (100 x 96 x 90, a wall: 44.1 us an iteration, staged 50.8),
+    // with many it is not (80^3, a wall: 38.2, fused 33.6; 64^3, a wall every
+    // five planes: 41.7 and 26.0).  Timed one after the other, bulk and listed
+    // sites say little about the two beside each other, so the best split
+    // candidate and the best of the others are replayed as an iteration runs them.
     const bool try_split = split_ok && (auto_mode || h->fire_mode == QMIN_FIRE_SPLIT);
     const bool try_sep = l6 || auto_mode || h->fire_mode == QMIN_FIRE_SEPARATE ||
                          (h->fire_mode == QMIN_FIRE_SPLIT && !split_ok);
-    const bool try_tiled = !l6 && sizeof(T) == 4 && ((auto_mode && !split_ok) || h->fire_mode == QMIN_FIRE_TILED);
-    const bool try_fused = !l6 && ((auto_mode && !split_ok) || h->fire_mode == QMIN_FIRE_FUSED);
+    const bool run_off = auto_mode && split_ok && sizeof(T) == 4 && !L.multi && h->n_split_sites > 0;
+    const bool others = (auto_mode && !split_ok) || run_off;
+    const bool try_tiled = !l6 && sizeof(T) == 4 && (others || h->fire_mode == QMIN_FIRE_TILED);
+    const bool try_fused = !l6 && (others || h->fire_mode == QMIN_FIRE_FUSED);
+    float best_split = kNoBudget;  // where the two are replayed; else `best` is the best of all
     if (try_sep || try_tiled || try_split) {
         const float t_plain = timed([&]() { return launch_fire_pred<T>(LB, h->fire, h->stream); }, kNoBudget);
         const size_t bytes = 5 * (size_t)h->P * h->esz;
@@ -1175,9 +1184,10 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
             budget_for(0.f));
         if (cudaGetLastError() != cudaSuccess) continue;
         h->tune_ms[kSepVariants + 2 * kFusedConfigs + 2 * kTiledConfigs + cap] = ms;
-        if (ms < best) {
-            best = ms;
-            h->path = 3;
+        float &least = run_off ? best_split : best;
+        if (ms < least) {
+            least = ms;
+            if (!run_off) h->path = 3;
             h->split_cap = cap;
         }
     }
@@ -1213,6 +1223,64 @@ template <class T> static int tune_fire(qmin_ctx *h, const Lat<T> &L)
             }
             if (zc >= h->Lz) break;
         }
+    }
+    if (run_off && best_split < kNoBudget && h->path >= 0) {
+        if ((r = ensure_aux(h))) return r;
+        // mean time of a launch over a graph of kReplay of them
+        constexpr int kReplay = 6;
+        auto replayed = [&](auto &&launch) -> float {
+            cudaGraph_t g = nullptr;
+            cudaGraphExec_t x = nullptr;
+            float ms = kNoBudget;
+            if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return ms;
+            int n = 0;
+            for (int k = 0; k < kReplay; ++k) n += launch();
+            if (cudaStreamEndCapture(h->stream, &g) == cudaSuccess &&
+                cudaGraphInstantiate(&x, g, cudaGraphInstantiateFlagUseNodePriority) == cudaSuccess) {
+                cudaGraphLaunch(x, h->stream);
+                ms = elapsed([&]() { cudaGraphLaunch(x, h->stream); }) / kReplay;
+                h->launches += 2 * n;
+            }
+            if (x) cudaGraphExecDestroy(x);
+            if (g) cudaGraphDestroy(g);
+            return ms;
+        };
+        const SplitLists sl = split_lists(h);
+        // writes the second set, as the fused kernel does
+        const float t_split = replayed([&]() {
+            cudaEventRecord(h->ev_fork, h->stream);
+            cudaStreamWaitEvent(h->aux, h->ev_fork, 0);
+            const int nd = launch_split_fused_deep<T>(L, (T *)h->Q2, (T *)h->V2, (T *)h->F2, sl, h->fire, h->partials,
+                                                      h->split_cap - kSplitFusedFirst, h->stream);
+            int nl = 0;
+            const int n = 1 + launch_split_fused_list<T>(L, (T *)h->V2, (T *)h->F2, sl, h->fire,
+                                                         h->partials + 3 * std::max(nd, 0), h->aux, &nl);
+            cudaEventRecord(h->ev_join, h->aux);
+            cudaStreamWaitEvent(h->stream, h->ev_join, 0);
+            return n;
+        });
+        float t_other = 0.f;
+        int nb = 0;
+        if (h->path == 1) {
+            t_other = replayed([&]() {
+                return launch_fire_fused<T>(h->fused_cfg, L, (T *)h->Q2, (T *)h->V2, (T *)h->F2, h->fire, h->partials,
+                                            h->fused_zc, h->stream, &nb);
+            });
+        } else {
+            const size_t bytes = 5 * (size_t)h->P * h->esz;
+            t_other = replayed([&]() { return launch_fire_pred<T>(LB, h->fire, h->stream); });
+            // the kick moves V
+            CK(cudaMemcpyAsync(h->V2, h->V, bytes, cudaMemcpyDeviceToDevice, h->stream));
+            CK(cudaMemcpyAsync(h->F2, h->F, bytes, cudaMemcpyDeviceToDevice, h->stream));
+            t_other += replayed([&]() {
+                return h->path == 2 ? launch_force_kick_tiled<T>(h->tiled_cfg, L, h->fire, h->partials, h->tiled_zc,
+                                                                 h->stream, &nb)
+                                    : launch_force_kick_only<T>(L, h->fire, h->partials, h->grid, h->stream, h->sep_cap);
+            });
+            CK(cudaMemcpyAsync(h->V, h->V2, bytes, cudaMemcpyDeviceToDevice, h->stream));
+            CK(cudaMemcpyAsync(h->F, h->F2, bytes, cudaMemcpyDeviceToDevice, h->stream));
+        }
+        if (t_split < t_other) h->path = 3;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
