@@ -24,6 +24,7 @@ def test_fixed_point_force_asks_for_no_planes(qmin, oracle, tmp_path):
         assert sum(n == planes for n in sizes()) == 4, "the staging buffer"
         assert rel_err(lat.force(), s.force()) <= 1e-12
         assert sum(n >= planes for n in sizes()) == 4
+        lat.set_fire_kernel(qmin.FIRE_SPLIT)
         lat.fire_init()
         r, ro = lat.fire_run(9), s.fire(9)
         assert lat.fire_tuning()["path"] == "split"
@@ -47,6 +48,7 @@ def test_no_room_for_the_fixed_point_form(qmin, oracle, tmp_path):
         for room in (True, False, True):
             s = system()
             lat = gpu_lattice(qmin, s, qmin.FP64)
+            lat.set_fire_kernel(qmin.FIRE_SPLIT)  # the separate kernels where there is none
             shim.shim_fail(8, 8, 0, 0 if room else 1000)
             lat.fire_init()
             r, ro = lat.fire_run(9), s.fire(9)

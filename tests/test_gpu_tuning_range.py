@@ -1,6 +1,6 @@
 """The strategy of an FP64 lattice does not hang on where its field is at the
 first run: a quench from noise below the fixed-point range, and a field with one
-value above it, take the strategy that a nematic start takes.  (64 x 56 x 60,
+value above it, take the strategy that a nematic start takes.  (96 x 80 x 88,
 where the fixed-point force is more than twice as fast as any other candidate.)"""
 import numpy as np
 import pytest
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("Ls", [(2.32, 0, 0, 0, 0), (2.32, 1.0, 0.5, 0, 0)], ids=["one", "multi"])
 @pytest.mark.parametrize("start", ["noise", "wide"])
 def test_choice_outside_the_range(qmin, oracle, start, Ls):
-    s = oracle.System((64, 56, 60), Ls=Ls)
+    s = oracle.System((96, 80, 88), Ls=Ls)
     s.random_nematic(5)
     s.add_wall(2, 0, 0, 5.3)
     nematic = s.Q.copy()
