@@ -188,7 +188,7 @@ def make_lattice(q, consts, g, precision):
 # the older strategies on a 128^3 case, scaled by the number of sites (their
 # traffic grows in proportion to the sites they process).
 DRAM_BYTES_PER_LAUNCH = {
-    ("force_kick_split", "f64"): 1031700000.0,   # 129.0 B/site (fixed-point force, 128^3 capture; 161 algorithmic)
+    ("force_kick_split", "f64"): 1270000000.0,   # 158.8 B/site (fixed-point force and listed sites; 161 algorithmic)
     ("force_kick_split", "f32"): 648814080.0,    # 81.1 B/site (81 algorithmic)
     ("fire_fused_split", "f32"): 939452544.0,    # 117.4 B/site (121 algorithmic)
     ("force_kick_reduce", "f64"): 2872800000.0,  # 359.1 B/site

@@ -52,8 +52,9 @@ template <class T> struct BatchArgs {
     // tile of its box (tx ty tz = 256, powers of two: lx = log2 tx, lxy = log2 tx ty)
     // cut where it overhangs the box
     int tx, ty, tz, lx, lxy;
-    // multi-constant: site classes (0 deep bulk, 1 other LC site, 2 object) and
-    // the sites whose derivative planes the class-1 forms read
+    // site classes (0 deep bulk, one-constant: LC sites without an object
+    // neighbour; 1 other LC site, 2 object); multi-constant: the sites whose
+    // derivative planes the class-1 forms read
     const uint8_t *cls, *needd;
 };
 
@@ -126,10 +127,12 @@ template <class T> struct BatchAcc {
 
 constexpr int kBatchWarps = kBlock / 32;  // warp partial sums per chunk
 // Blocks per SM of the FP64 iteration: three (80 registers, the listed sites'
-// form spills) take 367 us an iteration for 40 uneven one-constant solves (2.5 M
-// sites) and 442 for eight 64^3 multi-constant ones (2.1 M), two 401 and 475,
-// four 357 and 493: what bounds it is memory latency between its barriers
-// (floor at the measured HBM rate: 132 us and 109).
+// form spills) take 386 us an iteration for 40 uneven one-constant solves (2.5 M
+// sites), 496 for eight 64^3 multi-constant ones (2.1 M) and 133 for eight of 16
+// to 24; two 483 and 143 for the last two.  Before the low halves' products and
+// with read-only loads the first took 367, with two 401, with four 357: what
+// bounds it is memory latency between its barriers (floor at the measured HBM
+// rate: 132 us and 109).
 constexpr int kFixedPerSm = 3;
 
 // one set of packed state planes (Q, V, F)
@@ -564,7 +567,7 @@ constexpr int kMaxBatchSolves = 16384;  // the lists take 8 (nsolves + 1) bytes 
 // kept by every block in shared memory
 struct ActiveList {
     int *act, *pre;
-    int n, all;  // active solves; whether that is every solve
+    int n;  // active solves
 };
 
 // one warp's ballot over the solves in order; count(s): the work of solve s
@@ -593,7 +596,6 @@ template <class COUNT> __device__ __forceinline__ void b_rebuild(ActiveList *al,
         }
         if (threadIdx.x == 0) {
             al->n = n;
-            al->all = n == nsolves;
             al->pre[n] = tot;
         }
     }
@@ -675,10 +677,10 @@ struct TileItems {
 // FP64: predictor, (derivative planes,) force + kick, a grid barrier after
 // each; the block that finishes a solve's last item does its control.  The
 // bulk force runs in fixed point (the FP64 pipe took 948 us an iteration for
-// 2.5 M one-constant sites and 1420 for 2.1 M multi-constant ones, 367 and 442
+// 2.5 M one-constant sites and 1420 for 2.1 M multi-constant ones, 386 and 496
 // now); listed sites are items of their own, taken first, so that no warp waits
 // for one of them (546 with them inside the bulk runs, each chunk of 256 an
-// item; control as a phase with two more barriers 573).
+// item; control as a phase with two more barriers 573; 367 without either).
 // FP32 multi-constant solves come here when there is no room for the second
 // state set of k_b_fire_tiled.
 template <class T, bool MULTI>
@@ -1098,7 +1100,8 @@ static int classify_solves(qmin_batch_ctx *b)
 // 32 wide and 32 high), z chunks of 4 to 16 planes so that there are about four
 // items per resident block (two, three and six measured within 5 %).  Otherwise
 // runs of 1 to 8 blocks' sites, by the same rule (40 uneven solves, 2.5 M sites:
-// 431 us with runs of one block's sites, 389 two, 370 four, 367 eight, 382 ten).
+// 431 us with runs of one block's sites, 389 two, 370 four, 367 eight, 382 ten,
+// when it was 367).
 static int lay_out_items(qmin_batch_ctx *b, bool multi, bool tiled)
 {
     if (!b->tiles_h.empty() && b->tiles_multi == multi && b->tiles_tiled == tiled) return QMIN_OK;

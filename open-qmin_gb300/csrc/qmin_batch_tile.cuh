@@ -19,14 +19,15 @@
 namespace qmin {
 
 // 128 threads, three blocks per SM (168 registers; the multi-constant form
-// spills 270 bytes): 64 uneven one-constant solves (4.4 M sites) take 180 us an
-// iteration and eight 64^3 multi-constant ones (2.1 M sites) 183; four blocks per SM 183 and 199 (864
+// spills 284 bytes): 64 uneven one-constant solves (4.4 M sites) take 176 us an
+// iteration and eight 64^3 multi-constant ones (2.1 M sites) 185; when it was
+// 180 and 183, four blocks per SM took 183 and 199 (864
 // bytes spilled), five 235 and 202, 256 threads 182 and 210, tiles at most 16
 // wide 202 and 221.  The site-by-site form this replaced took 290 and 465:
 // every neighbour's prediction formed again (one-constant), derivative planes
-// at every site and 91 stencil reads through L1 (multi-constant).  Now 34 % of
-// the issue slots and 44 % of the measured HBM rate: plane loads one plane
-// ahead at 12 warps per SM.
+// at every site and 91 stencil reads through L1 (multi-constant).  Now 34 %
+// of the issue slots and 47 % of the measured HBM rate (one-constant), 26 % and
+// 26 % (multi-constant): plane loads one plane ahead at 12 warps per SM.
 constexpr int kTileThreads = 128, kTileWarps = kTileThreads / 32, kTilePerSm = 3, kTileWide = 32;
 constexpr int kTilePlane = 204;  // sites of a staged plane: at most (32 + 2) x (4 + 2)
 constexpr int kTileHalo = 96;  // halo entries of a plane: at most 2 (32 + 2) + 2 x 8, 2 (4 + 2) + 2 x 32

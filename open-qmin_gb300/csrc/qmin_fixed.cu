@@ -63,12 +63,12 @@ __global__ void __launch_bounds__(kBlock)
 // Multi-constant lattices leave it to k_force_kick_deep: with both forms in one
 // kernel the fixed-point one spills (83 x 61 x 97: 8.3 ms instead of 7.3).
 //
-// 1,080 instructions per warp and site group against 173 FP64 operations (2,770
+// 1,400 instructions per warp and site group against 173 FP64 operations (2,770
 // cycles of the FP64 pipe) of k_force_kick_deep; 26 FP64 operations are left
 // (metric 4, kick 5, sums 17), about half of the time they would need alone.
 // What bounds it is the latency of its 91 stencil reads and its chains at 16
 // warps per SM.  A grid of the resident blocks takes the sites in order:
-// 128-thread blocks four to an SM are 0.56 ms at 200^3 (256-thread ones 0.57,
+// 128-thread blocks four to an SM are 0.55 to 0.56 ms at 200^3 (256-thread ones 0.57,
 // boxes of 32 x 4 x 2 sites 0.62, 4 grids' worth of blocks 0.61), and no box
 // is left partly empty on a small or odd lattice.
 template <bool MULTI, bool KICK>

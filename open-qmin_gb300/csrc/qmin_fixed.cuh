@@ -92,7 +92,8 @@ QMIN_DEV int fix_mul_high(int a, int b, int c)
 // farther from quadruple precision than with the FP64 force, with them 1 % +-
 // 2 % (means over 400 starts; from smooth fields 27 and 38 % nearer).  They
 // cost 1.3 to 1.8 % of a run (50^3 one-constant, 100 iterations: 3.10 -> 3.14
-// ms, 83 x 61 x 97, 60: 7.42 -> 7.53, 200^3, 40: 41.9 -> 42.7).
+// ms, 83 x 61 x 97, 60: 7.42 -> 7.53, 200^3, 40: 41.9 -> 42.7), 5.5 % of a
+// multi-constant batch (eight 64^3: 470 -> 496 us an iteration).
 struct FixAcc {
     long long hi, mid;
     int lo;

@@ -880,12 +880,13 @@ __global__ void __launch_bounds__(kBlock) k_lb_close(IterDev *it, int m, const d
     it->active = (it->iterations < it->max_iters && it->forceMax > it->fcut) ? 1 : 0;
 }
 
-// FP32 and up to kLbGram pairs: the two-loop recursion on coefficients.  The
+// FP32 and up to kLbGram pairs: the two-loop recursion on coefficients (the
+// vector-free L-BFGS of Chen, Wang and Zhou, 2014).  The
 // step is p = F + sum cy_j y_j + sum cs_j s_j, and every dot product the
 // recursion takes is a sum over s_i . y_j, y_i . y_j, s_i . F and y_i . F.  Of
 // these an iteration changes those of the new pair and of F: one pass over the
 // pairs after the force forms them (k_lbg_post), one block runs the recursion in
-// FP64 (k_lbg_solve), one pass applies it with the step (k_lbg_step): 6 m - 1
+// FP64 (k_lbg_solve), one pass applies it with the step (k_lbg_step): 4 m + 7
 // vectors of 5 N values move, force aside, instead of the 8 m + 7 of the passes above.
 // Bound by HBM: at 200^3 and m = 5 0.67 ms (6.9 and 6.3 TB/s) instead of 1.24.
 // FP64 keeps the passes: 5 m + 1 products a value would bound it on the FP64 pipe.
@@ -925,7 +926,7 @@ __global__ void __launch_bounds__(kBlock)
     }
 }
 
-// hi + lo += x, exact up to the rounding of lo
+// hi + lo += x, exact up to the rounding of lo (Knuth's two-sum)
 __device__ __forceinline__ void add_twice(float &hi, float &lo, float x)
 {
     const float s = __fadd_rn(hi, x), b = __fsub_rn(s, hi);
