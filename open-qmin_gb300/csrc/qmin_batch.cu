@@ -893,6 +893,8 @@ struct qmin_batch_ctx {
     std::vector<SolveLists> lists;
     bool tiles_multi = false, tiles_tiled = false, classified_multi = false;
     void *geo_scratch = nullptr;
+    size_t geo_bytes = 0;
+    std::vector<int *> list_mem;  // what the lists are cut from
     long long *X = nullptr;  // FP64: Q 2^56 of the fixed-point force
     int2 *range = nullptr;
     int *done = nullptr;  // per solve: items of the phase that are done
@@ -1055,43 +1057,99 @@ template <class T> static int tune_shape(qmin_batch_ctx *b)
 
 // Site classes of every solve whose types changed since they were last taken,
 // on the device: classes, the derivative-plane marks and the two lists
-// (multi-constant), or the boundary sites (one-constant).
+// (multi-constant), or the boundary sites (one-constant).  The solves go in
+// groups of up to kGeoScratch bytes of scratch, each one set of launches, one
+// wait for the list sizes and one allocation (a solve at a time: 107 us for
+// each of 600 multi-constant ones of 6 to 8 cubed, 64 ms of their first run).
+constexpr size_t kGeoScratch = 8u << 20;
 static int classify_solves(qmin_batch_ctx *b)
 {
     const bool multi = b->params.multi_constant != 0;
     if (b->classified_multi != multi)
         for (auto &l : b->lists) l.classified = false;
     b->classified_multi = multi;
+    std::vector<int> todo;  // a solve that was never set is all type 0
+    for (int s = 0; s < b->nsolves; ++s)
+        if (!b->lists[s].classified) todo.push_back(s);
+    if (!todo.empty()) b->tiles_h.clear();
 
-    for (int s = 0; s < b->nsolves; ++s) {
-        auto &l = b->lists[s];
-        if (l.classified) continue;  // a solve that was never set is all type 0
+    constexpr size_t kRow = 32 * sizeof(int);  // a job's totals
+    auto bytes_of = [&](int s) {
         const SolveDesc &sd = b->solves_h[s];
-        if (!b->geo_scratch && cudaMalloc(&b->geo_scratch, split_scratch_bytes(b->maxN)) != cudaSuccess) {
-            cudaGetLastError();
-            return bfail(QMIN_ENOMEM, "batch site lists: scratch allocation failed");
+        return (split_scratch_bytes(sd.Lx * sd.Ly * sd.Lz) + 255) / 256 * 256 + sizeof(GeoJob) + kRow;
+    };
+    for (size_t g0 = 0, g1 = 0; g0 < todo.size(); g0 = g1) {
+        size_t bytes = 0;
+        for (g1 = g0; g1 < todo.size() && (g1 == g0 || bytes + bytes_of(todo[g1]) <= kGeoScratch); ++g1)
+            bytes += bytes_of(todo[g1]);
+        const int nj = (int)(g1 - g0);
+        if (b->geo_bytes < bytes) {
+            if (b->geo_scratch) cudaFree(b->geo_scratch);
+            b->geo_scratch = nullptr;
+            b->geo_bytes = 0;
+            if (cudaMalloc(&b->geo_scratch, bytes) != cudaSuccess) {
+                cudaGetLastError();
+                return bfail(QMIN_ENOMEM, "batch site lists: scratch allocation failed");
+            }
+            b->geo_bytes = bytes;
         }
-        int totals[32];
-        int n = multi ? build_split_lists_dev(b->types + sd.off, sd.Lx, sd.Ly, sd.Lz, b->cls + sd.off, b->geo_scratch,
-                                            totals, &l.sites, &l.sites_cap, &l.n_sites, &l.derivs, &l.derivs_cap,
-                                            &l.n_derivs, b->stream)
-                          : build_boundary_list_dev(b->types + sd.off, sd.Lx, sd.Ly, sd.Lz, b->cls + sd.off,
-                                                    b->geo_scratch, &l.sites, &l.sites_cap, &l.n_sites, b->stream);
-        if (n == -2) {
-            cudaGetLastError();
-            return bfail(QMIN_ENOMEM, "batch site lists: allocation failed");
+        // per-job scratch (256-byte steps), totals, jobs
+        std::vector<GeoJob> jobs((size_t)nj);
+        std::vector<int> totals((size_t)nj * 32);
+        char *p = (char *)b->geo_scratch;
+        size_t largest = 0;
+        for (int k = 0; k < nj; ++k) {
+            const SolveDesc &sd = b->solves_h[todo[g0 + k]];
+            GeoJob &J = jobs[k] = geo_job(b->types + sd.off, sd.Lx, sd.Ly, sd.Lz, b->cls + sd.off, p);
+            p += (split_scratch_bytes(J.N) + 255) / 256 * 256;
+            J.need = b->needd + sd.off;
+            J.D = multi ? (char *)b->D + (size_t)sd.off * b->esz : nullptr;
+            if (J.N > jobs[largest].N) largest = (size_t)k;
         }
-        if (n < 0) return bfail(QMIN_ECUDA, std::string("batch site lists: ") + cudaGetErrorString(cudaGetLastError()));
-        b->launches += n;
-        if (multi) {
-            b->launches += launch_need_marks(b->geo_scratch, sd.Lx * sd.Ly * sd.Lz, b->needd + sd.off, b->stream);
-            // derivative planes of a previous geometry: object sites' are read as zero and never written
-            for (int k = 0; k < 15; ++k)
-                BCK(cudaMemsetAsync((char *)b->D + ((size_t)k * b->P + sd.off) * b->esz, 0,
-                                    (size_t)sd.Lx * sd.Ly * sd.Lz * b->esz, b->stream));
+        int *dtotals = (int *)p;
+        for (int k = 0; k < nj; ++k) jobs[k].totals = dtotals + 32 * k;
+        GeoJob *djobs = (GeoJob *)(p + kRow * (size_t)nj);
+        BCK(cudaMemcpyAsync(djobs, jobs.data(), sizeof(GeoJob) * (size_t)nj, cudaMemcpyHostToDevice, b->stream));
+        b->launches += launch_geo_count(multi, jobs[largest], djobs, nj, b->stream);
+        BCK(cudaMemcpyAsync(totals.data(), dtotals, kRow * (size_t)nj, cudaMemcpyDeviceToHost, b->stream));
+        BCK(cudaStreamSynchronize(b->stream));
+        // room for the lists that outgrew theirs (half as much again, so that a changing geometry settles)
+        std::vector<int> ns((size_t)nj), nd((size_t)nj);
+        auto room = [](int n, int cap) { return n <= cap ? 0 : (cap ? n + n / 2 : n); };
+        size_t more = 0;
+        for (int k = 0; k < nj; ++k) {
+            const auto &l = b->lists[todo[g0 + k]];
+            geo_sizes(multi, &totals[(size_t)32 * k], &ns[k], &nd[k]);
+            more += (size_t)room(ns[k], l.sites_cap) + (size_t)room(nd[k], l.derivs_cap);
         }
-        l.classified = true;
-        b->tiles_h.clear();
+        int *at = nullptr;
+        if (more > 0) {
+            if (cudaMalloc(&at, sizeof(int) * more) != cudaSuccess) {
+                cudaGetLastError();
+                return bfail(QMIN_ENOMEM, "batch site lists: allocation failed");
+            }
+            b->list_mem.push_back(at);
+        }
+        bool any = false, anyd = false;
+        for (int k = 0; k < nj; ++k) {
+            auto &l = b->lists[todo[g0 + k]];
+            if (const int r = room(ns[k], l.sites_cap)) l.sites = at, l.sites_cap = r, at += r;
+            if (const int r = room(nd[k], l.derivs_cap)) l.derivs = at, l.derivs_cap = r, at += r;
+            l.n_sites = ns[k];
+            l.n_derivs = nd[k];
+            l.classified = true;
+            jobs[k].sites = l.sites;
+            jobs[k].derivs = l.derivs;
+            any = any || ns[k] > 0;
+            anyd = anyd || nd[k] > 0;
+        }
+        BCK(cudaMemcpyAsync(djobs, jobs.data(), sizeof(GeoJob) * (size_t)nj, cudaMemcpyHostToDevice, b->stream));
+        b->launches += launch_geo_fill(multi, jobs[largest], djobs, nj, any, anyd, b->stream);
+        if (multi)
+            b->launches += b->prec == QMIN_FP64
+                               ? launch_need_marks<double>(jobs[largest], djobs, nj, b->P, b->stream)
+                               : launch_need_marks<float>(jobs[largest], djobs, nj, b->P, b->stream);
+        BCK(cudaGetLastError());
     }
     return QMIN_OK;
 }
@@ -1322,10 +1380,7 @@ int qmin_batch_destroy(qmin_batch b)
                     b->tiles, b->coefs, b->tile_partials, b->geo_scratch, b->X, b->range, b->done};
     for (void *p : bufs)
         if (p) cudaFree(p);
-    for (auto &l : b->lists) {
-        if (l.sites) cudaFree(l.sites);
-        if (l.derivs) cudaFree(l.derivs);
-    }
+    for (int *p : b->list_mem) cudaFree(p);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return QMIN_OK;

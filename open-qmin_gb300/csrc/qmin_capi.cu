@@ -556,9 +556,7 @@ static int build_split_lists(qmin_ctx *h)
         }
         h->geo_scratch_bytes = need;
     }
-    int totals[32];
-    const int n = build_split_lists_dev(h->types, h->Lx, h->Ly, h->Lz, h->split_cls, h->geo_scratch, totals,
-                                        &h->split_sites, &h->split_sites_cap, &h->n_split_sites, &h->split_derivs,
+    const int n = build_split_lists_dev(h->types, h->Lx, h->Ly, h->Lz, h->split_cls, h->geo_scratch, &h->split_sites, &h->split_sites_cap, &h->n_split_sites, &h->split_derivs,
                                         &h->split_derivs_cap, &h->n_split_derivs, h->stream);
     if (n == -2) {
         cudaGetLastError();

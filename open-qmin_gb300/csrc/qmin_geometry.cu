@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 #include <string>
 
 #include "qmin_internal.h"
@@ -103,11 +104,21 @@ __device__ __forceinline__ void site_xyz(int i, int Lx, int Ly, int &x, int &y, 
     z = r / Ly;
 }
 
+// The kernels below do one lattice (`one`, many null) or, of several, the one of
+// their blockIdx.y: a batch's new geometries take one set of launches.
+__device__ __forceinline__ GeoJob job_of(const GeoJob &one, const GeoJob *many)
+{
+    return many ? many[blockIdx.y] : one;
+}
+
 // class of every site and the form key of the listed sites (kNoBucket otherwise)
 __global__ void __launch_bounds__(kScanBlock)
-    k_split_classify(const int8_t *__restrict__ t8, int Lx, int Ly, int Lz, uint8_t *cls, uint8_t *key)
+    k_split_classify(const __grid_constant__ GeoJob one, const GeoJob *many)
 {
-    const int N = Lx * Ly * Lz;
+    const GeoJob J = job_of(one, many);
+    const int8_t *__restrict__ t8 = J.t8;
+    uint8_t *cls = J.cls, *key = J.key;
+    const int Lx = J.Lx, Ly = J.Ly, Lz = J.Lz, N = J.N;
     for (int i = blockIdx.x * kScanBlock + threadIdx.x; i < N; i += gridDim.x * kScanBlock) {
         const int t = t8[i];
         if (t > 0) {
@@ -152,9 +163,12 @@ __global__ void __launch_bounds__(kScanBlock)
 // key 0 at every LC site one of whose six neighbours is a listed site (an
 // object site's derivative planes are zero, and stay so: they are never listed)
 __global__ void __launch_bounds__(kScanBlock)
-    k_split_need(const uint8_t *__restrict__ cls, int Lx, int Ly, int Lz, uint8_t *key)
+    k_split_need(const __grid_constant__ GeoJob one, const GeoJob *many)
 {
-    const int N = Lx * Ly * Lz;
+    const GeoJob J = job_of(one, many);
+    const uint8_t *__restrict__ cls = J.cls;
+    uint8_t *key = J.key2;
+    const int Lx = J.Lx, Ly = J.Ly, Lz = J.Lz, N = J.N;
     for (int i = blockIdx.x * kScanBlock + threadIdx.x; i < N; i += gridDim.x * kScanBlock) {
         int x, y, z;
         site_xyz(i, Lx, Ly, x, y, z);
@@ -168,10 +182,15 @@ __global__ void __launch_bounds__(kScanBlock)
     }
 }
 
-// per-chunk histogram of the keys below NB
-template <int NB>
-__global__ void __launch_bounds__(kScanBlock) k_bucket_count(const uint8_t *__restrict__ key, int N, int *counts)
+// per-chunk histogram of the keys below NB; LIST 0: the listed sites, 1: the derivative sites
+template <int NB, int LIST>
+__global__ void __launch_bounds__(kScanBlock) k_bucket_count(const __grid_constant__ GeoJob one, const GeoJob *many)
 {
+    const GeoJob J = job_of(one, many);
+    if (blockIdx.x >= J.nch) return;
+    const uint8_t *__restrict__ key = LIST ? J.key2 : J.key;
+    int *counts = LIST ? J.counts2 : J.counts;
+    const int N = J.N;
     __shared__ int h[NB];
     for (int b = threadIdx.x; b < NB; b += kScanBlock) h[b] = 0;
     __syncthreads();
@@ -187,9 +206,13 @@ __global__ void __launch_bounds__(kScanBlock) k_bucket_count(const uint8_t *__re
 // offsets[chunk][bucket]: the list is bucket-major, chunk order within a bucket;
 // totals[bucket] the bucket sizes.  One block; each bucket is an exclusive scan
 // over the chunks, in fixed order.
-template <int NB>
-__global__ void __launch_bounds__(1024) k_bucket_offsets(const int *counts, int nchunks, int *offsets, int *totals)
+template <int NB, int LIST>
+__global__ void __launch_bounds__(1024) k_bucket_offsets(const __grid_constant__ GeoJob one, const GeoJob *many)
 {
+    const GeoJob J = job_of(one, many);
+    const int *counts = LIST ? J.counts2 : J.counts;
+    int *offsets = LIST ? J.offsets2 : J.offsets, *totals = J.totals + (LIST ? kForms : 0);
+    const int nchunks = J.nch;
     __shared__ int carry;
     __shared__ int warp_sums[32];
     if (threadIdx.x == 0) carry = 0;
@@ -233,10 +256,15 @@ __global__ void __launch_bounds__(1024) k_bucket_offsets(const int *counts, int 
 
 // one warp per chunk: every site with key k < NB goes to offsets[chunk][k] +
 // (its rank among the chunk's earlier sites with key k)
-template <int NB>
-__global__ void __launch_bounds__(32)
-    k_bucket_scatter(const uint8_t *__restrict__ key, int N, const int *__restrict__ offsets, int *out)
+template <int NB, int LIST>
+__global__ void __launch_bounds__(32) k_bucket_scatter(const __grid_constant__ GeoJob one, const GeoJob *many)
 {
+    const GeoJob J = job_of(one, many);
+    if (blockIdx.x >= J.nch) return;
+    const uint8_t *__restrict__ key = LIST ? J.key2 : J.key;
+    const int *__restrict__ offsets = LIST ? J.offsets2 : J.offsets;
+    int *out = LIST ? J.derivs : J.sites;
+    const int N = J.N;
     __shared__ int run[NB];
     for (int b = threadIdx.x; b < NB; b += 32) run[b] = offsets[blockIdx.x * NB + b];
     __syncwarp();
@@ -259,7 +287,6 @@ __global__ void __launch_bounds__(32)
     }
 }
 
-constexpr int kForms = 28;  // listed-site forms: bulk-like and the 27 boundary cases
 
 }  // namespace
 
@@ -279,9 +306,12 @@ template int scan_types<int8_t>(const int8_t *, const int8_t *, int, int *, int 
 
 // class (0 type-0 sites without an object neighbour, 1 other LC sites, 2 objects) and key 0 at the class-1 sites
 __global__ void __launch_bounds__(kScanBlock)
-    k_boundary_classify(const int8_t *__restrict__ t8, int Lx, int Ly, int Lz, uint8_t *cls, uint8_t *key)
+    k_boundary_classify(const __grid_constant__ GeoJob one, const GeoJob *many)
 {
-    const int N = Lx * Ly * Lz;
+    const GeoJob J = job_of(one, many);
+    const int8_t *__restrict__ t8 = J.t8;
+    uint8_t *cls = J.cls, *key = J.key;
+    const int Lx = J.Lx, Ly = J.Ly, Lz = J.Lz, N = J.N;
     for (int i = blockIdx.x * kScanBlock + threadIdx.x; i < N; i += gridDim.x * kScanBlock) {
         const int t = t8[i];
         int c = t > 0 ? 2 : (t < 0 ? 1 : 0);
@@ -299,17 +329,19 @@ __global__ void __launch_bounds__(kScanBlock)
     }
 }
 
-// 1 where the derivative list of the build_split_lists_dev call that filled `scratch` holds the site
-__global__ void __launch_bounds__(kScanBlock) k_need_marks(const uint8_t *__restrict__ key, int N, uint8_t *need)
+// 1 where the derivative list holds the site; the derivative planes of object
+// sites zero (they are read and never written; a previous geometry may have)
+template <class T>
+__global__ void __launch_bounds__(kScanBlock) k_need_marks(const GeoJob *many, long long P)
 {
-    for (int i = blockIdx.x * kScanBlock + threadIdx.x; i < N; i += gridDim.x * kScanBlock) need[i] = key[i] == 0;
-}
-
-int launch_need_marks(const void *scratch, int N, uint8_t *need, cudaStream_t s)
-{
-    const int grid = std::max(1, std::min((N + kScanBlock - 1) / kScanBlock, 152 * 8));
-    k_need_marks<<<grid, kScanBlock, 0, s>>>(reinterpret_cast<const uint8_t *>(scratch) + N, N, need);
-    return 1;
+    const GeoJob J = many[blockIdx.y];
+    T *D = (T *)J.D;
+    for (int i = blockIdx.x * kScanBlock + threadIdx.x; i < J.N; i += gridDim.x * kScanBlock) {
+        J.need[i] = J.key2[i] == 0;
+        if (J.cls[i] == 2)
+#pragma unroll
+            for (int k = 0; k < 15; ++k) D[k * P + i] = T(0);
+    }
 }
 
 size_t split_scratch_bytes(int N)
@@ -330,63 +362,86 @@ static bool ensure_list(int **p, int *cap, int need)
     return true;
 }
 
-int build_boundary_list_dev(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch, int **sites,
-                            int *sites_cap, int *n_sites, cudaStream_t s)
+GeoJob geo_job(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch)
 {
-    const int N = Lx * Ly * Lz;
-    const int nch = (N + kBucketChunk - 1) / kBucketChunk;
-    uint8_t *key = reinterpret_cast<uint8_t *>(scratch);
-    int *counts = reinterpret_cast<int *>(reinterpret_cast<uintptr_t>(key + N + 15) & ~(uintptr_t)15),
-        *offsets = counts + nch, *total = offsets + nch;
-    const int grid = std::max(1, std::min((N + kScanBlock - 1) / kScanBlock, 152 * 8));
-    k_boundary_classify<<<grid, kScanBlock, 0, s>>>(t8, Lx, Ly, Lz, cls, key);
-    k_bucket_count<1><<<nch, kScanBlock, 0, s>>>(key, N, counts);
-    k_bucket_offsets<1><<<1, 1024, 0, s>>>(counts, nch, offsets, total);
-    int n = 0;
-    if (cudaMemcpyAsync(&n, total, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-        return -1;
-    if (!ensure_list(sites, sites_cap, n)) return -2;
-    if (n > 0) k_bucket_scatter<1><<<nch, 32, 0, s>>>(key, N, offsets, *sites);
-    *n_sites = n;
-    return cudaGetLastError() == cudaSuccess ? 3 + (n > 0) : -1;
+    GeoJob j;
+    memset(&j, 0, sizeof j);
+    j.t8 = t8;
+    j.Lx = Lx;
+    j.Ly = Ly;
+    j.Lz = Lz;
+    j.N = Lx * Ly * Lz;
+    j.nch = (j.N + kBucketChunk - 1) / kBucketChunk;
+    j.cls = cls;
+    j.key = reinterpret_cast<uint8_t *>(scratch);
+    j.key2 = j.key + j.N;
+    j.counts = reinterpret_cast<int *>(reinterpret_cast<uintptr_t>(j.key2 + j.N + 15) & ~(uintptr_t)15);
+    j.offsets = j.counts + (size_t)j.nch * kForms;
+    j.counts2 = j.offsets + (size_t)j.nch * kForms;
+    j.offsets2 = j.counts2 + j.nch;
+    j.totals = j.offsets2 + j.nch;
+    return j;
 }
 
-int build_split_lists_dev(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch, int *host_totals,
-                          int **sites, int *sites_cap, int *n_sites, int **derivs, int *derivs_cap, int *n_derivs,
-                          cudaStream_t s)
+int launch_geo_count(bool multi, const GeoJob &one, const GeoJob *many, int njobs, cudaStream_t s)
 {
-    const int N = Lx * Ly * Lz;
-    const int nch = (N + kBucketChunk - 1) / kBucketChunk;
-    uint8_t *key = reinterpret_cast<uint8_t *>(scratch);
-    uint8_t *key2 = key + N;
-    int *ib = reinterpret_cast<int *>(reinterpret_cast<uintptr_t>(key2 + N + 15) & ~(uintptr_t)15);
-    int *counts = ib, *offsets = counts + (size_t)nch * kForms, *counts2 = offsets + (size_t)nch * kForms,
-        *offsets2 = counts2 + nch, *totals = offsets2 + nch;  // totals: kForms + 1 ints
-    const int grid = std::max(1, std::min((N + kScanBlock - 1) / kScanBlock, 152 * 8));
-    int n = 0;
-    k_split_classify<<<grid, kScanBlock, 0, s>>>(t8, Lx, Ly, Lz, cls, key);
-    k_split_need<<<grid, kScanBlock, 0, s>>>(cls, Lx, Ly, Lz, key2);
-    k_bucket_count<kForms><<<nch, kScanBlock, 0, s>>>(key, N, counts);
-    k_bucket_count<1><<<nch, kScanBlock, 0, s>>>(key2, N, counts2);
-    k_bucket_offsets<kForms><<<1, 1024, 0, s>>>(counts, nch, offsets, totals);
-    k_bucket_offsets<1><<<1, 1024, 0, s>>>(counts2, nch, offsets2, totals + kForms);
-    n += 6;
-    if (cudaMemcpyAsync(host_totals, totals, (kForms + 1) * sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+    const dim3 g(std::max(1, std::min((one.N + kScanBlock - 1) / kScanBlock, 152 * 8)), njobs), gc(one.nch, njobs),
+        g1(1, njobs);
+    if (!multi) {
+        k_boundary_classify<<<g, kScanBlock, 0, s>>>(one, many);
+        k_bucket_count<1, 0><<<gc, kScanBlock, 0, s>>>(one, many);
+        k_bucket_offsets<1, 0><<<g1, 1024, 0, s>>>(one, many);
+        return 3;
+    }
+    k_split_classify<<<g, kScanBlock, 0, s>>>(one, many);
+    k_split_need<<<g, kScanBlock, 0, s>>>(one, many);
+    k_bucket_count<kForms, 0><<<gc, kScanBlock, 0, s>>>(one, many);
+    k_bucket_count<1, 1><<<gc, kScanBlock, 0, s>>>(one, many);
+    k_bucket_offsets<kForms, 0><<<g1, 1024, 0, s>>>(one, many);
+    k_bucket_offsets<1, 1><<<g1, 1024, 0, s>>>(one, many);
+    return 6;
+}
+
+void geo_sizes(bool multi, const int *totals, int *n_sites, int *n_derivs)
+{
+    *n_sites = 0;
+    for (int b = 0; b < (multi ? kForms : 1); ++b) *n_sites += totals[b];
+    *n_derivs = multi ? totals[kForms] : 0;
+}
+
+int launch_geo_fill(bool multi, const GeoJob &one, const GeoJob *many, int njobs, bool sites, bool derivs,
+                    cudaStream_t s)
+{
+    const dim3 gc(one.nch, njobs);
+    if (sites && multi) k_bucket_scatter<kForms, 0><<<gc, 32, 0, s>>>(one, many);
+    else if (sites) k_bucket_scatter<1, 0><<<gc, 32, 0, s>>>(one, many);
+    if (derivs) k_bucket_scatter<1, 1><<<gc, 32, 0, s>>>(one, many);
+    return (sites ? 1 : 0) + (derivs ? 1 : 0);
+}
+
+template <class T> int launch_need_marks(const GeoJob &largest, const GeoJob *many, int njobs, long long P, cudaStream_t s)
+{
+    const dim3 g(std::max(1, std::min((largest.N + kScanBlock - 1) / kScanBlock, 152 * 8)), njobs);
+    k_need_marks<T><<<g, kScanBlock, 0, s>>>(many, P);
+    return 1;
+}
+template int launch_need_marks<float>(const GeoJob &, const GeoJob *, int, long long, cudaStream_t);
+template int launch_need_marks<double>(const GeoJob &, const GeoJob *, int, long long, cudaStream_t);
+
+int build_split_lists_dev(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch, int **sites,
+                          int *sites_cap, int *n_sites, int **derivs, int *derivs_cap, int *n_derivs, cudaStream_t s)
+{
+    GeoJob j = geo_job(t8, Lx, Ly, Lz, cls, scratch);
+    int totals[kForms + 1], ns = 0, nd = 0;
+    int n = launch_geo_count(true, j, nullptr, 1, s);
+    if (cudaMemcpyAsync(totals, j.totals, sizeof totals, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return -1;
-    int ns = 0;
-    for (int b = 0; b < kForms; ++b) ns += host_totals[b];
-    const int nd = host_totals[kForms];
+    geo_sizes(true, totals, &ns, &nd);
     if (!ensure_list(sites, sites_cap, ns) || !ensure_list(derivs, derivs_cap, nd)) return -2;
-    if (ns > 0) {
-        k_bucket_scatter<kForms><<<nch, 32, 0, s>>>(key, N, offsets, *sites);
-        ++n;
-    }
-    if (nd > 0) {
-        k_bucket_scatter<1><<<nch, 32, 0, s>>>(key2, N, offsets2, *derivs);
-        ++n;
-    }
+    j.sites = *sites;
+    j.derivs = *derivs;
+    n += launch_geo_fill(true, j, nullptr, 1, ns > 0, nd > 0, s);
     *n_sites = ns;
     *n_derivs = nd;
     if (cudaGetLastError() != cudaSuccess) return -1;

@@ -218,19 +218,36 @@ int launch_split_deep(const Lat<T> &L, const SplitLists &sl, FireDev *fd, double
 // call synchronises the stream; part: 4 * 608 ints, out_dev: 4 ints)
 template <class TT>
 int scan_types(const TT *t, const int8_t *old8, int N, int *part, int *out_dev, int *out_host, cudaStream_t s);
-// the split path's classes and lists from the device types (qmin_geometry.cu):
-// cls (N bytes) written, *sites / *derivs grown as needed, host_totals: 29 ints;
-// scratch of split_scratch_bytes(N).  Returns the launch count, < 0 on failure.
+// Classes and lists from the device types (qmin_geometry.cu).  One lattice's
+// part: its types and classes (N bytes each), its scratch (split_scratch_bytes(N)
+// behind geo_job's pointers), its lists, and in a batch the derivative marks and planes.
+struct GeoJob {
+    const int8_t *t8;
+    uint8_t *cls, *key, *key2;
+    int *counts, *offsets, *counts2, *offsets2, *totals;  // totals: kForms + 1 ints
+    int *sites, *derivs;
+    uint8_t *need;
+    void *D;
+    int Lx, Ly, Lz, N, nch;
+};
+constexpr int kForms = 28;  // listed-site forms: bulk-like and the 27 boundary cases
 size_t split_scratch_bytes(int N);
-// one-constant classes (0 type 0 without an object neighbour, 1 other LC sites, 2 objects) and the class-1 sites in
-// site order; same scratch and returns
-int build_boundary_list_dev(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch, int **sites,
-                            int *sites_cap, int *n_sites, cudaStream_t s);
-// after build_split_lists_dev, from the same scratch: 1 where a site is in the derivative list
-int launch_need_marks(const void *scratch, int N, uint8_t *need, cudaStream_t s);
-int build_split_lists_dev(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch, int *host_totals,
-                          int **sites, int *sites_cap, int *n_sites, int **derivs, int *derivs_cap, int *n_derivs,
-                          cudaStream_t s);
+GeoJob geo_job(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch);
+// Of one job (many null) or the njobs at `many` on the device, `one` then the
+// largest of them: classes and list sizes into totals (multi: the split path's;
+// else 0 type 0 without an object neighbour, 1 other LC sites, 2 objects, and
+// the class-1 sites in site order), then the lists.  Return the launch count.
+int launch_geo_count(bool multi, const GeoJob &one, const GeoJob *many, int njobs, cudaStream_t s);
+int launch_geo_fill(bool multi, const GeoJob &one, const GeoJob *many, int njobs, bool sites, bool derivs,
+                    cudaStream_t s);
+void geo_sizes(bool multi, const int *totals, int *n_sites, int *n_derivs);
+// need: 1 where a site is in the derivative list; D of object sites zero
+template <class T>
+int launch_need_marks(const GeoJob &largest, const GeoJob *many, int njobs, long long P, cudaStream_t s);
+// the split path's classes and lists of one lattice, *sites / *derivs grown as
+// needed (the call synchronises the stream); the launch count, < 0 on failure
+int build_split_lists_dev(const int8_t *t8, int Lx, int Ly, int Lz, uint8_t *cls, void *scratch, int **sites,
+                          int *sites_cap, int *n_sites, int **derivs, int *derivs_cap, int *n_derivs, cudaStream_t s);
 template <class T>
 int launch_split_fused_deep(const Lat<T> &Lin, T *Qo, T *Vo, T *Fo, const SplitLists &sl, FireDev *fd,
                             double *partials, int variant, cudaStream_t s);
